@@ -4,8 +4,7 @@
 // blocks D_i and couplings L_i (to block i-1) and U_i (to block i+1).  One reduction
 // level eliminates the blocks at odd positions j of the active sequence:
 //
-//     Gauss-Jordan on [D_j | L_j | U_j | I]  ->  [I | G_j | H_j | D_j^-1]
-//          G_j = D_j^-1 L_j,   H_j = D_j^-1 U_j
+//          D_j^-1 by Gauss-Jordan,   G_j = D_j^-1 L_j,   H_j = D_j^-1 U_j
 //     for the even neighbours i (odd neighbours jl = left, jr = right):
 //          D_i <- D_i - L_i H_jl - U_i G_jr
 //          L_i <- -L_i G_jl        (couples i to the even block left of jl)
@@ -19,13 +18,15 @@
 // (L and U sparse: the even-block update is a sparse x dense product); the dense
 // updates of the higher levels are batched complex GEMMs.
 //
-// Gauss-Jordan is blocked: one CTA per block reduces a panel of NB columns in shared
-// memory (pivot search over the rows not yet used as pivots, in-place elimination that
-// turns the panel into the columns of the accumulated elementary transform E), then the
-// trailing columns t of every block are updated by t <- E t, i.e.
-// t[r] += sum_c E[r,c] t[piv_c], with the pivot rows themselves replaced.  Rows are
-// never swapped: the pivot row of column k is recorded and the outputs are gathered
-// by it.  Pivoting stays inside each diagonal block.
+// Gauss-Jordan is blocked and in place: one CTA per block reduces a panel of NB columns
+// in registers (pivot search over the rows not yet used as pivots, elimination that turns
+// the panel into the columns of the accumulated elementary transform E), then every other
+// column t of the block is updated by t <- E t, i.e. t[r] += sum_c E[r,c] t[piv_c], with
+// the pivot rows themselves replaced.  The columns left of the panel are then columns of
+// the inverse built so far (E applied to the columns of the identity that an [D | I] work
+// matrix would carry), so the work matrix is S x S and a block costs 8 S^3 real operations
+// instead of 12.  Rows are never swapped: the pivot row of column k is recorded and the
+// inverse is gathered by it.  Pivoting stays inside each diagonal block.
 //
 // Many shifts (forcing frequencies, targets) of one pencil are factorised together:
 // every kernel carries the shift as one more grid dimension, and shift s uses its own
@@ -189,154 +190,202 @@ __global__ void k_Dw_scatter(FV<C> v, int nshift) {
     }
 }
 
-// T_o = [Dw_j | I] for the odd blocks j of level lv, all shifts.  stride 0 selects
-// block 0 (the top of the reduction).
+// T_o = Dw_j for the odd blocks j of level lv, all shifts.  stride 0 selects block 0 (the
+// top of the reduction).
 template <typename C>
 __global__ void k_T_fill(FV<C> v, BcrLevel lv, int nodd, int nshift) {
     const int S = v.S;
-    const int64_t SS = (int64_t)S * S, per = 2 * SS, pershift = (int64_t)nodd * per, total = pershift * nshift;
+    const int64_t SS = (int64_t)S * S, pershift = (int64_t)nodd * SS, total = pershift * nshift;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
         const int64_t s = idx / pershift;
         const int64_t ws = idx - s * pershift;
-        const int64_t o = ws / per;
-        const int64_t e = ws - o * per;
-        const int part = (int)(e / SS);
-        const int64_t w = e - (int64_t)part * SS;
-        const int64_t q = 2 * o + 1;               // position of the odd block
-        const int64_t j = q * lv.stride;           // original block
-        C val;
-        if (part == 0) val = v.Dw[s * v.f_stride + j * SS + w];
-        else {
-            const int c = (int)(w / S), r = (int)(w - (int64_t)c * S);
-            val = (r == c) ? cone<C>() : czero<C>();
-        }
-        v.T[s * v.t_stride + o * per + e] = val;
+        const int64_t o = ws / SS;
+        const int64_t w = ws - o * SS;
+        const int64_t j = (2 * o + 1) * lv.stride;   // original block of position 2 o + 1
+        v.T[s * v.t_stride + o * 2 * SS + w] = v.Dw[s * v.f_stride + j * SS + w];
     }
+}
+
+// Pivot keys: |x|^2 as the bits of a non-negative number, whose integer order is the
+// numeric one, so the search runs on the integer units (on this GPU an FP64 comparison
+// costs as much as an FP64 product).  0 (a zero, a NaN or a used row) is never a pivot.
+__device__ __forceinline__ unsigned long long pivot_key(float2 x) {
+    const float v = abs2(x);
+    return v > 0.f ? (unsigned long long)__float_as_uint(v) : 0ull;
+}
+__device__ __forceinline__ unsigned long long pivot_key(double2 x) {
+    const double v = abs2(x);
+    const long long b = __double_as_longlong(v);
+    return (b > 0 && b <= 0x7ff0000000000000ll) ? (unsigned long long)b : 0ull;   // +0, NaN: 0
+}
+// The largest key of a warp and the lowest lane that holds it.
+template <typename C>
+__device__ __forceinline__ unsigned long long warp_argmax(unsigned long long key, int &lane_of) {
+    const unsigned lo = (unsigned)key;
+    if (sizeof(C) == 8) {
+        const unsigned m = __reduce_max_sync(0xffffffffu, lo);
+        lane_of = __ffs(__ballot_sync(0xffffffffu, lo == m)) - 1;
+        return m;
+    }
+    const unsigned hi = (unsigned)(key >> 32);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned l2 = hi == mh ? lo : 0u;
+    const unsigned ml = __reduce_max_sync(0xffffffffu, l2);
+    lane_of = __ffs(__ballot_sync(0xffffffffu, hi == mh && lo == ml)) - 1;
+    return ((unsigned long long)mh << 32) | ml;
 }
 
 // Panel reduction of columns [k0, k0+nb) of T_o; one CTA per (odd block o = blockIdx.x,
-// shift = blockIdx.y).
-template <typename C, int NB>
-__global__ void __launch_bounds__(1024) k_panel(FV<C> v, int k0) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int S = v.S;
-    C *P = reinterpret_cast<C *>(smem_raw);
-    int *u = reinterpret_cast<int *>(P + (size_t)S * NB);
-    __shared__ C prow[NB];
-    __shared__ double rv[32];
-    __shared__ int ri[32];
-    __shared__ int s_p;
-    __shared__ C s_dinv;
+// shift = blockIdx.y), one thread per row, which holds its NB entries of the panel in
+// registers.  Every elimination step works on register 0 and shifts the others down by
+// one, the finished column of E entering at the top: after nb steps column j of the
+// panel is register NB - nb + j, and the loop body needs no indexed registers.
+// The panel is a chain of S dependent steps per block: with the panel in shared memory,
+// one step cost four barriers, an FP64 pivot search and two shared-memory accesses per
+// product; here it is two barriers, an integer search and one broadcast load per two
+// columns.
+template <typename C, int NB, int MAXT>
+__global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0) {
+    __shared__ __align__(16) C prow[NB];
+    __shared__ unsigned long long wkey[32];
+    __shared__ int wrow[32];
     __shared__ int s_piv[NB];
+    const int S = v.S;
     const int64_t o = blockIdx.x, sh = blockIdx.y;
-    C *T = v.T + sh * v.t_stride + o * 2 * (int64_t)S * S;
+    C *T = v.T + sh * v.t_stride + o * 2 * (int64_t)S * S + (int64_t)k0 * S;
     int *piv = v.piv + sh * v.p_stride + o * S, *pidx = v.pidx + sh * v.p_stride + o * S;
     int *used = v.used + sh * v.p_stride + o * S;
-    const int tid = threadIdx.x, nt = blockDim.x;
+    const int r = threadIdx.x, lane = r & 31, w = r >> 5, nw = blockDim.x >> 5;
     const int nb = min(NB, S - k0);
+    const bool in = r < S;
 
-    for (int idx = tid; idx < S * nb; idx += nt) P[idx] = T[(int64_t)k0 * S + idx];
-    for (int r = tid; r < S; r += nt) u[r] = (k0 == 0) ? 0 : used[r];
-    __syncthreads();
-
+    C P[NB];
+#pragma unroll
+    for (int c = 0; c < NB; ++c) P[c] = (in && c < nb) ? T[r + (int64_t)c * S] : czero<C>();
+    bool u = !in || (k0 != 0 && used[r] != 0);
+    int mine = -1;   // the panel column this row became the pivot of
     int c = 0;
     for (; c < nb; ++c) {
-        double best = -1.0;
-        int bi = INT_MAX;
-        for (int r = tid; r < S; r += nt)
-            if (!u[r]) {
-                const double val = (double)abs2(P[c * S + r]);
-                if (val > best) { best = val; bi = r; }
-            }
-        for (int off = 16; off > 0; off >>= 1) {
-            const double ov = __shfl_down_sync(0xffffffffu, best, off);
-            const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-            if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+        int l;
+        const unsigned long long k = warp_argmax<C>(u ? 0ull : pivot_key(P[0]), l);
+        if (lane == 0) { wkey[w] = k; wrow[w] = w * 32 + l; }
+        __syncthreads();
+        int wl;
+        const unsigned long long best = warp_argmax<C>(lane < nw ? wkey[lane] : 0ull, wl);
+        if (best == 0ull) {   // uniform over the CTA
+            if (r == 0) atomicCAS(v.err, 0, KORE_DEVERR_PIVOT);
+            break;
         }
-        if ((tid & 31) == 0) { rv[tid >> 5] = best; ri[tid >> 5] = bi; }
-        __syncthreads();
-        if (tid < 32) {
-            const int nw = nt >> 5;
-            best = (tid < nw) ? rv[tid] : -1.0;
-            bi = (tid < nw) ? ri[tid] : INT_MAX;
-            for (int off = 16; off > 0; off >>= 1) {
-                const double ov = __shfl_down_sync(0xffffffffu, best, off);
-                const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-                if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-            }
-            if (tid == 0) {
-                int p = bi;
-                if (p >= S || !(best > 0.0)) {
-                    atomicCAS(v.err, 0, KORE_DEVERR_PIVOT);
-                    p = -1;
-                } else {
-                    u[p] = 1;
-                    s_dinv = cdiv(cone<C>(), P[c * S + p]);
-                }
-                s_p = p;
-                s_piv[c] = p;
-            }
-        }
-        __syncthreads();
-        const int p = s_p;
-        if (p < 0) break;
-        const C dinv = s_dinv;
-        if (tid < nb) prow[tid] = (tid == c) ? dinv : P[tid * S + p] * dinv;
-        __syncthreads();
-        for (int r = tid; r < S; r += nt) {
-            const C mult = P[c * S + r];
+        const int p = wrow[wl];
+        if (w == p >> 5) {   // the pivot row's warp publishes the row, scaled by 1 / pivot
             if (r == p) {
-                for (int cc = 0; cc < nb; ++cc) if (cc != c) P[cc * S + r] = prow[cc];
-            } else {
-                for (int cc = 0; cc < nb; ++cc) if (cc != c) P[cc * S + r] = cfms(P[cc * S + r], mult, prow[cc]);
+                u = true;
+                mine = c;
+                s_piv[c] = p;
+#pragma unroll
+                for (int q = 0; q < NB; ++q) prow[q] = P[q];
             }
-            P[c * S + r] = (r == p) ? dinv : -(mult * dinv);
+            __syncwarp();
+            const C dinv = cdiv(cone<C>(), prow[0]);
+            const C own = lane < NB ? prow[lane] : czero<C>();
+            __syncwarp();
+            if (lane < NB) prow[lane] = lane == 0 ? dinv : own * dinv;
         }
         __syncthreads();
+        const C dinv = prow[0], mult = P[0];
+        if (r == p) {
+#pragma unroll
+            for (int q = 1; q < NB; ++q) P[q - 1] = prow[q];
+            P[NB - 1] = dinv;
+        } else {
+#pragma unroll
+            for (int q = 1; q < NB; ++q) P[q - 1] = cfms(P[q], mult, prow[q]);
+            P[NB - 1] = -(mult * dinv);
+        }
     }
     const int done = c;
-    for (int idx = tid; idx < S * nb; idx += nt) T[(int64_t)k0 * S + idx] = P[idx];
-    for (int r = tid; r < S; r += nt) { used[r] = u[r]; pidx[r] = -1; }
-    __syncthreads();
-    if (tid < done) { piv[k0 + tid] = s_piv[tid]; pidx[s_piv[tid]] = tid; }
+    if (in) {
+        if (done == nb) {
+#pragma unroll
+            for (int q = 0; q < NB; ++q)
+                if (q >= NB - nb) T[r + (int64_t)(q - (NB - nb)) * S] = P[q];
+        }
+        used[r] = u ? 1 : 0;
+        pidx[r] = mine;
+    }
+    if (r < done) piv[k0 + r] = s_piv[r];
     // after a zero pivot the remaining columns keep an in-range row index so that the
     // update and extraction kernels stay in bounds (the error flag is already set)
-    if (tid >= done && tid < nb) piv[k0 + tid] = 0;
+    if (r >= done && r < nb) piv[k0 + r] = 0;
 }
 
-// Trailing update of TW columns per CTA (blockIdx.x) of odd block blockIdx.y, shift blockIdx.z.
+// Update of the columns outside the panel [k0, k0+nb): t <- t + E t[piv] for TW columns
+// per CTA (blockIdx.x) of odd block blockIdx.y, shift blockIdx.z; a column t left of the
+// panel is a finished column of the inverse, one right of it is still to be eliminated.
+// The CTA owns its columns whole (their pivot rows are read before they are replaced)
+// and walks the rows in chunks of 128: a thread holds 4 rows x TW / 8 columns, so that
+// one step of the sum costs 4 + TW / 8 shared-memory loads for TW / 2 complex products
+// and FP32 arithmetic, not shared memory, is the bound (complex128: the FP64 pipe).
+constexpr int kUpdRows = 128;
 template <typename C, int NB, int TW>
-__global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb, int col_begin, int col_end) {
-    __shared__ C tp[TW][NB];
+__global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb) {
+    constexpr int CT = TW / 8;   // columns per thread
+    __shared__ __align__(16) C tp[NB][TW];
+    __shared__ __align__(16) C es[NB][kUpdRows];
     const int S = v.S;
     const int64_t o = blockIdx.y, sh = blockIdx.z;
     C *T = v.T + sh * v.t_stride + o * 2 * (int64_t)S * S;
     const int *piv = v.piv + sh * v.p_stride + o * S, *pidx = v.pidx + sh * v.p_stride + o * S;
-    const int j0 = col_begin + blockIdx.x * TW;
-    const int tw = min(TW, col_end - j0);
-    for (int idx = threadIdx.x; idx < TW * NB; idx += blockDim.x) {
-        const int t = idx / NB, c = idx - t * NB;
-        tp[t][c] = (t < tw && c < nb) ? T[piv[k0 + c] + (int64_t)(j0 + t) * S] : czero<C>();
+    // columns of this CTA, counted without the panel's own
+    const int j0 = blockIdx.x * TW, ncols = S - nb;
+    auto column = [&](int t) { const int j = j0 + t; return j < k0 ? j : j + nb; };
+    for (int idx = threadIdx.x; idx < TW * NB; idx += 256) {
+        const int c = idx % NB, t = idx / NB;
+        tp[c][t] = (j0 + t < ncols && c < nb) ? T[piv[k0 + c] + (int64_t)column(t) * S] : czero<C>();
     }
-    __syncthreads();
     const C *E = T + (int64_t)k0 * S;
-    for (int r = threadIdx.x; r < S; r += blockDim.x) {
-        C er[NB];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int r0 = 0; r0 < S; r0 += kUpdRows) {
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < NB * kUpdRows; idx += 256) {
+            const int rr = idx % kUpdRows, c = idx / kUpdRows;
+            es[c][rr] = (r0 + rr < S && c < nb) ? E[r0 + rr + (int64_t)c * S] : czero<C>();
+        }
+        C acc[4][CT];
 #pragma unroll
-        for (int c = 0; c < NB; ++c) er[c] = (c < nb) ? E[r + (int64_t)c * S] : czero<C>();
-        const bool isp = pidx[r] >= 0;
-        for (int t = 0; t < tw; ++t) {
-            const int64_t idx = r + (int64_t)(j0 + t) * S;
-            C acc = isp ? czero<C>() : T[idx];
+        for (int i = 0; i < 4; ++i) {
+            const int r = r0 + tx + 32 * i;
+            const bool keep = r < S && pidx[r] < 0;   // a pivot row starts from zero
 #pragma unroll
-            for (int c = 0; c < NB; ++c) acc = cfma(acc, er[c], tp[t][c]);
-            T[idx] = acc;
+            for (int t = 0; t < CT; ++t)
+                acc[i][t] = (keep && j0 + ty * CT + t < ncols) ? T[r + (int64_t)column(ty * CT + t) * S] : czero<C>();
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int c = 0; c < NB; ++c) {
+            C e[4], t4[CT];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) e[i] = es[c][tx + 32 * i];
+#pragma unroll
+            for (int t = 0; t < CT; ++t) t4[t] = tp[c][ty * CT + t];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int t = 0; t < CT; ++t) acc[i][t] = cfma(acc[i][t], e[i], t4[t]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = r0 + tx + 32 * i;
+#pragma unroll
+            for (int t = 0; t < CT; ++t)
+                if (r < S && j0 + ty * CT + t < ncols) T[r + (int64_t)column(ty * CT + t) * S] = acc[i][t];
         }
     }
 }
 
-// Solution rows by pivot: Dinv_j[k,:] = T[piv[k], S:2S)  (column-major S x S), all shifts.
+// The inverse from the reduced work matrix: row piv[k] of T is row k of the inverse and
+// column k of T is its column piv[k] (column-major S x S, all shifts).
 template <typename C>
 __global__ void k_extract(FV<C> v, BcrLevel lv, int nodd, int top, int nshift) {
     const int S = v.S;
@@ -349,9 +398,9 @@ __global__ void k_extract(FV<C> v, BcrLevel lv, int nodd, int top, int nshift) {
         const int64_t w = ws - o * SS;
         const int c = (int)(w / S), k = (int)(w - (int64_t)c * S);
         const C *T = v.T + sh * v.t_stride + o * 2 * SS;
-        const int p = v.piv[sh * v.p_stride + o * S + k];
+        const int *piv = v.piv + sh * v.p_stride + o * S;
         const int64_t j = top ? 0 : (2 * o + 1) * lv.stride;
-        v.Dinv[sh * v.f_stride + j * SS + w] = T[p + (int64_t)(S + c) * S];
+        v.Dinv[sh * v.f_stride + j * SS + k + (int64_t)piv[c] * S] = T[piv[k] + (int64_t)c * S];
     }
 }
 
@@ -581,27 +630,26 @@ __global__ void __launch_bounds__(512) k_gh_l0(FV<C> v) {
     }
 }
 
-constexpr int kUpdTW = 8;
-
 unsigned grid_for(int64_t work, int threads, int num_sms) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>((work + threads - 1) / threads, 16LL * num_sms));
 }
 
 // Gauss-Jordan of the nodd work matrices T_o of every shift (all panels), then extraction.
-template <typename C, int NB>
+template <typename C, int NB, int MAXT>
 int gauss_jordan(kore_plan *p, const FV<C> &v, const BcrLevel &lv, int nodd, int top, int nshift) {
     const int S = p->S;
-    const size_t smem = (size_t)S * NB * sizeof(C) + (size_t)S * sizeof(int);
-    KORE_TRY(kore_allow_max_dyn_smem(k_panel<C, NB>, p->device));
-    const int pthreads = std::min(1024, ((S + 31) / 32) * 32);
+    const int pthreads = ((S + 31) / 32) * 32;
     for (int k0 = 0; k0 < S; k0 += NB) {
         const int nb = std::min(NB, S - k0);
-        k_panel<C, NB><<<dim3(nodd, nshift), pthreads, smem, p->stream>>>(v, k0);
+        k_panel<C, NB, MAXT><<<dim3(nodd, nshift), pthreads, 0, p->stream>>>(v, k0);
         KORE_LAUNCHED(1);
-        const int cb = k0 + nb;
-        // trailing columns: the rest of D, then the identity columns
-        dim3 g(kore_div_up(2 * S - cb, kUpdTW), nodd, nshift);
-        k_update<C, NB, kUpdTW><<<g, 256, 0, p->stream>>>(v, k0, nb, cb, 2 * S);
+        if (S == nb) break;
+        // 32 columns per CTA re-read the panel least; levels with few blocks take 8, so
+        // that their CTAs still cover the GPU
+        if ((int64_t)nodd * nshift * kore_div_up(S - nb, 32) >= 2 * p->num_sms)
+            k_update<C, NB, 32><<<dim3(kore_div_up(S - nb, 32), nodd, nshift), 256, 0, p->stream>>>(v, k0, nb);
+        else
+            k_update<C, NB, 8><<<dim3(kore_div_up(S - nb, 8), nodd, nshift), 256, 0, p->stream>>>(v, k0, nb);
         KORE_LAUNCHED(1);
     }
     k_extract<C><<<grid_for((int64_t)nodd * S * S * nshift, 256, p->num_sms), 256, 0, p->stream>>>(v, lv, nodd, top,
@@ -611,7 +659,7 @@ int gauss_jordan(kore_plan *p, const FV<C> &v, const BcrLevel &lv, int nodd, int
     return KORE_OK;
 }
 
-template <typename C, int NB>
+template <typename C, int NB, int MAXT>
 int factor_levels(kore_plan *p) {
     const int S = p->S, K = p->K, ns = p->fw_n;
     const int64_t SS = (int64_t)S * S;
@@ -623,10 +671,10 @@ int factor_levels(kore_plan *p) {
     KORE_LAUNCHED(2);
     for (int l = 0; l < p->nlev; ++l) {
         const BcrLevel &lv = p->lev[l];
-        k_T_fill<C><<<grid_for((int64_t)lv.nodd * 2 * SS * ns, 256, p->num_sms), 256, 0, st>>>(v, lv, lv.nodd, ns);
+        k_T_fill<C><<<grid_for((int64_t)lv.nodd * SS * ns, 256, p->num_sms), 256, 0, st>>>(v, lv, lv.nodd, ns);
         KORE_LAUNCHED(1);
-        // D_j^-1 of the odd blocks by Gauss-Jordan on [D_j | I]
-        KORE_TRY((gauss_jordan<C, NB>(p, v, lv, lv.nodd, 0, ns)));
+        // D_j^-1 of the odd blocks by Gauss-Jordan
+        KORE_TRY((gauss_jordan<C, NB, MAXT>(p, v, lv, lv.nodd, 0, ns)));
         const int th = std::min(512, ((S + 31) / 32) * 32);   // rows per pass (S <= 1024: two passes at most)
         if (l == 0) {
             // G_j, H_j from the sparse couplings (complex64: refined on the tensor cores),
@@ -657,26 +705,25 @@ int factor_levels(kore_plan *p) {
         }
         KORE_CUDA_TRY(cudaGetLastError());
     }
-    // the last active block (block 0): T = [Dw_0 | I]; stride 0 maps odd index 0 to block 0
+    // the last active block (block 0); stride 0 maps odd index 0 to block 0
     BcrLevel top{};
     top.Kl = 1;
     top.stride = 0;
     top.lu_L = top.lu_U = top.lu_nL = top.lu_nU = -1;
-    k_T_fill<C><<<grid_for(2 * SS * ns, 256, p->num_sms), 256, 0, st>>>(v, top, 1, ns);
+    k_T_fill<C><<<grid_for(SS * ns, 256, p->num_sms), 256, 0, st>>>(v, top, 1, ns);
     KORE_LAUNCHED(1);
-    KORE_TRY((gauss_jordan<C, NB>(p, v, top, 1, 1, ns)));
+    KORE_TRY((gauss_jordan<C, NB, MAXT>(p, v, top, 1, 1, ns)));
     return KORE_OK;
 }
 
+// A panel row lives in one thread's registers: NB complex values.  512 threads leave 128
+// registers each (NB = 32 complex64, 16 complex128), 1024 leave 64.
 template <typename C>
 int factor_dispatch(kore_plan *p) {
-    const size_t cap = 220 * 1024;
-    auto fits = [&](int nb) { return (size_t)p->S * nb * sizeof(C) + (size_t)p->S * sizeof(int) <= cap; };
-    if (sizeof(C) == 8 && fits(32)) return factor_levels<C, 32>(p);
-    if (fits(16)) return factor_levels<C, 16>(p);
-    if (fits(8)) return factor_levels<C, 8>(p);
-    if (fits(4)) return factor_levels<C, 4>(p);
-    return KORE_EINVAL;
+    constexpr int NB = sizeof(C) == 8 ? 32 : 16;
+    if (p->S <= 256) return factor_levels<C, NB, 256>(p);
+    if (p->S <= 512) return factor_levels<C, NB, 512>(p);
+    return factor_levels<C, NB / 2, 1024>(p);
 }
 
 }  // namespace

@@ -95,7 +95,7 @@ struct kore_plan {
     // S x S column-major blocks, indexed by original block number, per shift
     void *d_Dinv = nullptr, *d_Gm = nullptr, *d_Hm = nullptr, *d_Dw = nullptr;
     void *d_LU = nullptr;             // lu_mats blocks per shift
-    void *d_T = nullptr;              // nodd_max x (S x 2S) Gauss-Jordan work [D | I] per shift, column-major
+    void *d_T = nullptr;              // nodd_max x (S x 2S) per shift, column-major: Gauss-Jordan work (first S columns), then residuals of G, H
     double *d_rscale = nullptr;       // np row equilibration factors per shift
     int *d_piv = nullptr;             // nodd_max x S per shift: pivot row chosen for column k
     int *d_pidx = nullptr;            // nodd_max x S per shift: position of a row in the current panel or -1

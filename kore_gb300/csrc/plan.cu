@@ -524,15 +524,15 @@ int kore_profile(kore_plan *p, int enable, double *out) {
         }
         out[4] = (mats + lu) * S * S * e + (double)p->ell_nnz * (e + 4.0) + np * (16.0 + 8.0 + 16.0) +
                  6.0 * np * e;
-        // Gauss-Jordan on [D_j | L_j | U_j | I] for every eliminated block (trailing update
-        // 8 S nb (4S - k0 - nb) real flops per panel, ~28 S^3 per block) and four dense
-        // S^3 complex products (8 S^3 real flops each) per surviving block of levels >= 1
-        double gj = 0.0, gm = 0.0;
+        // in-place Gauss-Jordan of every eliminated block and the top (8 S^3 real flops
+        // each), and at levels >= 1 dense S^3 complex products (8 S^3): G, H of the
+        // eliminated blocks, four per surviving block
+        double gj = 1.0, gm = 0.0;
         for (int l = 0; l < p->nlev; ++l) {
             gj += p->lev[l].nodd;
-            if (l > 0) gm += 4.0 * p->lev[l].neven;
+            if (l > 0) gm += 2.0 * p->lev[l].nodd + 4.0 * p->lev[l].neven;
         }
-        out[5] = (gj + 1.0) * 28.0 * S * S * S + gm * 8.0 * S * S * S;
+        out[5] = (gj + gm) * 8.0 * S * S * S;
         for (int k = 2; k < 5; ++k) {
             out[6 + 2 * (k - 2)] = p->prof_ms[k];
             out[7 + 2 * (k - 2)] = (double)p->prof_n[k];
