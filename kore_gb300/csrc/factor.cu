@@ -770,7 +770,7 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
                      (void **)&p->d_rscale, (void **)&p->d_piv, (void **)&p->d_pidx, (void **)&p->d_used,
                      (void **)&p->d_sigma, (void **)&p->d_minf, (void **)&p->d_bb, (void **)&p->d_xb, (void **)&p->d_rb,
                      (void **)&p->d_bn, (void **)&p->d_rn, (void **)&p->d_part, (void **)&p->d_ir,
-                     (void **)&p->d_cnt, &p->d_ell_val, &p->d_tcplanes, &p->d_tctab};
+                     (void **)&p->d_cnt, &p->d_ell_val, &p->d_tctab};
     for (void **b : bufs) {
         if (*b) cudaFree(*b);
         *b = nullptr;
@@ -806,12 +806,7 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
     KORE_TRY(kore_alloc(p, (void **)&p->d_ir, c * sizeof(IrState)));
     KORE_TRY(kore_alloc(p, (void **)&p->d_cnt, c * (size_t)p->sweep_stages() * p->K * sizeof(int)));
     KORE_TRY(kore_alloc(p, &p->d_ell_val, c * std::max<int64_t>(p->ell_stride(), 1) * elt));
-    if (elt == sizeof(float2)) {
-        int64_t pl = 0, tb = 0;
-        kore_tc_level_bytes(p, cap, &pl, &tb);
-        KORE_TRY(kore_alloc(p, &p->d_tcplanes, (size_t)pl));
-        KORE_TRY(kore_alloc(p, &p->d_tctab, (size_t)tb));
-    }
+    if (elt == sizeof(float2)) KORE_TRY(kore_alloc(p, &p->d_tctab, (size_t)kore_tc_table_bytes(p, cap)));
     KORE_CUDA_TRY(cudaMemset(p->d_LU, 0, c * p->lu_stride() * elt));
     KORE_CUDA_TRY(cudaMemset(p->d_piv, 0, c * p->p_stride() * sizeof(int)));
     KORE_CUDA_TRY(cudaMemset(p->d_pidx, 0xff, c * p->p_stride() * sizeof(int)));

@@ -3,26 +3,27 @@
 //     x = x_hi + x_lo,  x_hi = x rounded to TF32,  x_lo = x - x_hi (exact in FP32),
 //     a b ~ a_hi b_hi + a_hi b_lo + a_lo b_hi      (FP32 accumulation in tensor memory)
 // and each complex product as four real ones,
-//     Re(AB) = Ar Br - Ai Bi,  Im(AB) = Ar Bi + Ai Br,
-// the subtraction done by the -Im planes of the B operand (below), so every MMA adds.
+//     Re(AB) = Ar Br - Ai Bi,  Im(AB) = Ar Bi + Ai Br
+// (the MMA's negate bit makes the subtraction).
 //
-// Data flow of one 128 x 64 tile of C = beta C + alpha (A1 B1 [+ A2 B2]):
-//   * k_tc_split writes, once per matrix, K-major FP32 planes: Re hi, Re lo, Im hi, Im lo
-//     of the A operands (transposed: K contiguous per row of A) and the same plus -Im hi,
-//     -Im lo of the B operands (as stored: K contiguous per column of B), K padded with
-//     zeros to Kp = 32 k;
-//   * one producer thread streams the planes of each 32-wide K slice into a two-stage
-//     shared-memory ring with cp.async.bulk.tensor (128-byte swizzle, the layout the MMA
-//     descriptors describe), each stage guarded by a "full" and an "empty" mbarrier.  The
-//     B planes of a stage lie as [-Bi | Br | Bi] (hi, then lo), so the 128-row windows
-//     W1 = [Br | Bi] and W2 = [-Bi | Br] are B operands of single MMAs:
-//         [Re | Im](C) += Ar W1 + Ai W2;
-//   * one thread issues tcgen05.mma (M = 128, N = 128, K = 8 per instruction, 6 per K
-//     step: 3xTF32 of the two products) into one tensor-memory accumulator (Re: columns
-//     0-63, Im: 64-127) and frees each stage with tcgen05.commit;
-//   * the four warps read their 32 lanes (rows) back with tcgen05.ld and write C.
+// Data flow of one 128 x 128 tile of C = beta C + alpha (A1 B1 [+ A2 B2]), one CTA:
+//   * the operands are split inside the kernel, 32 columns of K at a time: four warps load
+//     the 128 rows of A (one thread per row, coalesced along the column-major rows) and
+//     write the planes Re hi, Re lo, Im hi, Im lo to tensor memory, where the MMA takes
+//     its A operand from; four warps load the columns of B (K contiguous) and write the
+//     same four planes to shared memory in the 128-byte swizzled K-major layout;
+//   * each of the two stages has a "full" mbarrier (one arrival per converting warp) and an
+//     "empty" one (tcgen05.commit); the next slice's loads are in flight while a stage waits;
+//   * one thread issues tcgen05.mma (M = 128, N up to 128, K = 8, twelve per step of K) into
+//     the tensor-memory accumulators Re (columns 0-127) and Im (128-255);
+//   * the eight converting warps read the accumulators back with tcgen05.ld and write C.
+// What bounds it: the MMAs (a 32-wide slice takes 48 of them, about 3,070 cycles).  Both
+// operands from shared memory kept it at the shared-memory bandwidth (8 KB per MMA of 64
+// cycles, plus the copies), and planes split beforehand by another kernel made the copies
+// 2.3 times the operands: with A in tensor memory and the split in the kernel a slice
+// moves 64 KB from L2 per 3,070 cycles and shared memory serves B alone.
 // Every wait is bounded (error flag, then the kernel carries on to release its tensor
-// memory); tensor memory is allocated and freed by warp 0.
+// memory); tensor memory is allocated and freed by warp 8.
 #include "kore_internal.cuh"
 #include "kore_tma.cuh"
 #include <algorithm>
@@ -31,31 +32,29 @@
 
 namespace {
 
-constexpr int kTcM = 128, kTcN = 64, kTcK = 32, kTcStages = 2, kTcThreads = 128;
-constexpr int kPlanesA = 4, kPlanesB = 6;         // A: Re hi, Re lo, Im hi, Im lo; B: + -Im hi, -Im lo
-constexpr int kPlaneA = kTcM * kTcK * 4;          // 16 KB: one plane of an A slice
-constexpr int kPlaneB = kTcN * kTcK * 4;          // 8 KB
-constexpr int kStageA = kPlanesA * kPlaneA;
-constexpr int kStageBytes = kStageA + kPlanesB * kPlaneB;   // 112 KB
-constexpr uint32_t kTmemCols = 2 * kTcN;          // [Re | Im] accumulator: columns [0, 64) and [64, 128)
-constexpr size_t kTcSmem = (size_t)kTcStages * kStageBytes + 1024 + 128;
-// Order of the B planes in a stage: [-Im hi][Re hi][Im hi][-Im lo][Re lo][Im lo]; stage
-// slot of global plane p (Re hi, Re lo, Im hi, Im lo, -Im hi, -Im lo).
-__host__ __device__ constexpr int slot_b(int p) {
-    return p == 0 ? 1 : p == 1 ? 4 : p == 2 ? 2 : p == 3 ? 5 : p == 4 ? 0 : 3;
-}
+constexpr int kTcM = 128, kTcN = 128, kTcK = 32, kTcStages = 2;
+constexpr int kTcConvWarps = 8;                   // 4 for A, 4 for B; warp 8 issues the MMAs
+constexpr int kTcThreads = 32 * (kTcConvWarps + 1);
+constexpr int kPlanes = 4;                        // Re hi, Re lo, Im hi, Im lo
+constexpr int kPlaneB = kTcN * kTcK * 4;          // 16 KB: one plane of a B slice
+constexpr int kStageB = kPlanes * kPlaneB;
+// tensor memory: Re and Im accumulators, then the A planes (32 columns each) of the stages
+constexpr uint32_t kTmemA = 2 * kTcN;
+constexpr uint32_t kTmemCols = kTmemA + kTcStages * kPlanes * kTcK;   // 512, all of it
+// more than half of an SM's shared memory, so that no second CTA waits there for tensor memory
+constexpr size_t kTcSmem = (size_t)kTcStages * kStageB + 1024 + 128;
+static_assert(kTmemCols == 512 && 2 * kTcSmem > 227 * 1024, "one CTA per SM");
 
 struct TcJob {
-    int a1, b1, a2, b2;   // matrix indices into the A and B plane sets (a2 < 0: one product)
-    float2 *C;            // column-major S x S
-    float alpha;          // C = beta C + alpha (A1 B1 + A2 B2)
+    const float2 *A1, *B1, *A2, *B2;   // column-major S x S (A2 null: one product)
+    float2 *C;                         // column-major S x S
+    float alpha;                       // C = beta C + alpha (A1 B1 + A2 B2)
     int beta;
 };
 
 struct TcParams {
-    CUtensorMap amap, bmap;   // planes {Kp, S, 4 * matrices}, boxes {32, 128, 1} and {32, 64, 1}
     const TcJob *jobs;
-    int S, Kp, tiles_n;
+    int S, tiles_n;
     int *err;
 };
 
@@ -72,13 +71,13 @@ __device__ __forceinline__ void tc_dealloc(uint32_t taddr, uint32_t ncols) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] B[smem]; accumulate = 0 overwrites D
-__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[tmem] B[smem]; accumulate = 0 overwrites D
+__device__ __forceinline__ void tc_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+        "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 
@@ -101,6 +100,21 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
+// write 32 consecutive 32-bit columns of this warp's 32 lanes
+__device__ __forceinline__ void tc_st32(uint32_t taddr, const float (&v)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};" ::"f"(v[0]),
+        "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
+        "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]), "f"(v[16]), "f"(v[17]), "f"(v[18]),
+        "f"(v[19]), "f"(v[20]), "f"(v[21]), "f"(v[22]), "f"(v[23]), "f"(v[24]), "f"(v[25]), "f"(v[26]), "f"(v[27]),
+        "f"(v[28]), "f"(v[29]), "f"(v[30]), "f"(v[31]), "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// generic-proxy writes to shared memory visible to the MMA (async proxy)
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptor of a K-major operand in the 128-byte swizzled layout:
@@ -114,10 +128,11 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
 }
 
 // Instruction descriptor of kind::tf32: D F32 (bits 4-5 = 1), A and B TF32 (bits 7-9,
-// 10-12 = 2), no negation (bits 13, 14), both operands K-major (bits 15, 16 = 0),
-// N >> 3 at bits 17-22 (N = 128: the [Re | Im] window), M >> 4 at bits 24-28.
-__host__ __device__ constexpr uint32_t tf32_idesc() {
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)((2 * kTcN) >> 3) << 17) | ((uint32_t)(kTcM >> 4) << 24);
+// 10-12 = 2), A negated (bit 13), both operands K-major (bits 15, 16 = 0), N >> 3 at bits
+// 17-22, M >> 4 at bits 24-28.
+__device__ __forceinline__ uint32_t tf32_idesc(int n, int negate_a) {
+    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)negate_a << 13) | ((uint32_t)(n >> 3) << 17) |
+           ((uint32_t)(kTcM >> 4) << 24);
 }
 
 __device__ __forceinline__ float tf32_rna(float x) {
@@ -126,194 +141,210 @@ __device__ __forceinline__ float tf32_rna(float x) {
     return __uint_as_float(r);
 }
 
-// ----------------------------------------------------------------------------- split planes
-// planes[((m * P + p) * S + row) * Kp + k], p = Re hi, Re lo, Im hi, Im lo (P = 4, A
-// operands) and -Im hi, -Im lo (P = 6, B operands).  TRANS (A operand): row = row of X,
-// k = column of X.  !TRANS (B operand): row = column of X, k = row of X.  X is
-// column-major S x S; k in [S, Kp) is zero.
-template <bool TRANS>
-__global__ void __launch_bounds__(256) k_tc_split(const float2 *const *__restrict__ src, int S, int Kp,
-                                                  float *__restrict__ planes) {
-    __shared__ float2 t[32][33];
-    const int m = blockIdx.z;
-    const float2 *X = src[m];
-    const int k0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-    const int tx = threadIdx.x, ty = threadIdx.y;   // 32 x 8
-    const int64_t plane = (int64_t)S * Kp;
-    float *base = planes + (int64_t)m * (TRANS ? kPlanesA : kPlanesB) * plane;
-    auto put = [&](int row, int k, float2 v) {
-        const float rh = tf32_rna(v.x), ih = tf32_rna(v.y);
-        const int64_t o = (int64_t)row * Kp + k;
-        base[o] = rh;
-        base[plane + o] = v.x - rh;
-        base[2 * plane + o] = ih;
-        base[3 * plane + o] = v.y - ih;
-        if (!TRANS) {
-            base[4 * plane + o] = -ih;
-            base[5 * plane + o] = -(v.y - ih);
-        }
-    };
-    if (TRANS) {
-        // read X(r0 + tx, k0 + j) along its rows, write row r0 + j along k
-        for (int j = ty; j < 32; j += 8) {
-            const int r = r0 + tx, k = k0 + j;
-            t[j][tx] = (r < S && k < S) ? X[r + (int64_t)k * S] : make_float2(0.f, 0.f);
-        }
-        __syncthreads();
-        for (int j = ty; j < 32; j += 8) {
-            const int r = r0 + j, k = k0 + tx;
-            if (r < S && k < Kp) put(r, k, t[tx][j]);
-        }
-    } else {
-        for (int j = ty; j < 32; j += 8) {
-            const int n = r0 + j, k = k0 + tx;
-            if (n < S && k < Kp) put(n, k, (k < S) ? X[k + (int64_t)n * S] : make_float2(0.f, 0.f));
-        }
-    }
-}
-
 // ----------------------------------------------------------------------------- GEMM
-__global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const __grid_constant__ TcParams P) {
+__global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcParams P) {
     extern __shared__ unsigned char smem_raw[];
     // 1024-byte aligned stages (the 128-byte swizzle pattern repeats every 1024 bytes)
     unsigned char *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + kTcStages * kStageBytes);
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + kTcStages * kStageB);
     uint64_t *empty = full + kTcStages;
     uint64_t *accum = empty + kTcStages;
     uint32_t *holder = reinterpret_cast<uint32_t *>(accum + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const TcJob job = P.jobs[blockIdx.y];
+    const int S = P.S;
     const int tm = blockIdx.x / P.tiles_n, tn = blockIdx.x - tm * P.tiles_n;
-    const int nk = P.Kp / kTcK;
-    const int nstage = (job.a2 >= 0 ? 2 : 1) * nk;
+    const int nk = (S + kTcK - 1) / kTcK;
+    const int nstage = (job.A2 ? 2 : 1) * nk;
+    const int m0 = tm * kTcM, n0 = tn * kTcN;
+    const int n_eff = min(kTcN, (S - n0 + 15) & ~15);   // columns the MMAs compute
     if (tid == 0) {
         for (int s = 0; s < kTcStages; ++s) {
-            mbar_init(&full[s], 1);
+            mbar_init(&full[s], kTcConvWarps);
             mbar_init(&empty[s], 1);
         }
         mbar_init(accum, 1);
         mbar_fence_init();
     }
-    if (warp == 0) tc_alloc(holder, kTmemCols);
+    if (warp == kTcConvWarps) tc_alloc(holder, kTmemCols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *holder;
 
-    if (warp == 0) {
-        if (lane == 0) {
-            // producer: the four planes of A and of B for each 32-wide K slice
-            for (int ks = 0; ks < nstage; ++ks) {
-                const int s = ks % kTcStages;
-                const uint32_t ph = (uint32_t)(ks / kTcStages) & 1u;
-                if (!mbar_wait(&empty[s], ph ^ 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
-                mbar_arrive_expect_tx(&full[s], kStageBytes);
-                const int pair = ks / nk, kq = ks - pair * nk;
-                const int ia = pair ? job.a2 : job.a1, ib = pair ? job.b2 : job.b1;
-                unsigned char *sa = smem + (size_t)s * kStageBytes, *sb = sa + kStageA;
+    if (warp < 4) {
+        // A: thread = row, its 32 entries of the slice in registers, planes to tensor memory
+        const int row = m0 + warp * 32 + lane;
+        float2 v[kTcK];
+        auto load = [&](int ks) {
+            const float2 *A = (ks >= nk ? job.A2 : job.A1) + row;
+            const int k0 = (ks >= nk ? ks - nk : ks) * kTcK;
 #pragma unroll
-                for (int p = 0; p < kPlanesA; ++p)
-                    tma_load_3d(sa + p * kPlaneA, &P.amap, &full[s], kq * kTcK, tm * kTcM, ia * kPlanesA + p);
+            for (int k = 0; k < kTcK; ++k)
+                v[k] = (row < S && k0 + k < S) ? __ldg(A + (int64_t)(k0 + k) * S) : make_float2(0.f, 0.f);
+        };
+        load(0);
+        for (int ks = 0; ks < nstage; ++ks) {
+            const int s = ks % kTcStages;
+            if (!mbar_wait(&empty[s], ((uint32_t)(ks / kTcStages) & 1u) ^ 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
+            tc_fence_after();
+            const uint32_t ta = tmem + kTmemA + (uint32_t)(s * kPlanes * kTcK) + ((uint32_t)(warp * 32) << 16);
+            float r[kTcK];
 #pragma unroll
-                for (int p = 0; p < kPlanesB; ++p)
-                    tma_load_3d(sb + slot_b(p) * kPlaneB, &P.bmap, &full[s], kq * kTcK, tn * kTcN, ib * kPlanesB + p);
-            }
+            for (int k = 0; k < kTcK; ++k) r[k] = tf32_rna(v[k].x);
+            tc_st32(ta, r);
+#pragma unroll
+            for (int k = 0; k < kTcK; ++k) r[k] = v[k].x - tf32_rna(v[k].x);
+            tc_st32(ta + kTcK, r);
+#pragma unroll
+            for (int k = 0; k < kTcK; ++k) r[k] = tf32_rna(v[k].y);
+            tc_st32(ta + 2 * kTcK, r);
+#pragma unroll
+            for (int k = 0; k < kTcK; ++k) r[k] = v[k].y - tf32_rna(v[k].y);
+            tc_st32(ta + 3 * kTcK, r);
+            if (ks + 1 < nstage) load(ks + 1);
+            tc_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s]);
         }
-        __syncwarp();
-    } else if (warp == 1) {
-        if (lane == 0) {
-            // MMA issuer
-            const uint32_t id = tf32_idesc();
-            for (int ks = 0; ks < nstage; ++ks) {
-                const int s = ks % kTcStages;
-                const uint32_t ph = (uint32_t)(ks / kTcStages) & 1u;
-                if (!mbar_wait(&full[s], ph)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
-                tc_fence_after();
-                const uint32_t sa = smem_u32(smem + (size_t)s * kStageBytes), sb = sa + kStageA;
+    } else if (warp < kTcConvWarps) {
+        // B: thread = four entries of K (chunk ch) of columns n, n + 16, ..., planes to shared
+        // memory: row n of a plane is 128 bytes of K, its 16-byte chunk ch at ch ^ (n & 7)
+        const int ch = lane & 7, nb = (warp - 4) * 4 + (lane >> 3);
+        const bool vec = (S & 3) == 0;   // every column starts on a 32-byte boundary
+        float4 v[8][2];
+        auto load = [&](int ks) {
+            const float2 *B = ks >= nk ? job.B2 : job.B1;
+            const int k0 = (ks >= nk ? ks - nk : ks) * kTcK + 4 * ch;
 #pragma unroll
-                for (int k8 = 0; k8 < kTcK / 8; ++k8) {
-                    uint64_t a[kPlanesA];
-#pragma unroll
-                    for (int p = 0; p < kPlanesA; ++p) a[p] = sw128_desc(sa + p * kPlaneA) + (uint64_t)(2 * k8);
-                    // 128-row windows of the B planes (+ 32 bytes of K per step of 8)
-                    const uint64_t w1h = sw128_desc(sb + 1 * kPlaneB) + (uint64_t)(2 * k8);   // [Br hi | Bi hi]
-                    const uint64_t w2h = sw128_desc(sb + 0 * kPlaneB) + (uint64_t)(2 * k8);   // [-Bi hi | Br hi]
-                    const uint64_t w1l = sw128_desc(sb + 4 * kPlaneB) + (uint64_t)(2 * k8);   // [Br lo | Bi lo]
-                    const uint64_t w2l = sw128_desc(sb + 3 * kPlaneB) + (uint64_t)(2 * k8);   // [-Bi lo | Br lo]
-                    const uint32_t acc = (ks == 0 && k8 == 0) ? 0u : 1u;
-                    // [Re | Im] += Ar [Br | Bi]
-                    tc_mma(tmem, a[0], w1h, id, acc);
-                    tc_mma(tmem, a[0], w1l, id, 1u);
-                    tc_mma(tmem, a[1], w1h, id, 1u);
-                    // [Re | Im] += Ai [-Bi | Br]
-                    tc_mma(tmem, a[2], w2h, id, 1u);
-                    tc_mma(tmem, a[2], w2l, id, 1u);
-                    tc_mma(tmem, a[3], w2h, id, 1u);
-                }
-                tc_commit(&empty[s]);   // the slot is free once these MMAs have read it
-            }
-            tc_commit(accum);
-        }
-        __syncwarp();
-    }
-
-    // epilogue: warp w holds rows 32 w .. 32 w + 31 of the tile in its tensor-memory lanes
-    if (!mbar_wait(accum, 0)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
-    tc_fence_after();
-    const int row = tm * kTcM + warp * 32 + lane;
-    const uint32_t tl = tmem + ((uint32_t)(warp * 32) << 16);
-#pragma unroll
-    for (int c0 = 0; c0 < kTcN; c0 += 16) {
-        float re[16], im[16];
-        tc_ld16(tl + (uint32_t)c0, re);
-        tc_ld16(tl + (uint32_t)(kTcN + c0), im);
-        tc_ld_wait();
-        if (row < P.S) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const int col = tn * kTcN + c0 + j;
-                if (col < P.S) {
-                    float2 *c = job.C + row + (int64_t)col * P.S;
-                    float2 v = make_float2(job.alpha * re[j], job.alpha * im[j]);
-                    if (job.beta) {
-                        const float2 o = *c;
-                        v.x += o.x;
-                        v.y += o.y;
+            for (int i = 0; i < 8; ++i) {
+                const int n = n0 + nb + 16 * i;
+                v[i][0] = v[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (n < S && k0 < S) {
+                    const float2 *b = B + (int64_t)n * S + k0;
+                    if (vec) {
+                        v[i][0] = __ldg(reinterpret_cast<const float4 *>(b));
+                        v[i][1] = __ldg(reinterpret_cast<const float4 *>(b) + 1);
+                    } else {
+                        const float2 z = make_float2(0.f, 0.f);
+                        const float2 b0 = b[0], b1 = k0 + 1 < S ? b[1] : z, b2 = k0 + 2 < S ? b[2] : z,
+                                     b3 = k0 + 3 < S ? b[3] : z;
+                        v[i][0] = make_float4(b0.x, b0.y, b1.x, b1.y);
+                        v[i][1] = make_float4(b2.x, b2.y, b3.x, b3.y);
                     }
-                    *c = v;
+                }
+            }
+        };
+        load(0);
+        for (int ks = 0; ks < nstage; ++ks) {
+            const int s = ks % kTcStages;
+            if (!mbar_wait(&empty[s], ((uint32_t)(ks / kTcStages) & 1u) ^ 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
+            unsigned char *sb = smem + (size_t)s * kStageB;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int n = nb + 16 * i;
+                if (n >= n_eff) continue;
+                float4 *d = reinterpret_cast<float4 *>(sb + n * 128 + ((ch ^ (n & 7)) << 4));
+                const float4 re = make_float4(v[i][0].x, v[i][0].z, v[i][1].x, v[i][1].z);
+                const float4 im = make_float4(v[i][0].y, v[i][0].w, v[i][1].y, v[i][1].w);
+                const float4 rh = make_float4(tf32_rna(re.x), tf32_rna(re.y), tf32_rna(re.z), tf32_rna(re.w));
+                const float4 ih = make_float4(tf32_rna(im.x), tf32_rna(im.y), tf32_rna(im.z), tf32_rna(im.w));
+                d[0] = rh;
+                d[1 * kPlaneB / 16] = make_float4(re.x - rh.x, re.y - rh.y, re.z - rh.z, re.w - rh.w);
+                d[2 * kPlaneB / 16] = ih;
+                d[3 * kPlaneB / 16] = make_float4(im.x - ih.x, im.y - ih.y, im.z - ih.z, im.w - ih.w);
+            }
+            if (ks + 1 < nstage) load(ks + 1);
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s]);
+        }
+    } else if (lane == 0) {
+        // MMA issuer
+        const uint32_t ip = tf32_idesc(n_eff, 0), in = tf32_idesc(n_eff, 1);
+        const uint32_t re = tmem, im = tmem + kTcN;
+        for (int ks = 0; ks < nstage; ++ks) {
+            const int s = ks % kTcStages;
+            if (!mbar_wait(&full[s], (uint32_t)(ks / kTcStages) & 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
+            tc_fence_after();
+            const uint32_t ta = tmem + kTmemA + (uint32_t)(s * kPlanes * kTcK);
+            const uint32_t sb = smem_u32(smem + (size_t)s * kStageB);
+#pragma unroll
+            for (int k8 = 0; k8 < kTcK / 8; ++k8) {
+                uint32_t a[kPlanes];
+                uint64_t b[kPlanes];
+#pragma unroll
+                for (int p = 0; p < kPlanes; ++p) {
+                    a[p] = ta + (uint32_t)(p * kTcK + 8 * k8);
+                    b[p] = sw128_desc(sb + p * kPlaneB) + (uint64_t)(2 * k8);   // + 32 bytes of K
+                }
+                const uint32_t acc = (ks == 0 && k8 == 0) ? 0u : 1u;
+                // Re += Ar Br - Ai Bi, Im += Ar Bi + Ai Br; hi hi, hi lo, lo hi of each
+                tc_mma_ts(re, a[0], b[0], ip, acc);
+                tc_mma_ts(im, a[0], b[2], ip, acc);
+                tc_mma_ts(re, a[0], b[1], ip, 1u);
+                tc_mma_ts(im, a[0], b[3], ip, 1u);
+                tc_mma_ts(re, a[1], b[0], ip, 1u);
+                tc_mma_ts(im, a[1], b[2], ip, 1u);
+                tc_mma_ts(re, a[2], b[2], in, 1u);
+                tc_mma_ts(im, a[2], b[0], ip, 1u);
+                tc_mma_ts(re, a[2], b[3], in, 1u);
+                tc_mma_ts(im, a[2], b[1], ip, 1u);
+                tc_mma_ts(re, a[3], b[2], in, 1u);
+                tc_mma_ts(im, a[3], b[0], ip, 1u);
+            }
+            tc_commit(&empty[s]);   // the stage is free once these MMAs have read it
+        }
+        tc_commit(accum);
+    }
+    __syncwarp();
+
+    // epilogue: converting warp w reads rows 32 (w % 4) .. + 31 (the tensor-memory lanes it
+    // can reach) of columns 64 (w / 4) .. + 63
+    if (warp < kTcConvWarps) {
+        if (!mbar_wait(accum, 0)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
+        tc_fence_after();
+        const int row = m0 + (warp & 3) * 32 + lane;
+        const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        const int cb = (warp >> 2) * (kTcN / 2);
+#pragma unroll
+        for (int c0 = cb; c0 < cb + kTcN / 2; c0 += 16) {
+            if (c0 >= n_eff) break;
+            float re[16], im[16];
+            tc_ld16(tl + (uint32_t)c0, re);
+            tc_ld16(tl + (uint32_t)(kTcN + c0), im);
+            tc_ld_wait();
+            if (row < S) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const int col = n0 + c0 + j;
+                    if (col < S) {
+                        float2 *c = job.C + row + (int64_t)col * S;
+                        float2 v = make_float2(job.alpha * re[j], job.alpha * im[j]);
+                        if (job.beta) {
+                            const float2 o = *c;
+                            v.x += o.x;
+                            v.y += o.y;
+                        }
+                        *c = v;
+                    }
                 }
             }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tc_dealloc(tmem, kTmemCols);
+    if (warp == kTcConvWarps) tc_dealloc(tmem, kTmemCols);
 }
 
 // ----------------------------------------------------------------------------- host
-int tc_kp(int S) { return (S + kTcK - 1) / kTcK * kTcK; }
-
-// Splits srcA / srcB (device arrays of nA / nB matrix pointers, already on the device),
-// encodes the tensor maps and runs the jobs (device array of njobs).
-int tc_run(cudaStream_t st, int device, int S, const float2 *const *srcA, int nA, const float2 *const *srcB, int nB,
-           const TcJob *jobs, int njobs, float *planes, int *err) {
+// Runs the jobs (device array of njobs).  No job may read what another of the same call
+// writes.
+int tc_run(cudaStream_t st, int device, int S, const TcJob *jobs, int njobs, int *err) {
     if (njobs == 0) return KORE_OK;
-    if (nA > 65535 || nB > 65535) return KORE_EINVAL;
-    const int Kp = tc_kp(S);
-    float *pa = planes, *pb = planes + (int64_t)nA * kPlanesA * S * Kp;
-    const dim3 sg(Kp / 32, kore_div_up(S, 32));
-    k_tc_split<true><<<dim3(sg.x, sg.y, nA), dim3(32, 8), 0, st>>>(srcA, S, Kp, pa);
-    k_tc_split<false><<<dim3(sg.x, sg.y, nB), dim3(32, 8), 0, st>>>(srcB, S, Kp, pb);
-    KORE_LAUNCHED(2);
     TcParams P;
-    const uint64_t da[3] = {(uint64_t)Kp, (uint64_t)S, (uint64_t)kPlanesA * nA};
-    const uint64_t db[3] = {(uint64_t)Kp, (uint64_t)S, (uint64_t)kPlanesB * nB};
-    const uint64_t sd[2] = {(uint64_t)Kp * 4, (uint64_t)S * Kp * 4};
-    const uint32_t ba[3] = {kTcK, kTcM, 1}, bb[3] = {kTcK, kTcN, 1};
-    KORE_TRY(kore_encode_f32_3d(&P.amap, pa, da, sd, ba, 1));
-    KORE_TRY(kore_encode_f32_3d(&P.bmap, pb, db, sd, bb, 1));
     P.S = S;
-    P.Kp = Kp;
     P.tiles_n = kore_div_up(S, kTcN);
     P.err = err;
     const int tiles = kore_div_up(S, kTcM) * P.tiles_n;
@@ -329,8 +360,7 @@ int tc_run(cudaStream_t st, int device, int S, const float2 *const *srcA, int nA
 
 // FP64 reference of the self-test: C_ref(r, c) = beta C0 + alpha sum of the products
 // and the magnitude bound sum |a| |b| (one thread per element).
-__global__ void k_tc_ref(int S, const float2 *A, const float2 *B, const TcJob *jobs, int njobs, const float2 *C0,
-                         double *err) {
+__global__ void k_tc_ref(int S, const TcJob *jobs, int njobs, const float2 *C0, double *err) {
     const int j = blockIdx.y;
     if (j >= njobs) return;
     const TcJob jb = jobs[j];
@@ -339,10 +369,10 @@ __global__ void k_tc_ref(int S, const float2 *A, const float2 *B, const TcJob *j
         const int r = (int)(e % S), c = (int)(e / S);
         double sr = 0, si = 0, mag = 0;
         for (int pr = 0; pr < 2; ++pr) {
-            const int ia = pr ? jb.a2 : jb.a1, ib = pr ? jb.b2 : jb.b1;
-            if (ia < 0) continue;
+            const float2 *A = pr ? jb.A2 : jb.A1, *B = pr ? jb.B2 : jb.B1;
+            if (!A) continue;
             for (int k = 0; k < S; ++k) {
-                const float2 a = A[ia * SS + r + (int64_t)k * S], b = B[ib * SS + k + (int64_t)c * S];
+                const float2 a = A[r + (int64_t)k * S], b = B[k + (int64_t)c * S];
                 sr += (double)a.x * b.x - (double)a.y * b.y;
                 si += (double)a.x * b.y + (double)a.y * b.x;
                 mag += (fabs((double)a.x) + fabs((double)a.y)) * (fabs((double)b.x) + fabs((double)b.y));
@@ -370,26 +400,20 @@ __global__ void k_tc_fill(float2 *x, int64_t n, uint64_t seed) {
 }  // namespace
 
 // ----------------------------------------------------------------------------- factorisation use
-int tc_upload_run(kore_plan *p, const std::vector<const float2 *> &src, int64_t nA, const std::vector<TcJob> &jobs);
-// Bytes of the split planes and the job table for one reduction level's even-block update
-// (levels >= 1) of `cap` shifts; the plan allocates the largest over its levels.
-void kore_tc_level_bytes(const kore_plan *p, int cap, int64_t *plane_bytes, int64_t *table_bytes) {
-    int64_t pl = 0, tb = 0;
-    const int64_t S = p->S, Kp = tc_kp(p->S);
-    for (int l = 0; l < p->nlev; ++l) {
-        const int64_t ne = p->lev[l].neven, no = p->lev[l].nodd;
-        // even update (levels >= 1): 2 neven A + 2 nodd B matrices, 3 neven jobs;
-        // G, H and their refinement (every level): nodd A + 2 nodd B matrices, 2 nodd jobs
-        // planes: 4 per A and 6 per B matrix
-        const int64_t np_ = std::max(l > 0 ? 2 * ne * kPlanesA + 2 * no * kPlanesB : 0,
-                                     no * kPlanesA + 2 * no * kPlanesB) * cap;
-        const int64_t nm = std::max(l > 0 ? 2 * (ne + no) : 0, 3 * no) * cap;
-        const int64_t nj = std::max(l > 0 ? 3 * ne : 0, 2 * no) * cap;
-        pl = std::max(pl, np_ * S * Kp * 4);
-        tb = std::max(tb, nm * 8 + nj * (int64_t)sizeof(TcJob) + 64);
-    }
-    *plane_bytes = pl;
-    *table_bytes = tb;
+// Bytes of the job table for one reduction level of `cap` shifts; the plan allocates the
+// largest over its levels.
+int64_t kore_tc_table_bytes(const kore_plan *p, int cap) {
+    int64_t nj = 0;
+    for (int l = 0; l < p->nlev; ++l)
+        // even update (levels >= 1): 3 neven jobs; G, H and their refinement: 2 nodd jobs
+        nj = std::max<int64_t>(nj, std::max(l > 0 ? 3 * p->lev[l].neven : 0, 2 * p->lev[l].nodd));
+    return nj * cap * (int64_t)sizeof(TcJob) + 64;
+}
+
+static int tc_upload_run(kore_plan *p, const std::vector<TcJob> &jobs) {
+    KORE_CUDA_TRY(cudaMemcpyAsync(p->d_tctab, jobs.data(), jobs.size() * sizeof(TcJob), cudaMemcpyHostToDevice,
+                                  p->stream));
+    return tc_run(p->stream, p->device, p->S, static_cast<const TcJob *>(p->d_tctab), (int)jobs.size(), p->d_err);
 }
 
 // Even-block update of level l >= 1 for every shift (complex64 factors), the
@@ -399,50 +423,27 @@ int kore_even_update_tc(kore_plan *p, const BcrLevel &lv) {
     const int S = p->S, ns = p->fw_n;
     const int64_t lo = p->fw_lo;   // shift sh of the factor window is shift lo + sh of the plan
     const int64_t SS = (int64_t)S * S;
-    std::vector<const float2 *> src;   // A operands, then B operands
     std::vector<TcJob> jobs;
-    const int64_t nA = 2 * (int64_t)lv.neven * ns, nB = 2 * (int64_t)lv.nodd * ns;
-    src.reserve(nA + nB);
-    for (int sh = 0; sh < ns; ++sh) {
-        const float2 *LU = static_cast<const float2 *>(p->d_LU) + (lo + sh) * p->lu_stride();
-        for (int e = 0; e < lv.neven; ++e) {
-            src.push_back(LU + (lv.lu_L + 2 * e) * SS);   // A index (sh neven + e) 2 + 0: L_q
-            src.push_back(LU + (lv.lu_U + 2 * e) * SS);   //                            + 1: U_q
-        }
-    }
-    for (int sh = 0; sh < ns; ++sh) {
-        const float2 *G = static_cast<const float2 *>(p->d_Gm) + (lo + sh) * p->f_stride();
-        const float2 *H = static_cast<const float2 *>(p->d_Hm) + (lo + sh) * p->f_stride();
-        for (int o = 0; o < lv.nodd; ++o) {
-            const int64_t j = (int64_t)(2 * o + 1) * lv.stride;
-            src.push_back(G + j * SS);                    // B index (sh nodd + o) 2 + 0: G_j
-            src.push_back(H + j * SS);                    //                         + 1: H_j
-        }
-    }
     for (int sh = 0; sh < ns; ++sh) {
         float2 *LU = static_cast<float2 *>(p->d_LU) + (lo + sh) * p->lu_stride();
         float2 *Dw = static_cast<float2 *>(p->d_Dw) + (lo + sh) * p->f_stride();
+        const float2 *G = static_cast<const float2 *>(p->d_Gm) + (lo + sh) * p->f_stride();
+        const float2 *H = static_cast<const float2 *>(p->d_Hm) + (lo + sh) * p->f_stride();
         for (int e = 0; e < lv.neven; ++e) {
-            const int q = 2 * e;
+            const int64_t q = 2 * e, jl = (q - 1) * lv.stride * SS, jr = (q + 1) * lv.stride * SS;
             const bool hasl = q >= 1, hasr = q + 1 < lv.Kl;
-            const int aL = (sh * lv.neven + e) * 2, aU = aL + 1;
-            const int bl = (sh * lv.nodd + e - 1) * 2, br = (sh * lv.nodd + e) * 2;   // + 0: G, + 1: H
-            if (hasl || hasr) {
-                TcJob j{-1, -1, -1, -1, Dw + (int64_t)q * lv.stride * SS, -1.f, 1};
-                if (hasl) { j.a1 = aL; j.b1 = bl + 1; }
-                if (hasr) {
-                    if (j.a1 < 0) { j.a1 = aU; j.b1 = br; }
-                    else { j.a2 = aU; j.b2 = br; }
-                }
-                jobs.push_back(j);
-            }
-            if (lv.lu_nL >= 0 && q >= 2) jobs.push_back(TcJob{aL, bl, -1, -1, LU + (lv.lu_nL + e) * SS, -1.f, 0});
+            const float2 *Lq = LU + (lv.lu_L + q) * SS, *Uq = LU + (lv.lu_U + q) * SS;
+            float2 *D = Dw + q * lv.stride * SS;
+            if (hasl && hasr) jobs.push_back(TcJob{Lq, H + jl, Uq, G + jr, D, -1.f, 1});
+            else if (hasl) jobs.push_back(TcJob{Lq, H + jl, nullptr, nullptr, D, -1.f, 1});
+            else if (hasr) jobs.push_back(TcJob{Uq, G + jr, nullptr, nullptr, D, -1.f, 1});
+            if (lv.lu_nL >= 0 && q >= 2)
+                jobs.push_back(TcJob{Lq, G + jl, nullptr, nullptr, LU + (lv.lu_nL + e) * SS, -1.f, 0});
             if (lv.lu_nU >= 0 && q + 2 < lv.Kl)
-                jobs.push_back(TcJob{aU, br + 1, -1, -1, LU + (lv.lu_nU + e) * SS, -1.f, 0});
+                jobs.push_back(TcJob{Uq, H + jr, nullptr, nullptr, LU + (lv.lu_nU + e) * SS, -1.f, 0});
         }
     }
-    (void)nB;
-    return tc_upload_run(p, src, nA, jobs);
+    return tc_upload_run(p, jobs);
 }
 
 // R(k, c) += rs_k a_e for the level-0 couplings of the odd blocks (side 0: L_j into
@@ -464,17 +465,6 @@ __global__ void k_add_couplings(const int *__restrict__ cc_ptr, const int *__res
             float2 &r = R[k + (int64_t)c * S];
             r = make_float2((float)((double)r.x + a.x), (float)((double)r.y + a.y));
         }
-}
-
-int tc_upload_run(kore_plan *p, const std::vector<const float2 *> &src, int64_t nA, const std::vector<TcJob> &jobs) {
-    const size_t pbytes = src.size() * sizeof(void *), jbytes = jobs.size() * sizeof(TcJob);
-    unsigned char *tab = static_cast<unsigned char *>(p->d_tctab);
-    KORE_CUDA_TRY(cudaMemcpyAsync(tab, src.data(), pbytes, cudaMemcpyHostToDevice, p->stream));
-    KORE_CUDA_TRY(cudaMemcpyAsync(tab + pbytes, jobs.data(), jbytes, cudaMemcpyHostToDevice, p->stream));
-    const float2 *const *dsrc = reinterpret_cast<const float2 *const *>(tab);
-    return tc_run(p->stream, p->device, p->S, dsrc, (int)nA, dsrc + nA, (int)(src.size() - nA),
-                  reinterpret_cast<const TcJob *>(tab + pbytes), (int)jobs.size(), static_cast<float *>(p->d_tcplanes),
-                  p->d_err);
 }
 
 // G_j = D_j^-1 L_j and H_j = D_j^-1 U_j of the odd blocks of a level for every shift
@@ -503,37 +493,22 @@ int kore_gh_update_tc(kore_plan *p, const BcrLevel &lv, int level0) {
         return LU + (lo + sh) * p->lu_stride() + ((side ? lv.lu_U : lv.lu_L) + 2 * o + 1) * SS;
     };
     auto hasr = [&](int64_t o) { return 2 * o + 2 < lv.Kl; };
-    std::vector<const float2 *> src;
+    // one job per (shift, odd block, side): C = beta C + alpha A B with A the block's matrix
     std::vector<TcJob> jobs;
-    // stage 1 (levels >= 1): G0 = D^-1 L, H0 = D^-1 U
-    if (!level0) {
-        for (int sh = 0; sh < ns; ++sh)
-            for (int64_t o = 0; o < no; ++o) src.push_back(blk(Dinv, sh, o));
-        for (int sh = 0; sh < ns; ++sh)
-            for (int64_t o = 0; o < no; ++o) { src.push_back(rstore(sh, o, 0)); src.push_back(rstore(sh, o, 1)); }
+    auto run = [&](float2 *A, auto B, auto Cm, float alpha, int beta) {
+        jobs.clear();
         for (int sh = 0; sh < ns; ++sh)
             for (int64_t o = 0; o < no; ++o) {
-                const int a = (int)(sh * no + o);
-                jobs.push_back(TcJob{a, 2 * a, -1, -1, blk(G, sh, o), 1.f, 0});
-                if (hasr(o)) jobs.push_back(TcJob{a, 2 * a + 1, -1, -1, blk(H, sh, o), 1.f, 0});
+                jobs.push_back(TcJob{blk(A, sh, o), B(sh, o, 0), nullptr, nullptr, Cm(sh, o, 0), alpha, beta});
+                if (hasr(o)) jobs.push_back(TcJob{blk(A, sh, o), B(sh, o, 1), nullptr, nullptr, Cm(sh, o, 1), alpha, beta});
             }
-        KORE_TRY(tc_upload_run(p, src, ns * no, jobs));
-    }
-    // stage 2: R = L - D G0 (level 0: R = -D G0, then + L from the sparse couplings)
-    src.clear();
-    jobs.clear();
-    for (int sh = 0; sh < ns; ++sh)
-        for (int64_t o = 0; o < no; ++o) src.push_back(blk(Dw, sh, o));
-    for (int sh = 0; sh < ns; ++sh)
-        for (int64_t o = 0; o < no; ++o) { src.push_back(blk(G, sh, o)); src.push_back(blk(H, sh, o)); }
-    for (int sh = 0; sh < ns; ++sh)
-        for (int64_t o = 0; o < no; ++o) {
-            const int a = (int)(sh * no + o);
-            const int beta = level0 ? 0 : 1;
-            jobs.push_back(TcJob{a, 2 * a, -1, -1, rstore(sh, o, 0), -1.f, beta});
-            if (hasr(o)) jobs.push_back(TcJob{a, 2 * a + 1, -1, -1, rstore(sh, o, 1), -1.f, beta});
-        }
-    KORE_TRY(tc_upload_run(p, src, ns * no, jobs));
+        return tc_upload_run(p, jobs);
+    };
+    auto gh = [&](int sh, int64_t o, int side) { return blk(side ? H : G, sh, o); };
+    // levels >= 1: G0 = D^-1 L, H0 = D^-1 U
+    if (!level0) KORE_TRY(run(Dinv, rstore, gh, 1.f, 0));
+    // R = L - D G0 (level 0: R = -D G0, then + L from the sparse couplings)
+    KORE_TRY(run(Dw, gh, rstore, -1.f, level0 ? 0 : 1));
     if (level0) {
         k_add_couplings<<<dim3((unsigned)no, 2, ns), 256, 0, p->stream>>>(p->d_cc_ptr, p->d_cc_row, p->d_cc_src,
                                                                           p->d_aval, p->d_rscale + lo * p->np, S,
@@ -541,20 +516,8 @@ int kore_gh_update_tc(kore_plan *p, const BcrLevel &lv, int level0) {
                                                                           p->t_stride());
         KORE_LAUNCHED(1);
     }
-    // stage 3: G = G0 + D^-1 R
-    src.clear();
-    jobs.clear();
-    for (int sh = 0; sh < ns; ++sh)
-        for (int64_t o = 0; o < no; ++o) src.push_back(blk(Dinv, sh, o));
-    for (int sh = 0; sh < ns; ++sh)
-        for (int64_t o = 0; o < no; ++o) { src.push_back(rstore(sh, o, 0)); src.push_back(rstore(sh, o, 1)); }
-    for (int sh = 0; sh < ns; ++sh)
-        for (int64_t o = 0; o < no; ++o) {
-            const int a = (int)(sh * no + o);
-            jobs.push_back(TcJob{a, 2 * a, -1, -1, blk(G, sh, o), 1.f, 1});
-            if (hasr(o)) jobs.push_back(TcJob{a, 2 * a + 1, -1, -1, blk(H, sh, o), 1.f, 1});
-        }
-    return tc_upload_run(p, src, ns * no, jobs);
+    // G = G0 + D^-1 R
+    return run(Dinv, rstore, gh, 1.f, 1);
 }
 
 extern "C" int kore_tc_selftest(int device, int S, int nmat, double *max_rel_err) {
@@ -562,10 +525,9 @@ extern "C" int kore_tc_selftest(int device, int S, int nmat, double *max_rel_err
     int prev = -1;
     cudaGetDevice(&prev);
     KORE_CUDA_TRY(cudaSetDevice(device));
-    const int64_t SS = (int64_t)S * S, Kp = tc_kp(S);
+    const int64_t SS = (int64_t)S * S;
     float2 *A = nullptr, *B = nullptr, *C = nullptr, *C0 = nullptr;
-    float *planes = nullptr;
-    unsigned char *tab = nullptr;
+    TcJob *tab = nullptr;
     double *err = nullptr;
     int *flag = nullptr;
     int rc = KORE_OK;
@@ -574,8 +536,7 @@ extern "C" int kore_tc_selftest(int device, int S, int nmat, double *max_rel_err
     ck(cudaMalloc(&B, nmat * SS * sizeof(float2)));
     ck(cudaMalloc(&C, nmat * SS * sizeof(float2)));
     ck(cudaMalloc(&C0, nmat * SS * sizeof(float2)));
-    ck(cudaMalloc(&planes, (size_t)nmat * (kPlanesA + kPlanesB) * S * Kp * sizeof(float)));
-    ck(cudaMalloc(&tab, (size_t)2 * nmat * 8 + (size_t)nmat * sizeof(TcJob)));
+    ck(cudaMalloc(&tab, (size_t)nmat * sizeof(TcJob)));
     ck(cudaMalloc(&err, sizeof(double)));
     ck(cudaMalloc(&flag, sizeof(int)));
     if (rc == KORE_OK) {
@@ -585,22 +546,16 @@ extern "C" int kore_tc_selftest(int device, int S, int nmat, double *max_rel_err
         ck(cudaMemcpy(C0, C, nmat * SS * sizeof(float2), cudaMemcpyDeviceToDevice));
         ck(cudaMemset(err, 0, sizeof(double)));
         ck(cudaMemset(flag, 0, sizeof(int)));
-        std::vector<const float2 *> src;
-        for (int m = 0; m < nmat; ++m) src.push_back(A + m * SS);
-        for (int m = 0; m < nmat; ++m) src.push_back(B + m * SS);
         // job m: even m: C_m = A_m B_m;  odd m: C_m -= A_m B_m + A_{m-1} B_{m+1 mod n}
         std::vector<TcJob> jobs;
         for (int m = 0; m < nmat; ++m) {
-            if (m % 2 == 0) jobs.push_back(TcJob{m, m, -1, -1, C + m * SS, 1.f, 0});
-            else jobs.push_back(TcJob{m, m, m - 1, (m + 1) % nmat, C + m * SS, -1.f, 1});
+            if (m % 2 == 0) jobs.push_back(TcJob{A + m * SS, B + m * SS, nullptr, nullptr, C + m * SS, 1.f, 0});
+            else jobs.push_back(TcJob{A + m * SS, B + m * SS, A + (m - 1) * SS, B + (m + 1) % nmat * SS, C + m * SS, -1.f, 1});
         }
-        ck(cudaMemcpy(tab, src.data(), src.size() * 8, cudaMemcpyHostToDevice));
-        ck(cudaMemcpy(tab + src.size() * 8, jobs.data(), jobs.size() * sizeof(TcJob), cudaMemcpyHostToDevice));
-        const float2 *const *dsrc = reinterpret_cast<const float2 *const *>(tab);
-        const TcJob *djobs = reinterpret_cast<const TcJob *>(tab + src.size() * 8);
-        if (rc == KORE_OK) rc = tc_run(0, device, S, dsrc, nmat, dsrc + nmat, nmat, djobs, nmat, planes, flag);
+        ck(cudaMemcpy(tab, jobs.data(), jobs.size() * sizeof(TcJob), cudaMemcpyHostToDevice));
+        if (rc == KORE_OK) rc = tc_run(0, device, S, tab, nmat, flag);
         if (rc == KORE_OK) {
-            k_tc_ref<<<dim3(64, nmat), 256>>>(S, A, B, djobs, nmat, C0, err);
+            k_tc_ref<<<dim3(64, nmat), 256>>>(S, tab, nmat, C0, err);
             ck(cudaGetLastError());
             ck(cudaDeviceSynchronize());
             int h = 0;
@@ -609,7 +564,7 @@ extern "C" int kore_tc_selftest(int device, int S, int nmat, double *max_rel_err
             if (rc == KORE_OK && h != 0) rc = KORE_ETIMEOUT;
         }
     }
-    cudaFree(A); cudaFree(B); cudaFree(C); cudaFree(C0); cudaFree(planes); cudaFree(tab); cudaFree(err); cudaFree(flag);
+    cudaFree(A); cudaFree(B); cudaFree(C); cudaFree(C0); cudaFree(tab); cudaFree(err); cudaFree(flag);
     if (prev >= 0) cudaSetDevice(prev);
     return rc;
 }

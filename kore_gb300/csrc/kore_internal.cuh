@@ -117,9 +117,8 @@ struct kore_plan {
     int *d_ell_col = nullptr;         // padded slot of the coupled unknown, -1 for padding
     int *d_ell_src = nullptr;         // entry of A in the permuted CSR, -1 for padding
     void *d_ell_val = nullptr;        // per shift: rscale_row * A entry, factor precision
-    // complex64 factorisation: TF32 split planes and job table of the tensor-core
-    // even-block updates (gemm_tc.cu), sized for the largest level
-    void *d_tcplanes = nullptr;
+    // complex64 factorisation: job table of the tensor-core products (gemm_tc.cu), sized
+    // for the largest level
     void *d_tctab = nullptr;
 
     int64_t f_stride() const { return (int64_t)K * S * S; }
@@ -196,7 +195,8 @@ int kore_even_update_tc(kore_plan *p, const BcrLevel &lv);
 // G_j, H_j of the odd blocks with one refinement step (level0: G0, H0 already formed
 // from the sparse couplings)
 int kore_gh_update_tc(kore_plan *p, const BcrLevel &lv, int level0);
-void kore_tc_level_bytes(const kore_plan *p, int cap, int64_t *plane_bytes, int64_t *table_bytes);
+// bytes of the job table of `cap` shifts
+int64_t kore_tc_table_bytes(const kore_plan *p, int cap);
 
 // sweep.cu
 // x_s = (A - sigma_s B)^-1 b_s for every factorised shift s on padded l-major

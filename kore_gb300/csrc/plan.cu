@@ -98,7 +98,7 @@ void free_plan(kore_plan *p) {
                     p->d_red, p->d_part, p->d_err, p->d_bar, p->d_ir, p->d_V, p->d_Vtmp, p->d_ksx, p->d_small, p->d_warm,
                     p->d_sigma, p->d_minf, p->d_bb, p->d_xb, p->d_rb, p->d_bn, p->d_rn, p->d_cnt,
                     p->d_ell_col, p->d_ell_src, p->d_ell_val, p->d_long_rows, p->d_srow, p->d_smid,
-                    p->d_scol, p->d_sval, p->d_cc_ptr, p->d_cc_row, p->d_cc_src};
+                    p->d_scol, p->d_sval, p->d_cc_ptr, p->d_cc_row, p->d_cc_src, p->d_tctab};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     for (auto &v : p->d_v)
@@ -588,18 +588,9 @@ int kore_plan_estimate_bytes(const kore_pencil_desc *d, int precision, int nshif
     b += np * 8 + K * 4 + nlev * (int64_t)sizeof(BcrLevel) + 6 * np * 16 + 8192 * 8 + 1024;
     // factors and solve workspace of c shifts
     b += c * (4 * K * SS * e + lu * SS * e + nodd_max * 2 * SS * e + 3 * np * e + np * 8 + 3 * nodd_max * S * 4);
-    // level-0 couplings by column; split planes and job table of the tensor-core updates
+    // level-0 couplings by column; job table of the tensor-core products
     b += (2 * (K / 2 + 1) * (S + 1) + 2 * na) * 4;
-    if (precision == KORE_PREC_MIXED) {
-        const int64_t Kp = (S + 31) / 32 * 32;
-        int64_t nm = 0, nj = 0;
-        for (int64_t l = 0; l < nlev; ++l) {
-            const int64_t ne = Ks[l] - Ks[l] / 2, no = Ks[l] / 2;
-            nm = std::max<int64_t>(nm, std::max<int64_t>(l > 0 ? 4 * ne + 6 * no : 0, 4 * no + 6 * no) * 2);
-            nj = std::max<int64_t>(nj, std::max<int64_t>(l > 0 ? 3 * ne : 0, 2 * no));
-        }
-        b += c * (nm / 2 * S * Kp * 4 + nm * 8 + nj * 32 + 64);   // nm / 2 planes of S x Kp floats
-    }
+    if (precision == KORE_PREC_MIXED) b += c * (3 * (K + 1) * 48 + 64);
     b += c * (3 * np * 16 + 2 * (np / 64 + np / 8 + 1024) * 8 + (nlev > 0 ? 3 * nlev + 2 : 1) * K * 4 + ell * e + 128);
     b += 2 * d->n * c * 16;   // kore_solve's device copies of b and x
     // per target (one per shift): Krylov basis, its restart copy, a gathered input vector,

@@ -57,3 +57,15 @@ def test_block_shapes(gpu_lib, sizes, nshift, precision):
         assert solve_residual(M, x[:, s], b[:, s]) <= tol, s
         xr = forced_solve(M, b[:, s])
         assert np.linalg.norm(x[:, s] - xr) <= 1e-10 * np.linalg.norm(xr), s
+
+
+@pytest.mark.parametrize("S", [1, 5, 16, 33, 67, 127, 128, 129, 144, 256, 260, 513, 1024])
+def test_tc_gemm_tile_edges(gpu_lib, S):
+    """The complex64 tensor-core product around its 128 x 128 x 32 tile and at odd sizes
+    (columns off the 16-byte boundary).  3xTF32 with FP32 accumulation relative to
+    sum |a||b|: the dropped lo lo product and the rounding of lo (2^-21 each) and the
+    accumulation of S terms and twelve products, sqrt(12 S) 2^-24."""
+    import ctypes
+    err = ctypes.c_double(-1.0)
+    assert gpu_lib.kore_tc_selftest(0, S, 6, ctypes.byref(err)) == 0
+    assert 0.0 <= err.value < 2 * 2.0 ** -21 + (12 * S) ** 0.5 * 2.0 ** -24, err.value
