@@ -32,6 +32,8 @@
 
 namespace {
 
+// A 128 x 64 tile with one stage and two CTAs per SM, meant to overlap one CTA's epilogue
+// with the other's MMAs, took 2.5 times as long: each slice then waits for its conversion.
 constexpr int kTcM = 128, kTcN = 128, kTcK = 32, kTcStages = 2;
 constexpr int kTcConvWarps = 8;                   // 4 for A, 4 for B; warp 8 issues the MMAs
 constexpr int kTcThreads = 32 * (kTcConvWarps + 1);
@@ -100,16 +102,13 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
-// write 32 consecutive 32-bit columns of this warp's 32 lanes
-__device__ __forceinline__ void tc_st32(uint32_t taddr, const float (&v)[32]) {
+// write 16 consecutive 32-bit columns of this warp's 32 lanes
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const float (&v)[16]) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};" ::"f"(v[0]),
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"f"(v[0]),
         "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
-        "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]), "f"(v[16]), "f"(v[17]), "f"(v[18]),
-        "f"(v[19]), "f"(v[20]), "f"(v[21]), "f"(v[22]), "f"(v[23]), "f"(v[24]), "f"(v[25]), "f"(v[26]), "f"(v[27]),
-        "f"(v[28]), "f"(v[29]), "f"(v[30]), "f"(v[31]), "r"(taddr)
+        "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15]), "r"(taddr)
         : "memory");
 }
 __device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -189,19 +188,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcParams P) {
             if (!mbar_wait(&empty[s], ((uint32_t)(ks / kTcStages) & 1u) ^ 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
             tc_fence_after();
             const uint32_t ta = tmem + kTmemA + (uint32_t)(s * kPlanes * kTcK) + ((uint32_t)(warp * 32) << 16);
-            float r[kTcK];
 #pragma unroll
-            for (int k = 0; k < kTcK; ++k) r[k] = tf32_rna(v[k].x);
-            tc_st32(ta, r);
+            for (int p = 0; p < kPlanes; ++p)
 #pragma unroll
-            for (int k = 0; k < kTcK; ++k) r[k] = v[k].x - tf32_rna(v[k].x);
-            tc_st32(ta + kTcK, r);
+                for (int h = 0; h < kTcK; h += 16) {
+                    float r[16];
 #pragma unroll
-            for (int k = 0; k < kTcK; ++k) r[k] = tf32_rna(v[k].y);
-            tc_st32(ta + 2 * kTcK, r);
-#pragma unroll
-            for (int k = 0; k < kTcK; ++k) r[k] = v[k].y - tf32_rna(v[k].y);
-            tc_st32(ta + 3 * kTcK, r);
+                    for (int k = 0; k < 16; ++k) {
+                        const float x = p < 2 ? v[h + k].x : v[h + k].y, hi = tf32_rna(x);
+                        r[k] = (p & 1) ? x - hi : hi;
+                    }
+                    tc_st16(ta + (uint32_t)(p * kTcK + h), r);
+                }
             if (ks + 1 < nstage) load(ks + 1);
             tc_st_wait();
             tc_fence_before();
@@ -213,12 +211,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcParams P) {
         // memory: row n of a plane is 128 bytes of K, its 16-byte chunk ch at ch ^ (n & 7)
         const int ch = lane & 7, nb = (warp - 4) * 4 + (lane >> 3);
         const bool vec = (S & 3) == 0;   // every column starts on a 32-byte boundary
-        float4 v[8][2];
+        float4 v[kTcN / 16][2];
         auto load = [&](int ks) {
             const float2 *B = ks >= nk ? job.B2 : job.B1;
             const int k0 = (ks >= nk ? ks - nk : ks) * kTcK + 4 * ch;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < kTcN / 16; ++i) {
                 const int n = n0 + nb + 16 * i;
                 v[i][0] = v[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (n < S && k0 < S) {
@@ -242,7 +240,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcParams P) {
             if (!mbar_wait(&empty[s], ((uint32_t)(ks / kTcStages) & 1u) ^ 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
             unsigned char *sb = smem + (size_t)s * kStageB;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < kTcN / 16; ++i) {
                 const int n = nb + 16 * i;
                 if (n >= n_eff) continue;
                 float4 *d = reinterpret_cast<float4 *>(sb + n * 128 + ((ch ^ (n & 7)) << 4));
@@ -311,25 +309,27 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcParams P) {
 #pragma unroll
         for (int c0 = cb; c0 < cb + kTcN / 2; c0 += 16) {
             if (c0 >= n_eff) break;
+            // C's old entries are loaded together, ahead of the stores they must not wait for
+            float2 o[16];
+            float2 *c = job.C + row + (int64_t)(n0 + c0) * S;
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                o[j] = (job.beta && row < S && n0 + c0 + j < S) ? c[(int64_t)j * S] : make_float2(0.f, 0.f);
             float re[16], im[16];
             tc_ld16(tl + (uint32_t)c0, re);
             tc_ld16(tl + (uint32_t)(kTcN + c0), im);
             tc_ld_wait();
             if (row < S) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int col = n0 + c0 + j;
-                    if (col < S) {
-                        float2 *c = job.C + row + (int64_t)col * S;
+                for (int j = 0; j < 16; ++j)
+                    if (n0 + c0 + j < S) {
                         float2 v = make_float2(job.alpha * re[j], job.alpha * im[j]);
                         if (job.beta) {
-                            const float2 o = *c;
-                            v.x += o.x;
-                            v.y += o.y;
+                            v.x += o[j].x;
+                            v.y += o[j].y;
                         }
-                        *c = v;
+                        c[(int64_t)j * S] = v;
                     }
-                }
             }
         }
     }
