@@ -88,39 +88,63 @@ FV<C> make_fv(kore_plan *p) {
 
 // Row equilibration by powers of two (exact): rscale[p] = 2^-e with
 // e = exponent of max(max_e |a_pe|, |sigma| max_e |b_pe|); also the row 1-norms of
-// |A| + |sigma||B| whose maximum bounds ||A - sigma B||_inf.  Shift = blockIdx.y;
-// per-CTA maxima to red[s * gridDim.x + blockIdx.x].
+// |A| + |sigma||B| whose maximum bounds ||A - sigma B||_inf.  The entries are read once for
+// all shifts (one thread per row; their square roots run on the FP64 pipe).  Per-CTA maxima
+// to red[s * gridDim.x + blockIdx.x].
 template <typename C>
-__global__ void k_rowinfo(FV<C> v, double *__restrict__ red) {
-    const int s = blockIdx.y;
-    const double2 sg = v.sigma[s];
-    const double sabs = sqrt(abs2(sg));
-    double *rscale = v.rscale + (int64_t)s * v.np;
-    double mx = 0.0;
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < v.np; p += (int64_t)gridDim.x * blockDim.x) {
-        double am = 0.0, sum = 0.0;
-        for (int e = v.arow[p]; e < v.arow[p + 1]; ++e) {
-            const double t = sqrt(abs2(v.aval[e]));
-            am = fmax(am, t);
-            sum += t;
+__global__ void __launch_bounds__(256) k_rowinfo(FV<C> v, int nshift, double *__restrict__ red) {
+    __shared__ double sm[8];
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    double amax = 0.0, asum = 0.0, bmax = 0.0, bsum = 0.0;
+    if (p < v.np) {
+        const int a1 = v.arow[p + 1];
+#pragma unroll 4
+        for (int e = v.arow[p]; e < a1; ++e) {
+            const double2 a = v.aval[e];
+            const double t = a.y == 0.0 ? fabs(a.x) : a.x == 0.0 ? fabs(a.y) : sqrt(abs2(a));
+            amax = fmax(amax, t);
+            asum += t;
         }
-        if (v.has_b)
-            for (int e = v.brow[p]; e < v.brow[p + 1]; ++e) {
-                const double t = sabs * fabs(v.bval[e]);
-                am = fmax(am, t);
-                sum += t;
+        if (v.has_b) {
+            const int b1 = v.brow[p + 1];
+#pragma unroll 4
+            for (int e = v.brow[p]; e < b1; ++e) {
+                const double t = fabs(v.bval[e]);
+                bmax = fmax(bmax, t);
+                bsum += t;
             }
-        rscale[p] = (am > 0.0) ? ldexp(1.0, -ilogb(am)) : 1.0;
-        mx = fmax(mx, sum);
+        }
     }
+    for (int s = 0; s < nshift; ++s) {
+        const double sabs = sqrt(abs2(v.sigma[s]));
+        double mx = 0.0;
+        if (p < v.np) {
+            const double am = fmax(amax, sabs * bmax);
+            v.rscale[(int64_t)s * v.np + p] = (am > 0.0) ? ldexp(1.0, -ilogb(am)) : 1.0;
+            mx = asum + sabs * bsum;
+        }
+        mx = warp_max_d(mx);
+        if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = mx;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < 8; ++w) mx = fmax(mx, sm[w]);
+            red[(int64_t)s * gridDim.x + blockIdx.x] = mx;
+        }
+        __syncthreads();
+    }
+}
+
+// minf[s] = max of red[s * n .. s * n + n), one CTA per shift
+__global__ void k_minf(const double *__restrict__ red, int n, double *__restrict__ minf) {
+    __shared__ double sm[8];
+    double mx = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) mx = fmax(mx, red[(int64_t)blockIdx.x * n + i]);
     mx = warp_max_d(mx);
-    __shared__ double sm[32];
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = mx;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        double t = (threadIdx.x < (blockDim.x >> 5)) ? sm[threadIdx.x] : 0.0;
-        t = warp_max_d(t);
-        if (threadIdx.x == 0) red[(int64_t)s * gridDim.x + blockIdx.x] = t;
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) mx = fmax(mx, sm[w]);
+        minf[blockIdx.x] = mx;
     }
 }
 
@@ -190,23 +214,6 @@ __global__ void k_Dw_scatter(FV<C> v, int nshift) {
     }
 }
 
-// T_o = Dw_j for the odd blocks j of level lv, all shifts.  stride 0 selects block 0 (the
-// top of the reduction).
-template <typename C>
-__global__ void k_T_fill(FV<C> v, BcrLevel lv, int nodd, int nshift) {
-    const int S = v.S;
-    const int64_t SS = (int64_t)S * S, pershift = (int64_t)nodd * SS, total = pershift * nshift;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t s = idx / pershift;
-        const int64_t ws = idx - s * pershift;
-        const int64_t o = ws / SS;
-        const int64_t w = ws - o * SS;
-        const int64_t j = (2 * o + 1) * lv.stride;   // original block of position 2 o + 1
-        v.T[s * v.t_stride + o * 2 * SS + w] = v.Dw[s * v.f_stride + j * SS + w];
-    }
-}
-
 // Pivot keys: |x|^2 as the bits of a non-negative number, whose integer order is the
 // numeric one, so the search runs on the integer units (on this GPU an FP64 comparison
 // costs as much as an FP64 product).  0 (a zero, a NaN or a used row) is never a pivot.
@@ -236,6 +243,14 @@ __device__ __forceinline__ unsigned long long warp_argmax(unsigned long long key
     return ((unsigned long long)mh << 32) | ml;
 }
 
+// The diagonal block that work matrix o of shift sh inverts: the odd block at position
+// 2 o + 1 of a level (original block (2 o + 1) stride), or with stride 0 block 0, the top
+// of the reduction.
+template <typename C>
+__device__ __forceinline__ const C *diag_block(const FV<C> &v, int64_t o, int64_t sh, int stride) {
+    return v.Dw + sh * v.f_stride + (2 * o + 1) * stride * (int64_t)v.S * v.S;
+}
+
 // Panel reduction of columns [k0, k0+nb) of T_o; one CTA per (odd block o = blockIdx.x,
 // shift = blockIdx.y), one thread per row, which holds its NB entries of the panel in
 // registers.  Every elimination step works on register 0 and shifts the others down by
@@ -244,9 +259,10 @@ __device__ __forceinline__ unsigned long long warp_argmax(unsigned long long key
 // The panel is a chain of S dependent steps per block: with the panel in shared memory,
 // one step cost four barriers, an FP64 pivot search and two shared-memory accesses per
 // product; here it is two barriers, an integer search and one broadcast load per two
-// columns.
+// columns.  The first panel and its update
+// read the diagonal block itself, which stays as it is.
 template <typename C, int NB, int MAXT>
-__global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0) {
+__global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0, int stride) {
     __shared__ __align__(16) C prow[NB];
     __shared__ unsigned long long wkey[32];
     __shared__ int wrow[32];
@@ -254,6 +270,7 @@ __global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0) {
     const int S = v.S;
     const int64_t o = blockIdx.x, sh = blockIdx.y;
     C *T = v.T + sh * v.t_stride + o * 2 * (int64_t)S * S + (int64_t)k0 * S;
+    const C *src = k0 == 0 ? diag_block(v, o, sh, stride) : T;
     int *piv = v.piv + sh * v.p_stride + o * S, *pidx = v.pidx + sh * v.p_stride + o * S;
     int *used = v.used + sh * v.p_stride + o * S;
     const int r = threadIdx.x, lane = r & 31, w = r >> 5, nw = blockDim.x >> 5;
@@ -262,7 +279,7 @@ __global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0) {
 
     C P[NB];
 #pragma unroll
-    for (int c = 0; c < NB; ++c) P[c] = (in && c < nb) ? T[r + (int64_t)c * S] : czero<C>();
+    for (int c = 0; c < NB; ++c) P[c] = (in && c < nb) ? src[r + (int64_t)c * S] : czero<C>();
     bool u = !in || (k0 != 0 && used[r] != 0);
     int mine = -1;   // the panel column this row became the pivot of
     int c = 0;
@@ -329,20 +346,21 @@ __global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0) {
 // and FP32 arithmetic, not shared memory, is the bound (complex128: the FP64 pipe).
 constexpr int kUpdRows = 128;
 template <typename C, int NB, int TW>
-__global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb) {
+__global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb, int stride) {
     constexpr int CT = TW / 8;   // columns per thread
     __shared__ __align__(16) C tp[NB][TW];
     __shared__ __align__(16) C es[NB][kUpdRows];
     const int S = v.S;
     const int64_t o = blockIdx.y, sh = blockIdx.z;
     C *T = v.T + sh * v.t_stride + o * 2 * (int64_t)S * S;
+    const C *src = k0 == 0 ? diag_block(v, o, sh, stride) : T;
     const int *piv = v.piv + sh * v.p_stride + o * S, *pidx = v.pidx + sh * v.p_stride + o * S;
     // columns of this CTA, counted without the panel's own
     const int j0 = blockIdx.x * TW, ncols = S - nb;
     auto column = [&](int t) { const int j = j0 + t; return j < k0 ? j : j + nb; };
     for (int idx = threadIdx.x; idx < TW * NB; idx += 256) {
         const int c = idx % NB, t = idx / NB;
-        tp[c][t] = (j0 + t < ncols && c < nb) ? T[piv[k0 + c] + (int64_t)column(t) * S] : czero<C>();
+        tp[c][t] = (j0 + t < ncols && c < nb) ? src[piv[k0 + c] + (int64_t)column(t) * S] : czero<C>();
     }
     const C *E = T + (int64_t)k0 * S;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -359,7 +377,7 @@ __global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb) {
             const bool keep = r < S && pidx[r] < 0;   // a pivot row starts from zero
 #pragma unroll
             for (int t = 0; t < CT; ++t)
-                acc[i][t] = (keep && j0 + ty * CT + t < ncols) ? T[r + (int64_t)column(ty * CT + t) * S] : czero<C>();
+                acc[i][t] = (keep && j0 + ty * CT + t < ncols) ? src[r + (int64_t)column(ty * CT + t) * S] : czero<C>();
         }
         __syncthreads();
 #pragma unroll 4
@@ -404,57 +422,80 @@ __global__ void k_extract(FV<C> v, BcrLevel lv, int nodd, int top, int nshift) {
     }
 }
 
+// acc += a b; complex128 skips the products with a zero part of a (most couplings are
+// real or imaginary, and every FP64 product costs its pipe slot; the sums are the same).
+__device__ __forceinline__ float2 couple(float2 acc, float2 a, float2 b) { return cfma(acc, a, b); }
+__device__ __forceinline__ double2 couple(double2 acc, double2 a, double2 b) {
+    if (a.y == 0.0) return mk(fma(a.x, b.x, acc.x), fma(a.x, b.y, acc.y));
+    if (a.x == 0.0) return mk(fma(-a.y, b.y, acc.x), fma(a.y, b.x, acc.y));
+    return cfma(acc, a, b);
+}
+
 // Level 0 update of the even blocks with their sparse couplings:
 //   Dw_i -= rs (L_i H_jl + U_i G_jr),  L'_i = -rs L_i G_jl,  U'_i = -rs U_i H_jr.
-// CTA = (chunk of kEvenCW columns, even index e, shift); one thread per row, which reads
-// its row's coupling entries once, as padded rows (the level-0 rows of the sweep, with
-// the row scale folded in), and accumulates the kEvenCW columns in registers.
-constexpr int kEvenCW = 8;
-template <typename C>
+// CTA = (chunk of CW columns, even index e, shift); one thread per row, which reads its
+// row's coupling entries once, as padded rows (the level-0 rows of the sweep, with the row
+// scale folded in), and accumulates the CW columns in registers.  The CW columns of the
+// four matrices are staged in shared memory: an entry (about 30 per row) costs 2 CW reads
+// of them, and gathered from L2 those reads were what the kernel took its time for
+// (14.0 ms for 16 shifts of the 72k-unknown shell in complex64; complex128 is bound by
+// the FP64 pipe).
+template <typename C, int CW>
 __global__ void __launch_bounds__(512) k_even_l0(FV<C> v, BcrLevel lv) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C *sm = reinterpret_cast<C *>(smem_raw);   // [left H | left G | right G | right H], CW x S each
     const int S = v.S;
     const int64_t SS = (int64_t)S * S;
     const int64_t e = blockIdx.y, sh = blockIdx.z;
     const int64_t q = 2 * e;                 // position = original block at level 0
+    const bool hasl = q >= 1, hasr = q + 1 < lv.Kl;
     const bool outl = (lv.lu_nL >= 0) && q >= 2, outr = (lv.lu_nU >= 0) && q + 2 < lv.Kl;
-    const int c0 = blockIdx.x * kEvenCW;
-    const int cn = min(kEvenCW, S - c0);
+    const int c0 = blockIdx.x * CW;
+    const int cn = min(CW, S - c0);
     const int ntile = (S + 31) / 32;
     C *Di = v.Dw + sh * v.f_stride + q * SS;
     const C *G = v.G + sh * v.f_stride, *H = v.H + sh * v.f_stride;
-    const C *Hl = H + (q - 1) * SS, *Gl = G + (q - 1) * SS, *Gr = G + (q + 1) * SS, *Hr = H + (q + 1) * SS;
+    {
+        const int64_t off = (int64_t)c0 * S;
+        const C *src[4] = {hasl ? H + (q - 1) * SS + off : nullptr, outl ? G + (q - 1) * SS + off : nullptr,
+                           hasr ? G + (q + 1) * SS + off : nullptr, outr ? H + (q + 1) * SS + off : nullptr};
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+            if (src[m])
+                for (int i = threadIdx.x; i < cn * S; i += blockDim.x) sm[m * CW * S + i] = src[m][i];
+    }
+    __syncthreads();
     C *LU = v.LU + sh * v.lu_stride;
     const C *ev = v.ell_val + sh * v.ell_stride;
+    const int first = (int)(q * S);   // padded slot of the block's first row
     for (int r = threadIdx.x; r < S; r += blockDim.x) {
-        C dsum[kEvenCW], lsum[kEvenCW], usum[kEvenCW];
+        C dsum[CW], lsum[CW], usum[CW];
 #pragma unroll
-        for (int t = 0; t < kEvenCW; ++t) dsum[t] = lsum[t] = usum[t] = czero<C>();
+        for (int t = 0; t < CW; ++t) dsum[t] = lsum[t] = usum[t] = czero<C>();
         const int64_t ebase = ((q * ntile + r / 32) * (int64_t)v.ell_w) * 32 + (r & 31);
+#pragma unroll 4
         for (int k = 0; k < v.ell_w; ++k) {
             const int col = v.ell_col[ebase + (int64_t)k * 32];
-            if (col < 0) continue;
             const C a = ev[ebase + (int64_t)k * 32];
-            const int64_t blk = col / S, cr = col - blk * S;
-            if (blk < q) {   // left neighbour j = q - 1
+            if (col < 0) continue;
+            if (col < first) {   // left neighbour j = q - 1
+                const C *x = sm + (col - first + S);
 #pragma unroll
-                for (int t = 0; t < kEvenCW; ++t)
-                    if (t < cn) {
-                        const int64_t o = cr + (int64_t)(c0 + t) * S;
-                        dsum[t] = cfma(dsum[t], a, Hl[o]);
-                        if (outl) lsum[t] = cfma(lsum[t], a, Gl[o]);
-                    }
-            } else {         // right neighbour j = q + 1
+                for (int t = 0; t < CW; ++t) {
+                    dsum[t] = couple(dsum[t], a, x[t * S]);
+                    if (outl) lsum[t] = couple(lsum[t], a, x[(CW + t) * S]);
+                }
+            } else {             // right neighbour j = q + 1
+                const C *x = sm + 2 * CW * S + (col - first - S);
 #pragma unroll
-                for (int t = 0; t < kEvenCW; ++t)
-                    if (t < cn) {
-                        const int64_t o = cr + (int64_t)(c0 + t) * S;
-                        dsum[t] = cfma(dsum[t], a, Gr[o]);
-                        if (outr) usum[t] = cfma(usum[t], a, Hr[o]);
-                    }
+                for (int t = 0; t < CW; ++t) {
+                    dsum[t] = couple(dsum[t], a, x[t * S]);
+                    if (outr) usum[t] = couple(usum[t], a, x[(CW + t) * S]);
+                }
             }
         }
 #pragma unroll
-        for (int t = 0; t < kEvenCW; ++t)
+        for (int t = 0; t < CW; ++t)
             if (t < cn) {
                 const int64_t col = (int64_t)(c0 + t) * S;
                 Di[r + col] = Di[r + col] - dsum[t];
@@ -641,15 +682,15 @@ int gauss_jordan(kore_plan *p, const FV<C> &v, const BcrLevel &lv, int nodd, int
     const int pthreads = ((S + 31) / 32) * 32;
     for (int k0 = 0; k0 < S; k0 += NB) {
         const int nb = std::min(NB, S - k0);
-        k_panel<C, NB, MAXT><<<dim3(nodd, nshift), pthreads, 0, p->stream>>>(v, k0);
+        k_panel<C, NB, MAXT><<<dim3(nodd, nshift), pthreads, 0, p->stream>>>(v, k0, lv.stride);
         KORE_LAUNCHED(1);
         if (S == nb) break;
         // 32 columns per CTA re-read the panel least; levels with few blocks take 8, so
         // that their CTAs still cover the GPU
         if ((int64_t)nodd * nshift * kore_div_up(S - nb, 32) >= 2 * p->num_sms)
-            k_update<C, NB, 32><<<dim3(kore_div_up(S - nb, 32), nodd, nshift), 256, 0, p->stream>>>(v, k0, nb);
+            k_update<C, NB, 32><<<dim3(kore_div_up(S - nb, 32), nodd, nshift), 256, 0, p->stream>>>(v, k0, nb, lv.stride);
         else
-            k_update<C, NB, 8><<<dim3(kore_div_up(S - nb, 8), nodd, nshift), 256, 0, p->stream>>>(v, k0, nb);
+            k_update<C, NB, 8><<<dim3(kore_div_up(S - nb, 8), nodd, nshift), 256, 0, p->stream>>>(v, k0, nb, lv.stride);
         KORE_LAUNCHED(1);
     }
     k_extract<C><<<grid_for((int64_t)nodd * S * S * nshift, 256, p->num_sms), 256, 0, p->stream>>>(v, lv, nodd, top,
@@ -671,8 +712,6 @@ int factor_levels(kore_plan *p) {
     KORE_LAUNCHED(2);
     for (int l = 0; l < p->nlev; ++l) {
         const BcrLevel &lv = p->lev[l];
-        k_T_fill<C><<<grid_for((int64_t)lv.nodd * SS * ns, 256, p->num_sms), 256, 0, st>>>(v, lv, lv.nodd, ns);
-        KORE_LAUNCHED(1);
         // D_j^-1 of the odd blocks by Gauss-Jordan
         KORE_TRY((gauss_jordan<C, NB, MAXT>(p, v, lv, lv.nodd, 0, ns)));
         const int th = std::min(512, ((S + 31) / 32) * 32);   // rows per pass (S <= 1024: two passes at most)
@@ -682,8 +721,13 @@ int factor_levels(kore_plan *p) {
             k_gh_l0<C><<<dim3(kore_div_up(S, kGhCW), lv.nodd, ns), th, 0, st>>>(v);
             KORE_LAUNCHED(1);
             if (sizeof(C) == sizeof(float2)) KORE_TRY(kore_gh_update_tc(p, lv, 1));
-            dim3 g(kore_div_up(S, kEvenCW), lv.neven, ns);
-            k_even_l0<C><<<g, th, 0, st>>>(v, lv);
+            // columns per CTA: 8 while four blocks of 8 columns leave room for two CTAs per SM
+            // in shared memory (S = 400 in complex64: 102 KB), else fewer
+            const size_t per = (size_t)4 * S * sizeof(C);
+            const int cw = 8 * per <= 110 * 1024 ? 8 : 4 * per <= 110 * 1024 ? 4 : 2;
+            auto even = cw == 8 ? k_even_l0<C, 8> : cw == 4 ? k_even_l0<C, 4> : k_even_l0<C, 2>;
+            KORE_TRY(kore_allow_max_dyn_smem(even, p->device));
+            even<<<dim3(kore_div_up(S, cw), lv.neven, ns), th, cw * per, st>>>(v, lv);
             KORE_LAUNCHED(1);
         } else if (sizeof(C) == sizeof(float2)) {
             // complex64: tensor cores (3xTF32)
@@ -710,8 +754,6 @@ int factor_levels(kore_plan *p) {
     top.Kl = 1;
     top.stride = 0;
     top.lu_L = top.lu_U = top.lu_nL = top.lu_nU = -1;
-    k_T_fill<C><<<grid_for(SS * ns, 256, p->num_sms), 256, 0, st>>>(v, top, 1, ns);
-    KORE_LAUNCHED(1);
     KORE_TRY((gauss_jordan<C, NB, MAXT>(p, v, top, 1, 1, ns)));
     return KORE_OK;
 }
@@ -820,6 +862,40 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
 
 }  // namespace
 
+namespace {
+
+// Row scales, norms and level-0 couplings of the factor window, then its levels.
+template <typename C>
+int factor_window(kore_plan *p) {
+    const int lo = p->fw_lo, ns = p->fw_n;
+    const unsigned grid = kore_div_up(p->np, 256);
+    double *red = p->d_part;   // scratch: grid x ns doubles fit the residual partials buffer
+    k_rowinfo<C><<<grid, 256, 0, p->stream>>>(make_fv<C>(p), ns, red);
+    k_minf<<<ns, 256, 0, p->stream>>>(red, (int)grid, p->d_minf + lo);
+    KORE_LAUNCHED(2);
+    if (p->ell_stride() > 0) {
+        k_ell_fill<C><<<dim3(std::min<unsigned>(kore_div_up(p->ell_stride(), 256), 4096u), ns), 256, 0, p->stream>>>(
+            p->ell_stride(), p->ell_w, (p->S + 31) / 32, p->S, p->np, p->d_ell_src, p->d_aval,
+            p->d_rscale + (int64_t)lo * p->np, static_cast<C *>(p->d_ell_val) + (int64_t)lo * p->ell_stride());
+        KORE_LAUNCHED(1);
+    }
+    return factor_dispatch<C>(p);
+}
+
+// Factorises the factor window; the norms of its shifts come back with the one wait at the end.
+int run_window(kore_plan *p) {
+    if (p->prof) KORE_TRY(kore_prof_mark(p, 1, true));
+    KORE_TRY(p->prec == KORE_PREC_FP64 ? factor_window<double2>(p) : factor_window<float2>(p));
+    if (p->prof) KORE_TRY(kore_prof_mark(p, 1, false));
+    KORE_CUDA_TRY(cudaMemcpyAsync(p->minfs.data() + p->fw_lo, p->d_minf + p->fw_lo, p->fw_n * sizeof(double),
+                                  cudaMemcpyDeviceToHost, p->stream));
+    KORE_CUDA_TRY(cudaStreamSynchronize(p->stream));
+    p->minf = p->minfs[0];
+    return kore_check_device_error(p);
+}
+
+}  // namespace
+
 int kore_factor_impl(kore_plan *p, int nshift, const double *sigmas, int precision) {
     if (precision != KORE_PREC_FP64 && precision != KORE_PREC_MIXED) return KORE_EINVAL;
     if (nshift <= 0 || !sigmas) return KORE_EINVAL;
@@ -831,47 +907,13 @@ int kore_factor_impl(kore_plan *p, int nshift, const double *sigmas, int precisi
     p->fw_lo = 0;
     p->fw_n = nshift;
     p->sigmas.assign(nshift, mk(0.0, 0.0));
+    p->minfs.assign(nshift, 0.0);
     for (int s = 0; s < nshift; ++s) p->sigmas[s] = mk(sigmas[2 * s], sigmas[2 * s + 1]);
     p->sigma_re = sigmas[0];
     p->sigma_im = sigmas[1];
     KORE_CUDA_TRY(cudaMemcpyAsync(p->d_sigma, p->sigmas.data(), nshift * sizeof(double2), cudaMemcpyHostToDevice,
                                   p->stream));
-    const unsigned grid = std::min<unsigned>(kore_div_up(p->np, 256), 64u);
-    std::vector<double> red((size_t)grid * nshift);
-    double *d_red = p->d_part;   // scratch: grid x nshift doubles fit the residual partials buffer
-    if (p->prof) KORE_TRY(kore_prof_mark(p, 1, true));
-    int s;
-    if (precision == KORE_PREC_FP64) {
-        k_rowinfo<double2><<<dim3(grid, nshift), 256, 0, p->stream>>>(make_fv<double2>(p), d_red);
-        if (p->ell_stride() > 0)
-            k_ell_fill<double2><<<dim3(std::min<unsigned>(kore_div_up(p->ell_stride(), 256), 4096u), nshift), 256, 0,
-                              p->stream>>>(p->ell_stride(), p->ell_w, (p->S + 31) / 32, p->S, p->np, p->d_ell_src,
-                                           p->d_aval, p->d_rscale, static_cast<double2 *>(p->d_ell_val));
-        KORE_LAUNCHED(2);
-        KORE_CUDA_TRY(cudaMemcpyAsync(red.data(), d_red, red.size() * sizeof(double), cudaMemcpyDeviceToHost, p->stream));
-        KORE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-        s = factor_dispatch<double2>(p);
-    } else {
-        k_rowinfo<float2><<<dim3(grid, nshift), 256, 0, p->stream>>>(make_fv<float2>(p), d_red);
-        if (p->ell_stride() > 0)
-            k_ell_fill<float2><<<dim3(std::min<unsigned>(kore_div_up(p->ell_stride(), 256), 4096u), nshift), 256, 0,
-                              p->stream>>>(p->ell_stride(), p->ell_w, (p->S + 31) / 32, p->S, p->np, p->d_ell_src,
-                                           p->d_aval, p->d_rscale, static_cast<float2 *>(p->d_ell_val));
-        KORE_LAUNCHED(2);
-        KORE_CUDA_TRY(cudaMemcpyAsync(red.data(), d_red, red.size() * sizeof(double), cudaMemcpyDeviceToHost, p->stream));
-        KORE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-        s = factor_dispatch<float2>(p);
-    }
-    if (s != KORE_OK) return s;
-    if (p->prof) KORE_TRY(kore_prof_mark(p, 1, false));
-    p->minfs.assign(nshift, 0.0);
-    for (int sh = 0; sh < nshift; ++sh)
-        for (unsigned b = 0; b < grid; ++b) p->minfs[sh] = std::max(p->minfs[sh], red[(size_t)sh * grid + b]);
-    p->minf = p->minfs[0];
-    KORE_CUDA_TRY(cudaMemcpyAsync(p->d_minf, p->minfs.data(), nshift * sizeof(double), cudaMemcpyHostToDevice,
-                                  p->stream));
-    KORE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-    KORE_TRY(kore_check_device_error(p));
+    KORE_TRY(run_window(p));
     p->factored = true;
     return KORE_OK;
 }
@@ -889,44 +931,10 @@ int kore_factor_slot(kore_plan *p, int slot, double sigma_re, double sigma_im) {
                                   p->stream));
     p->fw_lo = slot;
     p->fw_n = 1;
-    const unsigned grid = std::min<unsigned>(kore_div_up(p->np, 256), 64u);
-    std::vector<double> red(grid);
-    double *d_red = p->d_part;
-    if (p->prof) KORE_TRY(kore_prof_mark(p, 1, true));
-    int s;
-    if (p->prec == KORE_PREC_FP64) {
-        k_rowinfo<double2><<<dim3(grid, 1), 256, 0, p->stream>>>(make_fv<double2>(p), d_red);
-        if (p->ell_stride() > 0)
-            k_ell_fill<double2><<<dim3(std::min<unsigned>(kore_div_up(p->ell_stride(), 256), 4096u), 1), 256, 0,
-                              p->stream>>>(p->ell_stride(), p->ell_w, (p->S + 31) / 32, p->S, p->np, p->d_ell_src,
-                                           p->d_aval, p->d_rscale + (int64_t)slot * p->np,
-                                           static_cast<double2 *>(p->d_ell_val) + (int64_t)slot * p->ell_stride());
-        KORE_LAUNCHED(2);
-        s = factor_dispatch<double2>(p);
-    } else {
-        k_rowinfo<float2><<<dim3(grid, 1), 256, 0, p->stream>>>(make_fv<float2>(p), d_red);
-        if (p->ell_stride() > 0)
-            k_ell_fill<float2><<<dim3(std::min<unsigned>(kore_div_up(p->ell_stride(), 256), 4096u), 1), 256, 0,
-                              p->stream>>>(p->ell_stride(), p->ell_w, (p->S + 31) / 32, p->S, p->np, p->d_ell_src,
-                                           p->d_aval, p->d_rscale + (int64_t)slot * p->np,
-                                           static_cast<float2 *>(p->d_ell_val) + (int64_t)slot * p->ell_stride());
-        KORE_LAUNCHED(2);
-        s = factor_dispatch<float2>(p);
-    }
+    const int s = run_window(p);
     p->fw_lo = 0;
     p->fw_n = p->nshift;
     if (s != KORE_OK) return s;
-    if (p->prof) KORE_TRY(kore_prof_mark(p, 1, false));
-    KORE_CUDA_TRY(cudaMemcpyAsync(red.data(), d_red, red.size() * sizeof(double), cudaMemcpyDeviceToHost, p->stream));
-    KORE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-    double mx = 0.0;
-    for (unsigned b = 0; b < grid; ++b) mx = std::max(mx, red[b]);
-    p->minfs[slot] = mx;
-    if (slot == 0) p->minf = mx;
-    KORE_CUDA_TRY(cudaMemcpyAsync(p->d_minf + slot, &p->minfs[slot], sizeof(double), cudaMemcpyHostToDevice,
-                                  p->stream));
-    KORE_CUDA_TRY(cudaStreamSynchronize(p->stream));
-    KORE_TRY(kore_check_device_error(p));
     p->factored = true;
     return KORE_OK;
 }
