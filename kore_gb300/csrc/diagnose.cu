@@ -12,28 +12,41 @@
 // The sums over l, the scaling by OmgTau Ek and the power-balance residuals
 // (bin/spin_doctor.py:148-160, 225-236) are left to the caller (kore_gb300/diagnostics.py).
 //
-// Layout: k_cheb_eval writes E[j][i][k] = d^j T_k / dr^j (x_i) for j = 0..3 (one thread
-// per point, three-term recurrences of T_k and its x-derivatives); k_flow_integrals
-// runs one CTA per (degree block, eigenvector), the block's coefficients in shared
-// memory, threads over the points, and reduces the three integrals in a fixed order.
+// Chebyshev polynomials and their derivatives are even or odd, d^j T_k(-x) =
+// (-1)^(k+j) d^j T_k(x), and the points are symmetric, so a pair of points x, -x takes one
+// pass over the coefficients: the sums over even and over odd k, added for x and subtracted
+// for -x.  That is half of the FP64 products, whose pipe (two multiply-adds per SM per clock)
+// bounds the kernel: 16 modes of the 240k-unknown shell took 19.2 ms with every point on its
+// own, of which 17 ms at the pipe's rate.
+// Layout: k_cheb_eval writes E[j][k][i] = d^j T_k / dr^j (x_i), j = 0..3, for the points
+// i < nh = ceil(N / 2) with x_i >= 0 (threads over points, three-term recurrences of T_k and
+// its x-derivatives), then x_i and the quadrature weights.  k_flow_integrals runs one CTA per
+// (degree block, kVec eigenvectors), the coefficients in shared memory, threads over the
+// point pairs, and reduces the three integrals in a fixed order.
 #include "kore_internal.cuh"
+#include <algorithm>
 #include <vector>
 
 namespace {
 
 constexpr int kDiagThreads = 256;
+constexpr int kVec = 2;   // eigenvectors per CTA: they share its reads of E (L2 traffic)
 
 __global__ void k_cheb_eval(int N, double ricb, double rcmb, double *__restrict__ E) {
+    const int nh = (N + 1) / 2;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
-    const double x = cos((i + 0.5) * 3.14159265358979323846 / N);
+    if (i >= nh) return;
+    // the middle point of an odd N is 0 (cos(pi / 2) rounds to 6e-17)
+    const double x = (2 * i + 1 == N) ? 0.0 : cos((i + 0.5) * 3.14159265358979323846 / N);
     const double dr = 2.0 / (rcmb - ricb);   // dx/dr
-    const int64_t NN = (int64_t)N * N;
+    const int64_t NN = (int64_t)N * nh;
+    E[4 * NN + i] = x;
+    E[4 * NN + nh + i] = sqrt(1.0 - x * x);
     // T_k and its first three x-derivatives: T_{k+1} = 2x T_k - T_{k-1} differentiated
     double t0 = 1.0, t1 = x;            // T_{k-1}, T_k
-    double d10 = 0.0, d11 = 1.0;        // T'
-    double d20 = 0.0, d21 = 0.0;        // T''
-    double d30 = 0.0, d31 = 0.0;        // T'''
+    double d10 = 0.0, d11 = 1.0;        // first derivative
+    double d20 = 0.0, d21 = 0.0;        // second
+    double d30 = 0.0, d31 = 0.0;        // third
     for (int k = 0; k < N; ++k) {
         double v0, v1, v2, v3;
         if (k == 0) { v0 = 1.0; v1 = 0.0; v2 = 0.0; v3 = 0.0; }
@@ -46,93 +59,140 @@ __global__ void k_cheb_eval(int N, double ricb, double rcmb, double *__restrict_
             t0 = t1; t1 = n0; d10 = d11; d11 = n1; d20 = d21; d21 = n2; d30 = d31; d31 = n3;
             v0 = n0; v1 = n1; v2 = n2; v3 = n3;
         }
-        E[(int64_t)i * N + k] = v0;
-        E[NN + (int64_t)i * N + k] = v1 * dr;
-        E[2 * NN + (int64_t)i * N + k] = v2 * dr * dr;
-        E[3 * NN + (int64_t)i * N + k] = v3 * dr * dr * dr;
+        const int64_t at = (int64_t)k * nh + i;
+        E[at] = v0;
+        E[NN + at] = v1 * dr;
+        E[2 * NN + at] = v2 * dr * dr;
+        E[3 * NN + at] = v3 * dr * dr * dr;
     }
 }
 
 struct FlowArgs {
-    int N, npol, ntor;
+    int N, npol, ntor, nvec;
     double ricb, rcmb;
     const int *lpol, *ltor;      // degrees of the poloidal and toroidal blocks
     const double2 *x;            // nvec vectors of (npol + ntor) N complex coefficients
-    const double *E;             // 4 N N evaluation matrices
+    const double *E;             // evaluation matrices, points and weights (k_cheb_eval)
     double *out;                 // per (vector, block): energy, diffusion, internal dissipation
 };
 
+// Integrands (energy, diffusion, internal dissipation) at radius rk from the radial
+// function and its derivatives p.
+__device__ __forceinline__ void flow_integrands(bool tor, int l, double rk, const double2 (&p)[4], double (&f)[3]) {
+    const double L = (double)l * (l + 1), f0 = 4.0 * 3.14159265358979323846 / (2 * l + 1);
+    const double r2 = rk * rk;
+    if (!tor) {
+        const double ri = 1.0 / rk, li = 1.0 / L;
+        const double2 q0 = (L / rk) * p[0];
+        const double2 s0 = p[1] + ri * p[0];
+        const double2 q1 = ri * (L * p[1] - q0);
+        const double2 s1 = p[2] + li * q1;
+        const double2 q2 = ri * (L * p[2] - 2.0 * q1);
+        const double2 s2 = p[3] + li * q2;
+        f[0] = f0 * (r2 * abs2(q0) + r2 * L * abs2(s0));
+        const double2 t = L * r2 * (conjg(s0) * s2) + (2.0 * rk * L) * (conjg(s0) * s1) +
+                          (-(L * L)) * (conjg(s0) * s0) + (-((double)l * l + l + 2)) * (conjg(q0) * q0) +
+                          (2.0 * rk) * (conjg(q0) * q1) + r2 * (conjg(q0) * q2) +
+                          (2.0 * L) * (conjg(q0) * s0 + q0 * conjg(s0));
+        f[1] = 2.0 * f0 * t.x;
+        const double2 u = q0 + rk * s1 - s0;
+        f[2] = 2.0 * f0 * (L * abs2(u) + 3.0 * abs2(rk * q1) + L * (l - 1) * (l + 2) * abs2(s0));
+    } else {
+        const double2 t0 = p[0], t1 = p[1], t2 = p[2];
+        f[0] = f0 * r2 * L * abs2(t0);
+        const double2 t = L * r2 * (conjg(t0) * t2) + (2.0 * rk * L) * (conjg(t0) * t1) + (-(L * L)) * (conjg(t0) * t0);
+        f[1] = 2.0 * f0 * t.x;
+        f[2] = 2.0 * f0 * (L * abs2(rk * t1 - t0) + L * (l - 1) * (l + 2) * abs2(t0));
+    }
+}
+
+// Sums over even (e) and odd (o) k of E_j[k][i] c_k for ND derivatives and kVec vectors.
+template <int ND>
+__device__ __forceinline__ void parity_sums(const double *__restrict__ E, int64_t NN, int nh, int N, int i,
+                                            const double2 *cs, double2 (&e)[kVec][4], double2 (&o)[kVec][4]) {
+    for (int k = 0; k < N; k += 2) {
+        const bool odd = k + 1 < N;
+        double ev[ND], ov[ND];
+#pragma unroll
+        for (int j = 0; j < ND; ++j) {
+            ev[j] = __ldg(E + j * NN + (int64_t)k * nh + i);
+            ov[j] = odd ? __ldg(E + j * NN + (int64_t)(k + 1) * nh + i) : 0.0;
+        }
+#pragma unroll
+        for (int v = 0; v < kVec; ++v) {
+            const double2 c0 = cs[v * (N + 1) + k], c1 = cs[v * (N + 1) + k + 1];   // entry N is zero
+#pragma unroll
+            for (int j = 0; j < ND; ++j) {
+                e[v][j].x = fma(ev[j], c0.x, e[v][j].x);
+                e[v][j].y = fma(ev[j], c0.y, e[v][j].y);
+                o[v][j].x = fma(ov[j], c1.x, o[v][j].x);
+                o[v][j].y = fma(ov[j], c1.y, o[v][j].y);
+            }
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kDiagThreads) k_flow_integrals(FlowArgs a) {
-    extern __shared__ double2 cs[];   // the block's N coefficients
-    __shared__ double red[3][kDiagThreads / 32];
-    const int b = blockIdx.x, v = blockIdx.y, N = a.N;
+    extern __shared__ double2 cs[];   // kVec x (N + 1) coefficients
+    __shared__ double red[kVec][3][kDiagThreads / 32];
+    const int b = blockIdx.x, v0 = blockIdx.y * kVec, N = a.N, nh = (N + 1) / 2;
     const int nblk = a.npol + a.ntor;
     const bool tor = b >= a.npol;
     const int l = tor ? a.ltor[b - a.npol] : a.lpol[b];
-    const double2 *c = a.x + ((int64_t)v * nblk + b) * N;
-    for (int k = threadIdx.x; k < N; k += blockDim.x) cs[k] = c[k];
+    for (int v = 0; v < kVec; ++v) {
+        const double2 *c = a.x + ((int64_t)(v0 + v) * nblk + b) * N;
+        for (int k = threadIdx.x; k <= N; k += blockDim.x)
+            cs[v * (N + 1) + k] = (k < N && v0 + v < a.nvec) ? c[k] : mk(0.0, 0.0);
+    }
     __syncthreads();
-    const int64_t NN = (int64_t)N * N;
-    const double L = (double)l * (l + 1), f0 = 4.0 * 3.14159265358979323846 / (2 * l + 1);
-    double ke = 0.0, dk = 0.0, di = 0.0;
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-        const double xk = cos((i + 0.5) * 3.14159265358979323846 / N);
-        const double rk = 0.5 * (a.rcmb - a.ricb) * (xk + 1.0) + a.ricb;
-        const double w = sqrt(1.0 - xk * xk);
-        const int nd = tor ? 3 : 4;
-        double2 p[4] = {mk(0, 0), mk(0, 0), mk(0, 0), mk(0, 0)};
-        for (int j = 0; j < nd; ++j) {
-            const double *e = a.E + j * NN + (int64_t)i * N;
-            double2 acc = mk(0.0, 0.0);
-            for (int k = 0; k < N; ++k) {
-                const double ev = __ldg(e + k);
-                acc.x = fma(ev, cs[k].x, acc.x);
-                acc.y = fma(ev, cs[k].y, acc.y);
+    const int64_t NN = (int64_t)N * nh;
+    double sum[kVec][3];
+#pragma unroll
+    for (int v = 0; v < kVec; ++v) sum[v][0] = sum[v][1] = sum[v][2] = 0.0;
+    for (int i = threadIdx.x; i < nh; i += blockDim.x) {
+        double2 e[kVec][4], o[kVec][4];
+#pragma unroll
+        for (int v = 0; v < kVec; ++v)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) e[v][j] = o[v][j] = mk(0.0, 0.0);
+        if (tor) parity_sums<3>(a.E, NN, nh, N, i, cs, e, o);
+        else parity_sums<4>(a.E, NN, nh, N, i, cs, e, o);
+        const double x = a.E[4 * NN + i], w = a.E[4 * NN + nh + i];
+        const int npt = (2 * i + 1 == N) ? 1 : 2;   // the middle point of an odd N is its own mirror
+        for (int m = 0; m < npt; ++m) {
+            const double xk = m ? -x : x;
+            const double rk = 0.5 * (a.rcmb - a.ricb) * (xk + 1.0) + a.ricb;
+#pragma unroll
+            for (int v = 0; v < kVec; ++v) {
+                double2 p[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    p[j] = m ? e[v][j] - o[v][j] : e[v][j] + o[v][j];
+                    if (m && (j & 1)) p[j] = -p[j];
+                }
+                double f[3];
+                flow_integrands(tor, l, rk, p, f);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) sum[v][q] += w * f[q];
             }
-            p[j] = acc;
         }
-        const double r2 = rk * rk;
-        double fke, fdk, fdi;
-        if (!tor) {
-            const double2 q0 = (L / rk) * p[0];
-            const double2 s0 = p[1] + (1.0 / rk) * p[0];
-            const double2 q1 = (1.0 / rk) * (L * p[1] - q0);
-            const double2 s1 = p[2] + (1.0 / L) * q1;
-            const double2 q2 = (1.0 / rk) * (L * p[2] - 2.0 * q1);
-            const double2 s2 = p[3] + (1.0 / L) * q2;
-            fke = f0 * (r2 * abs2(q0) + r2 * L * abs2(s0));
-            const double2 t = L * r2 * (conjg(s0) * s2) + (2.0 * rk * L) * (conjg(s0) * s1) +
-                              (-(L * L)) * (conjg(s0) * s0) + (-((double)l * l + l + 2)) * (conjg(q0) * q0) +
-                              (2.0 * rk) * (conjg(q0) * q1) + r2 * (conjg(q0) * q2) +
-                              (2.0 * L) * (conjg(q0) * s0 + q0 * conjg(s0));
-            fdk = 2.0 * f0 * t.x;
-            const double2 u = q0 + rk * s1 - s0;
-            fdi = 2.0 * f0 * (L * abs2(u) + 3.0 * abs2(rk * q1) + L * (l - 1) * (l + 2) * abs2(s0));
-        } else {
-            const double2 t0 = p[0], t1 = p[1], t2 = p[2];
-            fke = f0 * r2 * L * abs2(t0);
-            const double2 t = L * r2 * (conjg(t0) * t2) + (2.0 * rk * L) * (conjg(t0) * t1) + (-(L * L)) * (conjg(t0) * t0);
-            fdk = 2.0 * f0 * t.x;
-            fdi = 2.0 * f0 * (L * abs2(rk * t1 - t0) + L * (l - 1) * (l + 2) * abs2(t0));
+    }
+#pragma unroll
+    for (int v = 0; v < kVec; ++v)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const double t = warp_sum_d(sum[v][q]);
+            if ((threadIdx.x & 31) == 0) red[v][q][threadIdx.x >> 5] = t;
         }
-        ke += w * fke;
-        dk += w * fdk;
-        di += w * fdi;
-    }
-    ke = warp_sum_d(ke);
-    dk = warp_sum_d(dk);
-    di = warp_sum_d(di);
-    if ((threadIdx.x & 31) == 0) {
-        red[0][threadIdx.x >> 5] = ke;
-        red[1][threadIdx.x >> 5] = dk;
-        red[2][threadIdx.x >> 5] = di;
-    }
     __syncthreads();
-    if (threadIdx.x < 3) {
-        double s = 0.0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += red[threadIdx.x][q];
-        const double quad = (3.14159265358979323846 / N) * (a.rcmb - a.ricb) / 2.0;
-        a.out[((int64_t)v * nblk + b) * 3 + threadIdx.x] = quad * s;
+    if (threadIdx.x < 3 * kVec) {
+        const int v = threadIdx.x / 3, q = threadIdx.x - 3 * v;
+        if (v0 + v < a.nvec) {
+            double s = 0.0;
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[v][q][w];
+            const double quad = (3.14159265358979323846 / N) * (a.rcmb - a.ricb) / 2.0;
+            a.out[((int64_t)(v0 + v) * nblk + b) * 3 + q] = quad * s;
+        }
     }
 }
 
@@ -158,7 +218,8 @@ extern "C" int kore_flow_diagnostics(int device, int N, double ricb, int npol, c
     auto ck = [&](cudaError_t e) {
         if (e != cudaSuccess && rc == KORE_OK) rc = (e == cudaErrorMemoryAllocation) ? KORE_ENOMEM : KORE_ECUDA;
     };
-    ck(cudaMalloc(&dE, (size_t)4 * N * N * sizeof(double)));
+    const int nh = (N + 1) / 2;
+    ck(cudaMalloc(&dE, ((size_t)4 * N * nh + 2 * nh) * sizeof(double)));
     ck(cudaMalloc(&dx, xbytes));
     ck(cudaMalloc(&dout, obytes));
     ck(cudaMalloc(&dl, (size_t)nblk * sizeof(int)));
@@ -167,9 +228,12 @@ extern "C" int kore_flow_diagnostics(int device, int N, double ricb, int npol, c
         ls.insert(ls.end(), ltor, ltor + ntor);
         ck(cudaMemcpy(dl, ls.data(), ls.size() * sizeof(int), cudaMemcpyHostToDevice));
         ck(cudaMemcpy(dx, x, xbytes, cudaMemcpyHostToDevice));
-        k_cheb_eval<<<kore_div_up(N, 128), 128>>>(N, ricb, 1.0, dE);
-        FlowArgs a{N, npol, ntor, ricb, 1.0, dl, dl + npol, dx, dE, dout};
-        k_flow_integrals<<<dim3(nblk, nvec), kDiagThreads, N * sizeof(double2)>>>(a);
+        k_cheb_eval<<<kore_div_up(nh, 32), 32>>>(N, ricb, 1.0, dE);
+        FlowArgs a{N, npol, ntor, nvec, ricb, 1.0, dl, dl + npol, dx, dE, dout};
+        const size_t smem = (size_t)kVec * (N + 1) * sizeof(double2);
+        if (rc == KORE_OK) rc = kore_allow_max_dyn_smem(k_flow_integrals, device);
+        const int threads = std::min(kDiagThreads, (nh + 31) / 32 * 32);
+        k_flow_integrals<<<dim3(nblk, kore_div_up(nvec, kVec)), threads, smem>>>(a);
         KORE_LAUNCHED(2);
         ck(cudaGetLastError());
         ck(cudaMemcpy(out, dout, obytes, cudaMemcpyDeviceToHost));
