@@ -60,7 +60,7 @@ struct FV {
     const C *ell_val;
     int ell_w;
     int64_t ell_stride;
-    int64_t f_stride, lu_stride, t_stride, p_stride;
+    int64_t f_stride, lu_stride, t_stride, t_block, p_stride;
 };
 
 // View of the plan's factor storage starting at the factor window's first shift (shift
@@ -82,7 +82,7 @@ FV<C> make_fv(kore_plan *p) {
     v.ell_col = p->d_ell_col; v.ell_val = static_cast<const C *>(p->d_ell_val) + lo * p->ell_stride();
     v.ell_w = p->ell_w;
     v.ell_stride = p->ell_stride();
-    v.f_stride = p->f_stride(); v.lu_stride = p->lu_stride(); v.t_stride = p->t_stride(); v.p_stride = p->p_stride();
+    v.f_stride = p->f_stride(); v.lu_stride = p->lu_stride(); v.t_stride = p->t_stride(); v.t_block = p->t_block(sizeof(C)); v.p_stride = p->p_stride();
     return v;
 }
 
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0, int stride) {
     __shared__ int s_piv[NB];
     const int S = v.S;
     const int64_t o = blockIdx.x, sh = blockIdx.y;
-    C *T = v.T + sh * v.t_stride + o * 2 * (int64_t)S * S + (int64_t)k0 * S;
+    C *T = v.T + sh * v.t_stride + o * v.t_block + (int64_t)k0 * S;
     const C *src = k0 == 0 ? diag_block(v, o, sh, stride) : T;
     int *piv = v.piv + sh * v.p_stride + o * S, *pidx = v.pidx + sh * v.p_stride + o * S;
     int *used = v.used + sh * v.p_stride + o * S;
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb, int str
     __shared__ __align__(16) C es[NB][kUpdRows];
     const int S = v.S;
     const int64_t o = blockIdx.y, sh = blockIdx.z;
-    C *T = v.T + sh * v.t_stride + o * 2 * (int64_t)S * S;
+    C *T = v.T + sh * v.t_stride + o * v.t_block;
     const C *src = k0 == 0 ? diag_block(v, o, sh, stride) : T;
     const int *piv = v.piv + sh * v.p_stride + o * S, *pidx = v.pidx + sh * v.p_stride + o * S;
     // columns of this CTA, counted without the panel's own
@@ -415,7 +415,7 @@ __global__ void k_extract(FV<C> v, BcrLevel lv, int nodd, int top, int nshift) {
         const int64_t o = ws / SS;
         const int64_t w = ws - o * SS;
         const int c = (int)(w / S), k = (int)(w - (int64_t)c * S);
-        const C *T = v.T + sh * v.t_stride + o * 2 * SS;
+        const C *T = v.T + sh * v.t_stride + o * v.t_block;
         const int *piv = v.piv + sh * v.p_stride + o * S;
         const int64_t j = top ? 0 : (2 * o + 1) * lv.stride;
         v.Dinv[sh * v.f_stride + j * SS + k + (int64_t)piv[c] * S] = T[piv[k] + (int64_t)c * S];
@@ -503,125 +503,6 @@ __global__ void __launch_bounds__(512) k_even_l0(FV<C> v, BcrLevel lv) {
                 if (outr) LU[(lv.lu_nU + e) * SS + r + col] = -usum[t];
             }
     }
-}
-
-// One 64 x 64 tile (blockIdx.x, blockIdx.y) of Cm = [Cm] +- (A1 B1 + A2 B2) for
-// column-major S x S complex operands (A2 may be null), 4 x 4 outputs per thread,
-// FP64/FP32 CUDA cores.
-constexpr int kGT = 64, kGK = 16;
-template <typename C>
-__device__ __forceinline__ void gemm_tile(const C *A1, const C *B1, const C *A2, const C *B2, C *Cm, int S,
-                                          bool accumulate, bool negate) {
-    __shared__ C As[kGK][kGT + 1];
-    __shared__ C Bs[kGK][kGT + 1];
-    const int m0 = blockIdx.x * kGT, n0 = blockIdx.y * kGT;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 x 16 threads
-    C acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = czero<C>();
-    for (int pass = 0; pass < 2; ++pass) {
-        const C *A = pass ? A2 : A1;
-        const C *B = pass ? B2 : B1;
-        if (!A) continue;
-        for (int k0 = 0; k0 < S; k0 += kGK) {
-            for (int idx = threadIdx.x; idx < kGK * kGT; idx += blockDim.x) {
-                const int kk = idx / kGT, mm = idx - kk * kGT;
-                const int gm = m0 + mm, gk = k0 + kk;
-                As[kk][mm] = (gm < S && gk < S) ? A[gm + (int64_t)gk * S] : czero<C>();
-                const int nn = idx / kGK, kb = idx - nn * kGK;
-                const int gn = n0 + nn, gk2 = k0 + kb;
-                Bs[kb][nn] = (gn < S && gk2 < S) ? B[gk2 + (int64_t)gn * S] : czero<C>();
-            }
-            __syncthreads();
-#pragma unroll
-            for (int kk = 0; kk < kGK; ++kk) {
-                C av[4], bv[4];
-#pragma unroll
-                for (int a = 0; a < 4; ++a) av[a] = As[kk][tx + 16 * a];
-#pragma unroll
-                for (int b = 0; b < 4; ++b) bv[b] = Bs[kk][ty + 16 * b];
-#pragma unroll
-                for (int a = 0; a < 4; ++a)
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) acc[a][b] = cfma(acc[a][b], av[a], bv[b]);
-            }
-            __syncthreads();
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int gm = m0 + tx + 16 * a, gn = n0 + ty + 16 * b;
-            if (gm < S && gn < S) {
-                const int64_t idx = gm + (int64_t)gn * S;
-                const C d = negate ? -acc[a][b] : acc[a][b];
-                Cm[idx] = accumulate ? Cm[idx] + d : d;
-            }
-        }
-}
-
-// Batched dense update of the even blocks at levels >= 1 (complex128; the complex64
-// factorisation runs it on the tensor cores, gemm_tc.cu), one GEMM job per
-// (shift, even block, kind): kind 0: Dw_i -= L_q H_jl + U_q G_jr;  kind 1: L' = -L_q G_jl;
-// kind 2: U' = -U_q H_jr.
-template <typename C>
-__global__ void __launch_bounds__(256) k_even_gemm(FV<C> v, BcrLevel lv, int job0) {
-    const int S = v.S;
-    const int64_t SS = (int64_t)S * S;
-    const int job = job0 + blockIdx.z;
-    const int per = 3 * lv.neven;
-    const int64_t sh = job / per;
-    const int jj = job - (int)sh * per;
-    const int64_t e = jj / 3;
-    const int kind = jj - 3 * (int)e;
-    const int64_t q = 2 * e;
-    const bool hasl = q >= 1, hasr = q + 1 < lv.Kl;
-    const C *A1 = nullptr, *B1 = nullptr, *A2 = nullptr, *B2 = nullptr;
-    C *Cm = nullptr;
-    bool accumulate = false;
-    C *LU = v.LU + sh * v.lu_stride;
-    const C *G = v.G + sh * v.f_stride, *H = v.H + sh * v.f_stride;
-    const C *Lq = LU + (lv.lu_L + q) * SS, *Uq = LU + (lv.lu_U + q) * SS;
-    const int64_t jl = (q - 1) * lv.stride, jr = (q + 1) * lv.stride;
-    if (kind == 0) {
-        Cm = v.Dw + sh * v.f_stride + q * lv.stride * SS;
-        accumulate = true;
-        if (hasl) { A1 = Lq; B1 = H + jl * SS; }
-        if (hasr) { A2 = Uq; B2 = G + jr * SS; }
-    } else if (kind == 1) {
-        if (lv.lu_nL < 0 || q < 2) return;
-        Cm = LU + (lv.lu_nL + e) * SS;
-        A1 = Lq; B1 = G + jl * SS;
-    } else {
-        if (lv.lu_nU < 0 || q + 2 >= lv.Kl) return;
-        Cm = LU + (lv.lu_nU + e) * SS;
-        A1 = Uq; B1 = H + jr * SS;
-    }
-    if (!A1) { A1 = A2; B1 = B2; A2 = nullptr; B2 = nullptr; }
-    if (!A1) return;
-    gemm_tile<C>(A1, B1, A2, B2, Cm, S, accumulate, true);
-}
-
-// G_j = D_j^-1 L_q and H_j = D_j^-1 U_q of the odd blocks of a level >= 1 (complex128;
-// complex64 on the tensor cores), one job per (shift, odd block, G or H).
-template <typename C>
-__global__ void __launch_bounds__(256) k_gh_gemm(FV<C> v, BcrLevel lv, int job0) {
-    const int S = v.S;
-    const int64_t SS = (int64_t)S * S;
-    const int job = job0 + blockIdx.z;
-    const int64_t sh = job / (2 * lv.nodd);
-    const int jj = job - (int)sh * 2 * lv.nodd;
-    const int64_t o = jj / 2;
-    const int which = jj - 2 * (int)o;
-    const int64_t q = 2 * o + 1, j = q * lv.stride;
-    if (which == 1 && q + 1 >= lv.Kl) return;   // no right neighbour: H_j is never read
-    const C *Di = v.Dinv + sh * v.f_stride + j * SS;
-    const C *Bm = v.LU + sh * v.lu_stride + ((which ? lv.lu_U : lv.lu_L) + q) * SS;
-    C *Cm = (which ? v.H : v.G) + sh * v.f_stride + j * SS;
-    gemm_tile<C>(Di, Bm, nullptr, nullptr, Cm, S, false, false);
 }
 
 // Level 0: G_j = D_j^-1 (R L_j) and H_j = D_j^-1 (R U_j) from the couplings by column:
@@ -734,18 +615,9 @@ int factor_levels(kore_plan *p) {
             KORE_TRY(kore_gh_update_tc(p, lv, 0));
             KORE_TRY(kore_even_update_tc(p, lv));
         } else {
-            // complex128: FP64 CUDA cores
-            const dim3 tg(kore_div_up(S, kGT), kore_div_up(S, kGT));
-            const int gjobs = 2 * lv.nodd * ns;
-            for (int j0 = 0; j0 < gjobs; j0 += 65535) {
-                k_gh_gemm<C><<<dim3(tg.x, tg.y, std::min(65535, gjobs - j0)), 256, 0, st>>>(v, lv, j0);
-                KORE_LAUNCHED(1);
-            }
-            const int jobs = 3 * lv.neven * ns;
-            for (int j0 = 0; j0 < jobs; j0 += 65535) {
-                k_even_gemm<C><<<dim3(tg.x, tg.y, std::min(65535, jobs - j0)), 256, 0, st>>>(v, lv, j0);
-                KORE_LAUNCHED(1);
-            }
+            // complex128: tensor cores (digits)
+            KORE_TRY(kore_gh_update_oz(p, lv));
+            KORE_TRY(kore_even_update_oz(p, lv));
         }
         KORE_CUDA_TRY(cudaGetLastError());
     }
@@ -812,7 +684,7 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
                      (void **)&p->d_rscale, (void **)&p->d_piv, (void **)&p->d_pidx, (void **)&p->d_used,
                      (void **)&p->d_sigma, (void **)&p->d_minf, (void **)&p->d_bb, (void **)&p->d_xb, (void **)&p->d_rb,
                      (void **)&p->d_bn, (void **)&p->d_rn, (void **)&p->d_part, (void **)&p->d_ir,
-                     (void **)&p->d_cnt, &p->d_ell_val, &p->d_tctab};
+                     (void **)&p->d_cnt, &p->d_ell_val, &p->d_tctab, &p->d_oz};
     for (void **b : bufs) {
         if (*b) cudaFree(*b);
         *b = nullptr;
@@ -821,6 +693,7 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
     p->factor_bytes = 0;
     p->factor_elt = 0;
     p->shift_cap = 0;
+    p->oz_bytes = 0;
     const size_t before = p->bytes;
     const size_t c = (size_t)cap;
     KORE_TRY(kore_alloc(p, &p->d_Dinv, c * p->f_stride() * elt));
@@ -828,7 +701,7 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
     KORE_TRY(kore_alloc(p, &p->d_Hm, c * p->f_stride() * elt));
     KORE_TRY(kore_alloc(p, &p->d_Dw, c * p->f_stride() * elt));
     KORE_TRY(kore_alloc(p, &p->d_LU, c * p->lu_stride() * elt));
-    KORE_TRY(kore_alloc(p, &p->d_T, c * p->t_stride() * elt));
+    KORE_TRY(kore_alloc(p, &p->d_T, c * p->nodd_max * p->t_block(elt) * elt));
     KORE_TRY(kore_alloc(p, &p->d_zlo, c * p->np * elt));
     KORE_TRY(kore_alloc(p, &p->d_xlo, c * p->np * elt));
     KORE_TRY(kore_alloc(p, &p->d_flo, c * p->np * elt));
@@ -849,6 +722,11 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
     KORE_TRY(kore_alloc(p, (void **)&p->d_cnt, c * (size_t)p->sweep_stages() * p->K * sizeof(int)));
     KORE_TRY(kore_alloc(p, &p->d_ell_val, c * std::max<int64_t>(p->ell_stride(), 1) * elt));
     if (elt == sizeof(float2)) KORE_TRY(kore_alloc(p, &p->d_tctab, (size_t)kore_tc_table_bytes(p, cap)));
+    else {
+        const int64_t oz = kore_oz_workspace_bytes(p->S, p->K, cap);
+        KORE_TRY(kore_alloc(p, &p->d_oz, (size_t)oz));
+        p->oz_bytes = oz;
+    }
     KORE_CUDA_TRY(cudaMemset(p->d_LU, 0, c * p->lu_stride() * elt));
     KORE_CUDA_TRY(cudaMemset(p->d_piv, 0, c * p->p_stride() * sizeof(int)));
     KORE_CUDA_TRY(cudaMemset(p->d_pidx, 0xff, c * p->p_stride() * sizeof(int)));

@@ -1,0 +1,656 @@
+// Complex128 GEMMs of the FP64 factorisation on the 5th-generation tensor cores, by
+// splitting into integer digits (the error-free transformation of Ozaki, Ogita, Oishi and
+// Rump, Numer. Algorithms 59, 2012): GB300's FP64 pipe does two multiply-adds per SM and
+// clock, its FP16 tensor cores about four thousand.
+//
+// Scaling.  C = A B with inner index k: row k of B is divided by 2^rho_k, its largest
+// exponent (taken over the two matrices, G and H or L and U, that meet the same A), column
+// k of A is multiplied by it, then every row i of A and column j of B by its own power of
+// two, so that all entries lie in (-1, 1).  The powers are exact; rho keeps an unknown of
+// another magnitude from losing its digits (the columns of L grow as the fourth power of
+// the radial order, the rows of G fall as fast).
+//
+// Digits.  An entry is rounded to 63 bits and written as nine digits in [-64, 64] of base
+// 128, exact in FP16:  x = sum_i x_i 128^-(i+1).  The product keeps the 45 digit pairs with
+// i + i' = d <= 8:  sum_d 128^-(d+2) (sum over pairs and k of x_i y_i').  Each inner sum is
+// a sum of at most 9 K products of at most 2^12, hence an integer below 2^24 for K <= 448,
+// and exact in the MMA's FP32 accumulators; longer inner dimensions are cut into pieces of
+// 448.  The nine sums are put together as integers and rounded to FP64 once.  What is lost
+// is below K 2^-60 of (largest entry of A's row) x (largest of B's column): in solves with
+// these factors the error against 64 bits is that of FP64 products or smaller.
+//
+// Data flow.  k_oz_rho finds rho; k_oz_split_a and k_oz_split_b write the digit planes in
+// the order the MMA reads them (8 x 16-byte core matrices, K-major, no swizzle), nine slices
+// of a 16-wide step of K one after another, so a step is one contiguous bulk copy.
+// k_oz_gemm computes a 128 x 64 tile: the tensor memory holds the accumulators of three
+// values of d (Re and Im: 384 columns), so the tile takes three passes over K, d = 8-6 with
+// nine slices, 5-3 with six, 2-0 with three; one thread issues tcgen05.mma (kind::f16), one
+// the bulk copies into a two-stage ring (108 KB per stage), and sixteen warps move the
+// sums into 64-bit integers between the passes.
+// What bounds it: shared-memory bandwidth (an MMA of 128 x 64 x 16 reads 6 KB), about 48
+// cycles per MMA, 180 MMAs per step of K.
+#include "kore_internal.cuh"
+#include "kore_tma.cuh"
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+namespace {
+
+constexpr int kOzSlices = 9, kOzBits = 7;
+constexpr int kOzM = 128, kOzN = 64, kOzK = 16;
+constexpr int kOzMaxSteps = 28;                    // steps of K whose sums stay below 2^24
+constexpr int kOzSliceA = 2 * kOzM * kOzK * 2;     // bytes of one slice of a step: Re, Im
+constexpr int kOzSliceB = 2 * kOzN * kOzK * 2;
+constexpr int kOzStepA = kOzSlices * kOzSliceA, kOzStepB = kOzSlices * kOzSliceB;
+constexpr int kOzStages = 2;
+constexpr int kOzStage = kOzStepA + kOzStepB;      // 108 KB
+constexpr int kOzEpiWarps = 16;
+constexpr int kOzThreads = 32 * (kOzEpiWarps + 2); // + the copying and the MMA warp
+constexpr size_t kOzSmem = (size_t)kOzStages * kOzStage + 128 + 128;
+constexpr int kOzNone = -100000;                   // exponent of an all-zero row
+constexpr int kOzBad = 100000;                     // exponent of a row with an infinity or NaN
+
+static_assert((int64_t)kOzSlices * kOzMaxSteps * kOzK * 4096 <= (1 << 24), "exact FP32 sums");
+
+int oz_mt(int S) { return (S + kOzM - 1) / kOzM; }
+int oz_nt(int S) { return (S + kOzN - 1) / kOzN; }
+__host__ __device__ inline int oz_steps(int S) { return (S + kOzK - 1) / kOzK; }
+int64_t oz_bytes_a(int S) { return (int64_t)oz_mt(S) * oz_steps(S) * kOzStepA; }
+int64_t oz_bytes_b(int S) { return (int64_t)oz_nt(S) * oz_steps(S) * kOzStepB; }
+
+// The scaling of an inner dimension: rows of X0 and X1 (X1 may be null).
+struct OzPair {
+    const double2 *X0, *X1;
+};
+// A matrix to split, and the pair whose rho scales it.
+struct OzOperand {
+    const double2 *X;
+    int pair;
+};
+// C = beta C + alpha (A1 B1 [+ A2 B2]): indices of split operands (a2 < 0: one product).
+struct OzJob {
+    int a1, b1, a2, b2;
+    double2 *C;
+    int negate, beta;
+};
+
+// exponent e with |v| < 2^e of a finite nonzero double, from its bits (subnormals count as zero)
+__device__ __forceinline__ int exp_of(double2 v) {
+    const int a = (__double2hiint(v.x) >> 20) & 0x7ff, b = (__double2hiint(v.y) >> 20) & 0x7ff;
+    const int m = max(a, b);
+    return m == 0x7ff ? kOzBad : m == 0 ? kOzNone : m - 1022;
+}
+
+// rho[pair][k] = largest exponent in row k of the pair's matrices.  CTA = 32 rows, warps
+// over the columns.
+__global__ void __launch_bounds__(256) k_oz_rho(const OzPair *__restrict__ pairs, int S, int *__restrict__ rho) {
+    __shared__ int sm[8][32];
+    const OzPair p = pairs[blockIdx.y];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = blockIdx.x * 32 + lane;
+    int e = kOzNone;
+    if (r < S)
+        for (int c = w; c < S; c += 8) {
+            e = max(e, exp_of(p.X0[r + (int64_t)c * S]));
+            if (p.X1) e = max(e, exp_of(p.X1[r + (int64_t)c * S]));
+        }
+    sm[w][lane] = e;
+    __syncthreads();
+    if (w == 0 && r < S) {
+#pragma unroll
+        for (int q = 1; q < 8; ++q) e = max(e, sm[q][lane]);
+        // a row without finite nonzero entries is left unscaled
+        rho[(int64_t)blockIdx.y * S + r] = (e == kOzNone || e == kOzBad) ? 0 : e;
+    }
+}
+
+// v 2^(62 - e) rounded to an integer (|v| < 2^e)
+__device__ __forceinline__ long long fixed63(double v, int e) {
+    const long long b = __double_as_longlong(v);
+    const int ex = (int)(b >> 52) & 0x7ff;
+    if (ex == 0 || ex == 0x7ff) return 0;
+    const long long m = (b & 0xfffffffffffffll) | (1ll << 52);
+    const int sh = ex - 1075 + 62 - e;
+    long long x;
+    if (sh >= 0) x = sh < 10 ? m << sh : 0;   // sh <= 9 by |v| < 2^e
+    else x = sh > -55 ? (m + (1ll << (-sh - 1))) >> -sh : 0;
+    return b < 0 ? -x : x;
+}
+
+// The nine digits of eight fixed-point numbers x, packed as the eight FP16 values (16 bytes)
+// of each slice.
+__device__ __forceinline__ void put_digits(long long (&x)[8], unsigned char *out, int64_t stride) {
+#pragma unroll
+    for (int s = kOzSlices - 1; s >= 0; --s) {
+        uint32_t h[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            int d;
+            if (s > 0) {
+                d = (((int)x[u] + 64) & 127) - 64;
+                x[u] = (x[u] - d) >> kOzBits;
+            } else d = (int)x[u];
+            h[u] = (uint32_t)(0x6600 + d);   // FP16 bits of 1536 + d
+        }
+        uint4 v;
+        uint32_t *p = &v.x;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t w = h[2 * u] | (h[2 * u + 1] << 16);
+            uint32_t r;
+            asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(w), "r"(0x66006600u));   // exact
+            p[u] = r;
+        }
+        *reinterpret_cast<uint4 *>(out + s * stride) = v;
+    }
+}
+
+// Planes and row exponents of an A operand: 32 rows per CTA (grid x), operand = blockIdx.y.
+// The planes' order: [row tile of 128][step of K][slice][Re, Im][8 rows][half step][row][8 k].
+__global__ void __launch_bounds__(256) k_oz_split_a(const OzOperand *__restrict__ ops, int S,
+                                                    const int *__restrict__ rho0, unsigned char *__restrict__ planes,
+                                                    int64_t bytes, int *__restrict__ exps) {
+    __shared__ int sm[8][32];
+    const OzOperand op = ops[blockIdx.y];
+    const int *rho = rho0 + (int64_t)op.pair * S;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = blockIdx.x * 32 + lane;
+    int e = kOzNone;
+    if (r < S)
+        for (int k = w; k < S; k += 8) {
+            const int x = exp_of(op.X[r + (int64_t)k * S]);
+            e = max(e, (x == kOzNone || x == kOzBad) ? x : x + rho[k]);
+        }
+    sm[w][lane] = e;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) e = max(e, sm[q][lane]);
+    if (w == 0 && r < S) exps[(int64_t)blockIdx.y * S + r] = e;
+    if (r >= S) return;
+    const int steps = oz_steps(S);
+    unsigned char *base = planes + (int64_t)blockIdx.y * bytes + (int64_t)(r / kOzM) * steps * kOzStepA +
+                          ((r % kOzM) / 8) * 256 + (r % 8) * 16;
+    for (int kg = w; kg < 2 * steps; kg += 8) {
+        long long re[8], im[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int k = kg * 8 + u;
+            const double2 v = k < S ? op.X[r + (int64_t)k * S] : mk(0.0, 0.0);
+            const int ek = k < S ? e - rho[k] : 0;
+            re[u] = fixed63(v.x, ek);
+            im[u] = fixed63(v.y, ek);
+        }
+        unsigned char *o = base + (int64_t)(kg >> 1) * kOzStepA + (kg & 1) * 128;
+        put_digits(re, o, kOzSliceA);
+        put_digits(im, o + kOzSliceA / 2, kOzSliceA);
+    }
+}
+
+// Planes and column exponents of a B operand: 8 columns per CTA (grid x), a warp's lanes
+// over the columns; the planes' order as above with columns in the place of rows and tiles
+// of 64.
+__global__ void __launch_bounds__(256) k_oz_split_b(const OzOperand *__restrict__ ops, int S,
+                                                    const int *__restrict__ rho0, unsigned char *__restrict__ planes,
+                                                    int64_t bytes, int *__restrict__ exps) {
+    __shared__ int sm[32][8];
+    const OzOperand op = ops[blockIdx.y];
+    const int *rho = rho0 + (int64_t)op.pair * S;
+    const int c8 = threadIdx.x & 7, t = threadIdx.x >> 3, c = blockIdx.x * 8 + c8;   // 8 columns x 32
+    const double2 *X = op.X + (int64_t)c * S;
+    int e = kOzNone;
+    if (c < S)
+        for (int k = t; k < S; k += 32) {
+            const int x = exp_of(X[k]);
+            e = max(e, (x == kOzNone || x == kOzBad) ? x : x - rho[k]);
+        }
+    sm[t][c8] = e;
+    __syncthreads();
+#pragma unroll 8
+    for (int q = 0; q < 32; ++q) e = max(e, sm[q][c8]);
+    if (t == 0 && c < S) exps[(int64_t)blockIdx.y * S + c] = e;
+    if (c >= S) return;
+    const int steps = oz_steps(S);
+    unsigned char *base = planes + (int64_t)blockIdx.y * bytes + (int64_t)(c / kOzN) * steps * kOzStepB +
+                          ((c % kOzN) / 8) * 256 + (c % 8) * 16;
+    for (int kg = t; kg < 2 * steps; kg += 32) {
+        long long re[8], im[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int k = kg * 8 + u;
+            const double2 v = k < S ? X[k] : mk(0.0, 0.0);
+            const int ek = k < S ? e + rho[k] : 0;
+            re[u] = fixed63(v.x, ek);
+            im[u] = fixed63(v.y, ek);
+        }
+        unsigned char *o = base + (int64_t)(kg >> 1) * kOzStepB + (kg & 1) * 128;
+        put_digits(re, o, kOzSliceB);
+        put_digits(im, o + kOzSliceB / 2, kOzSliceB);
+    }
+}
+
+// ----------------------------------------------------------------------------- tcgen05 PTX
+__device__ __forceinline__ void oz_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void oz_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void oz_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void oz_commit(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void oz_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void oz_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// bulk copy of `bytes` (a multiple of 16) contiguous bytes global -> shared, completing on bar
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(bar))
+        : "memory");
+}
+// Shared-memory descriptor of a K-major operand of 8 x 16-byte core matrices without
+// swizzle: leading byte offset (the next core matrix along K) 128, stride byte offset (the
+// next 8 rows) 256, version 1.
+__device__ __forceinline__ uint64_t core_desc(uint32_t saddr) {
+    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(256 >> 4) << 32) |
+           ((uint64_t)1 << 46);
+}
+// Instruction descriptor of kind::f16: D F32 (bits 4-5 = 1), A and B F16 (0), A negated
+// (bit 13), N >> 3 at bits 17-22, M >> 4 at bits 24-28.
+__host__ __device__ constexpr uint32_t f16_idesc(int negate_a) {
+    return (1u << 4) | ((uint32_t)negate_a << 13) | ((uint32_t)(kOzN >> 3) << 17) | ((uint32_t)(kOzM >> 4) << 24);
+}
+
+struct OzParams {
+    const OzJob *jobs;
+    const unsigned char *pa, *pb;     // split operands
+    const int *ea, *eb;               // their exponents, S each
+    int64_t bytes_a, bytes_b;         // of one split operand
+    int S, nt;
+    int *err;
+};
+
+// (h 2^42 + g) 2^(e - 68) rounded to FP64
+__device__ __forceinline__ double from_digits(long long h, long long g, int e) {
+    const __int128 v = ((__int128)h << 42) + g;
+    const bool neg = v < 0;
+    unsigned __int128 u = neg ? -(unsigned __int128)v : (unsigned __int128)v;
+    const unsigned long long hi = (unsigned long long)(u >> 64), lo = (unsigned long long)u;
+    if ((hi | lo) == 0) return 0.0;
+    const int lz = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
+    u <<= lz;
+    const unsigned long long m = (unsigned long long)(u >> 64);           // v = m 2^(64 - lz)
+    const unsigned long long m53 = (m >> 11) + ((m >> 10) & 1);           // = m53 2^(75 - lz)
+    const int q = 75 - lz + e - 68, be = q + 1075;
+    double r;
+    if (be >= 1 && be < 2046)   // m53 = 2^53 carries into the exponent
+        r = __longlong_as_double((long long)(((unsigned long long)be << 52) + (m53 - (1ull << 52))));
+    else r = ldexp((double)m53, q);
+    return neg ? -r : r;
+}
+
+// One 128 x 64 tile (blockIdx.x) of job blockIdx.y.
+__global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzParams P) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char *smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + kOzStages * kOzStage);
+    uint64_t *empty = full + kOzStages;
+    uint64_t *accum = empty + kOzStages;     // a pass's sums are complete
+    uint64_t *drained = accum + 1;           // and have been read
+    uint32_t *holder = reinterpret_cast<uint32_t *>(drained + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const OzJob job = P.jobs[blockIdx.y];
+    const int S = P.S, steps = oz_steps(S);
+    const int mt = blockIdx.x / P.nt, nt = blockIdx.x - mt * P.nt;
+    const int pieces = (steps + kOzMaxSteps - 1) / kOzMaxSteps;   // of the inner dimension
+    const int nseg = (job.a2 >= 0 ? 2 : 1) * pieces;              // pieces of all products
+    if (tid == 0) {
+        for (int s = 0; s < kOzStages; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(accum, 1);
+        mbar_init(drained, kOzEpiWarps);
+        mbar_fence_init();
+    }
+    if (warp == kOzEpiWarps + 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(holder))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    oz_fence_before();
+    __syncthreads();
+    oz_fence_after();
+    const uint32_t tmem = *holder;
+
+    if (warp == kOzEpiWarps) {
+        if (lane == 0) {
+            uint32_t it = 0;
+            for (int sg = 0; sg < nseg; ++sg) {
+                const int prod = sg / pieces, k0 = (sg - prod * pieces) * kOzMaxSteps;
+                const int k1 = min(steps, k0 + kOzMaxSteps);
+                const unsigned char *pa = P.pa + (prod ? job.a2 : job.a1) * P.bytes_a + (int64_t)mt * steps * kOzStepA;
+                const unsigned char *pb = P.pb + (prod ? job.b2 : job.b1) * P.bytes_b + (int64_t)nt * steps * kOzStepB;
+                for (int g = 0; g < 3; ++g) {
+                    const uint32_t ns = kOzSlices - 3 * g;
+                    for (int k = k0; k < k1; ++k, ++it) {
+                        const int s = it % kOzStages;
+                        if (!mbar_wait(&empty[s], ((it / kOzStages) & 1u) ^ 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
+                        mbar_arrive_expect_tx(&full[s], ns * (kOzSliceA + kOzSliceB));
+                        unsigned char *sa = smem + (size_t)s * kOzStage;
+                        bulk_load(sa, pa + (int64_t)k * kOzStepA, ns * kOzSliceA, &full[s]);
+                        bulk_load(sa + kOzStepA, pb + (int64_t)k * kOzStepB, ns * kOzSliceB, &full[s]);
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == kOzEpiWarps + 1) {
+        if (lane == 0) {
+            uint32_t it = 0, pass = 0;
+            for (int sg = 0; sg < nseg; ++sg) {
+                const int prod = sg / pieces, k0 = (sg - prod * pieces) * kOzMaxSteps;
+                const int k1 = min(steps, k0 + kOzMaxSteps);
+                for (int g = 0; g < 3; ++g, ++pass) {
+                    if (pass > 0 && !mbar_wait(drained, (pass - 1) & 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
+                    oz_fence_after();
+                    for (int k = k0; k < k1; ++k, ++it) {
+                        const int s = it % kOzStages;
+                        if (!mbar_wait(&full[s], (it / kOzStages) & 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
+                        oz_fence_after();
+                        const uint64_t da = core_desc(smem_u32(smem + (size_t)s * kOzStage));
+                        const uint64_t db = core_desc(smem_u32(smem + (size_t)s * kOzStage + kOzStepA));
+                        // descriptor steps: slice 2 x part, part Im after Re
+                        constexpr uint64_t sa = kOzSliceA >> 4, sb = kOzSliceB >> 4;
+                        for (int q = 0; q < 3; ++q) {
+                            const int d = 8 - 3 * g - q;
+                            const uint32_t re = tmem + (uint32_t)(q * 2 * kOzN), im = re + kOzN;
+                            for (int i = 0; i <= d; ++i) {
+                                const uint64_t ar = da + i * sa, ai = ar + sa / 2;
+                                const uint64_t br = db + (d - i) * sb, bi = br + sb / 2;
+                                const uint32_t acc = (k == k0 && i == 0) ? 0u : 1u;
+                                oz_mma(re, ar, br, f16_idesc(0), acc);
+                                oz_mma(im, ar, bi, f16_idesc(0), acc);
+                                oz_mma(re, ai, bi, f16_idesc(1), 1u);
+                                oz_mma(im, ai, br, f16_idesc(0), 1u);
+                            }
+                        }
+                        oz_commit(&empty[s]);
+                    }
+                    oz_commit(accum);
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        // rows 32 (warp % 4) .. + 31 (the tensor-memory lanes this warp reaches), columns
+        // 16 (warp / 4) .. + 15 of the tile
+        const int row = mt * kOzM + (warp & 3) * 32 + lane, cb = (warp >> 2) * 16;
+        const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cb;
+        uint32_t pass = 0;
+        for (int sg = 0; sg < nseg; ++sg) {
+            const int prod = sg / pieces;
+            long long gr[16], gi[16];   // sums of d = 3 .. 8 in units of 128^-10
+#pragma unroll
+            for (int c = 0; c < 16; ++c) gr[c] = gi[c] = 0;
+#pragma unroll
+            for (int g = 0; g < 2; ++g, ++pass) {
+                if (!mbar_wait(accum, pass & 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
+                oz_fence_after();
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const int sh = kOzBits * (3 * g + q);
+#pragma unroll
+                    for (int h = 0; h < 16; h += 8) {
+                        float vr[8], vi[8];
+                        oz_ld8(tl + (uint32_t)(q * 2 * kOzN + h), vr);
+                        oz_ld8(tl + (uint32_t)(q * 2 * kOzN + kOzN + h), vi);
+                        oz_ld_wait();
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) {
+                            gr[h + c] += (long long)__float2int_rn(vr[c]) << sh;
+                            gi[h + c] += (long long)__float2int_rn(vi[c]) << sh;
+                        }
+                    }
+                }
+                oz_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(drained);
+            }
+            if (!mbar_wait(accum, pass & 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
+            oz_fence_after();
+            const int *ea = P.ea + (int64_t)(prod ? job.a2 : job.a1) * S, *eb = P.eb + (int64_t)(prod ? job.b2 : job.b1) * S;
+            const int er = row < S ? ea[row] : kOzNone;
+            const bool add = sg > 0 || job.beta;
+#pragma unroll
+            for (int h = 0; h < 16; h += 4) {
+                // d = 2, 1, 0 in units of 128^-4; four columns at a time
+                long long tr[4], ti[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tr[c] = ti[c] = 0;
+                uint32_t r[3][2][4];
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+#pragma unroll
+                    for (int z = 0; z < 2; ++z)
+                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                                     : "=r"(r[q][z][0]), "=r"(r[q][z][1]), "=r"(r[q][z][2]), "=r"(r[q][z][3])
+                                     : "r"(tl + (uint32_t)(q * 2 * kOzN + z * kOzN + h))
+                                     : "memory");
+                oz_ld_wait();
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        tr[c] += (long long)__float2int_rn(__uint_as_float(r[q][0][c])) << (kOzBits * q);
+                        ti[c] += (long long)__float2int_rn(__uint_as_float(r[q][1][c])) << (kOzBits * q);
+                    }
+                double2 old[4];
+                const int col0 = nt * kOzN + cb + h;
+                double2 *C = job.C + row + (int64_t)col0 * S;
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    old[c] = (add && row < S && col0 + c < S) ? C[(int64_t)c * S] : mk(0.0, 0.0);
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (row < S && col0 + c < S) {
+                        const int ec = eb[col0 + c];
+                        double2 v;
+                        if (er == kOzBad || ec == kOzBad) v = mk(NAN, NAN);
+                        else if (er == kOzNone || ec == kOzNone) v = mk(0.0, 0.0);
+                        else v = mk(from_digits(tr[c], gr[h + c], er + ec), from_digits(ti[c], gi[h + c], er + ec));
+                        if (job.negate) v = -v;
+                        C[(int64_t)c * S] = add ? old[c] + v : v;
+                    }
+            }
+            oz_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(drained);
+            ++pass;
+        }
+    }
+    oz_fence_before();
+    __syncthreads();
+    if (warp == kOzEpiWarps + 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
+// Operands and jobs of one batch, and its place in the workspace.
+struct OzBatch {
+    std::vector<OzPair> pairs;
+    std::vector<OzOperand> a, b;
+    std::vector<OzJob> jobs;
+    void clear() { pairs.clear(); a.clear(); b.clear(); jobs.clear(); }
+};
+
+int64_t round256(int64_t x) { return (x + 255) & ~(int64_t)255; }
+
+// workspace bytes of a batch of np pairs, na and nb operands and nj jobs
+int64_t oz_batch_bytes(int S, int64_t np, int64_t na, int64_t nb, int64_t nj) {
+    return round256(na * oz_bytes_a(S)) + round256(nb * oz_bytes_b(S)) + round256((np + na + nb) * S * 4) +
+           round256(np * sizeof(OzPair)) + round256((na + nb) * sizeof(OzOperand)) + round256(nj * sizeof(OzJob));
+}
+
+int oz_run(cudaStream_t st, int device, int S, const OzBatch &w, unsigned char *ws, int *err) {
+    if (w.jobs.empty()) return KORE_OK;
+    const int64_t np = (int64_t)w.pairs.size(), na = (int64_t)w.a.size(), nb = (int64_t)w.b.size();
+    unsigned char *pa = ws, *pb = pa + round256(na * oz_bytes_a(S));
+    int *rho = reinterpret_cast<int *>(pb + round256(nb * oz_bytes_b(S)));
+    int *ea = rho + np * S, *eb = ea + na * S;
+    unsigned char *tab = reinterpret_cast<unsigned char *>(rho) + round256((np + na + nb) * S * 4);
+    // one upload of the tables
+    std::vector<unsigned char> h(round256(np * sizeof(OzPair)) + round256((na + nb) * sizeof(OzOperand)) +
+                                 w.jobs.size() * sizeof(OzJob));
+    auto put = [&](size_t at, const void *src, size_t n) { if (n) memcpy(h.data() + at, src, n); };
+    const size_t at_ops = round256(np * sizeof(OzPair)), at_jobs = at_ops + round256((na + nb) * sizeof(OzOperand));
+    put(0, w.pairs.data(), np * sizeof(OzPair));
+    put(at_ops, w.a.data(), na * sizeof(OzOperand));
+    put(at_ops + na * sizeof(OzOperand), w.b.data(), nb * sizeof(OzOperand));
+    put(at_jobs, w.jobs.data(), w.jobs.size() * sizeof(OzJob));
+    KORE_CUDA_TRY(cudaMemcpyAsync(tab, h.data(), h.size(), cudaMemcpyHostToDevice, st));
+    const OzOperand *da = reinterpret_cast<const OzOperand *>(tab + at_ops);
+    k_oz_rho<<<dim3(kore_div_up(S, 32), (unsigned)np), 256, 0, st>>>(reinterpret_cast<const OzPair *>(tab), S, rho);
+    k_oz_split_a<<<dim3(kore_div_up(S, 32), (unsigned)na), 256, 0, st>>>(da, S, rho, pa, oz_bytes_a(S), ea);
+    k_oz_split_b<<<dim3(kore_div_up(S, 8), (unsigned)nb), 256, 0, st>>>(da + na, S, rho, pb, oz_bytes_b(S), eb);
+    OzParams P;
+    P.jobs = reinterpret_cast<const OzJob *>(tab + at_jobs);
+    P.pa = pa; P.pb = pb; P.ea = ea; P.eb = eb;
+    P.bytes_a = oz_bytes_a(S); P.bytes_b = oz_bytes_b(S);
+    P.S = S; P.nt = oz_nt(S); P.err = err;
+    KORE_TRY(kore_allow_max_dyn_smem(k_oz_gemm, device));
+    k_oz_gemm<<<dim3(oz_mt(S) * oz_nt(S), (unsigned)w.jobs.size()), kOzThreads, kOzSmem, st>>>(P);
+    KORE_LAUNCHED(4);
+    KORE_CUDA_TRY(cudaGetLastError());
+    return KORE_OK;
+}
+
+}  // namespace
+
+// ----------------------------------------------------------------------------- factorisation use
+// The products run in batches that share a workspace of at most 512 MB (several waves of
+// tiles at the largest blocks; the planes take 2.3 times the matrices).
+constexpr int64_t kOzWorkspace = 512ll << 20;
+
+int64_t kore_oz_workspace_bytes(int S, int64_t K, int64_t cap) {
+    int64_t need = 0;
+    for (int64_t Kl = K - K / 2; Kl > 1; Kl -= Kl / 2) {   // levels >= 1
+        const int64_t no = Kl / 2 * cap, ne = (Kl - Kl / 2) * cap;
+        need = std::max({need, oz_batch_bytes(S, no, no, 2 * no, 2 * no),
+                         oz_batch_bytes(S, no, 2 * ne, 2 * no, 3 * ne)});
+    }
+    // one block's products always fit
+    return need == 0 ? 0 : std::max(std::min(need, kOzWorkspace), oz_batch_bytes(S, 2, 2, 4, 3));
+}
+
+namespace {
+
+struct OzQueue {
+    kore_plan *p;
+    OzBatch w;
+    // room for a unit of np pairs, na and nb operands and nj jobs: runs the batch when it
+    // would not fit with it
+    int room(int64_t np, int64_t na, int64_t nb, int64_t nj, bool *flushed) {
+        *flushed = false;
+        if (oz_batch_bytes(p->S, (int64_t)w.pairs.size() + np, (int64_t)w.a.size() + na, (int64_t)w.b.size() + nb,
+                           (int64_t)w.jobs.size() + nj) <= p->oz_bytes)
+            return KORE_OK;
+        *flushed = true;
+        return run();
+    }
+    int run() {
+        KORE_TRY(oz_run(p->stream, p->device, p->S, w, static_cast<unsigned char *>(p->d_oz), p->d_err));
+        w.clear();
+        return KORE_OK;
+    }
+    int pair(const double2 *x0, const double2 *x1) {
+        w.pairs.push_back({x0, x1});
+        return (int)w.pairs.size() - 1;
+    }
+    int a(const double2 *x, int pr) {
+        w.a.push_back({x, pr});
+        return (int)w.a.size() - 1;
+    }
+    int b(const double2 *x, int pr) {
+        w.b.push_back({x, pr});
+        return (int)w.b.size() - 1;
+    }
+};
+
+}  // namespace
+
+// G_j = D_j^-1 L_q and H_j = D_j^-1 U_q of the odd blocks of a level >= 1 (complex128).
+int kore_gh_update_oz(kore_plan *p, const BcrLevel &lv) {
+    const int64_t SS = (int64_t)p->S * p->S;
+    OzQueue z{p, {}};
+    bool flushed;
+    for (int sh = p->fw_lo; sh < p->fw_lo + p->fw_n; ++sh) {
+        const double2 *LU = static_cast<const double2 *>(p->d_LU) + sh * p->lu_stride();
+        const int64_t f = sh * p->f_stride();
+        for (int o = 0; o < lv.nodd; ++o) {
+            const int64_t q = 2 * o + 1, j = f + q * lv.stride * SS;
+            const bool hasr = q + 1 < lv.Kl;   // no right neighbour: H_j is never read
+            const double2 *L = LU + (lv.lu_L + q) * SS, *U = hasr ? LU + (lv.lu_U + q) * SS : nullptr;
+            KORE_TRY(z.room(1, 1, 2, 2, &flushed));
+            const int pr = z.pair(L, U), a = z.a(static_cast<const double2 *>(p->d_Dinv) + j, pr);
+            z.w.jobs.push_back({a, z.b(L, pr), -1, -1, static_cast<double2 *>(p->d_Gm) + j, 0, 0});
+            if (hasr) z.w.jobs.push_back({a, z.b(U, pr), -1, -1, static_cast<double2 *>(p->d_Hm) + j, 0, 0});
+        }
+    }
+    return z.run();
+}
+
+// Even-block update of a level >= 1 (complex128): D_i -= L_q H_jl + U_q G_jr; L' = -L_q G_jl;
+// U' = -U_q H_jr.
+int kore_even_update_oz(kore_plan *p, const BcrLevel &lv) {
+    const int64_t SS = (int64_t)p->S * p->S;
+    OzQueue z{p, {}};
+    bool flushed;
+    for (int sh = p->fw_lo; sh < p->fw_lo + p->fw_n; ++sh) {
+        double2 *LU = static_cast<double2 *>(p->d_LU) + sh * p->lu_stride();
+        double2 *Dw = static_cast<double2 *>(p->d_Dw) + sh * p->f_stride();
+        const double2 *G = static_cast<const double2 *>(p->d_Gm) + sh * p->f_stride();
+        const double2 *H = static_cast<const double2 *>(p->d_Hm) + sh * p->f_stride();
+        // the split G and H of the last odd block queued: the left neighbour of the next even one
+        int opr = -1, og = -1, oh = -1;
+        auto odd = [&](int64_t q) {   // position q
+            const int64_t j = q * lv.stride * SS;
+            const bool hasr = q + 1 < lv.Kl;
+            opr = z.pair(G + j, hasr ? H + j : nullptr);
+            og = z.b(G + j, opr);
+            oh = hasr ? z.b(H + j, opr) : -1;
+        };
+        for (int e = 0; e < lv.neven; ++e) {
+            const int64_t q = 2 * e;
+            const bool hasl = q >= 1, hasr = q + 1 < lv.Kl;
+            KORE_TRY(z.room(2, 2, 4, 3, &flushed));
+            OzJob d{-1, -1, -1, -1, Dw + q * lv.stride * SS, 1, 1};
+            if (hasl) {
+                if (flushed || opr < 0) odd(q - 1);
+                const int a = z.a(LU + (lv.lu_L + q) * SS, opr);
+                d.a1 = a;
+                d.b1 = oh;
+                if (lv.lu_nL >= 0) z.w.jobs.push_back({a, og, -1, -1, LU + (lv.lu_nL + e) * SS, 1, 0});
+            }
+            if (hasr) {
+                odd(q + 1);
+                const int a = z.a(LU + (lv.lu_U + q) * SS, opr);
+                (hasl ? d.a2 : d.a1) = a;
+                (hasl ? d.b2 : d.b1) = og;
+                if (lv.lu_nU >= 0 && q + 2 < lv.Kl) z.w.jobs.push_back({a, oh, -1, -1, LU + (lv.lu_nU + e) * SS, 1, 0});
+            }
+            if (hasl || hasr) z.w.jobs.push_back(d);
+        }
+    }
+    return z.run();
+}

@@ -95,7 +95,7 @@ struct kore_plan {
     // S x S column-major blocks, indexed by original block number, per shift
     void *d_Dinv = nullptr, *d_Gm = nullptr, *d_Hm = nullptr, *d_Dw = nullptr;
     void *d_LU = nullptr;             // lu_mats blocks per shift
-    void *d_T = nullptr;              // nodd_max x (S x 2S) per shift, column-major: Gauss-Jordan work (first S columns), then residuals of G, H
+    void *d_T = nullptr;              // nodd_max x t_block() per shift, column-major: Gauss-Jordan work, then (complex64) residuals of G, H
     double *d_rscale = nullptr;       // np row equilibration factors per shift
     int *d_piv = nullptr;             // nodd_max x S per shift: pivot row chosen for column k
     int *d_pidx = nullptr;            // nodd_max x S per shift: position of a row in the current panel or -1
@@ -120,10 +120,15 @@ struct kore_plan {
     // complex64 factorisation: job table of the tensor-core products (gemm_tc.cu), sized
     // for the largest level
     void *d_tctab = nullptr;
+    // complex128 factorisation: digit planes and tables of one batch of products (gemm_oz.cu)
+    void *d_oz = nullptr;
+    int64_t oz_bytes = 0;
 
     int64_t f_stride() const { return (int64_t)K * S * S; }
     int64_t lu_stride() const { return lu_mats * (int64_t)S * S; }
-    int64_t t_stride() const { return (int64_t)nodd_max * 2 * S * S; }
+    // Gauss-Jordan work of one block: complex64 keeps the residuals of G and H there too
+    int64_t t_block(size_t elt) const { return (elt == 8 ? 2 : 1) * (int64_t)S * S; }
+    int64_t t_stride() const { return nodd_max * t_block(factor_elt); }
     int64_t p_stride() const { return (int64_t)nodd_max * S; }
     int64_t ell_stride() const { return ell_rows * ell_w; }
     // stages of one sweep: A_l, B_l (l < nlev), the top block, C_l (nlev > l >= 1), E_0, C_0
@@ -197,6 +202,12 @@ int kore_even_update_tc(kore_plan *p, const BcrLevel &lv);
 int kore_gh_update_tc(kore_plan *p, const BcrLevel &lv, int level0);
 // bytes of the job table of `cap` shifts
 int64_t kore_tc_table_bytes(const kore_plan *p, int cap);
+
+// gemm_oz.cu: complex128 products of a level >= 1 on the tensor cores, split into digits
+int kore_gh_update_oz(kore_plan *p, const BcrLevel &lv);
+int kore_even_update_oz(kore_plan *p, const BcrLevel &lv);
+// bytes of their workspace for blocks of S, K blocks and cap shifts
+int64_t kore_oz_workspace_bytes(int S, int64_t K, int64_t cap);
 
 // sweep.cu
 // x_s = (A - sigma_s B)^-1 b_s for every factorised shift s on padded l-major

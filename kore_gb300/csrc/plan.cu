@@ -98,7 +98,7 @@ void free_plan(kore_plan *p) {
                     p->d_red, p->d_part, p->d_err, p->d_bar, p->d_ir, p->d_V, p->d_Vtmp, p->d_ksx, p->d_small, p->d_warm,
                     p->d_sigma, p->d_minf, p->d_bb, p->d_xb, p->d_rb, p->d_bn, p->d_rn, p->d_cnt,
                     p->d_ell_col, p->d_ell_src, p->d_ell_val, p->d_long_rows, p->d_srow, p->d_smid,
-                    p->d_scol, p->d_sval, p->d_cc_ptr, p->d_cc_row, p->d_cc_src, p->d_tctab};
+                    p->d_scol, p->d_sval, p->d_cc_ptr, p->d_cc_row, p->d_cc_src, p->d_tctab, p->d_oz};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     for (auto &v : p->d_v)
@@ -587,10 +587,10 @@ int kore_plan_estimate_bytes(const kore_pencil_desc *d, int precision, int nshif
     b += (np + 1) * 4 + nb * 12;
     b += np * 8 + K * 4 + nlev * (int64_t)sizeof(BcrLevel) + 6 * np * 16 + 8192 * 8 + 1024;
     // factors and solve workspace of c shifts
-    b += c * (4 * K * SS * e + lu * SS * e + nodd_max * 2 * SS * e + 3 * np * e + np * 8 + 3 * nodd_max * S * 4);
+    b += c * (4 * K * SS * e + lu * SS * e + nodd_max * (e == 8 ? 2 : 1) * SS * e + 3 * np * e + np * 8 + 3 * nodd_max * S * 4);
     // level-0 couplings by column; job table of the tensor-core products
     b += (2 * (K / 2 + 1) * (S + 1) + 2 * na) * 4;
-    if (precision == KORE_PREC_MIXED) b += c * (3 * (K + 1) * 48 + 64);
+    b += precision == KORE_PREC_MIXED ? c * (3 * (K + 1) * 48 + 64) : kore_oz_workspace_bytes((int)S, K, c);
     b += c * (3 * np * 16 + 2 * (np / 64 + np / 8 + 1024) * 8 + (nlev > 0 ? 3 * nlev + 2 : 1) * K * 4 + ell * e + 128);
     b += 2 * d->n * c * 16;   // kore_solve's device copies of b and x
     // per target (one per shift): Krylov basis, its restart copy, a gathered input vector,
