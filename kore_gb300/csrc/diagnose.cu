@@ -20,17 +20,17 @@
 // own, of which 17 ms at the pipe's rate.
 // Layout: k_cheb_eval writes E[j][k][i] = d^j T_k / dr^j (x_i), j = 0..3, for the points
 // i < nh = ceil(N / 2) with x_i >= 0 (threads over points, three-term recurrences of T_k and
-// its x-derivatives), then x_i and the quadrature weights.  k_flow_integrals runs one CTA per
-// (degree block, kVec eigenvectors), the coefficients in shared memory, threads over the
-// point pairs, and reduces the three integrals in a fixed order.
+// its r-derivatives), then x_i and the quadrature weights.  k_flow_integrals runs one CTA per
+// (degree block, KV eigenvectors), the coefficients in shared memory; R threads share a pair
+// of points, thread role r summing over k = r, r + R, ... (R even, so a role's k have one
+// parity), and the three integrals are reduced in a fixed order.
 #include "kore_internal.cuh"
 #include <algorithm>
 #include <vector>
 
 namespace {
 
-constexpr int kDiagThreads = 256;
-constexpr int kVec = 2;   // eigenvectors per CTA: they share its reads of E (L2 traffic)
+constexpr int kDiagThreads = 512;   // at most, roles x points
 
 __global__ void k_cheb_eval(int N, double ricb, double rcmb, double *__restrict__ E) {
     const int nh = (N + 1) / 2;
@@ -42,28 +42,24 @@ __global__ void k_cheb_eval(int N, double ricb, double rcmb, double *__restrict_
     const int64_t NN = (int64_t)N * nh;
     E[4 * NN + i] = x;
     E[4 * NN + nh + i] = sqrt(1.0 - x * x);
-    // T_k and its first three x-derivatives: T_{k+1} = 2x T_k - T_{k-1} differentiated
+    // T_k and its first three r-derivatives: T_{k+1} = 2x T_k - T_{k-1} differentiated
+    // (dx/dr = dr), seven FP64 operations per step
+    const double x2 = 2.0 * x, c1 = 2.0 * dr, c2 = 4.0 * dr, c3 = 6.0 * dr;
     double t0 = 1.0, t1 = x;            // T_{k-1}, T_k
-    double d10 = 0.0, d11 = 1.0;        // first derivative
+    double d10 = 0.0, d11 = dr;         // first derivative
     double d20 = 0.0, d21 = 0.0;        // second
     double d30 = 0.0, d31 = 0.0;        // third
-    for (int k = 0; k < N; ++k) {
-        double v0, v1, v2, v3;
-        if (k == 0) { v0 = 1.0; v1 = 0.0; v2 = 0.0; v3 = 0.0; }
-        else if (k == 1) { v0 = x; v1 = 1.0; v2 = 0.0; v3 = 0.0; }
-        else {
-            const double n0 = 2.0 * x * t1 - t0;
-            const double n1 = 2.0 * t1 + 2.0 * x * d11 - d10;
-            const double n2 = 4.0 * d11 + 2.0 * x * d21 - d20;
-            const double n3 = 6.0 * d21 + 2.0 * x * d31 - d30;
-            t0 = t1; t1 = n0; d10 = d11; d11 = n1; d20 = d21; d21 = n2; d30 = d31; d31 = n3;
-            v0 = n0; v1 = n1; v2 = n2; v3 = n3;
-        }
+    for (int k = 0; k < N; ++k) {       // (t0, d10, ...) belongs to k
         const int64_t at = (int64_t)k * nh + i;
-        E[at] = v0;
-        E[NN + at] = v1 * dr;
-        E[2 * NN + at] = v2 * dr * dr;
-        E[3 * NN + at] = v3 * dr * dr * dr;
+        E[at] = t0;
+        E[NN + at] = d10;
+        E[2 * NN + at] = d20;
+        E[3 * NN + at] = d30;
+        const double n0 = fma(x2, t1, -t0);
+        const double n1 = fma(c1, t1, fma(x2, d11, -d10));
+        const double n2 = fma(c2, d11, fma(x2, d21, -d20));
+        const double n3 = fma(c3, d21, fma(x2, d31, -d30));
+        t0 = t1; t1 = n0; d10 = d11; d11 = n1; d20 = d21; d21 = n2; d30 = d31; d31 = n3;
     }
 }
 
@@ -106,69 +102,81 @@ __device__ __forceinline__ void flow_integrands(bool tor, int l, double rk, cons
     }
 }
 
-// Sums over even (e) and odd (o) k of E_j[k][i] c_k for ND derivatives and kVec vectors.
-template <int ND>
-__device__ __forceinline__ void parity_sums(const double *__restrict__ E, int64_t NN, int nh, int N, int i,
-                                            const double2 *cs, double2 (&e)[kVec][4], double2 (&o)[kVec][4]) {
-    for (int k = 0; k < N; k += 2) {
-        const bool odd = k + 1 < N;
-        double ev[ND], ov[ND];
+// Sums over k = role, role + R, ... of E_j[k][i] c_k for ND derivatives and KV vectors.
+template <int ND, int KV, int R>
+__device__ __forceinline__ void role_sums(const double *__restrict__ E, int64_t NN, int nh, int N, int i, int role,
+                                          const double2 *cs, double2 (&s)[KV][4]) {
+#pragma unroll 2
+    for (int k = role; k < N; k += R) {
+        double ev[ND];
 #pragma unroll
-        for (int j = 0; j < ND; ++j) {
-            ev[j] = __ldg(E + j * NN + (int64_t)k * nh + i);
-            ov[j] = odd ? __ldg(E + j * NN + (int64_t)(k + 1) * nh + i) : 0.0;
-        }
+        for (int j = 0; j < ND; ++j) ev[j] = __ldg(E + j * NN + (int64_t)k * nh + i);
 #pragma unroll
-        for (int v = 0; v < kVec; ++v) {
-            const double2 c0 = cs[v * (N + 1) + k], c1 = cs[v * (N + 1) + k + 1];   // entry N is zero
+        for (int v = 0; v < KV; ++v) {
+            const double2 c = cs[v * N + k];
 #pragma unroll
             for (int j = 0; j < ND; ++j) {
-                e[v][j].x = fma(ev[j], c0.x, e[v][j].x);
-                e[v][j].y = fma(ev[j], c0.y, e[v][j].y);
-                o[v][j].x = fma(ov[j], c1.x, o[v][j].x);
-                o[v][j].y = fma(ov[j], c1.y, o[v][j].y);
+                s[v][j].x = fma(ev[j], c.x, s[v][j].x);
+                s[v][j].y = fma(ev[j], c.y, s[v][j].y);
             }
         }
     }
 }
 
-__global__ void __launch_bounds__(kDiagThreads) k_flow_integrals(FlowArgs a) {
-    extern __shared__ double2 cs[];   // kVec x (N + 1) coefficients
-    __shared__ double red[kVec][3][kDiagThreads / 32];
-    const int b = blockIdx.x, v0 = blockIdx.y * kVec, N = a.N, nh = (N + 1) / 2;
+// pts point pairs at a time (a multiple of 32), R threads each.
+template <int KV, int R>
+__global__ void __launch_bounds__(kDiagThreads) k_flow_integrals(FlowArgs a, int pts) {
+    extern __shared__ double2 cs[];      // KV x N coefficients, then the roles' sums
+    __shared__ double red[KV][3][kDiagThreads / 32];
+    const int b = blockIdx.x, v0 = blockIdx.y * KV, N = a.N, nh = (N + 1) / 2;
+    double2 *ps = cs + KV * N;           // [vector][derivative][role][point]
     const int nblk = a.npol + a.ntor;
     const bool tor = b >= a.npol;
     const int l = tor ? a.ltor[b - a.npol] : a.lpol[b];
-    for (int v = 0; v < kVec; ++v) {
+    for (int v = 0; v < KV; ++v) {
         const double2 *c = a.x + ((int64_t)(v0 + v) * nblk + b) * N;
-        for (int k = threadIdx.x; k <= N; k += blockDim.x)
-            cs[v * (N + 1) + k] = (k < N && v0 + v < a.nvec) ? c[k] : mk(0.0, 0.0);
+        for (int k = threadIdx.x; k < N; k += blockDim.x) cs[v * N + k] = v0 + v < a.nvec ? c[k] : mk(0.0, 0.0);
     }
     __syncthreads();
     const int64_t NN = (int64_t)N * nh;
-    double sum[kVec][3];
+    const int pt = threadIdx.x % pts, role = threadIdx.x / pts;
+    double sum[KV][3];
 #pragma unroll
-    for (int v = 0; v < kVec; ++v) sum[v][0] = sum[v][1] = sum[v][2] = 0.0;
-    for (int i = threadIdx.x; i < nh; i += blockDim.x) {
-        double2 e[kVec][4], o[kVec][4];
+    for (int v = 0; v < KV; ++v) sum[v][0] = sum[v][1] = sum[v][2] = 0.0;
+    for (int i0 = 0; i0 < nh; i0 += pts) {
+        const int i = i0 + pt;
+        double2 s[KV][4];
 #pragma unroll
-        for (int v = 0; v < kVec; ++v)
+        for (int v = 0; v < KV; ++v)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) e[v][j] = o[v][j] = mk(0.0, 0.0);
-        if (tor) parity_sums<3>(a.E, NN, nh, N, i, cs, e, o);
-        else parity_sums<4>(a.E, NN, nh, N, i, cs, e, o);
-        const double x = a.E[4 * NN + i], w = a.E[4 * NN + nh + i];
-        const int npt = (2 * i + 1 == N) ? 1 : 2;   // the middle point of an odd N is its own mirror
-        for (int m = 0; m < npt; ++m) {
-            const double xk = m ? -x : x;
-            const double rk = 0.5 * (a.rcmb - a.ricb) * (xk + 1.0) + a.ricb;
+            for (int j = 0; j < 4; ++j) s[v][j] = mk(0.0, 0.0);
+        if (i < nh) {
+            if (tor) role_sums<3, KV, R>(a.E, NN, nh, N, i, role, cs, s);
+            else role_sums<4, KV, R>(a.E, NN, nh, N, i, role, cs, s);
+        }
+        __syncthreads();
 #pragma unroll
-            for (int v = 0; v < kVec; ++v) {
+        for (int v = 0; v < KV; ++v)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) ps[((v * 4 + j) * R + role) * pts + pt] = s[v][j];
+        __syncthreads();
+        // role 0 takes x, role 1 its mirror image (the middle point of an odd N has none)
+        if (role < 2 && i < nh && !(role == 1 && 2 * i + 1 == N)) {
+            const double x = a.E[4 * NN + i], w = a.E[4 * NN + nh + i];
+            const double rk = 0.5 * (a.rcmb - a.ricb) * ((role ? -x : x) + 1.0) + a.ricb;
+#pragma unroll
+            for (int v = 0; v < KV; ++v) {
                 double2 p[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    p[j] = m ? e[v][j] - o[v][j] : e[v][j] + o[v][j];
-                    if (m && (j & 1)) p[j] = -p[j];
+                    double2 e = mk(0.0, 0.0), o = mk(0.0, 0.0);
+#pragma unroll
+                    for (int q = 0; q < R; q += 2) {
+                        e = e + ps[((v * 4 + j) * R + q) * pts + pt];
+                        o = o + ps[((v * 4 + j) * R + q + 1) * pts + pt];
+                    }
+                    p[j] = role ? e - o : e + o;
+                    if (role && (j & 1)) p[j] = -p[j];
                 }
                 double f[3];
                 flow_integrands(tor, l, rk, p, f);
@@ -178,22 +186,30 @@ __global__ void __launch_bounds__(kDiagThreads) k_flow_integrals(FlowArgs a) {
         }
     }
 #pragma unroll
-    for (int v = 0; v < kVec; ++v)
+    for (int v = 0; v < KV; ++v)
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             const double t = warp_sum_d(sum[v][q]);
             if ((threadIdx.x & 31) == 0) red[v][q][threadIdx.x >> 5] = t;
         }
     __syncthreads();
-    if (threadIdx.x < 3 * kVec) {
+    if (threadIdx.x < 3 * KV) {
         const int v = threadIdx.x / 3, q = threadIdx.x - 3 * v;
         if (v0 + v < a.nvec) {
-            double s = 0.0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[v][q][w];
+            double t = 0.0;
+            for (int w = 0; w < 2 * pts / 32; ++w) t += red[v][q][w];   // roles 0 and 1
             const double quad = (3.14159265358979323846 / N) * (a.rcmb - a.ricb) / 2.0;
-            a.out[((int64_t)(v0 + v) * nblk + b) * 3 + q] = quad * s;
+            a.out[((int64_t)(v0 + v) * nblk + b) * 3 + q] = quad * t;
         }
     }
+}
+
+template <int KV, int R>
+int launch_flow(const FlowArgs &a, int device, int pts) {
+    const size_t smem = ((size_t)KV * a.N + (size_t)KV * 4 * R * pts) * sizeof(double2);
+    KORE_TRY(kore_allow_max_dyn_smem(k_flow_integrals<KV, R>, device));
+    k_flow_integrals<KV, R><<<dim3(a.npol + a.ntor, kore_div_up(a.nvec, KV)), R * pts, smem>>>(a, pts);
+    return KORE_OK;
 }
 
 }  // namespace
@@ -230,10 +246,16 @@ extern "C" int kore_flow_diagnostics(int device, int N, double ricb, int npol, c
         ck(cudaMemcpy(dx, x, xbytes, cudaMemcpyHostToDevice));
         k_cheb_eval<<<kore_div_up(nh, 32), 32>>>(N, ricb, 1.0, dE);
         FlowArgs a{N, npol, ntor, nvec, ricb, 1.0, dl, dl + npol, dx, dE, dout};
-        const size_t smem = (size_t)kVec * (N + 1) * sizeof(double2);
-        if (rc == KORE_OK) rc = kore_allow_max_dyn_smem(k_flow_integrals, device);
-        const int threads = std::min(kDiagThreads, (nh + 31) / 32 * 32);
-        k_flow_integrals<<<dim3(nblk, kore_div_up(nvec, kVec)), threads, smem>>>(a);
+        int nsm = 0;
+        ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+        // Many blocks: two vectors share a CTA's reads of E.  Few: the chain of products of
+        // one thread is the time, so eight threads share a pair of points.  Whole calls, two
+        // vectors and two threads against one and eight: 60 blocks of N = 96, 8 vectors, 380
+        // and 417 us; 100 of N = 200, 4 vectors, 608 and 606 us; 300 of N = 240, one vector,
+        // 530 and 435 us; 600 of N = 400, one vector, 1,828 and 1,248 us.
+        const bool many = nvec > 1 && (int64_t)nblk * nvec >= 2LL * nsm;
+        const int pts = std::min(many ? 256 : 64, (nh + 31) / 32 * 32);
+        if (rc == KORE_OK) rc = many ? launch_flow<2, 2>(a, device, pts) : launch_flow<1, 8>(a, device, pts);
         KORE_LAUNCHED(2);
         ck(cudaGetLastError());
         ck(cudaMemcpy(out, dout, obytes, cudaMemcpyDeviceToHost));

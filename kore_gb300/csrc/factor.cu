@@ -54,7 +54,7 @@ struct FV {
     const double2 *sigma;
     double *rscale;
     C *Dinv, *G, *H, *Dw, *LU, *T;
-    int *piv, *pidx, *used, *err;
+    int *piv, *used, *err;
     const int *cc_ptr, *cc_row, *cc_src;
     const int *ell_col;      // level-0 coupling rows of every block (kore_plan::d_ell_*)
     const C *ell_val;
@@ -76,7 +76,7 @@ FV<C> make_fv(kore_plan *p) {
     v.Dinv = static_cast<C *>(p->d_Dinv) + lo * p->f_stride(); v.G = static_cast<C *>(p->d_Gm) + lo * p->f_stride();
     v.H = static_cast<C *>(p->d_Hm) + lo * p->f_stride(); v.Dw = static_cast<C *>(p->d_Dw) + lo * p->f_stride();
     v.LU = static_cast<C *>(p->d_LU) + lo * p->lu_stride(); v.T = static_cast<C *>(p->d_T) + lo * p->t_stride();
-    v.piv = p->d_piv + lo * p->p_stride(); v.pidx = p->d_pidx + lo * p->p_stride();
+    v.piv = p->d_piv + lo * p->p_stride();
     v.used = p->d_used + lo * p->p_stride(); v.err = p->d_err;
     v.cc_ptr = p->d_cc_ptr; v.cc_row = p->d_cc_row; v.cc_src = p->d_cc_src;
     v.ell_col = p->d_ell_col; v.ell_val = static_cast<const C *>(p->d_ell_val) + lo * p->ell_stride();
@@ -226,6 +226,18 @@ __device__ __forceinline__ unsigned long long pivot_key(double2 x) {
     const long long b = __double_as_longlong(v);
     return (b > 0 && b <= 0x7ff0000000000000ll) ? (unsigned long long)b : 0ull;   // +0, NaN: 0
 }
+// 1 / x.  complex128: conj(x) / |x|^2 of x scaled by a power of two to magnitude [1, 4), one
+// FP64 division (about a dozen steps of the pipe each) where the scaled quotient takes three.
+__device__ __forceinline__ float2 inverse(float2 x) { return cdiv(cone<float2>(), x); }
+__device__ __forceinline__ double2 inverse(double2 x) {
+    const int hx = (__double2hiint(x.x) >> 20) & 0x7ff, hy = (__double2hiint(x.y) >> 20) & 0x7ff;
+    const int e = max(hx, hy);
+    if (e < 64 || e > 1982) return cdiv(cone<double2>(), x);   // 2^-e itself near the range's ends
+    const double s = __hiloint2double((2046 - e) << 20, 0);    // 2^(1023 - e)
+    const double2 z = s * x;
+    const double r = 1.0 / abs2(z);
+    return mk(s * (z.x * r), -(s * (z.y * r)));
+}
 // The largest key of a warp and the lowest lane that holds it.
 template <typename C>
 __device__ __forceinline__ unsigned long long warp_argmax(unsigned long long key, int &lane_of) {
@@ -262,7 +274,7 @@ __device__ __forceinline__ const C *diag_block(const FV<C> &v, int64_t o, int64_
 // columns.  The first panel and its update
 // read the diagonal block itself, which stays as it is.
 template <typename C, int NB, int MAXT>
-__global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0, int stride) {
+__global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0, int nb, int stride) {
     __shared__ __align__(16) C prow[NB];
     __shared__ unsigned long long wkey[32];
     __shared__ int wrow[32];
@@ -271,17 +283,16 @@ __global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0, int stride) {
     const int64_t o = blockIdx.x, sh = blockIdx.y;
     C *T = v.T + sh * v.t_stride + o * v.t_block + (int64_t)k0 * S;
     const C *src = k0 == 0 ? diag_block(v, o, sh, stride) : T;
-    int *piv = v.piv + sh * v.p_stride + o * S, *pidx = v.pidx + sh * v.p_stride + o * S;
+    int *piv = v.piv + sh * v.p_stride + o * S;
     int *used = v.used + sh * v.p_stride + o * S;
     const int r = threadIdx.x, lane = r & 31, w = r >> 5, nw = blockDim.x >> 5;
-    const int nb = min(NB, S - k0);
     const bool in = r < S;
 
     C P[NB];
 #pragma unroll
     for (int c = 0; c < NB; ++c) P[c] = (in && c < nb) ? src[r + (int64_t)c * S] : czero<C>();
-    bool u = !in || (k0 != 0 && used[r] != 0);
-    int mine = -1;   // the panel column this row became the pivot of
+    int mine = (in && k0 != 0) ? used[r] : 0;   // 1 + the column this row is the pivot of, or 0
+    bool u = !in || mine != 0;
     int c = 0;
     for (; c < nb; ++c) {
         int l;
@@ -298,13 +309,13 @@ __global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0, int stride) {
         if (w == p >> 5) {   // the pivot row's warp publishes the row, scaled by 1 / pivot
             if (r == p) {
                 u = true;
-                mine = c;
+                mine = k0 + c + 1;
                 s_piv[c] = p;
 #pragma unroll
                 for (int q = 0; q < NB; ++q) prow[q] = P[q];
             }
             __syncwarp();
-            const C dinv = cdiv(cone<C>(), prow[0]);
+            const C dinv = inverse(prow[0]);
             const C own = lane < NB ? prow[lane] : czero<C>();
             __syncwarp();
             if (lane < NB) prow[lane] = lane == 0 ? dinv : own * dinv;
@@ -328,8 +339,7 @@ __global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0, int stride) {
             for (int q = 0; q < NB; ++q)
                 if (q >= NB - nb) T[r + (int64_t)(q - (NB - nb)) * S] = P[q];
         }
-        used[r] = u ? 1 : 0;
-        pidx[r] = mine;
+        used[r] = mine;
     }
     if (r < done) piv[k0 + r] = s_piv[r];
     // after a zero pivot the remaining columns keep an in-range row index so that the
@@ -337,16 +347,16 @@ __global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0, int stride) {
     if (r >= done && r < nb) piv[k0 + r] = 0;
 }
 
-// Update of the columns outside the panel [k0, k0+nb): t <- t + E t[piv] for TW columns
-// per CTA (blockIdx.x) of odd block blockIdx.y, shift blockIdx.z; a column t left of the
-// panel is a finished column of the inverse, one right of it is still to be eliminated.
+// Update of the columns [c0, c1) outside the panel [k0, k0+nb): t <- t + E t[piv] for TW
+// columns per CTA (blockIdx.x) of odd block blockIdx.y, shift blockIdx.z; a column t left of
+// the panel is a finished column of the inverse, one right of it is still to be eliminated.
 // The CTA owns its columns whole (their pivot rows are read before they are replaced)
 // and walks the rows in chunks of 128: a thread holds 4 rows x TW / 8 columns, so that
 // one step of the sum costs 4 + TW / 8 shared-memory loads for TW / 2 complex products
 // and FP32 arithmetic, not shared memory, is the bound (complex128: the FP64 pipe).
 constexpr int kUpdRows = 128;
 template <typename C, int NB, int TW>
-__global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb, int stride) {
+__global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb, int c0, int c1, int stride) {
     constexpr int CT = TW / 8;   // columns per thread
     __shared__ __align__(16) C tp[NB][TW];
     __shared__ __align__(16) C es[NB][kUpdRows];
@@ -354,10 +364,10 @@ __global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb, int str
     const int64_t o = blockIdx.y, sh = blockIdx.z;
     C *T = v.T + sh * v.t_stride + o * v.t_block;
     const C *src = k0 == 0 ? diag_block(v, o, sh, stride) : T;
-    const int *piv = v.piv + sh * v.p_stride + o * S, *pidx = v.pidx + sh * v.p_stride + o * S;
-    // columns of this CTA, counted without the panel's own
-    const int j0 = blockIdx.x * TW, ncols = S - nb;
-    auto column = [&](int t) { const int j = j0 + t; return j < k0 ? j : j + nb; };
+    const int *piv = v.piv + sh * v.p_stride + o * S, *used = v.used + sh * v.p_stride + o * S;
+    // columns of this CTA, counted from c0 without the panel's own
+    const int j0 = blockIdx.x * TW, ncols = c1 - c0 - nb;
+    auto column = [&](int t) { const int j = c0 + j0 + t; return j < k0 ? j : j + nb; };
     for (int idx = threadIdx.x; idx < TW * NB; idx += 256) {
         const int c = idx % NB, t = idx / NB;
         tp[c][t] = (j0 + t < ncols && c < nb) ? src[piv[k0 + c] + (int64_t)column(t) * S] : czero<C>();
@@ -374,7 +384,8 @@ __global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb, int str
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int r = r0 + tx + 32 * i;
-            const bool keep = r < S && pidx[r] < 0;   // a pivot row starts from zero
+            // a pivot row of the panel starts from zero
+            const bool keep = r < S && !(used[r] > k0 && used[r] <= k0 + nb);
 #pragma unroll
             for (int t = 0; t < CT; ++t)
                 acc[i][t] = (keep && j0 + ty * CT + t < ncols) ? src[r + (int64_t)column(ty * CT + t) * S] : czero<C>();
@@ -556,23 +567,42 @@ unsigned grid_for(int64_t work, int threads, int num_sms) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>((work + threads - 1) / threads, 16LL * num_sms));
 }
 
-// Gauss-Jordan of the nodd work matrices T_o of every shift (all panels), then extraction.
+// Gauss-Jordan of the nodd work matrices T_o of every shift, then extraction.  Complex64:
+// panels of NB columns, each followed by the update of all other columns.  Complex128, where
+// that update would keep the FP64 pipe busy: the panels' updates stay within a group of
+// kGroup columns, whose transform is then applied to the other columns as one product on
+// the tensor cores (gemm_oz.cu), so that the FP64 pipe does kGroup / S of the work.  Wider
+// groups leave more of it there, narrower ones make more products (four shifts of the
+// 72k-unknown shell, S = 240, factorised and solved: 104.6, 99.8 and 107.6 ms for 32, 48 and
+// 64; without groups 175 ms).
+constexpr int kGroup = 48;
 template <typename C, int NB, int MAXT>
 int gauss_jordan(kore_plan *p, const FV<C> &v, const BcrLevel &lv, int nodd, int top, int nshift) {
     const int S = p->S;
     const int pthreads = ((S + 31) / 32) * 32;
-    for (int k0 = 0; k0 < S; k0 += NB) {
-        const int nb = std::min(NB, S - k0);
-        k_panel<C, NB, MAXT><<<dim3(nodd, nshift), pthreads, 0, p->stream>>>(v, k0, lv.stride);
-        KORE_LAUNCHED(1);
-        if (S == nb) break;
-        // 32 columns per CTA re-read the panel least; levels with few blocks take 8, so
-        // that their CTAs still cover the GPU
-        if ((int64_t)nodd * nshift * kore_div_up(S - nb, 32) >= 2 * p->num_sms)
-            k_update<C, NB, 32><<<dim3(kore_div_up(S - nb, 32), nodd, nshift), 256, 0, p->stream>>>(v, k0, nb, lv.stride);
-        else
-            k_update<C, NB, 8><<<dim3(kore_div_up(S - nb, 8), nodd, nshift), 256, 0, p->stream>>>(v, k0, nb, lv.stride);
-        KORE_LAUNCHED(1);
+    // A group's product has fixed costs of about 50 us (four launches, one tile's chain); the
+    // FP64 products that it replaces, four multiply-adds each, run at two per SM and clock.
+    // (30 blocks of S = 96: 6.4 ms per solve with groups at every level, 5.9 without.)
+    const int64_t fma = 4LL * nodd * nshift * S * std::max(0, S - kGroup) * kGroup;
+    const int group = (sizeof(C) == 16 && fma / (2 * p->num_sms) > 200000) ? kGroup : S;
+    for (int g0 = 0; g0 < S; g0 += group) {
+        const int g1 = std::min(S, g0 + group);
+        for (int k0 = g0; k0 < g1; k0 += NB) {
+            const int nb = std::min(NB, g1 - k0), ncols = g1 - g0 - nb;
+            k_panel<C, NB, MAXT><<<dim3(nodd, nshift), pthreads, 0, p->stream>>>(v, k0, nb, lv.stride);
+            KORE_LAUNCHED(1);
+            if (ncols == 0) continue;
+            // 32 columns per CTA re-read the panel least; levels with few blocks take 8, so
+            // that their CTAs still cover the GPU
+            if ((int64_t)nodd * nshift * kore_div_up(ncols, 32) >= 2 * p->num_sms)
+                k_update<C, NB, 32><<<dim3(kore_div_up(ncols, 32), nodd, nshift), 256, 0, p->stream>>>(v, k0, nb, g0, g1,
+                                                                                                     lv.stride);
+            else
+                k_update<C, NB, 8><<<dim3(kore_div_up(ncols, 8), nodd, nshift), 256, 0, p->stream>>>(v, k0, nb, g0, g1,
+                                                                                                   lv.stride);
+            KORE_LAUNCHED(1);
+        }
+        if (g1 - g0 < S) KORE_TRY(kore_group_update_oz(p, lv, nodd, g0, g1));
     }
     k_extract<C><<<grid_for((int64_t)nodd * S * S * nshift, 256, p->num_sms), 256, 0, p->stream>>>(v, lv, nodd, top,
                                                                                                 nshift);
@@ -681,7 +711,7 @@ namespace {
 int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
     if (p->factor_elt == elt && p->shift_cap >= cap) return KORE_OK;
     void **bufs[] = {&p->d_Dinv, &p->d_Gm, &p->d_Hm, &p->d_Dw, &p->d_LU, &p->d_T, &p->d_zlo, &p->d_xlo, &p->d_flo,
-                     (void **)&p->d_rscale, (void **)&p->d_piv, (void **)&p->d_pidx, (void **)&p->d_used,
+                     (void **)&p->d_rscale, (void **)&p->d_piv, (void **)&p->d_used,
                      (void **)&p->d_sigma, (void **)&p->d_minf, (void **)&p->d_bb, (void **)&p->d_xb, (void **)&p->d_rb,
                      (void **)&p->d_bn, (void **)&p->d_rn, (void **)&p->d_part, (void **)&p->d_ir,
                      (void **)&p->d_cnt, &p->d_ell_val, &p->d_tctab, &p->d_oz};
@@ -707,7 +737,6 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
     KORE_TRY(kore_alloc(p, &p->d_flo, c * p->np * elt));
     KORE_TRY(kore_alloc(p, (void **)&p->d_rscale, c * p->np * sizeof(double)));
     KORE_TRY(kore_alloc(p, (void **)&p->d_piv, c * p->p_stride() * sizeof(int)));
-    KORE_TRY(kore_alloc(p, (void **)&p->d_pidx, c * p->p_stride() * sizeof(int)));
     KORE_TRY(kore_alloc(p, (void **)&p->d_used, c * p->p_stride() * sizeof(int)));
     KORE_TRY(kore_alloc(p, (void **)&p->d_sigma, c * sizeof(double2)));
     KORE_TRY(kore_alloc(p, (void **)&p->d_minf, c * sizeof(double)));
@@ -729,7 +758,6 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
     }
     KORE_CUDA_TRY(cudaMemset(p->d_LU, 0, c * p->lu_stride() * elt));
     KORE_CUDA_TRY(cudaMemset(p->d_piv, 0, c * p->p_stride() * sizeof(int)));
-    KORE_CUDA_TRY(cudaMemset(p->d_pidx, 0xff, c * p->p_stride() * sizeof(int)));
     KORE_CUDA_TRY(cudaMemset(p->d_used, 0, c * p->p_stride() * sizeof(int)));
     KORE_CUDA_TRY(cudaMemset(p->d_ir, 0, c * sizeof(IrState)));
     p->factor_bytes = p->bytes - before;

@@ -56,8 +56,9 @@ static_assert((int64_t)kOzSlices * kOzMaxSteps * kOzK * 4096 <= (1 << 24), "exac
 int oz_mt(int S) { return (S + kOzM - 1) / kOzM; }
 int oz_nt(int S) { return (S + kOzN - 1) / kOzN; }
 __host__ __device__ inline int oz_steps(int S) { return (S + kOzK - 1) / kOzK; }
-int64_t oz_bytes_a(int S) { return (int64_t)oz_mt(S) * oz_steps(S) * kOzStepA; }
-int64_t oz_bytes_b(int S) { return (int64_t)oz_nt(S) * oz_steps(S) * kOzStepB; }
+// planes of S rows (columns) and an inner dimension K
+int64_t oz_bytes_a(int S, int K) { return (int64_t)oz_mt(S) * oz_steps(K) * kOzStepA; }
+int64_t oz_bytes_b(int S, int K) { return (int64_t)oz_nt(S) * oz_steps(K) * kOzStepB; }
 
 // The scaling of an inner dimension: rows of X0 and X1 (X1 may be null).
 struct OzPair {
@@ -73,6 +74,32 @@ struct OzJob {
     int a1, b1, a2, b2;
     double2 *C;
     int negate, beta;
+};
+
+// The transform E of a group of columns [g0, g1) of the Gauss-Jordan work matrices and the
+// columns it is applied to: t <- t (zero in the group's pivot rows) + E t[pivot rows], for
+// block z = first + i (i: the batch's), shift z / nodd of the factor window, odd index
+// z % nodd.  Before the first group's update the columns are the diagonal block's.
+struct OzGroup {
+    double2 *T;
+    const double2 *D;
+    const int *piv, *used;
+    int64_t t_stride, t_block, f_stride, p_stride;
+    int nodd, stride, S, g0, g1, first;
+    __device__ double2 *work(int i) const {
+        const int z = first + i, sh = z / nodd, o = z - sh * nodd;
+        return T + sh * t_stride + o * t_block;
+    }
+    __device__ const double2 *source(int i) const {
+        if (g0 != 0) return work(i);
+        const int z = first + i, sh = z / nodd, o = z - sh * nodd;
+        return D + sh * f_stride + (2 * o + 1) * stride * (int64_t)S * S;
+    }
+    __device__ int64_t rows(int i) const {   // offset of the block's piv and used
+        const int z = first + i, sh = z / nodd, o = z - sh * nodd;
+        return sh * p_stride + (int64_t)o * S;
+    }
+    __device__ int column(int t) const { return t < g0 ? t : t + g1 - g0; }   // t-th column outside the group
 };
 
 // exponent e with |v| < 2^e of a finite nonzero double, from its bits (subnormals count as zero)
@@ -147,17 +174,14 @@ __device__ __forceinline__ void put_digits(long long (&x)[8], unsigned char *out
 
 // Planes and row exponents of an A operand: 32 rows per CTA (grid x), operand = blockIdx.y.
 // The planes' order: [row tile of 128][step of K][slice][Re, Im][8 rows][half step][row][8 k].
-__global__ void __launch_bounds__(256) k_oz_split_a(const OzOperand *__restrict__ ops, int S,
-                                                    const int *__restrict__ rho0, unsigned char *__restrict__ planes,
-                                                    int64_t bytes, int *__restrict__ exps) {
+__device__ __forceinline__ void split_a(const double2 *__restrict__ X, int S, int K, const int *__restrict__ rho,
+                                        unsigned char *__restrict__ planes, int64_t bytes, int *__restrict__ exps) {
     __shared__ int sm[8][32];
-    const OzOperand op = ops[blockIdx.y];
-    const int *rho = rho0 + (int64_t)op.pair * S;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = blockIdx.x * 32 + lane;
     int e = kOzNone;
     if (r < S)
-        for (int k = w; k < S; k += 8) {
-            const int x = exp_of(op.X[r + (int64_t)k * S]);
+        for (int k = w; k < K; k += 8) {
+            const int x = exp_of(X[r + (int64_t)k * S]);
             e = max(e, (x == kOzNone || x == kOzBad) ? x : x + rho[k]);
         }
     sm[w][lane] = e;
@@ -166,7 +190,7 @@ __global__ void __launch_bounds__(256) k_oz_split_a(const OzOperand *__restrict_
     for (int q = 0; q < 8; ++q) e = max(e, sm[q][lane]);
     if (w == 0 && r < S) exps[(int64_t)blockIdx.y * S + r] = e;
     if (r >= S) return;
-    const int steps = oz_steps(S);
+    const int steps = oz_steps(K);
     unsigned char *base = planes + (int64_t)blockIdx.y * bytes + (int64_t)(r / kOzM) * steps * kOzStepA +
                           ((r % kOzM) / 8) * 256 + (r % 8) * 16;
     for (int kg = w; kg < 2 * steps; kg += 8) {
@@ -174,8 +198,8 @@ __global__ void __launch_bounds__(256) k_oz_split_a(const OzOperand *__restrict_
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const int k = kg * 8 + u;
-            const double2 v = k < S ? op.X[r + (int64_t)k * S] : mk(0.0, 0.0);
-            const int ek = k < S ? e - rho[k] : 0;
+            const double2 v = k < K ? X[r + (int64_t)k * S] : mk(0.0, 0.0);
+            const int ek = k < K ? e - rho[k] : 0;
             re[u] = fixed63(v.x, ek);
             im[u] = fixed63(v.y, ek);
         }
@@ -185,30 +209,42 @@ __global__ void __launch_bounds__(256) k_oz_split_a(const OzOperand *__restrict_
     }
 }
 
+__global__ void __launch_bounds__(256) k_oz_split_a(const OzOperand *__restrict__ ops, int S,
+                                                    const int *__restrict__ rho, unsigned char *__restrict__ planes,
+                                                    int64_t bytes, int *__restrict__ exps) {
+    const OzOperand op = ops[blockIdx.y];
+    split_a(op.X, S, S, rho + (int64_t)op.pair * S, planes, bytes, exps);
+}
+__global__ void __launch_bounds__(256) k_oz_group_a(const OzGroup q, const int *__restrict__ rho,
+                                                    unsigned char *__restrict__ planes, int64_t bytes,
+                                                    int *__restrict__ exps) {
+    const int W = q.g1 - q.g0;
+    split_a(q.work(blockIdx.y) + (int64_t)q.g0 * q.S, q.S, W, rho + (int64_t)blockIdx.y * W, planes, bytes, exps);
+}
+
 // Planes and column exponents of a B operand: 8 columns per CTA (grid x), a warp's lanes
 // over the columns; the planes' order as above with columns in the place of rows and tiles
 // of 64.
-__global__ void __launch_bounds__(256) k_oz_split_b(const OzOperand *__restrict__ ops, int S,
-                                                    const int *__restrict__ rho0, unsigned char *__restrict__ planes,
-                                                    int64_t bytes, int *__restrict__ exps) {
+// Column c of n, entry k of K: X[row(k) + ld c], row(k) = k or the pivot row of k.
+__device__ __forceinline__ void split_b(const double2 *__restrict__ X, const int *__restrict__ piv, int c, int n, int K,
+                                        const int *__restrict__ rho, unsigned char *__restrict__ planes, int64_t bytes,
+                                        int *__restrict__ exps) {
     __shared__ int sm[32][8];
-    const OzOperand op = ops[blockIdx.y];
-    const int *rho = rho0 + (int64_t)op.pair * S;
-    const int c8 = threadIdx.x & 7, t = threadIdx.x >> 3, c = blockIdx.x * 8 + c8;   // 8 columns x 32
-    const double2 *X = op.X + (int64_t)c * S;
+    const int c8 = threadIdx.x & 7, t = threadIdx.x >> 3;   // 8 columns x 32
+    auto at = [&](int k) { return X[piv ? piv[k] : k]; };
     int e = kOzNone;
-    if (c < S)
-        for (int k = t; k < S; k += 32) {
-            const int x = exp_of(X[k]);
+    if (c < n)
+        for (int k = t; k < K; k += 32) {
+            const int x = exp_of(at(k));
             e = max(e, (x == kOzNone || x == kOzBad) ? x : x - rho[k]);
         }
     sm[t][c8] = e;
     __syncthreads();
 #pragma unroll 8
     for (int q = 0; q < 32; ++q) e = max(e, sm[q][c8]);
-    if (t == 0 && c < S) exps[(int64_t)blockIdx.y * S + c] = e;
-    if (c >= S) return;
-    const int steps = oz_steps(S);
+    if (t == 0 && c < n) exps[(int64_t)blockIdx.y * n + c] = e;
+    if (c >= n) return;
+    const int steps = oz_steps(K);
     unsigned char *base = planes + (int64_t)blockIdx.y * bytes + (int64_t)(c / kOzN) * steps * kOzStepB +
                           ((c % kOzN) / 8) * 256 + (c % 8) * 16;
     for (int kg = t; kg < 2 * steps; kg += 32) {
@@ -216,14 +252,41 @@ __global__ void __launch_bounds__(256) k_oz_split_b(const OzOperand *__restrict_
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const int k = kg * 8 + u;
-            const double2 v = k < S ? X[k] : mk(0.0, 0.0);
-            const int ek = k < S ? e + rho[k] : 0;
+            const double2 v = k < K ? at(k) : mk(0.0, 0.0);
+            const int ek = k < K ? e + rho[k] : 0;
             re[u] = fixed63(v.x, ek);
             im[u] = fixed63(v.y, ek);
         }
         unsigned char *o = base + (int64_t)(kg >> 1) * kOzStepB + (kg & 1) * 128;
         put_digits(re, o, kOzSliceB);
         put_digits(im, o + kOzSliceB / 2, kOzSliceB);
+    }
+}
+__global__ void __launch_bounds__(256) k_oz_split_b(const OzOperand *__restrict__ ops, int S,
+                                                    const int *__restrict__ rho, unsigned char *__restrict__ planes,
+                                                    int64_t bytes, int *__restrict__ exps) {
+    const OzOperand op = ops[blockIdx.y];
+    const int c = blockIdx.x * 8 + (threadIdx.x & 7);
+    split_b(op.X + (int64_t)c * S, nullptr, c, S, S, rho + (int64_t)op.pair * S, planes, bytes, exps);
+}
+__global__ void __launch_bounds__(256) k_oz_group_b(const OzGroup q, const int *__restrict__ rho,
+                                                    unsigned char *__restrict__ planes, int64_t bytes,
+                                                    int *__restrict__ exps) {
+    const int W = q.g1 - q.g0, c = blockIdx.x * 8 + (threadIdx.x & 7);
+    split_b(q.source(blockIdx.y) + (int64_t)q.column(c) * q.S, q.piv + q.rows(blockIdx.y) + q.g0, c, q.S - W, W,
+            rho + (int64_t)blockIdx.y * W, planes, bytes, exps);
+}
+// rho of a group: the largest exponent of each of its pivot rows outside the group.  One CTA
+// per block, a warp per pivot row.
+__global__ void __launch_bounds__(512) k_oz_group_rho(const OzGroup q, int *__restrict__ rho) {
+    const int W = q.g1 - q.g0, n = q.S - W, lane = threadIdx.x & 31;
+    const double2 *X = q.source(blockIdx.x);
+    const int *piv = q.piv + q.rows(blockIdx.x) + q.g0;
+    for (int k = threadIdx.x >> 5; k < W; k += 16) {
+        int e = kOzNone;
+        for (int t = lane; t < n; t += 32) e = max(e, exp_of(X[piv[k] + (int64_t)q.column(t) * q.S]));
+        e = __reduce_max_sync(0xffffffffu, e);
+        if (lane == 0) rho[(int64_t)blockIdx.x * W + k] = (e == kOzNone || e == kOzBad) ? 0 : e;
     }
 }
 
@@ -277,8 +340,9 @@ struct OzParams {
     const unsigned char *pa, *pb;     // split operands
     const int *ea, *eb;               // their exponents, S each
     int64_t bytes_a, bytes_b;         // of one split operand
-    int S, nt;
+    int S, nt, steps;                 // rows (and leading dimension) of C, column tiles, steps of K
     int *err;
+    OzGroup group;                    // group update: block blockIdx.y instead of a job
 };
 
 // (h 2^42 + g) 2^(e - 68) rounded to FP64
@@ -300,7 +364,8 @@ __device__ __forceinline__ double from_digits(long long h, long long g, int e) {
     return neg ? -r : r;
 }
 
-// One 128 x 64 tile (blockIdx.x) of job blockIdx.y.
+// One 128 x 64 tile (blockIdx.x) of job (of the group update: block) blockIdx.y.
+template <bool GROUP>
 __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzParams P) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
@@ -310,8 +375,16 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzParams P) {
     uint64_t *drained = accum + 1;           // and have been read
     uint32_t *holder = reinterpret_cast<uint32_t *>(drained + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const OzJob job = P.jobs[blockIdx.y];
-    const int S = P.S, steps = oz_steps(S);
+    const int S = P.S, steps = P.steps;
+    OzJob job;
+    if (GROUP) {
+        job.a1 = job.b1 = blockIdx.y;
+        job.a2 = job.b2 = -1;
+        job.C = P.group.work(blockIdx.y);
+        job.negate = 0;
+        job.beta = 1;
+    } else job = P.jobs[blockIdx.y];
+    const int ncols = GROUP ? S - (P.group.g1 - P.group.g0) : S;
     const int mt = blockIdx.x / P.nt, nt = blockIdx.x - mt * P.nt;
     const int pieces = (steps + kOzMaxSteps - 1) / kOzMaxSteps;   // of the inner dimension
     const int nseg = (job.a2 >= 0 ? 2 : 1) * pieces;              // pieces of all products
@@ -430,9 +503,17 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzParams P) {
             }
             if (!mbar_wait(accum, pass & 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
             oz_fence_after();
-            const int *ea = P.ea + (int64_t)(prod ? job.a2 : job.a1) * S, *eb = P.eb + (int64_t)(prod ? job.b2 : job.b1) * S;
+            const int *ea = P.ea + (int64_t)(prod ? job.a2 : job.a1) * S, *eb = P.eb + (int64_t)(prod ? job.b2 : job.b1) * ncols;
             const int er = row < S ? ea[row] : kOzNone;
             const bool add = sg > 0 || job.beta;
+            // the group update reads its source, zero in the group's pivot rows
+            const double2 *old_c = job.C;
+            bool keep = row < S;
+            if (GROUP) {
+                old_c = P.group.source(blockIdx.y);
+                const int u = row < S ? P.group.used[P.group.rows(blockIdx.y) + row] : 0;
+                keep = keep && !(u > P.group.g0 && u <= P.group.g1);
+            }
 #pragma unroll
             for (int h = 0; h < 16; h += 4) {
                 // d = 2, 1, 0 in units of 128^-4; four columns at a time
@@ -458,20 +539,22 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzParams P) {
                     }
                 double2 old[4];
                 const int col0 = nt * kOzN + cb + h;
-                double2 *C = job.C + row + (int64_t)col0 * S;
+                int64_t at[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    at[c] = row + (int64_t)(GROUP ? P.group.column(col0 + c) : col0 + c) * S;
+                    old[c] = (add && keep && col0 + c < ncols) ? old_c[at[c]] : mk(0.0, 0.0);
+                }
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
-                    old[c] = (add && row < S && col0 + c < S) ? C[(int64_t)c * S] : mk(0.0, 0.0);
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    if (row < S && col0 + c < S) {
+                    if (row < S && col0 + c < ncols) {
                         const int ec = eb[col0 + c];
                         double2 v;
                         if (er == kOzBad || ec == kOzBad) v = mk(NAN, NAN);
                         else if (er == kOzNone || ec == kOzNone) v = mk(0.0, 0.0);
                         else v = mk(from_digits(tr[c], gr[h + c], er + ec), from_digits(ti[c], gi[h + c], er + ec));
                         if (job.negate) v = -v;
-                        C[(int64_t)c * S] = add ? old[c] + v : v;
+                        job.C[at[c]] = add ? old[c] + v : v;
                     }
             }
             oz_fence_before();
@@ -498,15 +581,15 @@ int64_t round256(int64_t x) { return (x + 255) & ~(int64_t)255; }
 
 // workspace bytes of a batch of np pairs, na and nb operands and nj jobs
 int64_t oz_batch_bytes(int S, int64_t np, int64_t na, int64_t nb, int64_t nj) {
-    return round256(na * oz_bytes_a(S)) + round256(nb * oz_bytes_b(S)) + round256((np + na + nb) * S * 4) +
+    return round256(na * oz_bytes_a(S, S)) + round256(nb * oz_bytes_b(S, S)) + round256((np + na + nb) * S * 4) +
            round256(np * sizeof(OzPair)) + round256((na + nb) * sizeof(OzOperand)) + round256(nj * sizeof(OzJob));
 }
 
 int oz_run(cudaStream_t st, int device, int S, const OzBatch &w, unsigned char *ws, int *err) {
     if (w.jobs.empty()) return KORE_OK;
     const int64_t np = (int64_t)w.pairs.size(), na = (int64_t)w.a.size(), nb = (int64_t)w.b.size();
-    unsigned char *pa = ws, *pb = pa + round256(na * oz_bytes_a(S));
-    int *rho = reinterpret_cast<int *>(pb + round256(nb * oz_bytes_b(S)));
+    unsigned char *pa = ws, *pb = pa + round256(na * oz_bytes_a(S, S));
+    int *rho = reinterpret_cast<int *>(pb + round256(nb * oz_bytes_b(S, S)));
     int *ea = rho + np * S, *eb = ea + na * S;
     unsigned char *tab = reinterpret_cast<unsigned char *>(rho) + round256((np + na + nb) * S * 4);
     // one upload of the tables
@@ -521,15 +604,15 @@ int oz_run(cudaStream_t st, int device, int S, const OzBatch &w, unsigned char *
     KORE_CUDA_TRY(cudaMemcpyAsync(tab, h.data(), h.size(), cudaMemcpyHostToDevice, st));
     const OzOperand *da = reinterpret_cast<const OzOperand *>(tab + at_ops);
     k_oz_rho<<<dim3(kore_div_up(S, 32), (unsigned)np), 256, 0, st>>>(reinterpret_cast<const OzPair *>(tab), S, rho);
-    k_oz_split_a<<<dim3(kore_div_up(S, 32), (unsigned)na), 256, 0, st>>>(da, S, rho, pa, oz_bytes_a(S), ea);
-    k_oz_split_b<<<dim3(kore_div_up(S, 8), (unsigned)nb), 256, 0, st>>>(da + na, S, rho, pb, oz_bytes_b(S), eb);
-    OzParams P;
+    k_oz_split_a<<<dim3(kore_div_up(S, 32), (unsigned)na), 256, 0, st>>>(da, S, rho, pa, oz_bytes_a(S, S), ea);
+    k_oz_split_b<<<dim3(kore_div_up(S, 8), (unsigned)nb), 256, 0, st>>>(da + na, S, rho, pb, oz_bytes_b(S, S), eb);
+    OzParams P{};
     P.jobs = reinterpret_cast<const OzJob *>(tab + at_jobs);
     P.pa = pa; P.pb = pb; P.ea = ea; P.eb = eb;
-    P.bytes_a = oz_bytes_a(S); P.bytes_b = oz_bytes_b(S);
-    P.S = S; P.nt = oz_nt(S); P.err = err;
-    KORE_TRY(kore_allow_max_dyn_smem(k_oz_gemm, device));
-    k_oz_gemm<<<dim3(oz_mt(S) * oz_nt(S), (unsigned)w.jobs.size()), kOzThreads, kOzSmem, st>>>(P);
+    P.bytes_a = oz_bytes_a(S, S); P.bytes_b = oz_bytes_b(S, S);
+    P.S = S; P.nt = oz_nt(S); P.steps = oz_steps(S); P.err = err;
+    KORE_TRY(kore_allow_max_dyn_smem(k_oz_gemm<false>, device));
+    k_oz_gemm<false><<<dim3(oz_mt(S) * oz_nt(S), (unsigned)w.jobs.size()), kOzThreads, kOzSmem, st>>>(P);
     KORE_LAUNCHED(4);
     KORE_CUDA_TRY(cudaGetLastError());
     return KORE_OK;
@@ -542,6 +625,11 @@ int oz_run(cudaStream_t st, int device, int S, const OzBatch &w, unsigned char *
 // tiles at the largest blocks; the planes take 2.3 times the matrices).
 constexpr int64_t kOzWorkspace = 512ll << 20;
 
+// workspace bytes of one block's group update, W columns
+static int64_t oz_group_bytes(int S, int W) {
+    return oz_bytes_a(S, W) + oz_bytes_b(S, W) + round256((int64_t)(W + 2 * S) * 4);
+}
+
 int64_t kore_oz_workspace_bytes(int S, int64_t K, int64_t cap) {
     int64_t need = 0;
     for (int64_t Kl = K - K / 2; Kl > 1; Kl -= Kl / 2) {   // levels >= 1
@@ -549,8 +637,10 @@ int64_t kore_oz_workspace_bytes(int S, int64_t K, int64_t cap) {
         need = std::max({need, oz_batch_bytes(S, no, no, 2 * no, 2 * no),
                          oz_batch_bytes(S, no, 2 * ne, 2 * no, 3 * ne)});
     }
+    // the group updates of the eliminated blocks of level 0 (a group has at most 64 columns)
+    const int64_t group = std::max<int64_t>(K / 2, 1) * cap * oz_group_bytes(S, 64);
     // one block's products always fit
-    return need == 0 ? 0 : std::max(std::min(need, kOzWorkspace), oz_batch_bytes(S, 2, 2, 4, 3));
+    return std::max(std::min(std::max(need, group), kOzWorkspace), oz_batch_bytes(S, 2, 2, 4, 3));
 }
 
 namespace {
@@ -653,4 +743,33 @@ int kore_even_update_oz(kore_plan *p, const BcrLevel &lv) {
         }
     }
     return z.run();
+}
+
+int kore_group_update_oz(kore_plan *p, const BcrLevel &lv, int nodd, int g0, int g1) {
+    const int S = p->S, W = g1 - g0, n = S - W;
+    const int64_t lo = p->fw_lo;
+    OzGroup q{static_cast<double2 *>(p->d_T) + lo * p->t_stride(), static_cast<const double2 *>(p->d_Dw) + lo * p->f_stride(),
+              p->d_piv + lo * p->p_stride(), p->d_used + lo * p->p_stride(), p->t_stride(), p->t_block(sizeof(double2)),
+              p->f_stride(), p->p_stride(), nodd, lv.stride, S, g0, g1, 0};
+    const int total = nodd * p->fw_n;
+    const int per = (int)std::min<int64_t>(std::min(total, 65535), p->oz_bytes / oz_group_bytes(S, W));
+    if (per < 1) return KORE_EINVAL;
+    KORE_TRY(kore_allow_max_dyn_smem(k_oz_gemm<true>, p->device));
+    for (q.first = 0; q.first < total; q.first += per) {
+        const int nb = std::min(per, total - q.first);
+        unsigned char *pa = static_cast<unsigned char *>(p->d_oz), *pb = pa + nb * oz_bytes_a(S, W);
+        int *rho = reinterpret_cast<int *>(pb + nb * oz_bytes_b(S, W)), *ea = rho + (int64_t)nb * W,
+            *eb = ea + (int64_t)nb * S;
+        k_oz_group_rho<<<nb, 512, 0, p->stream>>>(q, rho);
+        k_oz_group_a<<<dim3(kore_div_up(S, 32), nb), 256, 0, p->stream>>>(q, rho, pa, oz_bytes_a(S, W), ea);
+        k_oz_group_b<<<dim3(kore_div_up(n, 8), nb), 256, 0, p->stream>>>(q, rho, pb, oz_bytes_b(S, W), eb);
+        OzParams P{};
+        P.pa = pa; P.pb = pb; P.ea = ea; P.eb = eb;
+        P.bytes_a = oz_bytes_a(S, W); P.bytes_b = oz_bytes_b(S, W);
+        P.S = S; P.nt = oz_nt(n); P.steps = oz_steps(W); P.err = p->d_err; P.group = q;
+        k_oz_gemm<true><<<dim3(oz_mt(S) * P.nt, nb), kOzThreads, kOzSmem, p->stream>>>(P);
+        KORE_LAUNCHED(4);
+    }
+    KORE_CUDA_TRY(cudaGetLastError());
+    return KORE_OK;
 }

@@ -98,8 +98,7 @@ struct kore_plan {
     void *d_T = nullptr;              // nodd_max x t_block() per shift, column-major: Gauss-Jordan work, then (complex64) residuals of G, H
     double *d_rscale = nullptr;       // np row equilibration factors per shift
     int *d_piv = nullptr;             // nodd_max x S per shift: pivot row chosen for column k
-    int *d_pidx = nullptr;            // nodd_max x S per shift: position of a row in the current panel or -1
-    int *d_used = nullptr;            // nodd_max x S per shift: row already used as a pivot
+    int *d_used = nullptr;            // nodd_max x S per shift: 1 + the column a row is the pivot of, or 0
     // Level-0 couplings (the entries of a block's rows in the columns of its two
     // neighbours) as padded rows, tile by tile: entry k of row r of tile t of block i at
     // ((i * ntile + t) * ell_w + k) * 32 + r % 32, ntile = ceil(S / 32).  The first
@@ -206,6 +205,10 @@ int64_t kore_tc_table_bytes(const kore_plan *p, int cap);
 // gemm_oz.cu: complex128 products of a level >= 1 on the tensor cores, split into digits
 int kore_gh_update_oz(kore_plan *p, const BcrLevel &lv);
 int kore_even_update_oz(kore_plan *p, const BcrLevel &lv);
+// Gauss-Jordan of the nodd blocks of the factor window (complex128): the transform of columns
+// [g0, g1) applied to the other columns; the blocks' work matrices from the diagonal blocks
+// when g0 = 0
+int kore_group_update_oz(kore_plan *p, const BcrLevel &lv, int nodd, int g0, int g1);
 // bytes of their workspace for blocks of S, K blocks and cap shifts
 int64_t kore_oz_workspace_bytes(int S, int64_t K, int64_t cap);
 
