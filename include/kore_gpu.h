@@ -164,6 +164,14 @@ int kore_factor_shifts(kore_plan *plan, int nshift, const double *sigmas, int pr
  */
 int kore_solve(kore_plan *plan, const double *b, double *x, int nrhs, double refine_tol,
                kore_stats *stats);
+/*
+ * kore_solve with the right-hand sides and the solutions as the columns of row-major host
+ * arrays: entry (i, k) of x at x + 2*(nrhs*i + k), of b likewise; with b_shared != 0, b is
+ * one vector of n entries used for every column.  The GPU gathers and scatters the columns,
+ * so a host that keeps them side by side need not transpose.
+ */
+int kore_solve_cols(kore_plan *plan, const double *b, int b_shared, double *x, int nrhs, double refine_tol,
+                    kore_stats *stats);
 int kore_solve_dev(kore_plan *plan, const void *b_dev, void *x_dev, int nrhs,
                    double refine_tol, void *stream, kore_stats *stats);
 
@@ -379,6 +387,11 @@ int kore_assemble_blocks(int device, int n1, int nops, const double *ops, int64_
 
 int kore_flow_diagnostics(int device, int N, double ricb, int npol, const int32_t *lpol, int ntor,
                           const int32_t *ltor, const double *x, int nvec, double *out);
+
+/* kore_flow_diagnostics of vectors stored side by side: coefficient i of vector v at
+ * x + 2*(nvec*i + v), i < (npol + ntor) N. */
+int kore_flow_diagnostics_cols(int device, int N, double ricb, int npol, const int32_t *lpol, int ntor,
+                               const int32_t *ltor, const double *x, int nvec, double *out);
 
 /* Number of kernels this library launched since load (for launch accounting). */
 int64_t kore_kernel_launches(void);

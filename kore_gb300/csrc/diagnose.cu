@@ -67,7 +67,8 @@ struct FlowArgs {
     int N, npol, ntor, nvec;
     double ricb, rcmb;
     const int *lpol, *ltor;      // degrees of the poloidal and toroidal blocks
-    const double2 *x;            // nvec vectors of (npol + ntor) N complex coefficients
+    const double2 *x;            // nvec vectors of (npol + ntor) N complex coefficients:
+    int64_t vstride, cstride;    // coefficient i of vector v at x[v vstride + i cstride]
     const double *E;             // evaluation matrices, points and weights (k_cheb_eval)
     double *out;                 // per (vector, block): energy, diffusion, internal dissipation
 };
@@ -134,8 +135,9 @@ __global__ void __launch_bounds__(kDiagThreads) k_flow_integrals(FlowArgs a, int
     const bool tor = b >= a.npol;
     const int l = tor ? a.ltor[b - a.npol] : a.lpol[b];
     for (int v = 0; v < KV; ++v) {
-        const double2 *c = a.x + ((int64_t)(v0 + v) * nblk + b) * N;
-        for (int k = threadIdx.x; k < N; k += blockDim.x) cs[v * N + k] = v0 + v < a.nvec ? c[k] : mk(0.0, 0.0);
+        const double2 *c = a.x + (v0 + v) * a.vstride + (int64_t)b * N * a.cstride;
+        for (int k = threadIdx.x; k < N; k += blockDim.x)
+            cs[v * N + k] = v0 + v < a.nvec ? c[k * a.cstride] : mk(0.0, 0.0);
     }
     __syncthreads();
     const int64_t NN = (int64_t)N * nh;
@@ -212,10 +214,8 @@ int launch_flow(const FlowArgs &a, int device, int pts) {
     return KORE_OK;
 }
 
-}  // namespace
-
-extern "C" int kore_flow_diagnostics(int device, int N, double ricb, int npol, const int32_t *lpol, int ntor,
-                                     const int32_t *ltor, const double *x, int nvec, double *out) {
+int flow_diagnostics(int device, int N, double ricb, int npol, const int32_t *lpol, int ntor, const int32_t *ltor,
+                     const double *x, int nvec, double *out, bool cols) {
     if (N < 2 || N > 3000 || !(ricb > 0.0 && ricb < 1.0) || npol < 0 || ntor < 0 || npol + ntor == 0 ||
         (npol && !lpol) || (ntor && !ltor) || !x || nvec <= 0 || !out)
         return KORE_EINVAL;
@@ -245,7 +245,8 @@ extern "C" int kore_flow_diagnostics(int device, int N, double ricb, int npol, c
         ck(cudaMemcpy(dl, ls.data(), ls.size() * sizeof(int), cudaMemcpyHostToDevice));
         ck(cudaMemcpy(dx, x, xbytes, cudaMemcpyHostToDevice));
         k_cheb_eval<<<kore_div_up(nh, 32), 32>>>(N, ricb, 1.0, dE);
-        FlowArgs a{N, npol, ntor, nvec, ricb, 1.0, dl, dl + npol, dx, dE, dout};
+        FlowArgs a{N, npol, ntor, nvec, ricb, 1.0, dl, dl + npol, dx, cols ? 1 : (int64_t)nblk * N, cols ? nvec : 1, dE,
+                   dout};
         int nsm = 0;
         ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
         // Many blocks: two vectors share a CTA's reads of E.  Few: the chain of products of
@@ -263,4 +264,16 @@ extern "C" int kore_flow_diagnostics(int device, int N, double ricb, int npol, c
     cudaFree(dE); cudaFree(dx); cudaFree(dout); cudaFree(dl);
     if (prev >= 0 && prev != device) cudaSetDevice(prev);
     return rc;
+}
+
+}  // namespace
+
+extern "C" int kore_flow_diagnostics(int device, int N, double ricb, int npol, const int32_t *lpol, int ntor,
+                                     const int32_t *ltor, const double *x, int nvec, double *out) {
+    return flow_diagnostics(device, N, ricb, npol, lpol, ntor, ltor, x, nvec, out, false);
+}
+
+extern "C" int kore_flow_diagnostics_cols(int device, int N, double ricb, int npol, const int32_t *lpol, int ntor,
+                                          const int32_t *ltor, const double *x, int nvec, double *out) {
+    return flow_diagnostics(device, N, ricb, npol, lpol, ntor, ltor, x, nvec, out, true);
 }

@@ -144,7 +144,7 @@ struct kore_plan {
     double *d_part = nullptr;         // per-CTA maxima of the residual kernel (2 per CTA, per shift)
     double *h_red = nullptr;          // pinned host mirror
     int *d_err = nullptr;
-    unsigned *d_bar = nullptr;
+    int *d_flag = nullptr;            // a solve's non-finite flag
     int *d_cnt = nullptr;             // sweep completion counters (shift_cap x sweep_stages() x K)
     IrState *d_ir = nullptr;          // one per shift
 
@@ -239,6 +239,11 @@ int kore_scatter(kore_plan *p, const double2 *padded, double2 *orig);
 // nshift vectors at once (original order: shift s at s * n; padded: at s * np)
 int kore_gather_shifts(kore_plan *p, const double2 *orig, double2 *padded);
 int kore_scatter_shifts(kore_plan *p, const double2 *padded, double2 *orig);
+// the same with entry o of shift s's vector at orig + ld * o + (shared ? 0 : s)
+int kore_gather_cols(kore_plan *p, const double2 *orig, int ld, bool shared, double2 *padded);
+int kore_scatter_cols(kore_plan *p, const double2 *padded, double2 *orig, int ld);
+// *flag = 1 when an entry of v (n complex) is not finite
+int kore_check_finite(kore_plan *p, const double2 *v, int64_t n, int *flag);
 
 // eigs.cu
 // ntarget Krylov-Schur runs, targets 0 .. nshift-1 around the factorised shifts, the

@@ -95,7 +95,7 @@ void free_plan(kore_plan *p) {
     void *ptrs[] = {p->d_arow, p->d_acol, p->d_asplit, p->d_aval, p->d_brow, p->d_bcol, p->d_bval,
                     p->d_slot2orig, p->d_bsz, p->d_Dinv, p->d_Gm, p->d_Hm, p->d_Dw, p->d_LU, p->d_lev,
                     p->d_rscale, p->d_T, p->d_piv, p->d_used, p->d_zlo, p->d_xlo, p->d_flo,
-                    p->d_red, p->d_part, p->d_err, p->d_bar, p->d_ir, p->d_V, p->d_Vtmp, p->d_ksx, p->d_small, p->d_warm,
+                    p->d_red, p->d_part, p->d_err, p->d_flag, p->d_ir, p->d_V, p->d_Vtmp, p->d_ksx, p->d_small, p->d_warm,
                     p->d_sigma, p->d_minf, p->d_bb, p->d_xb, p->d_rb, p->d_bn, p->d_rn, p->d_cnt,
                     p->d_ell_col, p->d_ell_src, p->d_ell_val, p->d_long_rows, p->d_srow, p->d_smid,
                     p->d_scol, p->d_sval, p->d_cc_ptr, p->d_cc_row, p->d_cc_src, p->d_tctab, p->d_oz};
@@ -360,7 +360,7 @@ int create(const kore_pencil_desc *d, int device, kore_plan **out) {
     for (auto &v : p->d_v) KORE_TRY(kore_alloc(p, (void **)&v, p->np * sizeof(double2)));
     KORE_TRY(kore_alloc(p, (void **)&p->d_red, 8192 * sizeof(double)));
     KORE_TRY(kore_alloc(p, (void **)&p->d_err, sizeof(int)));
-    KORE_TRY(kore_alloc(p, (void **)&p->d_bar, 64));
+    KORE_TRY(kore_alloc(p, (void **)&p->d_flag, 64));
     KORE_CUDA_TRY(cudaMemset(p->d_err, 0, sizeof(int)));
     KORE_CUDA_TRY(cudaMemset(p->d_red, 0, 8192 * sizeof(double)));
     KORE_CUDA_TRY(cudaMallocHost(&p->h_red, 8192 * sizeof(double)));
@@ -372,14 +372,18 @@ int create(const kore_pencil_desc *d, int device, kore_plan **out) {
 }
 
 // nrhs right-hand sides (original order, device) in groups of nshift: right-hand side k
-// is solved with shift k % nshift.
-int solve_dev_impl(kore_plan *p, const double2 *b, double2 *x, int nrhs, double tol, kore_stats *st) {
+// is solved with shift k % nshift.  ld = 0: one vector after another; else side by side,
+// entry o of vector k at ld * o + k (shared: b is one vector).
+int solve_dev_impl(kore_plan *p, const double2 *b, double2 *x, int nrhs, double tol, kore_stats *st, int ld = 0,
+                   bool shared = false) {
     if (nrhs % p->nshift != 0) return KORE_EINVAL;
     KORE_TRY(kore_ir_reset(p));
     for (int g = 0; g < nrhs; g += p->nshift) {
-        KORE_TRY(kore_gather_shifts(p, b + (int64_t)g * p->n, p->d_bb));
+        if (ld) KORE_TRY(kore_gather_cols(p, shared ? b : b + g, shared ? 1 : ld, shared, p->d_bb));
+        else KORE_TRY(kore_gather_shifts(p, b + (int64_t)g * p->n, p->d_bb));
         KORE_TRY(kore_apply_inverse(p, p->d_bb, p->d_xb, tol));
-        KORE_TRY(kore_scatter_shifts(p, p->d_xb, x + (int64_t)g * p->n));
+        if (ld) KORE_TRY(kore_scatter_cols(p, p->d_xb, x + g, ld));
+        else KORE_TRY(kore_scatter_shifts(p, p->d_xb, x + (int64_t)g * p->n));
     }
     IrState s;
     KORE_TRY(kore_ir_read(p, &s));
@@ -390,6 +394,40 @@ int solve_dev_impl(kore_plan *p, const double2 *b, double2 *x, int nrhs, double 
     }
     if (s.nan) return KORE_ENAN;
     return KORE_OK;
+}
+
+// The host-pointer solves: copies, solve, and the test of the solution for NaN or Inf
+// (bin/solve.py:263-268), which runs on the device ahead of the copy back.
+int solve_host(kore_plan *p, const double *b, double *x, int nrhs, double refine_tol, kore_stats *stats, bool cols,
+               bool shared) {
+    if (!p || !b || !x || nrhs <= 0) return KORE_EINVAL;
+    if (p->factored && nrhs % p->nshift != 0) return KORE_EINVAL;
+    if (!p->factored) return KORE_ENOTFACTORED;
+    DeviceGuard g(p->device);
+    auto t0 = std::chrono::steady_clock::now();
+    if (stats) *stats = kore_stats{};
+    double2 *db = nullptr, *dx = nullptr;
+    const size_t xbytes = (size_t)p->n * nrhs * sizeof(double2), bbytes = shared ? (size_t)p->n * sizeof(double2) : xbytes;
+    KORE_CUDA_TRY(cudaMallocAsync((void **)&db, bbytes, p->stream));
+    if (cudaMallocAsync((void **)&dx, xbytes, p->stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFreeAsync(db, p->stream);
+        return KORE_ENOMEM;
+    }
+    int s = KORE_OK, bad = 0;
+    if (cudaMemcpyAsync(db, b, bbytes, cudaMemcpyHostToDevice, p->stream) != cudaSuccess) s = KORE_ECUDA;
+    if (s == KORE_OK) s = solve_dev_impl(p, db, dx, nrhs, refine_tol, stats, cols ? nrhs : 0, shared);
+    if (s == KORE_OK) s = kore_check_finite(p, dx, p->n * nrhs, p->d_flag);
+    if (s == KORE_OK && (cudaMemcpyAsync(&bad, p->d_flag, sizeof(int), cudaMemcpyDeviceToHost, p->stream) != cudaSuccess ||
+                         cudaMemcpyAsync(x, dx, xbytes, cudaMemcpyDeviceToHost, p->stream) != cudaSuccess))
+        s = KORE_ECUDA;
+    cudaFreeAsync(db, p->stream);
+    cudaFreeAsync(dx, p->stream);
+    if (cudaStreamSynchronize(p->stream) != cudaSuccess && s == KORE_OK) s = KORE_ECUDA;
+    if (s == KORE_OK) s = kore_check_device_error(p);
+    if (s == KORE_OK && bad) s = KORE_ENAN;
+    if (stats) stats->iterate_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    return s;
 }
 
 }  // namespace
@@ -415,29 +453,12 @@ int kore_factor_shifts(kore_plan *plan, int nshift, const double *sigmas, int pr
 }
 
 int kore_solve(kore_plan *p, const double *b, double *x, int nrhs, double refine_tol, kore_stats *stats) {
-    if (!p || !b || !x || nrhs <= 0) return KORE_EINVAL;
-    if (p->factored && nrhs % p->nshift != 0) return KORE_EINVAL;
-    if (!p->factored) return KORE_ENOTFACTORED;
-    DeviceGuard g(p->device);
-    auto t0 = std::chrono::steady_clock::now();
-    if (stats) *stats = kore_stats{};
-    double2 *db = nullptr, *dx = nullptr;
-    const size_t bytes = (size_t)p->n * nrhs * sizeof(double2);
-    KORE_CUDA_TRY(cudaMallocAsync((void **)&db, bytes, p->stream));
-    KORE_CUDA_TRY(cudaMallocAsync((void **)&dx, bytes, p->stream));
-    int s = KORE_OK;
-    if (cudaMemcpyAsync(db, b, bytes, cudaMemcpyHostToDevice, p->stream) != cudaSuccess) s = KORE_ECUDA;
-    if (s == KORE_OK) s = solve_dev_impl(p, db, dx, nrhs, refine_tol, stats);
-    if (s == KORE_OK && cudaMemcpyAsync(x, dx, bytes, cudaMemcpyDeviceToHost, p->stream) != cudaSuccess) s = KORE_ECUDA;
-    cudaFreeAsync(db, p->stream);
-    cudaFreeAsync(dx, p->stream);
-    if (cudaStreamSynchronize(p->stream) != cudaSuccess && s == KORE_OK) s = KORE_ECUDA;
-    if (s == KORE_OK) s = kore_check_device_error(p);
-    if (s == KORE_OK)
-        for (int64_t i = 0; i < 2 * p->n * nrhs; ++i)
-            if (!std::isfinite(x[i])) { s = KORE_ENAN; break; }
-    if (stats) stats->iterate_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    return s;
+    return solve_host(p, b, x, nrhs, refine_tol, stats, false, false);
+}
+
+int kore_solve_cols(kore_plan *p, const double *b, int b_shared, double *x, int nrhs, double refine_tol,
+                    kore_stats *stats) {
+    return solve_host(p, b, x, nrhs, refine_tol, stats, true, b_shared != 0);
 }
 
 int kore_solve_dev(kore_plan *p, const void *b_dev, void *x_dev, int nrhs, double refine_tol, void *stream,

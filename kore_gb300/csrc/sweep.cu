@@ -1004,6 +1004,76 @@ int kore_scatter_shifts(kore_plan *p, const double2 *padded, double2 *orig) {
 
 namespace {
 
+// Vectors stored side by side: entry o of shift s's vector at orig[ld o + s] (shared: one
+// vector for all).  CTA = 32 padded rows x 8 shifts at a time through shared memory, so that
+// both sides are read and written in runs.
+__global__ void __launch_bounds__(256) k_gather_cols(int64_t np, int ns, const int64_t *__restrict__ s2o,
+                                                     const double2 *__restrict__ orig, int ld, int shared,
+                                                     double2 *__restrict__ padded) {
+    __shared__ double2 t[8][33];
+    const int64_t p0 = blockIdx.x * 32LL;
+    for (int s0 = 0; s0 < ns; s0 += 8) {
+        {
+            const int s = s0 + (threadIdx.x & 7), r = threadIdx.x >> 3;
+            const int64_t o = p0 + r < np ? s2o[p0 + r] : -1;
+            t[threadIdx.x & 7][r] = (o >= 0 && s < ns) ? orig[o * ld + (shared ? 0 : s)] : mk(0.0, 0.0);
+        }
+        __syncthreads();
+        const int s = s0 + (threadIdx.x >> 5), r = threadIdx.x & 31;
+        if (s < ns && p0 + r < np) padded[s * np + p0 + r] = t[threadIdx.x >> 5][r];
+        __syncthreads();
+    }
+}
+__global__ void __launch_bounds__(256) k_scatter_cols(int64_t np, int ns, const int64_t *__restrict__ s2o,
+                                                      const double2 *__restrict__ padded, double2 *__restrict__ orig,
+                                                      int ld) {
+    __shared__ double2 t[8][33];
+    const int64_t p0 = blockIdx.x * 32LL;
+    for (int s0 = 0; s0 < ns; s0 += 8) {
+        {
+            const int s = s0 + (threadIdx.x >> 5), r = threadIdx.x & 31;
+            if (s < ns && p0 + r < np) t[threadIdx.x >> 5][r] = padded[s * np + p0 + r];
+        }
+        __syncthreads();
+        const int s = s0 + (threadIdx.x & 7), r = threadIdx.x >> 3;
+        const int64_t o = p0 + r < np ? s2o[p0 + r] : -1;
+        if (o >= 0 && s < ns) orig[o * ld + s] = t[threadIdx.x & 7][r];
+        __syncthreads();
+    }
+}
+__global__ void k_check_finite(const double2 *__restrict__ v, int64_t n, int *flag) {
+    bool bad = false;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double2 x = v[i];
+        bad = bad || (__double2hiint(x.x) & 0x7ff00000) == 0x7ff00000 || (__double2hiint(x.y) & 0x7ff00000) == 0x7ff00000;
+    }
+    if (bad) *flag = 1;
+}
+
+}  // namespace
+
+int kore_gather_cols(kore_plan *p, const double2 *orig, int ld, bool shared, double2 *padded) {
+    k_gather_cols<<<kore_div_up(p->np, 32), 256, 0, p->stream>>>(p->np, p->nshift, p->d_slot2orig, orig, ld, shared, padded);
+    KORE_LAUNCHED(1);
+    KORE_CUDA_TRY(cudaGetLastError());
+    return KORE_OK;
+}
+int kore_scatter_cols(kore_plan *p, const double2 *padded, double2 *orig, int ld) {
+    k_scatter_cols<<<kore_div_up(p->np, 32), 256, 0, p->stream>>>(p->np, p->nshift, p->d_slot2orig, padded, orig, ld);
+    KORE_LAUNCHED(1);
+    KORE_CUDA_TRY(cudaGetLastError());
+    return KORE_OK;
+}
+int kore_check_finite(kore_plan *p, const double2 *v, int64_t n, int *flag) {
+    KORE_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), p->stream));
+    k_check_finite<<<std::min<unsigned>(kore_div_up(n, 256), 1024u), 256, 0, p->stream>>>(v, n, flag);
+    KORE_LAUNCHED(1);
+    KORE_CUDA_TRY(cudaGetLastError());
+    return KORE_OK;
+}
+
+namespace {
+
 // one thread per shift
 __global__ void k_ir_begin(IrState *st, int nshift, unsigned live_mask) {
     const int s = threadIdx.x;

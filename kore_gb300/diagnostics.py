@@ -32,12 +32,12 @@ def flow_integrals(X, m, symm, lmax, N, ricb, device=0):
     if X.ndim == 1:
         X = X[:, None]
     k = X.shape[1]
-    xs = np.ascontiguousarray(X[:nb * N, :].T, dtype=np.complex128)   # (k, nb N)
+    xs = L.as_c128(X[:nb * N, :])   # (nb N, k): no copy for complex C-ordered vectors
     out = np.zeros((k, nb, 3))
     lpi = L.as_i32(lp)
     lti = L.as_i32(lt)
-    L.check(L.load().kore_flow_diagnostics(int(device), int(N), float(ricb), len(lp), L.ptr(lpi), len(lt),
-                                           L.ptr(lti), L.ptr(xs), k, L.ptr(out)), "kore_flow_diagnostics")
+    L.check(L.load().kore_flow_diagnostics_cols(int(device), int(N), float(ricb), len(lp), L.ptr(lpi), len(lt),
+                                                L.ptr(lti), L.ptr(xs), k, L.ptr(out)), "kore_flow_diagnostics")
     return out, np.concatenate([lp, lt])
 
 

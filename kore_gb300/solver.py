@@ -119,12 +119,17 @@ class Pencil:
         """x = (A - sigma B)^-1 b for a vector or the columns of an (n, k) array."""
         b = np.asarray(b)
         one = b.ndim == 1
-        bc = L.as_c128(b.reshape(self.n, -1).T)  # (k, n) rows contiguous
-        x = np.empty_like(bc)
+        cols = b.reshape(self.n, -1)
+        k = cols.shape[1]
+        # the columns stay side by side (the GPU gathers and scatters them); one vector
+        # broadcast to several columns is copied once
+        shared = k > 1 and cols.strides[1] == 0
+        bc = L.as_c128(cols[:, 0] if shared else cols)
+        x = np.empty((self.n, k), dtype=np.complex128)
         st = L.Stats()
-        L.check(self.lib.kore_solve(self._plan, L.ptr(bc), L.ptr(x), bc.shape[0], float(refine_tol), C.byref(st)),
-                "kore_solve")
-        out = x[0] if one else np.ascontiguousarray(x.T)
+        L.check(self.lib.kore_solve_cols(self._plan, L.ptr(bc), int(shared), L.ptr(x), k, float(refine_tol),
+                                         C.byref(st)), "kore_solve")
+        out = x[:, 0] if one else x
         return (out, st.as_dict()) if stats else out
 
     def solve_dev(self, b_ptr, x_ptr, nrhs=1, refine_tol=0.0, stream=None):
@@ -212,21 +217,27 @@ def forced_sweep(pencil, omegas, b, precision="mixed", group=16, refine_tol=0.0,
     om = np.asarray(omegas, dtype=np.float64).ravel()
     F = len(om)
     b = np.asarray(b)
-    X = np.empty((pencil.n, F), dtype=np.complex128)
+    one = b.reshape(-1, 1) / scale if b.ndim != 2 else None   # one right-hand side for every frequency
+    X = None if 0 < F <= group else np.empty((pencil.n, F), dtype=np.complex128)
     times = []
     escalated, resid = 0, 0.0
     for g0 in range(0, F, group):
         sl = slice(g0, min(F, g0 + group))
+        k = sl.stop - sl.start
         t = time.perf_counter()
         pencil.factor_shifts(1j * om[sl], precision)
-        rhs = (b[:, sl] if b.ndim == 2 else np.repeat(b.reshape(-1, 1), sl.stop - sl.start, axis=1)) / scale
-        X[:, sl], st = pencil.solve(rhs, refine_tol=refine_tol, stats=True)
+        rhs = np.broadcast_to(one, (len(one), k)) if one is not None else b[:, sl] / scale
+        x, st = pencil.solve(rhs, refine_tol=refine_tol, stats=True)
         if precision == "mixed":
             resid = max(resid, st["solve_resid_max"])
             if escalate_tol and not st["solve_resid_max"] <= escalate_tol:
                 pencil.factor_shifts(1j * om[sl], "fp64")
-                X[:, sl] = pencil.solve(rhs)
-                escalated += sl.stop - sl.start
+                x = pencil.solve(rhs)
+                escalated += k
+        if X is None:
+            X = x   # a single group
+        else:
+            X[:, sl] = x
         times.append(time.perf_counter() - t)
     if info is not None:
         info.update(escalated=escalated, mixed_resid_max=resid)

@@ -69,3 +69,28 @@ def test_tc_gemm_tile_edges(gpu_lib, S):
     err = ctypes.c_double(-1.0)
     assert gpu_lib.kore_tc_selftest(0, S, 6, ctypes.byref(err)) == 0
     assert 0.0 <= err.value < 2 * 2.0 ** -21 + (12 * S) ** 0.5 * 2.0 ** -24, err.value
+
+
+@pytest.mark.parametrize("nshift,k", [(1, 1), (1, 3), (3, 9), (9, 9)])
+def test_columns_equal_vectors(gpu_lib, nshift, k):
+    """Right-hand sides side by side (kore_solve_cols, one vector for all included) give bit
+    for bit what the same vectors give one after another (kore_solve)."""
+    import ctypes
+    from kore_gb300 import _lib as L
+    A, B, p = pencil([33, 31, 32, 40], 5)
+    rng = np.random.default_rng(1)
+    n = A.shape[0]
+    b = rng.standard_normal((n, k)) + 1j * rng.standard_normal((n, k))
+    with p:
+        p.factor_shifts(1j * np.linspace(0.1, 1.0, nshift), "mixed")
+        rows, ref = np.ascontiguousarray(b.T), np.empty((k, n), dtype=complex)
+        assert p.lib.kore_solve(p._plan, L.ptr(rows), L.ptr(ref), k, 0.0, ctypes.byref(L.Stats())) == 0
+        np.testing.assert_array_equal(p.solve(b), ref.T)
+        np.testing.assert_array_equal(p.solve(np.asfortranarray(b)), ref.T)
+        one = np.broadcast_to(b[:, :1], (n, k))
+        np.testing.assert_array_equal(p.solve(one), p.solve(np.array(one)))
+        bad = b.copy()
+        bad[n // 2, k - 1] = np.inf
+        with pytest.raises(L.KoreError) as e:
+            p.solve(bad)
+        assert e.value.status == 8   # KORE_ENAN
