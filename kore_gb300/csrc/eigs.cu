@@ -76,10 +76,11 @@ struct SchurOut {
 
 __device__ inline double cabs_(double2 a) { return hypot(a.x, a.y); }
 
+// principal square root, scaled (any magnitude)
 __device__ inline double2 csqrt_(double2 z) {
     const double r = hypot(z.x, z.y);
     if (r == 0.0) return mk(0.0, 0.0);
-    double t = sqrt(0.5 * (r + fabs(z.x)));
+    const double t = sqrt(0.5 * (r + fabs(z.x)));
     if (z.x >= 0.0) return mk(t, z.y / (2.0 * t));
     return mk(fabs(z.y) / (2.0 * t), copysign(t, z.y));
 }
@@ -92,66 +93,119 @@ __device__ __forceinline__ double2 shfl_xor_c(double2 v, int o) {
     return v;
 }
 
-// G = [c s; -conj(s) c] with G [x; y] = [r; 0]; c = |x| / n, s = (x / |x|) conj(y) / n,
-// n = sqrt(|x|^2 + |y|^2), evaluated with two reciprocal square roots.
-__device__ __forceinline__ void givens_r(double2 x, double2 y, double &c, double2 &s) {
-    const double a2 = abs2(x), b2 = abs2(y);
-    if (b2 == 0.0) { c = 1.0; s = mk(0.0, 0.0); return; }
-    if (a2 == 0.0) { c = 0.0; s = mk(1.0, 0.0); return; }
-    const double rn = rsqrt(a2 + b2), ra = rsqrt(a2);
-    c = a2 * ra * rn;
-    s = (ra * rn) * (x * conjg(y));
+// ----------------------------------------------------------------------------- rotations
+// The projected problem is a chain of rotations G = [c s; -conj(s) c] with G [x; y] = [r; 0],
+// c = |x| / n, s = (x / |x|) conj(y) / n, n = sqrt(|x|^2 + |y|^2).  Each is formed from
+// entries that the one before it wrote, and on this GPU every FP64 warp instruction holds
+// its sub-partition's pipe for 64 cycles whatever the number of active lanes: the number of
+// instructions on that chain is the time.  One warp (the last) carries it: its lanes hold
+// the real and imaginary parts of the products side by side, so that a rotation's parameters
+// take 18 FP64 instructions and the 2 x 2 block where its row and column updates meet six
+// (32 and 36 when a lane did whole complex products), while the other warps apply the
+// rotation to the remaining entries.  One barrier per rotation.  (Calls of 40 vectors:
+// 7.5 ms with both, 3.9 now.)
+struct Rot {
+    double c, sx, sy;
+};
+
+// The rotation of (x, y), in every lane of a full warp.
+__device__ __forceinline__ Rot givens_warp(double2 x, double2 y) {
+    const int l = threadIdx.x & 3;
+    // lane 0: |x|^2, 1: |y|^2, 2: Re x conj(y), 3: Im x conj(y)
+    const double a1 = l == 1 ? y.x : (l == 3 ? x.y : x.x), b1 = l == 0 ? x.x : y.x;
+    const double a2 = l == 1 ? y.y : (l == 3 ? -x.x : x.y), b2 = l == 0 ? x.y : y.y;
+    const double v = fma(a1, b1, a2 * b2);
+    const double xx = __shfl_sync(0xffffffffu, v, 0), yy = __shfl_sync(0xffffffffu, v, 1);
+    Rot g;
+    if (__double_as_longlong(yy) == 0) {   // integer tests: a comparison costs an FP64 instruction
+        g.c = 1.0; g.sx = g.sy = 0.0;
+    } else if (__double_as_longlong(xx) == 0) {
+        g.c = 0.0; g.sx = 1.0; g.sy = 0.0;
+    } else {
+        const double r = rsqrt(l == 1 ? xx : xx + yy);   // lane 0: 1 / n, 1: 1 / |x|
+        const double t = __shfl_sync(0xffffffffu, r, 0) * __shfl_sync(0xffffffffu, r, 1);
+        double w = t * v;   // lane 0: c, 2: Re s, 3: Im s
+        // c^2 + |s|^2 = 1 to rounding: thousands of rotations accumulate in Q, and the
+        // reciprocal roots' errors would not average out
+        const double w2 = l == 1 ? 0.0 : w * w;
+        double n = w2 + __shfl_xor_sync(0xffffffffu, w2, 1);
+        n = n + __shfl_xor_sync(0xffffffffu, n, 2);
+        w = w * fma(-0.5, n, 1.5);
+        g.c = __shfl_sync(0xffffffffu, w, 0);
+        g.sx = __shfl_sync(0xffffffffu, w, 2);
+        g.sy = __shfl_sync(0xffffffffu, w, 3);
+    }
+    return g;
 }
 
-// Apply G from the left to rows k, k+1 and G^H from the right to columns k, k+1 of H
-// (rows [0, r1), columns [c0, m)), and G^H to columns k, k+1 of Q, in one parallel step.
-// The FP64 dependency chain of a rotation is its latency (about 64 cycles per FP64
-// operation on this GPU), so the 2 x 2 block where the row and column updates meet is
-// split over lanes 0-3 of the last warp, one entry each, while the other warps update
-// every other entry (one per thread): the two run on different SM sub-partitions.
-__device__ __forceinline__ void apply_rot(double2 *H, double2 *Q, int m, int k, int c0, int r1, double c, double2 s) {
-    const int tid = threadIdx.x, nt = blockDim.x - 32;
-    if (tid >= nt) {
-        if (tid >= nt + 4) return;
-        const double2 h00 = H[k + k * m], h01 = H[k + (k + 1) * m], h10 = H[k + 1 + k * m],
-                      h11 = H[k + 1 + (k + 1) * m];
-        const int r = tid & 1, cc = (tid >> 1) & 1;   // output row k + r, column k + cc
-        // rows of G [h]: row r of the rotated rows, at columns k and k+1
-        const double2 ta = r ? c * h10 - conjg(s) * h00 : c * h00 + s * h10;   // column k
-        const double2 tb = r ? c * h11 - conjg(s) * h01 : c * h01 + s * h11;   // column k+1
-        const double2 out = cc ? c * tb - ta * s : c * ta + tb * conjg(s);
-        __syncwarp(0xFu);
-        H[k + r + (k + cc) * m] = out;
-        return;
-    }
-    const int nrow = m - (k + 2);                     // columns k+2.. of rows k, k+1
-    const int ncol = (r1 > k) ? k : r1;                // rows 0..k-1 of columns k, k+1
-    const int nlow = (r1 > k + 2) ? 1 : 0;             // row k+2 of columns k, k+1
-    const int nleft = (c0 < k) ? 1 : 0;                // column k-1 of rows k, k+1
-    const int total = nrow + ncol + nlow + nleft + m;
-    // Every item is a pair (a, b) of one matrix: rows k, k+1 of a column (G from the left,
-    // u = s) or columns k, k+1 of a row (G^H from the right, u = conj(s)); both are
-    // a' = c a + u b, b' = c b - conj(u) a.  Only the addressing differs between items,
-    // so the FP64 arithmetic runs once per warp instead of once per divergent branch.
-    for (int t = tid; t < total; t += nt) {
+// The critical warp's share of rotation g of rows and columns k, k+1 of H: the 2 x 2 block
+// (G from the left, G^H from the right; lanes 0-7: component + 2 column + 4 row), columns k,
+// k+1 of row `row` (G^H from the right; lanes 8-11: component + 2 column) when row >= 0, and
+// with left >= 0 the entries (k, left), (k+1, left) that g was formed from, which become r
+// and 0 (lanes 12-13, and 14).  Returns the lane's new value.
+__device__ __forceinline__ double critical_rot(double2 *H2, int m, int k, int row, int left, const Rot &g) {
+    double *H = reinterpret_cast<double *>(H2);
+    const int lane = threadIdx.x & 31;
+    const int comp = lane & 1, j = (lane >> 1) & 1, i = (lane >> 2) & 1;
+    const bool blk = lane < 8, low = lane >= 8 && lane < 12 && row >= 0, lft = lane >= 12 && lane < 14 && left >= 0;
+    // left product: own entry and the other row's, same and other component
+    const int at = blk ? 2 * (k + i + (k + j) * m) + comp : low ? 2 * (row + (k + j) * m) + comp
+                                                        : lft ? 2 * (k + left * m) + comp : 0;
+    const int other = blk ? 2 * (k + 1 - i + (k + j) * m) : lft ? 2 * (k + 1 + left * m) : 0;
+    const double own = H[at], same = H[other + comp], cross = H[other + 1 - comp];
+    const int row1 = blk ? i : 0;
+    double t = fma(g.c, own, fma(row1 ? -g.sx : g.sx, same, (comp ? g.sy : -g.sy) * cross));
+    if (low) t = own;
+    // right product: the other column's value of the same row
+    const double rs = __shfl_xor_sync(0xffffffffu, t, 2), rc = __shfl_xor_sync(0xffffffffu, t, 3);
+    const double u = fma(g.c, t, fma(j ? -g.sx : g.sx, rs, (comp ? -g.sy : g.sy) * rc));
+    const double out = lft ? t : u;
+    __syncwarp();
+    if (blk || low || lft) H[at] = out;
+    if (lane == 14 && left >= 0) H2[k + 1 + left * m] = mk(0.0, 0.0);
+    return out;
+}
+
+// The other warps' share: every other entry of rows and columns k, k+1 of H (rows k, k+1 of
+// columns k+2 .. m-1; columns k, k+1 of rows 0 .. k-1 without row `skip`) and of columns k,
+// k+1 of Q.  Each item is a pair (a, b): a' = c a + u b, b' = c b - conj(u) a, u = s from the
+// left, conj(s) from the right; only the addressing differs between items.
+__device__ __forceinline__ void apply_rot(double2 *H, double2 *Q, int m, int k, int skip, const Rot &g) {
+    const int nt = blockDim.x - 32;
+    const int nrow = m - (k + 2), total = nrow + k + m;
+    for (int t = threadIdx.x; t < total; t += nt) {
         int u = t, ia, step;
-        bool left;
+        double sy = -g.sy;
         double2 *M = H;
         if (u < nrow) {
-            ia = k + (k + 2 + u) * m; step = 1; left = true;
-        } else if ((u -= nrow) < ncol + nlow) {
-            ia = ((u < ncol) ? u : k + 2) + k * m; step = m; left = false;
-        } else if ((u -= ncol + nlow) < nleft) {
-            ia = k + (k - 1) * m; step = 1; left = true;
+            ia = k + (k + 2 + u) * m; step = 1; sy = g.sy;
+        } else if ((u -= nrow) < k) {
+            if (u == skip) continue;
+            ia = u + k * m; step = m;
         } else {
-            u -= nleft;
-            M = Q; ia = u + k * m; step = m; left = false;
+            M = Q; ia = (u - k) + k * m; step = m;
         }
         const double2 a = M[ia], b = M[ia + step];
-        const double2 us = left ? s : conjg(s);
-        M[ia] = c * a + us * b;
-        M[ia + step] = c * b - conjg(us) * a;
+        const double2 us = mk(g.sx, sy);
+        M[ia] = g.c * a + us * b;
+        M[ia + step] = g.c * b - conjg(us) * a;
     }
+}
+
+// Eigenvalue of [a b; c d] nearer d (the Wilkinson shift).
+__device__ __forceinline__ double2 wilkinson(double2 a, double2 b, double2 c, double2 d) {
+    const double2 half = 0.5 * (a - d);
+    const double2 z = half * half + b * c;
+    const double n2 = abs2(z);
+    double2 disc;
+    if (n2 > 1e-280 && n2 < 1e280) {   // two reciprocal square roots instead of hypot, sqrt and a division
+        const double w = 0.5 * (n2 * rsqrt(n2) + fabs(z.x)), rw = rsqrt(w);
+        const double t = w * rw, o = 0.5 * rw;
+        disc = z.x >= 0.0 ? mk(t, z.y * o) : mk(fabs(z.y) * o, copysign(t, z.y));
+    } else disc = csqrt_(z);
+    // (a + d) / 2 +- disc - d = half +- disc
+    const double2 p = half + disc, q = half - disc;
+    return d + (abs2(p) < abs2(q) ? p : q);
 }
 
 // Per-target parameters of a batched k_schur launch: CTA t works on target t when bit t
@@ -256,6 +310,8 @@ __global__ void __launch_bounds__(kSchurT) k_schur(const double2 *__restrict__ H
     const double eps = 2.220446049250313e-16;
     int hi = m - 1, iter = 0, total = 0, fail = 0;
     __shared__ int lred[kSchurT / 32];
+    __shared__ Rot rot[2];
+    const bool crit = wid == kSchurT / 32 - 1;   // the warp of the rotations' chain
     while (hi > 0) {
         // l = the largest index in [1, hi] whose subdiagonal entry is negligible, else 0:
         // one thread per candidate, maximum over the CTA
@@ -275,31 +331,29 @@ __global__ void __launch_bounds__(kSchurT) k_schur(const double2 *__restrict__ H
         if (l == hi) { --hi; iter = 0; continue; }
         if (++total > 60 * m) { fail = 1; break; }
         ++iter;
-        double2 mu;
-        {
-            const double2 a = H[hi - 1 + (hi - 1) * m], b = H[hi - 1 + hi * m];
+        if (crit) {
             const double2 c = H[hi + (hi - 1) * m], d = H[hi + hi * m];
-            if (iter % 10 == 0) {
-                mu = d + mk(1.5 * fabs(c.x), 0.0);   // exceptional shift
-            } else {
-                const double2 half = 0.5 * (a - d);
-                const double2 disc = csqrt_(half * half + b * c);
-                const double2 m1 = 0.5 * (a + d) + disc, m2 = 0.5 * (a + d) - disc;
-                mu = (abs2(m1 - d) < abs2(m2 - d)) ? m1 : m2;
-            }
-        }
-        for (int k = l; k < hi; ++k) {
-            double2 x, y;
-            if (k == l) { x = H[l + l * m] - mu; y = H[l + 1 + l * m]; }
-            else { x = H[k + (k - 1) * m]; y = H[k + 1 + (k - 1) * m]; }
-            double c; double2 sn;
-            givens_r(x, y, c, sn);
-            __syncthreads();
-            apply_rot(H, Q, m, k, (k > l) ? k - 1 : l, min(k + 3, hi + 1), c, sn);
-            __syncthreads();
-            if (k > l && tid == 0) H[k + 1 + (k - 1) * m] = mk(0.0, 0.0);
+            // every tenth sweep an exceptional shift
+            const double2 mu = iter % 10 == 0 ? d + mk(1.5 * fabs(c.x), 0.0)
+                                              : wilkinson(H[hi - 1 + (hi - 1) * m], H[hi - 1 + hi * m], c, d);
+            const Rot g = givens_warp(H[l + l * m] - mu, H[l + 1 + l * m]);
+            if (lane == 0) rot[l & 1] = g;
         }
         __syncthreads();
+        for (int k = l; k < hi; ++k) {
+            const Rot g = rot[k & 1];
+            if (crit) {
+                const int row = k + 2 <= hi ? k + 2 : -1;
+                const double v = critical_rot(H, m, k, row, k > l ? k - 1 : -1, g);
+                if (k + 1 < hi) {   // the next rotation from (k + 1, k) and the bulge (k + 2, k)
+                    const double2 x = mk(__shfl_sync(0xffffffffu, v, 4), __shfl_sync(0xffffffffu, v, 5));
+                    const double2 y = mk(__shfl_sync(0xffffffffu, v, 8), __shfl_sync(0xffffffffu, v, 9));
+                    const Rot n = givens_warp(x, y);
+                    if (lane == 0) rot[(k + 1) & 1] = n;
+                }
+            } else apply_rot(H, Q, m, k, -1, g);
+            __syncthreads();
+        }
     }
     for (int idx = tid; idx < m * m; idx += kSchurT) {
         const int r = idx % m, c = idx / m;
@@ -315,19 +369,34 @@ __global__ void __launch_bounds__(kSchurT) k_schur(const double2 *__restrict__ H
         double bk = key[pos];
         for (int j = pos + 1; j < m; ++j)
             if (key[j] < bk) { bk = key[j]; best = j; }
+        if (best == pos) continue;
+        // swaps (k, k + 1), k = best - 1 .. pos; the next swap's t12 is in row k - 1 of column
+        // k, which the critical warp updates itself
+        if (crit) {
+            const int k = best - 1;
+            const Rot g = givens_warp(H[k + (k + 1) * m], H[k + 1 + (k + 1) * m] - H[k + k * m]);
+            if (lane == 0) rot[k & 1] = g;
+        }
+        __syncthreads();
         for (int k = best - 1; k >= pos; --k) {
-            const double2 t11 = H[k + k * m], t22 = H[k + 1 + (k + 1) * m], t12 = H[k + (k + 1) * m];
-            double c; double2 sn;
-            givens_r(t12, t22 - t11, c, sn);
-            __syncthreads();
-            apply_rot(H, Q, m, k, k, k + 2, c, sn);
-            __syncthreads();
-            if (tid == 0) {
-                H[k + 1 + k * m] = mk(0.0, 0.0);
-                const double t = key[k];
-                key[k] = key[k + 1];
-                key[k + 1] = t;
-            }
+            const Rot g = rot[k & 1];
+            if (crit) {
+                const bool more = k > pos;
+                const double v = critical_rot(H, m, k, more ? k - 1 : -1, -1, g);
+                __syncwarp();
+                if (lane == 0) {
+                    H[k + 1 + k * m] = mk(0.0, 0.0);
+                    const double t = key[k];
+                    key[k] = key[k + 1];
+                    key[k + 1] = t;
+                }
+                if (more) {
+                    const double2 t22 = mk(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 1));
+                    const double2 t12 = mk(__shfl_sync(0xffffffffu, v, 8), __shfl_sync(0xffffffffu, v, 9));
+                    const Rot n = givens_warp(t12, t22 - H[k - 1 + (k - 1) * m]);
+                    if (lane == 0) rot[(k - 1) & 1] = n;
+                }
+            } else apply_rot(H, Q, m, k, k > pos ? k - 1 : -1, g);
             __syncthreads();
         }
     }
