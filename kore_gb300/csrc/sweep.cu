@@ -35,6 +35,11 @@ __device__ __forceinline__ double2 ldg(const double2 *p) { return __ldg(p); }
 __device__ __forceinline__ float2 ldg(const float2 *p) { return __ldg(p); }
 __device__ __forceinline__ void stcg(double2 *p, double2 v) { __stcg(p, v); }
 __device__ __forceinline__ void stcg(float2 *p, float2 v) { __stcg(p, v); }
+template <typename C> __device__ __forceinline__ C shfl_xor(C v, int o) {
+    v.x = __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y = __shfl_xor_sync(0xffffffffu, v.y, o);
+    return v;
+}
 
 struct SweepArgs {
     int K, S, nlev, nshift;
@@ -76,17 +81,24 @@ __device__ __forceinline__ long long ld_acquire_cta(const long long *p) {
     return v;
 }
 
-// Thread 0 waits (bounded) until *c >= target; on timeout or an earlier error the
+// One arrival at a completion counter, after this thread's (and, by the barrier before it,
+// its warp's) writes.
+__device__ __forceinline__ void signal_count(int *c) {
+    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(c) : "memory");
+}
+
+// A thread waits (bounded) until *c >= target; on timeout or an earlier error the
 // error flag is set and the caller goes on (its result is then wrong, but the kernel
 // ends).
 __device__ __forceinline__ void wait_count(const int *c, int target, int *err) {
     unsigned spins = 0;
     while (ld_relaxed_i32(c) < target) {
+        if (++spins < 32) continue;
         if (ld_relaxed_i32(err) != 0) return;
-        if (++spins > KORE_SPIN_LIMIT) { atomicCAS(err, 0, KORE_DEVERR_FLAG); return; }
+        if (spins > KORE_SPIN_LIMIT) { atomicCAS(err, 0, KORE_DEVERR_FLAG); return; }
         __nanosleep(32);
     }
-    __threadfence();   // acquire: the producer's data is read after the counter
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");   // acquire: the producer's data is read after the counter
 }
 
 // ----------------------------------------------------------------------------- the sweep kernel
@@ -122,6 +134,14 @@ constexpr TmaVariant kTmaVariants[] = {{2, 16384}, {3, 16384}, {4, 16384}, {2, 8
 constexpr TmaVariant kTmaDefault = {4, 8192};
 constexpr int kTmaThreads = kTmaConsumers + 64;   // + one producer warp + one dependency-checker warp
 constexpr int kTileRows = 32;
+// Stages with few tiles take tiles of 8 rows instead: a chunk then holds four times the
+// columns and four times as many SMs work on the stage.  These stages are the chain of the
+// upper levels, where a tile's own time counts.  complex128: its products (10.5 us per matrix
+// of S = 240 on the FP64 pipe of one SM), so a warp's lanes share each row four ways (lane =
+// row + 8 x column mod 4).  complex64: its chunks' waits (2.8 us per matrix at S = 400; a
+// quarter of the chunks, 0.7 us); a warp keeps its columns and their order, so the sums are
+// those of 32-row tiles bit for bit.  See sweep_low_tiles for the rule.
+constexpr int kLowRows = 8;
 constexpr int kMaxRing = 24;
 constexpr int kEllReg = 4;   // level-0 coupling entries per thread held in registers (width 32)
 // input-vector loads in flight per consumer lane: a two-matrix tile's slice (about 2 S / 4
@@ -133,7 +153,9 @@ template <typename C, int CPS> constexpr int fill_of() { return (CPS == 2 || (CP
 enum { kMapDinv = 0, kMapG = 1, kMapH = 2, kMapLU = 3 };
 
 struct SweepTmaParams {
-    CUtensorMap maps[4];   // Dinv, G, H, LU: (2S reals, S columns, blocks, shifts)
+    CUtensorMap maps[8];   // Dinv, G, H, LU: (2S reals, S columns, blocks, shifts), boxes of 32
+                           // rows, then the same with boxes of 8
+    int low_tiles;         // a stage with at most this many 32-row tiles takes 8-row tiles
     SweepArgs a;
     int nst;               // ring slots
 };
@@ -147,6 +169,7 @@ template <typename C, int CHUNK> struct TmaShape {
 // of its rows, first row, and the blocks it multiplies (map, block index within the map).
 struct TileJob {
     int kind, l, nmat, r0;
+    bool low;            // 8 rows instead of 32
     int64_t s, blk;
     int map[2];
     int64_t mblk[2];
@@ -154,9 +177,19 @@ struct TileJob {
     bool hasl, hasr;
 };
 
+// Stage k of the tile order among the counters: A_l: l, B_l: L + l, top: 2 L, C_l: 2 L + 1 + l,
+// E_0: 3 L + 1.
+__device__ __forceinline__ int counter_of(int k, int L) {
+    if (k < 2 * L) return (k & 1) ? L + (k >> 1) : (k >> 1);
+    if (k == 2 * L) return 2 * L;
+    return k < 3 * L ? 2 * L + 1 + (3 * L - k) : k == 3 * L ? 3 * L + 1 : 2 * L + 1;
+}
+
+// tiles: tiles per block of each counter's stage
 __device__ __forceinline__ void decode_tile(int64_t g, int &k, const int64_t *st_begin, const BcrLevel *lv_s, int L,
-                                            int ntile, TileJob &t) {
+                                            const int *tiles, int S, TileJob &t) {
     while (g >= st_begin[k + 1]) ++k;
+    const int ntile = tiles[counter_of(k, L)];
     const int64_t loc = g - st_begin[k];
     if (k < 2 * L) { t.kind = (k & 1) ? 1 : 0; t.l = k >> 1; }
     else if (k == 2 * L) { t.kind = 2; t.l = L; }
@@ -167,7 +200,8 @@ __device__ __forceinline__ void decode_tile(int64_t g, int &k, const int64_t *st
     t.s = loc / ((int64_t)nblk * ntile);
     const int64_t rem = loc - t.s * nblk * ntile;
     const int64_t bi = rem / ntile;
-    t.r0 = (int)(rem - bi * ntile) * kTileRows;
+    t.low = ntile > (S + kTileRows - 1) / kTileRows;
+    t.r0 = (int)(rem - bi * ntile) * (t.low ? kLowRows : kTileRows);
     t.nmat = 0;
     t.hasl = t.hasr = false;
     if (t.kind == 0) {
@@ -220,12 +254,17 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
     using Shape = TmaShape<C, CHUNK>;
     constexpr int kCols = Shape::kCols, kCpw = Shape::kColsPerWarp;
     constexpr int kFill = fill_of<C, CPS>();
+    constexpr bool kSplit = sizeof(C) == 16;   // low tiles: lanes share a row
+    // Columns of a warp: runs of kRun, 4 kRun apart.  complex64: the same in every variant, so
+    // that a sweep's sums do not depend on the autotuner's choice (with 8 KB chunks of 32 rows
+    // a warp then works on every other chunk).
+    constexpr int kRun = sizeof(C) == 8 ? 16 : kCpw;
+    constexpr bool kHalf = kCols < 4 * kRun;
     const SweepArgs &a = P.a;
     const int nst = P.nst;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const int S = a.S, ns = a.nshift, L = a.nlev, K = a.K;
-    const int nc = (S + kCols - 1) / kCols;   // chunks per block
-    const int nvec = nc * kCols;
+    const int nvec = (S + 4 * kCols - 1) / (4 * kCols) * (4 * kCols);   // whole chunks of either height
     unsigned char *ring = smem_raw;
     uint64_t *full = reinterpret_cast<uint64_t *>(smem_raw + (size_t)nst * CHUNK);
     uint64_t *empty = full + nst;
@@ -233,6 +272,7 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
     __shared__ C red[2][kTmaConsumerWarps][33];   // per-warp partial sums, by tile parity
     __shared__ BcrLevel lv_s[kMaxLevels];
     __shared__ int64_t st_begin[3 * kMaxLevels + 2];
+    __shared__ int tiles[3 * kMaxLevels + 2];   // per block of a stage, by its counter
     __shared__ long long ready;      // highest tile of this CTA whose inputs are complete
     {
         bool all = true;
@@ -251,7 +291,7 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
         mbar_fence_init();
         ready = -1;
     }
-    if (tid == kTmaConsumers) for (int i = 0; i < 4; ++i) tma_prefetch_desc(&P.maps[i]);
+    if (tid == kTmaConsumers) for (int i = 0; i < 8; ++i) tma_prefetch_desc(&P.maps[i]);
     __syncthreads();
     if (tid == 0) {
         int64_t acc = 0;
@@ -262,7 +302,12 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
             else if (k == 2 * L) nblk = 1;
             else if (k < 3 * L) nblk = lv_s[3 * L - k].nodd;
             else nblk = lv_s[0].nodd;   // E_0, C_0
-            acc += (int64_t)nblk * ntile * ns;
+            // the sparse stages B_0 and E_0 keep 32 rows
+            const bool sparse = L > 0 && (k == 1 || k == 3 * L);
+            const bool low = !sparse && nblk * ntile * ns <= P.low_tiles;
+            const int nt = low ? (S + kLowRows - 1) / kLowRows : ntile;
+            tiles[counter_of(k, L)] = nt;
+            acc += (int64_t)nblk * nt * ns;
         }
         st_begin[nstage] = acc;
     }
@@ -272,11 +317,8 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
         return mask_has(a.live_mask, s) && !(a.skip && a.skip[s * a.skip_stride] != 0);
     };
     auto ctr = [&](int64_t s, int sid, int64_t blk) -> int * { return a.cnt + ((s * nstage + sid) * K + blk); };
-    auto xready = [&](int64_t s, int64_t blk) -> int * {
-        if (blk == 0) return ctr(s, 2 * L, 0);
-        const int lb = __ffsll(blk) - 1;
-        return ctr(s, 2 * L + 1 + lb, blk);
-    };
+    // counter of the stage that finishes x of a block
+    auto xstage = [&](int64_t blk) -> int { return blk == 0 ? 2 * L : 2 * L + __ffsll(blk); };
 
     if (w == kTmaConsumerWarps) {
         // ------------------------------------------------------------------ producer
@@ -286,16 +328,17 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
             uint64_t issued = 0;
             TileJob t;
             for (int64_t g = blockIdx.x; g < total; g += gridDim.x) {
-                decode_tile(g, k, st_begin, lv_s, L, ntile, t);
+                decode_tile(g, k, st_begin, lv_s, L, tiles, S, t);
                 if (!live(t.s)) continue;
 #pragma unroll
                 for (int m = 0; m < 2; ++m) {
                     if (m >= t.nmat) break;
-                    for (int ch = 0; ch < nc; ++ch) {
+                    const int cols = t.low ? 4 * kCols : kCols;
+                    for (int ch = 0; ch * cols < S; ++ch) {
                         if (!mbar_wait(&empty[slot], ph ^ 1)) atomicCAS(a.err, 0, KORE_DEVERR_FLAG);
                         mbar_arrive_expect_tx(&full[slot], CHUNK);
-                        tma_load_4d(ring + (size_t)slot * CHUNK, &P.maps[t.map[m]], &full[slot],
-                                    2 * t.r0, ch * kCols, (int)t.mblk[m], (int)t.s);
+                        tma_load_4d(ring + (size_t)slot * CHUNK, &P.maps[t.map[m] + (t.low ? 4 : 0)], &full[slot],
+                                    2 * t.r0, ch * cols, (int)t.mblk[m], (int)t.s);
                         ++issued;
                         if (++slot == (uint32_t)nst) { slot = 0; ph ^= 1; }
                     }
@@ -309,12 +352,6 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
         return;
     }
     auto vec = [&](void *base, int64_t s) -> C * { return static_cast<C *>(base) + s * np; };
-    auto rhs0 = [&](int64_t s, int64_t p) -> C {
-        const double bn = a.bnorm[s];
-        const double bscale = (bn > 0.0) ? 1.0 / bn : 1.0;
-        return from_c128<C>((a.rscale[s * np + p] * bscale) * a.b[s * np + p]);
-    };
-
     if (w == kTmaConsumerWarps + 1) {
         // ------------------------------------------------------------------ dependency checker
         // Runs ahead of the consumers through the CTA's tiles: waits (bounded, one lane
@@ -325,31 +362,28 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
         int k = 0;
         TileJob t;
         for (int64_t g = blockIdx.x; g < total; g += gridDim.x) {
-            decode_tile(g, k, st_begin, lv_s, L, ntile, t);
+            decode_tile(g, k, st_begin, lv_s, L, tiles, S, t);
             const int64_t s = t.s;
             if (live(s)) {
                 // the counters this tile needs (at most three), one lane waiting on each
-                const int *d0 = nullptr, *d1 = nullptr, *d2 = nullptr;
+                int sid = -1;
+                int64_t blk = t.blk;
                 if (t.kind == 0) {
-                    if (t.l > 0) d0 = ctr(s, L + t.l - 1, t.blk);
+                    if (t.l > 0 && lane == 0) sid = L + t.l - 1;
                 } else if (t.kind == 1) {
                     const int64_t st = lv_s[t.l].stride;
-                    if (t.hasl) d0 = ctr(s, t.l, t.blk - st);
-                    if (t.hasr) d1 = ctr(s, t.l, t.blk + st);
-                    if (t.l > 0) d2 = ctr(s, L + t.l - 1, t.blk);
+                    if (lane == 0 && t.hasl) { sid = t.l; blk = t.blk - st; }
+                    if (lane == 1 && t.hasr) { sid = t.l; blk = t.blk + st; }
+                    if (lane == 2 && t.l > 0) sid = L + t.l - 1;
                 } else if (t.kind == 2) {
-                    if (L > 0) d0 = ctr(s, 2 * L - 1, 0);
-                } else if (t.kind == 4) {
-                    d0 = xready(s, t.vblk[0]);
-                    if (t.hasr) d1 = xready(s, t.vblk[1]);
-                } else if (t.l == 0) {
-                    d0 = ctr(s, 3 * L + 1, t.blk);
-                } else {
-                    d0 = xready(s, t.vblk[0]);
-                    if (t.nmat > 1) d1 = xready(s, t.vblk[1]);
+                    if (L > 0 && lane == 0) { sid = 2 * L - 1; blk = 0; }
+                } else if (t.kind == 3 && t.l == 0) {
+                    if (lane == 0) sid = 3 * L + 1;
+                } else if (lane == 0 || (lane == 1 && t.hasr)) {   // E_0, C_l: x of the neighbours
+                    blk = lane == 0 ? t.vblk[0] : t.vblk[1];
+                    sid = xstage(blk);
                 }
-                const int *mine = lane == 0 ? d0 : (lane == 1 ? d1 : (lane == 2 ? d2 : nullptr));
-                if (mine) wait_count(mine, ntile, a.err);
+                if (sid >= 0) wait_count(ctr(s, sid, blk), tiles[sid], a.err);
                 __syncwarp();
             }
             if (lane == 0) st_release_cta(&ready, (long long)g);
@@ -373,8 +407,10 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
     int k = 0;
     TileJob t;
     int64_t i = 0;
+    int64_t scaled = -1;     // the shift of bscale (an FP64 division, kept off the tiles' path)
+    double bscale = 1.0;
     for (int64_t g = blockIdx.x; g < total; g += gridDim.x, ++i) {
-        decode_tile(g, k, st_begin, lv_s, L, ntile, t);
+        decode_tile(g, k, st_begin, lv_s, L, tiles, S, t);
         const int64_t s = t.s;
         const int sid = t.kind == 0 ? t.l
                       : (t.kind == 1 ? L + t.l : (t.kind == 2 ? 2 * L : (t.kind == 3 ? 2 * L + 1 + t.l : 3 * L + 1)));
@@ -395,22 +431,30 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
                 ecol[u] = in ? __ldg(a.ell_col + ebase + (int64_t)kk * 32) : -1;
                 eval[u] = in ? ldg(ellv + ebase + (int64_t)kk * 32) : czero<C>();
             }
+            // rows this tile writes; the right-hand side does not depend on the sweep
+            const int r = t.r0 + (t.low ? lane & 7 : lane);
+            const int64_t p = t.blk * S + r;
+            const bool wr = w == 0 && r < S && !(t.low && lane >= kLowRows);
+            C zf = czero<C>();
+            double2 prev = mk(0.0, 0.0);
+            const bool from_b = (t.kind == 0 && t.l == 0) || (t.kind == 2 && L == 0);
+            if ((from_b || ell) && scaled != s) {
+                const double bn = a.bnorm[s];
+                bscale = (bn > 0.0) ? 1.0 / bn : 1.0;
+                scaled = s;
+            }
+            if (wr && ell) zf = from_c128<C>((a.rscale[s * np + p] * bscale) * a.b[s * np + p]);
             if (lane == 0) {
                 // the checker has seen this tile's inputs complete (acquire; __syncwarp
                 // orders the rest of the warp after this lane)
                 unsigned spins = 0;
                 while (ld_acquire_cta(&ready) < (long long)g) {
                     if (++spins > KORE_SPIN_LIMIT) { atomicCAS(a.err, 0, KORE_DEVERR_FLAG); break; }
-                    __nanosleep(16);
+                    if (spins > 64) __nanosleep(16);
                 }
             }
             __syncwarp();
-            // rows this tile writes, and what the write combines with (read early)
-            const int r = t.r0 + lane;
-            const int64_t p = t.blk * S + r;
-            const bool wr = w == 0 && r < S;
-            C zf = czero<C>();
-            double2 prev = mk(0.0, 0.0);
+            // what the write combines with (read early)
             if (wr) {
                 if (t.kind == 1 && t.l > 0) zf = ldcg(vec(a.f, s) + p);
                 else if (t.kind == 3 && t.l > 0) zf = ldcg(vec(a.z, s) + p);
@@ -420,10 +464,8 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
                 // this warp's slice of the input vectors: columns ch kCols + w kCpw + u
                 const C *src = (t.kind == 0 || t.kind == 2 || (t.kind == 3 && t.l == 0))
                                    ? vec(a.f, s) : (t.kind == 1 ? vec(a.z, s) : vec(a.x, s));
-                const bool from_b = (t.kind == 0 && t.l == 0) || (t.kind == 2 && L == 0);
-                const double bn = a.bnorm[s];
-                const double bscale = (bn > 0.0) ? 1.0 / bn : 1.0;
-                const int per = nc * kCpw, ne = t.nmat * per;
+                const int per = nvec / kTmaConsumerWarps;   // zeros past S: the chunks reach there
+                const int ne = t.nmat * per;
                 const int64_t vb0 = t.vblk[0] * S, vb1 = t.vblk[1] * S;
                 for (int e0 = 0; e0 < ne; e0 += 32 * kFill) {
                     C v[kFill];
@@ -432,7 +474,9 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
                     for (int u = 0; u < kFill; ++u) {
                         const int e = e0 + u * 32 + lane;
                         const int m = e >= per ? 1 : 0, rem = e - m * per;
-                        const int c = (rem / kCpw) * kCols + w * kCpw + rem % kCpw;
+                        // low tiles of complex128: runs of kCols columns, 4 kCols apart
+                        const int c = t.low && kSplit ? (rem / kCols) * 4 * kCols + w * kCols + rem % kCols
+                                            : (rem / kRun) * 4 * kRun + w * kRun + rem % kRun;
                         cv[u] = (e < ne) ? m * nvec + c : -1;
                         v[u] = czero<C>();
                         if (e < ne && c < S) {
@@ -461,19 +505,43 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
 #pragma unroll
                 for (int m = 0; m < 2; ++m) {
                     if (m >= t.nmat) break;
-                    const C *vv = vbuf + m * nvec + w * kCpw;
-                    for (int ch = 0; ch < nc; ++ch) {
+                    // the warp's columns of a chunk; in low tiles of complex128 column
+                    // w kCols + 4 u + lane / 8
+                    const bool split = t.low && kSplit;
+                    const C *vv = vbuf + m * nvec;
+                    const int cols = t.low ? 4 * kCols : kCols;
+                    for (int ch = 0; ch * cols < S; ++ch) {
                         if (!mbar_wait(&full[slot], ph)) atomicCAS(a.err, 0, KORE_DEVERR_FLAG);
-                        const C *bc = reinterpret_cast<const C *>(ring + (size_t)slot * CHUNK) +
-                                      w * kCpw * kTileRows + lane;
-                        const C *vc = vv + ch * kCols;
+                        const C *cb = reinterpret_cast<const C *>(ring + (size_t)slot * CHUNK);
+                        const C *vc = vv + ch * cols;
+                        if (split) {
+                            const C *bc = cb + w * kCpw * kTileRows + lane;
+                            vc += w * kCols + (lane >> 3);
 #pragma unroll
-                        for (int u = 0; u < kCpw; ++u) acc = cfma(acc, bc[u * kTileRows], vc[u]);
+                            for (int u = 0; u < kCpw; ++u) acc = cfma(acc, bc[u * kTileRows], vc[4 * u]);
+                        } else if (t.low) {
+#pragma unroll
+                            for (int h = 0; h < kCols / kRun; ++h) {
+                                const int c0 = (4 * h + w) * kRun;
+                                const C *bc = cb + c0 * kLowRows + (lane & 7);
+#pragma unroll
+                                for (int u = 0; u < kRun; ++u) acc = cfma(acc, bc[u * kLowRows], vc[c0 + u]);
+                            }
+                        } else if (!kHalf || (ch & 1) == (w >> 1)) {
+                            const int c0 = kHalf ? (w & 1) * kRun : w * kRun;
+                            const C *bc = cb + c0 * kTileRows + lane;
+#pragma unroll
+                            for (int u = 0; u < kRun; ++u) acc = cfma(acc, bc[u * kTileRows], vc[c0 + u]);
+                        }
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&empty[slot]);
                         if (++slot == (uint32_t)nst) { slot = 0; ph ^= 1; }
                     }
                 }
+            }
+            if (t.low && kSplit) {   // the four column classes of a row
+                acc = acc + shfl_xor(acc, 8);
+                acc = acc + shfl_xor(acc, 16);
             }
             rd[w][lane] = acc;
             named_sync(1, kTmaConsumers);
@@ -482,7 +550,7 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
 #pragma unroll
                 for (int q = 0; q < kTmaConsumerWarps; ++q) val = val + rd[q][lane];
                 if (wr) {
-                    if (ell) stcg(vec(a.f, s) + p, rhs0(s, p) - val);
+                    if (ell) stcg(vec(a.f, s) + p, zf - val);
                     else if (t.kind == 0) stcg(vec(a.z, s) + p, val);
                     else if (t.kind == 1) stcg(vec(a.f, s) + p, zf - val);
                     else if (t.kind == 2 || t.l == 0) emit(s, p, val, prev);
@@ -492,10 +560,7 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
         }
         if (w == 0) {
             __syncwarp();
-            if (lane == 0) {
-                __threadfence();
-                atomicAdd(done, 1);
-            }
+            if (lane == 0) signal_count(done);
         }
     }
 }
@@ -729,7 +794,7 @@ __global__ void k_scatter(int64_t np, int64_t n, const int64_t *__restrict__ s2o
 template <typename C>
 size_t tma_smem(int S, int nst, int chunk) {
     const int kCols = chunk / (kTileRows * (int)sizeof(C));
-    const int nvec = ((S + kCols - 1) / kCols) * kCols;
+    const int nvec = (S + 4 * kCols - 1) / (4 * kCols) * (4 * kCols);
     return (size_t)nst * chunk + 2 * (size_t)nst * sizeof(uint64_t) + 2 * (size_t)nvec * sizeof(C);
 }
 
@@ -753,6 +818,13 @@ SweepArgs sweep_args(const kore_plan *p, int nshift) {
     return a;
 }
 
+// Largest number of 32-row tiles of a stage that takes 8-row tiles (kLowRows).  A lone tile
+// of complex128 fills its SM's FP64 pipe, so splitting pays while there are fewer tiles than
+// SMs; complex64 tiles wait on their chunks and still gain with two per SM.  Whole solves
+// with limits 0, 40, 76, 101, 152 and 304: 72k shell in complex128 918, 771, 756, 742, 721,
+// 730 us; 240k shell in complex64 (7 sweeps) 5.26, 5.06, 4.98, 4.98, 4.90, 4.88 ms.
+int sweep_low_tiles(const kore_plan *p) { return p->prec == KORE_PREC_FP64 ? p->num_sms : 2 * p->num_sms; }
+
 // Tensor maps, ring depth and the cooperative launch of the k_sweep_tma variant v (CTAs
 // per SM, chunk bytes); the completion counters a.cnt are zeroed first.
 template <typename C>
@@ -764,11 +836,15 @@ int launch_sweep(const kore_plan *p, const SweepArgs &a, cudaStream_t st, TmaVar
     if (v.chunk != 8192 && v.chunk != 16384) return KORE_EINVAL;
     const int kCols = v.chunk / (kTileRows * (int)sizeof(C));
     const int ns = a.nshift;
-    KORE_TRY(kore_encode_block_map(&P.maps[kMapDinv], p->d_Dinv, rb, p->S, p->K, ns, p->f_stride(), kTileRows, kCols));
-    KORE_TRY(kore_encode_block_map(&P.maps[kMapG], p->d_Gm, rb, p->S, p->K, ns, p->f_stride(), kTileRows, kCols));
-    KORE_TRY(kore_encode_block_map(&P.maps[kMapH], p->d_Hm, rb, p->S, p->K, ns, p->f_stride(), kTileRows, kCols));
-    KORE_TRY(kore_encode_block_map(&P.maps[kMapLU], p->d_LU, rb, p->S, p->lu_mats, ns, p->lu_stride(), kTileRows,
-                                   kCols));
+    for (int low = 0; low < 2; ++low) {
+        const int rows = low ? kLowRows : kTileRows, cols = low ? 4 * kCols : kCols, o = 4 * low;
+        KORE_TRY(kore_encode_block_map(&P.maps[o + kMapDinv], p->d_Dinv, rb, p->S, p->K, ns, p->f_stride(), rows, cols));
+        KORE_TRY(kore_encode_block_map(&P.maps[o + kMapG], p->d_Gm, rb, p->S, p->K, ns, p->f_stride(), rows, cols));
+        KORE_TRY(kore_encode_block_map(&P.maps[o + kMapH], p->d_Hm, rb, p->S, p->K, ns, p->f_stride(), rows, cols));
+        KORE_TRY(kore_encode_block_map(&P.maps[o + kMapLU], p->d_LU, rb, p->S, p->lu_mats, ns, p->lu_stride(), rows,
+                                       cols));
+    }
+    P.low_tiles = sweep_low_tiles(p);
     // ring depth: as many slots as fit cps CTAs in the SM's shared memory
     int smem_sm = 0, smem_blk = 0;
     KORE_CUDA_TRY(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, p->device));
