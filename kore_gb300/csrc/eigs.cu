@@ -484,7 +484,9 @@ __device__ __forceinline__ double warp_transpose_sum16(double (&v)[16], int lane
 
 // Target t: partial_t[b*nc + c] = sum over the CTA's rows of conj(V_t[:,c]) w_t for
 // c < ncol_t and, with with_norm, entry c = ncol_t = sum |w_t|^2 (nc = ncol_t + with_norm).
-// run (may be null): target t returns at once unless run[t] != 0.
+// run (may be null): target t returns at once unless run[t] != 0.  grid.z shares the chunks of
+// columns: with few rows the products of one SM's FP64 pipe are the time (1,920 rows, 40
+// columns: 28 us on 8 CTAs, 10 us with the chunks on CTAs of their own; the same sums).
 __global__ void __launch_bounds__(kDotThreads) k_mdot(int64_t np, TVec V, TVec w, double2 *__restrict__ partial0,
                                                       int with_norm, const int *__restrict__ run, TCols tc) {
     const int tg = blockIdx.y;
@@ -495,7 +497,7 @@ __global__ void __launch_bounds__(kDotThreads) k_mdot(int64_t np, TVec V, TVec w
     __shared__ double sm[kDotThreads / 32][2 * kDotChunk];
     const int ncol = tc.n[tg];
     const int nc = ncol + with_norm;
-    for (int c0 = 0; c0 < nc; c0 += kDotChunk) {
+    for (int c0 = blockIdx.z * kDotChunk; c0 < nc; c0 += gridDim.z * kDotChunk) {
         double2 acc[kDotChunk];
 #pragma unroll
         for (int t = 0; t < kDotChunk; ++t) acc[t] = mk(0.0, 0.0);
@@ -583,6 +585,31 @@ __global__ void k_mgs_update(int64_t np, TVec V, const double2 *__restrict__ h0,
         for (int c = 0; c < ncol; ++c) acc = cfms(acc, Vt[r + (int64_t)c * np], hs[c]);
         wt[r] = acc;
     }
+}
+
+// The same for few rows: a thread per real or imaginary part, so that twice as many warps,
+// on SMs of their own, share the FP64 work (the same operations in the same order).
+__global__ void __launch_bounds__(128) k_mgs_update_parts(int64_t np, TVec V, const double2 *__restrict__ h0, TVec w,
+                                                          const int *__restrict__ run, TCols tc) {
+    const int tg = blockIdx.y;
+    if (!in_mask(tc.mask, tg) || (run && run[tg] == 0)) return;
+    const double2 *__restrict__ Vt = V.p[tg];
+    double *__restrict__ wt = reinterpret_cast<double *>(w.p[tg]);
+    const int ncol = tc.n[tg];
+    __shared__ double2 hs[kMaxNcv + 1];
+    for (int c = threadIdx.x; c < ncol; c += blockDim.x) hs[c] = h0[tg * kHStride + c];
+    __syncthreads();
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= 2 * np) return;
+    const int64_t r = i >> 1;
+    const bool im = i & 1;
+    double acc = wt[i];
+#pragma unroll 8
+    for (int c = 0; c < ncol; ++c) {
+        const double2 v = Vt[r + (int64_t)c * np], h = hs[c];
+        acc = fma(-v.x, im ? h.y : h.x, fma(im ? -v.y : v.y, im ? h.x : h.y, acc));
+    }
+    wt[i] = acc;
 }
 
 // partial_t[b] = sum of |w_t|^2 over CTA b's rows (grid.y = target)
@@ -712,6 +739,8 @@ __global__ void k_copy_vecs(int64_t np, TVec src, TVec dst, unsigned mask) {
 
 // Target t: Vout_t[:, c] = V_t[:, 0:m_t] G_t[:, c] for c < ncol_t, with m_t = tc.n[t],
 // ncol_t = tc.j[t] and G_t column-major with leading dimension tc.ld[t].
+// grid.z shares the chunks of columns (few rows: as k_mdot; 1,920 rows, 40 vectors: 208 us
+// on 8 CTAs, 80 us with the chunks on CTAs of their own).
 constexpr int kGemmChunk = 8;
 __global__ void k_gemm_vg(int64_t np, TVec V, TVec G, TVec Vout, TCols tc) {
     const int tg = blockIdx.y;
@@ -721,7 +750,7 @@ __global__ void k_gemm_vg(int64_t np, TVec V, TVec G, TVec Vout, TCols tc) {
     const double2 *__restrict__ Gt = G.p[tg];
     double2 *__restrict__ Vo = Vout.p[tg];
     __shared__ double2 gs[kMaxNcv * kGemmChunk];
-    for (int c0 = 0; c0 < ncol; c0 += kGemmChunk) {
+    for (int c0 = blockIdx.z * kGemmChunk; c0 < ncol; c0 += gridDim.z * kGemmChunk) {
         __syncthreads();
         for (int idx = threadIdx.x; idx < m * kGemmChunk; idx += blockDim.x) {
             const int j = idx % m, t = idx / m;
@@ -904,6 +933,23 @@ int apply_op(Ctx &c, const TVec &v, unsigned mask, const double *shift_tols = nu
     return kore_apply_inverse(p, c.t1, c.w, c.refine_tol, mask, shift_tols);
 }
 
+// CTAs of a tall-skinny kernel along its chunks of columns: as many as keep two CTAs per SM
+// busy when the rows alone do not.
+unsigned chunk_grid(const Ctx &c, int chunks) {
+    const unsigned want = kore_div_up(2LL * c.p->num_sms, (long long)c.grid * c.T);
+    return std::max(1u, std::min((unsigned)chunks, want));
+}
+
+// w_t -= V_t h_t
+void mgs_update(Ctx &c, const TVec &V, const double2 *h, const TVec &w, const int *run, const TCols &tc) {
+    // one warp per SM sub-partition at most: below that the component form is the faster
+    if (2 * c.np * c.T <= 128LL * 4 * c.p->num_sms)
+        k_mgs_update_parts<<<dim3(kore_div_up(2 * c.np, 128), c.T), 128, 0, c.p->stream>>>(c.np, V, h, w, run, tc);
+    else
+        k_mgs_update<<<dim3(c.grid, c.T), 256, 0, c.p->stream>>>(c.np, V, h, w, run, tc);
+    KORE_LAUNCHED(1);
+}
+
 // For each target t in tc.mask: orthogonalise w_t against V_t[:, 0:ncol_t] (classical
 // Gram-Schmidt with refinement if needed), write h and beta into column j_t of Hbar_t and
 // set V_t[:, j_t + 1] = w_t / beta.
@@ -916,17 +962,18 @@ int orthonormalise(Ctx &c, const TVec &V, const TCols &tc) {
     const TVec w = contiguous(c.w, c.T, c.np);
     double2 *h1 = c.h, *h2 = c.h + (kMaxNcv + 1);
     const dim3 g2(c.grid, c.T);
+    const dim3 g3(c.grid, c.T, chunk_grid(c, kore_div_up(nmax + 1, kDotChunk)));
     // first pass, with ||w||^2 as entry ncol of h1
-    k_mdot<<<g2, kDotThreads, 0, p->stream>>>(c.np, V, w, c.partial, 1, nullptr, tc);
+    k_mdot<<<g3, kDotThreads, 0, p->stream>>>(c.np, V, w, c.partial, 1, nullptr, tc);
     k_mdot_reduce<<<dim3(nmax + 1, c.T), 256, 0, p->stream>>>((int)c.grid, c.partial, kPartStride, h1, 0, nullptr,
                                                                tc, 1);
-    k_mgs_update<<<g2, 256, 0, p->stream>>>(c.np, V, h1, w, nullptr, tc);
+    mgs_update(c, V, h1, w, nullptr, tc);
     k_refine_decide<<<c.T, 256, 0, p->stream>>>(c.h, c.run2, tc);
     // second pass if needed
-    k_mdot<<<g2, kDotThreads, 0, p->stream>>>(c.np, V, w, c.partial, 0, c.run2, tc);
+    k_mdot<<<g3, kDotThreads, 0, p->stream>>>(c.np, V, w, c.partial, 0, c.run2, tc);
     k_mdot_reduce<<<dim3(nmax, c.T), 256, 0, p->stream>>>((int)c.grid, c.partial, kPartStride, h2, 0, c.run2, tc, 0);
-    k_mgs_update<<<g2, 256, 0, p->stream>>>(c.np, V, h2, w, c.run2, tc);
-    KORE_LAUNCHED(7);
+    mgs_update(c, V, h2, w, c.run2, tc);
+    KORE_LAUNCHED(5);
     // h = h1 + h2
     k_mdot_reduce<<<dim3(nmax, c.T), 32, 0, p->stream>>>(1, h2, kHStride, h1, 1, nullptr, tc, 0);
     k_nrm2_partial<<<g2, 256, 0, p->stream>>>(c.np, w, c.dpart, tc.mask);
@@ -1191,9 +1238,10 @@ int begin_purify(Run &r, int s, const double2 *theta) {
     for (int u = 0; u < kMaxTargets; ++u) a.p[u] = b.p[u] = d.p[u] = nullptr;
     // G = Q Y[:, 0:nout] (m x nout) into T's storage, then X = V G
     a.p[s] = c.Q + s * kSqStride; b.p[s] = c.Y + s * kSqStride; d.p[s] = c.Tm + s * kSqStride;
-    k_gemm_vg<<<dim3(1, r.T), 256, 0, p->stream>>>(x.m, a, b, d, gc);
+    const unsigned gz = chunk_grid(c, kore_div_up(x.nout, kGemmChunk));
+    k_gemm_vg<<<dim3(1, r.T, gz), 256, 0, p->stream>>>(x.m, a, b, d, gc);
     a.p[s] = x.V; b.p[s] = c.Tm + s * kSqStride; d.p[s] = x.Vt;
-    k_gemm_vg<<<dim3(c.grid, r.T), 256, 0, p->stream>>>(c.np, a, b, d, gc);
+    k_gemm_vg<<<dim3(c.grid, r.T, gz), 256, 0, p->stream>>>(c.np, a, b, d, gc);
     KORE_LAUNCHED(2);
     x.phase = 1;
     x.k = 0;
@@ -1447,7 +1495,10 @@ int kore_eigs_engine(kore_plan *p, EigsSource *src, bool *valid, int max_ncv) {
         }
         if (rc.mask) {
             if (p->prof) KORE_TRY(kore_prof_mark(p, 4, true));
-            k_gemm_vg<<<dim3(c.grid, T), 256, 0, p->stream>>>(np, rV, rQ, rOut, rc);
+            int kmax = 0;
+            for (int s = 0; s < T; ++s) kmax = std::max(kmax, rc.j[s]);
+            k_gemm_vg<<<dim3(c.grid, T, chunk_grid(c, kore_div_up(kmax, kGemmChunk))), 256, 0, p->stream>>>(np, rV, rQ, rOut,
+                                                                                                         rc);
             k_copy_vecs<<<dim3(c.grid, T), 256, 0, p->stream>>>(np, rSrc, rDst, rc.mask);
             TCols hc = rc;
             for (int s = 0; s < T; ++s) { hc.n[s] = rc.j[s]; hc.ld[s] = r.sl[s].m + 1; }
