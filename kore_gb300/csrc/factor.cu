@@ -710,11 +710,11 @@ namespace {
 // (Re)allocate the per-shift buffers for `cap` shifts of elements of `elt` bytes.
 int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
     if (p->factor_elt == elt && p->shift_cap >= cap) return KORE_OK;
-    void **bufs[] = {&p->d_Dinv, &p->d_Gm, &p->d_Hm, &p->d_Dw, &p->d_LU, &p->d_T, &p->d_zlo, &p->d_xlo, &p->d_flo,
+    void **bufs[] = {&p->d_Dinv, &p->d_Gm, &p->d_Hm, &p->d_Dw, &p->d_LU, &p->d_T, &p->d_sweep,
                      (void **)&p->d_rscale, (void **)&p->d_piv, (void **)&p->d_used,
                      (void **)&p->d_sigma, (void **)&p->d_minf, (void **)&p->d_bb, (void **)&p->d_xb, (void **)&p->d_rb,
                      (void **)&p->d_bn, (void **)&p->d_rn, (void **)&p->d_part, (void **)&p->d_ir,
-                     (void **)&p->d_cnt, &p->d_ell_val, &p->d_tctab, &p->d_oz};
+                     &p->d_ell_val, &p->d_tctab, &p->d_oz};
     for (void **b : bufs) {
         if (*b) cudaFree(*b);
         *b = nullptr;
@@ -732,9 +732,7 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
     KORE_TRY(kore_alloc(p, &p->d_Dw, c * p->f_stride() * elt));
     KORE_TRY(kore_alloc(p, &p->d_LU, c * p->lu_stride() * elt));
     KORE_TRY(kore_alloc(p, &p->d_T, c * p->nodd_max * p->t_block(elt) * elt));
-    KORE_TRY(kore_alloc(p, &p->d_zlo, c * p->np * elt));
-    KORE_TRY(kore_alloc(p, &p->d_xlo, c * p->np * elt));
-    KORE_TRY(kore_alloc(p, &p->d_flo, c * p->np * elt));
+    KORE_TRY(kore_alloc(p, &p->d_sweep, c * p->sweep_vec_elems() * elt));
     KORE_TRY(kore_alloc(p, (void **)&p->d_rscale, c * p->np * sizeof(double)));
     KORE_TRY(kore_alloc(p, (void **)&p->d_piv, c * p->p_stride() * sizeof(int)));
     KORE_TRY(kore_alloc(p, (void **)&p->d_used, c * p->p_stride() * sizeof(int)));
@@ -748,7 +746,6 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
     // per-CTA maxima of the residual products: (np / 64 + np / 8 + 2) CTAs at most, 2 each
     KORE_TRY(kore_alloc(p, (void **)&p->d_part, c * 2 * (size_t)(p->np / 64 + p->np / 8 + 1024) * sizeof(double)));
     KORE_TRY(kore_alloc(p, (void **)&p->d_ir, c * sizeof(IrState)));
-    KORE_TRY(kore_alloc(p, (void **)&p->d_cnt, c * (size_t)p->sweep_stages() * p->K * sizeof(int)));
     KORE_TRY(kore_alloc(p, &p->d_ell_val, c * std::max<int64_t>(p->ell_stride(), 1) * elt));
     if (elt == sizeof(float2)) KORE_TRY(kore_alloc(p, &p->d_tctab, (size_t)kore_tc_table_bytes(p, cap)));
     else {

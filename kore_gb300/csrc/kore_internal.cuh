@@ -130,14 +130,18 @@ struct kore_plan {
     int64_t t_stride() const { return nodd_max * t_block(factor_elt); }
     int64_t p_stride() const { return (int64_t)nodd_max * S; }
     int64_t ell_stride() const { return ell_rows * ell_w; }
-    // stages of one sweep: A_l, B_l (l < nlev), the top block, C_l (nlev > l >= 1), E_0, C_0
-    int sweep_stages() const { return nlev > 0 ? 3 * nlev + 2 : 1; }
+    // entries of one shift's sweep vectors: z, x, g (np each) and f of every level >= 1
+    int64_t sweep_vec_elems() const {
+        int64_t f = 0;
+        for (const BcrLevel &l : lev) f += l.neven;
+        return 3 * np + f * S;
+    }
 
     // solve workspace (padded, complex128 unless noted)
     double2 *d_v[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     // per shift (shift_cap sets of np): sweep vectors in factor precision, and the
     // complex128 right-hand side, solution and residual of a batched solve
-    void *d_zlo = nullptr, *d_xlo = nullptr, *d_flo = nullptr;
+    void *d_sweep = nullptr;
     double2 *d_bb = nullptr, *d_xb = nullptr, *d_rb = nullptr;
     double *d_bn = nullptr, *d_rn = nullptr;   // per-shift ||b||_inf and ||r||_inf
     double *d_red = nullptr;          // reduction scratch (8192 doubles)
@@ -145,7 +149,6 @@ struct kore_plan {
     double *h_red = nullptr;          // pinned host mirror
     int *d_err = nullptr;
     int *d_flag = nullptr;            // a solve's non-finite flag
-    int *d_cnt = nullptr;             // sweep completion counters (shift_cap x sweep_stages() x K)
     IrState *d_ir = nullptr;          // one per shift
 
     // Krylov-Schur workspace (per target: basis and restart buffer of ncv + 1 columns)

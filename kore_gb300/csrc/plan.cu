@@ -94,9 +94,9 @@ void free_plan(kore_plan *p) {
     p->ev_pool.clear();
     void *ptrs[] = {p->d_arow, p->d_acol, p->d_asplit, p->d_aval, p->d_brow, p->d_bcol, p->d_bval,
                     p->d_slot2orig, p->d_bsz, p->d_Dinv, p->d_Gm, p->d_Hm, p->d_Dw, p->d_LU, p->d_lev,
-                    p->d_rscale, p->d_T, p->d_piv, p->d_used, p->d_zlo, p->d_xlo, p->d_flo,
+                    p->d_rscale, p->d_T, p->d_piv, p->d_used, p->d_sweep,
                     p->d_red, p->d_part, p->d_err, p->d_flag, p->d_ir, p->d_V, p->d_Vtmp, p->d_ksx, p->d_small, p->d_warm,
-                    p->d_sigma, p->d_minf, p->d_bb, p->d_xb, p->d_rb, p->d_bn, p->d_rn, p->d_cnt,
+                    p->d_sigma, p->d_minf, p->d_bb, p->d_xb, p->d_rb, p->d_bn, p->d_rn,
                     p->d_ell_col, p->d_ell_src, p->d_ell_val, p->d_long_rows, p->d_srow, p->d_smid,
                     p->d_scol, p->d_sval, p->d_cc_ptr, p->d_cc_row, p->d_cc_src, p->d_tctab, p->d_oz};
     for (void *q : ptrs)
@@ -608,11 +608,11 @@ int kore_plan_estimate_bytes(const kore_pencil_desc *d, int precision, int nshif
     b += (np + 1) * 4 + nb * 12;
     b += np * 8 + K * 4 + nlev * (int64_t)sizeof(BcrLevel) + 6 * np * 16 + 8192 * 8 + 1024;
     // factors and solve workspace of c shifts
-    b += c * (4 * K * SS * e + lu * SS * e + nodd_max * (e == 8 ? 2 : 1) * SS * e + 3 * np * e + np * 8 + 2 * nodd_max * S * 4);
+    b += c * (4 * K * SS * e + lu * SS * e + nodd_max * (e == 8 ? 2 : 1) * SS * e + (4 * np + nlev * S) * e + np * 8 + 2 * nodd_max * S * 4);
     // level-0 couplings by column; job table of the tensor-core products
     b += (2 * (K / 2 + 1) * (S + 1) + 2 * na) * 4;
     b += precision == KORE_PREC_MIXED ? c * (3 * (K + 1) * 48 + 64) : kore_oz_workspace_bytes((int)S, K, c);
-    b += c * (3 * np * 16 + 2 * (np / 64 + np / 8 + 1024) * 8 + (nlev > 0 ? 3 * nlev + 2 : 1) * K * 4 + ell * e + 128);
+    b += c * (3 * np * 16 + 2 * (np / 64 + np / 8 + 1024) * 8 + ell * e + 128);
     b += 2 * d->n * c * 16;   // kore_solve's device copies of b and x
     // per target (one per shift): Krylov basis, its restart copy, a gathered input vector,
     // the slot's warm-start vector and the projected-problem workspace

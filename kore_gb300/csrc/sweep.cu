@@ -29,12 +29,8 @@
 
 namespace {
 
-__device__ __forceinline__ double2 ldcg(const double2 *p) { return __ldcg(p); }
-__device__ __forceinline__ float2 ldcg(const float2 *p) { return __ldcg(p); }
 __device__ __forceinline__ double2 ldg(const double2 *p) { return __ldg(p); }
 __device__ __forceinline__ float2 ldg(const float2 *p) { return __ldg(p); }
-__device__ __forceinline__ void stcg(double2 *p, double2 v) { __stcg(p, v); }
-__device__ __forceinline__ void stcg(float2 *p, float2 v) { __stcg(p, v); }
 template <typename C> __device__ __forceinline__ C shfl_xor(C v, int o) {
     v.x = __shfl_xor_sync(0xffffffffu, v.x, o);
     v.y = __shfl_xor_sync(0xffffffffu, v.y, o);
@@ -53,10 +49,11 @@ struct SweepArgs {
     const double2 *b;                // nshift x np right-hand sides (complex128, padded)
     const double *rscale;            // nshift x np
     const double *bnorm;             // nshift scalings
-    void *f, *z, *x;                 // nshift x np reduction vectors (factor precision)
+    void *vecs;                      // per shift the sweep's vectors (sweep_vec_elems), all bits set
+                                     // before the launch
+    int64_t vec_stride;
     double2 *out;                    // nshift x np
     int accumulate;
-    int *cnt;                        // completion counters: nshift x stages x K, zeroed before the launch
     int *err;
     const int *skip;                 // shift s is skipped when skip[s * skip_stride] != 0
     int skip_stride;
@@ -72,33 +69,53 @@ __host__ __device__ __forceinline__ bool mask_has(unsigned mask, int64_t s) {
     return s >= 32 || ((mask >> s) & 1u);
 }
 
-__device__ __forceinline__ void st_release_cta(long long *p, long long v) {
-    asm volatile("st.release.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(p)), "l"(v) : "memory");
+// An entry of the sweep's vectors is written once per sweep.  Before the sweep all its bits
+// are set, a NaN that no arithmetic produces, so a reader sees by the entry itself whether
+// it is there: no counter, fence or flag stands between a tile's result and its use.  The 8
+// bytes of a complex64 entry and each half of a complex128 one are written and read as one
+// access (relaxed, at L2), and a complex128 entry is there when both halves are.
+__device__ __forceinline__ void st_entry(float2 *p, float2 v) {
+    const unsigned long long b = (unsigned long long)__float_as_uint(v.x) | ((unsigned long long)__float_as_uint(v.y) << 32);
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(b) : "memory");
 }
-__device__ __forceinline__ long long ld_acquire_cta(const long long *p) {
-    long long v;
-    asm volatile("ld.acquire.cta.shared::cta.b64 %0, [%1];" : "=l"(v) : "r"(smem_u32(p)) : "memory");
+__device__ __forceinline__ void st_entry(double2 *p, double2 v) {
+    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v.x), "d"(v.y) : "memory");
+}
+__device__ __forceinline__ float2 ld_entry(const float2 *p) {
+    unsigned long long b;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(b) : "l"(p) : "memory");
+    return make_float2(__uint_as_float((unsigned)b), __uint_as_float((unsigned)(b >> 32)));
+}
+__device__ __forceinline__ double2 ld_entry(const double2 *p) {
+    double2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
     return v;
 }
-
-// One arrival at a completion counter, after this thread's (and, by the barrier before it,
-// its warp's) writes.
-__device__ __forceinline__ void signal_count(int *c) {
-    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(c) : "memory");
+__device__ __forceinline__ bool unset(float2 v) { return __float_as_uint(v.x) == 0xffffffffu; }
+__device__ __forceinline__ bool unset(double2 v) {
+    return __double_as_longlong(v.x) == -1ll || __double_as_longlong(v.y) == -1ll;
 }
 
-// A thread waits (bounded) until *c >= target; on timeout or an earlier error the
-// error flag is set and the caller goes on (its result is then wrong, but the kernel
-// ends).
-__device__ __forceinline__ void wait_count(const int *c, int target, int *err) {
-    unsigned spins = 0;
-    while (ld_relaxed_i32(c) < target) {
-        if (++spins < 32) continue;
-        if (ld_relaxed_i32(err) != 0) return;
-        if (spins > KORE_SPIN_LIMIT) { atomicCAS(err, 0, KORE_DEVERR_FLAG); return; }
-        __nanosleep(32);
+// Iteration limit of a wait for an entry (about a microsecond each): seconds.
+constexpr unsigned kEntryLimit = 1u << 22;
+
+// Reads (bounded) an entry until it is there; on timeout or an earlier error the error flag
+// is set and the caller goes on (its result is then wrong, but the kernel ends).
+template <typename C>
+__device__ __noinline__ C wait_entry_long(const C *p, int *err) {
+    C v = ld_entry(p);
+    for (unsigned spins = 0; unset(v); v = ld_entry(p)) {
+        if (ld_relaxed_i32(err) != 0) break;
+        if (++spins > kEntryLimit) { atomicCAS(err, 0, KORE_DEVERR_FLAG); break; }
+        __nanosleep(64);
     }
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");   // acquire: the producer's data is read after the counter
+    return v;
+}
+template <typename C>
+__device__ __forceinline__ C wait_entry(const C *p, int *err) {
+    C v = ld_entry(p);
+    for (int spins = 0; unset(v) && spins < 16; ++spins) v = ld_entry(p);
+    return unset(v) ? wait_entry_long(p, err) : v;
 }
 
 // ----------------------------------------------------------------------------- the sweep kernel
@@ -106,11 +123,17 @@ __device__ __forceinline__ void wait_count(const int *c, int target, int *err) {
 //     A_0, B_0, A_1, B_1, ..., A_{L-1}, B_{L-1}, top, C_{L-1}, ..., C_1, E_0, C_0
 // (A: z_j = D_j^-1 f_j, B: f_i -= L_i z_jl + U_i z_jr, C: x_j = z_j - G_j x_jl - H_j x_jr
 // at levels >= 1; E_0: g_j = c_j - L_j x_jl - U_j x_jr and C_0: x_j = D_j^-1 g_j)
-// and CTA c takes tiles c, c + G, c + 2G, ...  A tile reads only blocks whose counters
-// are complete (e.g. a B tile needs A of its two neighbours), and after its rows are
-// written 1 is added to the counter of (stage, block).  Tiles are taken in increasing
-// order by co-resident CTAs, so every wait is on a tile of a lower number that some
-// CTA is processing or has processed: no deadlock, and adjacent stages overlap.
+// and CTA c takes tiles c, c + G, c + 2G, ...  A tile waits for the entries it reads, each
+// written by a tile of a lower number (st_entry, wait_entry).  Tiles are taken in increasing
+// order by co-resident CTAs, so every wait is on a tile that some CTA is processing or has
+// processed: no deadlock, and adjacent stages overlap.  Per shift there are four vectors: z
+// and x (a block of each is written once), g (E_0), and f, which every level has its own copy
+// of (level l's active blocks, l >= 1; level 0's is the right-hand side), so that every entry
+// is written once.
+//
+// With completion counters (a fence and an atomic per tile, a checker warp that polled them
+// and told the consumers, then the loads) a stage of the chain spent 2.9 us of its 4 us between
+// one tile's result and the next tile's inputs.
 //
 // A tile of A, C, top or B at levels >= 1 reads one or two S x S blocks (stored
 // column-major); they are cut into chunks of 32 rows x kCols columns (16 KB) that one
@@ -118,10 +141,9 @@ __device__ __forceinline__ void wait_count(const int *c, int target, int *err) {
 // each slot guarded by a "full" mbarrier (completed by the copy) and an "empty"
 // mbarrier (one arrival per consumer warp).  The producer runs ahead through the CTA's
 // tile sequence: the factor data of later tiles does not depend on the sweep, so it is
-// fetched while the consumer warps wait for their input vectors.  A dependency-checker
-// warp also runs ahead and publishes in shared memory which tiles have their inputs
-// complete.  B_0 and E_0 read the level-0 couplings as padded rows (at most a few
-// dozen entries per row) with plain coalesced loads instead.
+// fetched while the consumer warps wait for their input vectors.  B_0 and E_0 read the level-0
+// couplings as padded rows (at most a few dozen entries per row) with plain coalesced loads
+// instead.
 constexpr int kTmaConsumerWarps = 4;
 constexpr int kTmaConsumers = 32 * kTmaConsumerWarps;
 // Variants: 2, 3 or 4 CTAs per SM (deeper rings per CTA, or more CTAs whose per-tile
@@ -132,7 +154,7 @@ constexpr int kTmaConsumers = 32 * kTmaConsumerWarps;
 struct TmaVariant { int cps, chunk; };
 constexpr TmaVariant kTmaVariants[] = {{2, 16384}, {3, 16384}, {4, 16384}, {2, 8192}, {3, 8192}, {4, 8192}};
 constexpr TmaVariant kTmaDefault = {4, 8192};
-constexpr int kTmaThreads = kTmaConsumers + 64;   // + one producer warp + one dependency-checker warp
+constexpr int kTmaThreads = kTmaConsumers + 32;   // + one producer warp
 constexpr int kTileRows = 32;
 // Stages with few tiles take tiles of 8 rows instead: a chunk then holds four times the
 // columns and four times as many SMs work on the stage.  These stages are the chain of the
@@ -147,7 +169,7 @@ constexpr int kEllReg = 4;   // level-0 coupling entries per thread held in regi
 // input-vector loads in flight per consumer lane: a two-matrix tile's slice (about 2 S / 4
 // entries per warp: 2 x 7 x 16 at S = 400 with 16 KB chunks, 2 x 13 x 8 with 8 KB) takes
 // one round of L2 latency with 8, two with 4; the variants whose register budget
-// (65536 / (192 CPS)) cannot hold 8 keep 4
+// (65536 / (160 CPS)) cannot hold 8 keep 4
 template <typename C, int CPS> constexpr int fill_of() { return (CPS == 2 || (CPS == 3 && sizeof(C) == 8)) ? 8 : 4; }
 
 enum { kMapDinv = 0, kMapG = 1, kMapH = 2, kMapLU = 3 };
@@ -166,86 +188,101 @@ template <typename C, int CHUNK> struct TmaShape {
 };
 
 // One tile of the sweep: stage kind (0 A, 1 B, 2 top, 3 C, 4 E_0), level, shift, block
-// of its rows, first row, and the blocks it multiplies (map, block index within the map).
+// of its rows, first row, the blocks it multiplies (map, block index within the map), and
+// the blocks of its vectors, as element offsets into the shift's vectors.
 struct TileJob {
     int kind, l, nmat, r0;
     bool low;            // 8 rows instead of 32
+    bool from_b;         // its input vector is the right-hand side
     int64_t s, blk;
     int map[2];
     int64_t mblk[2];
-    int64_t vblk[2];     // block of the vector each matrix multiplies
-    bool hasl, hasr;
+    int64_t in[2];       // the vector each matrix multiplies (E_0, B_0: in[0] the vector gathered from)
+    int64_t add;         // what the product is subtracted from (-1: nothing or the right-hand side)
+    int64_t out;
 };
 
-// Stage k of the tile order among the counters: A_l: l, B_l: L + l, top: 2 L, C_l: 2 L + 1 + l,
-// E_0: 3 L + 1.
-__device__ __forceinline__ int counter_of(int k, int L) {
-    if (k < 2 * L) return (k & 1) ? L + (k >> 1) : (k >> 1);
-    if (k == 2 * L) return 2 * L;
-    return k < 3 * L ? 2 * L + 1 + (3 * L - k) : k == 3 * L ? 3 * L + 1 : 2 * L + 1;
-}
+// Shapes that decode_tile needs, in shared memory.
+struct SweepShape {
+    int S, L, K;
+    BcrLevel lv[kMaxLevels];
+    int64_t begin[3 * kMaxLevels + 3];   // first tile of each stage
+    int tiles[3 * kMaxLevels + 2];       // tiles per block of each stage
+    int64_t fo[kMaxLevels + 1];          // element offset of level l's f (l >= 1)
+    int64_t x, g;                        // element offsets of x and g (z: 0)
+};
 
-// tiles: tiles per block of each counter's stage
-__device__ __forceinline__ void decode_tile(int64_t g, int &k, const int64_t *st_begin, const BcrLevel *lv_s, int L,
-                                            const int *tiles, int S, TileJob &t) {
-    while (g >= st_begin[k + 1]) ++k;
-    const int ntile = tiles[counter_of(k, L)];
-    const int64_t loc = g - st_begin[k];
+__device__ __forceinline__ void decode_tile(int64_t n, int &k, const SweepShape &h, TileJob &t) {
+    while (n >= h.begin[k + 1]) ++k;
+    const int L = h.L, ntile = h.tiles[k];
+    const int64_t S = h.S, loc = n - h.begin[k];
     if (k < 2 * L) { t.kind = (k & 1) ? 1 : 0; t.l = k >> 1; }
     else if (k == 2 * L) { t.kind = 2; t.l = L; }
     else if (k < 3 * L) { t.kind = 3; t.l = 3 * L - k; }
     else if (k == 3 * L) { t.kind = 4; t.l = 0; }
     else { t.kind = 3; t.l = 0; }
-    const int nblk = (t.kind == 1) ? lv_s[t.l].neven : (t.kind == 2 ? 1 : lv_s[t.l].nodd);
+    const int nblk = (t.kind == 1) ? h.lv[t.l].neven : (t.kind == 2 ? 1 : h.lv[t.l].nodd);
     t.s = loc / ((int64_t)nblk * ntile);
     const int64_t rem = loc - t.s * nblk * ntile;
     const int64_t bi = rem / ntile;
     t.low = ntile > (S + kTileRows - 1) / kTileRows;
     t.r0 = (int)(rem - bi * ntile) * (t.low ? kLowRows : kTileRows);
-    t.nmat = 0;
-    t.hasl = t.hasr = false;
+    t.nmat = 1;
+    t.from_b = false;
+    t.add = -1;
     if (t.kind == 0) {
-        const int64_t j = (2 * bi + 1) * lv_s[t.l].stride;
+        const int64_t q = 2 * bi + 1, j = q * h.lv[t.l].stride;
         t.blk = j;
-        t.map[0] = kMapDinv; t.mblk[0] = j; t.vblk[0] = j; t.nmat = 1;
+        t.map[0] = kMapDinv; t.mblk[0] = j;
+        t.from_b = t.l == 0;
+        t.in[0] = t.l == 0 ? 0 : h.fo[t.l] + q * S;
+        t.out = j * S;
     } else if (t.kind == 1) {
-        const BcrLevel lv = lv_s[t.l];
+        const BcrLevel lv = h.lv[t.l];
         const int64_t q = 2 * bi;
         t.blk = q * lv.stride;
-        t.hasl = q >= 1;
-        t.hasr = q + 1 < lv.Kl;
+        t.out = h.fo[t.l + 1] + bi * S;
         if (t.l > 0) {
             // L_q z_jl first when it exists, then U_q z_jr
+            const bool hasl = q >= 1, hasr = q + 1 < lv.Kl;
             const int64_t jl = (q - 1) * lv.stride, jr = (q + 1) * lv.stride;
             t.map[0] = t.map[1] = kMapLU;
-            t.mblk[0] = t.hasl ? lv.lu_L + q : lv.lu_U + q;
-            t.vblk[0] = t.hasl ? jl : jr;
+            t.mblk[0] = hasl ? lv.lu_L + q : lv.lu_U + q;
+            t.in[0] = (hasl ? jl : jr) * S;
             t.mblk[1] = lv.lu_U + q;
-            t.vblk[1] = jr;
-            t.nmat = (int)t.hasl + (int)t.hasr;
+            t.in[1] = jr * S;
+            t.nmat = (int)hasl + (int)hasr;
+            t.add = h.fo[t.l] + q * S;
+        } else {
+            t.nmat = 0;
+            t.in[0] = 0;   // z
         }
     } else if (t.kind == 2) {
         t.blk = 0;
-        t.map[0] = kMapDinv; t.mblk[0] = 0; t.vblk[0] = 0; t.nmat = 1;
+        t.map[0] = kMapDinv; t.mblk[0] = 0;
+        t.from_b = L == 0;
+        t.in[0] = L == 0 ? 0 : h.fo[L];
+        t.out = h.x;
     } else if (t.kind == 3 && t.l > 0) {
-        const BcrLevel lv = lv_s[t.l];
+        const BcrLevel lv = h.lv[t.l];
         const int64_t q = 2 * bi + 1, j = q * lv.stride;
         t.blk = j;
-        t.hasr = q + 1 < lv.Kl;
-        t.map[0] = kMapG; t.mblk[0] = j; t.vblk[0] = j - lv.stride; t.nmat = 1;
-        if (t.hasr) { t.map[1] = kMapH; t.mblk[1] = j; t.vblk[1] = j + lv.stride; t.nmat = 2; }
+        t.map[0] = kMapG; t.mblk[0] = j; t.in[0] = h.x + (j - lv.stride) * S;
+        if (q + 1 < lv.Kl) { t.map[1] = kMapH; t.mblk[1] = j; t.in[1] = h.x + (j + lv.stride) * S; t.nmat = 2; }
+        t.add = j * S;
+        t.out = h.x + j * S;
     } else if (t.kind == 3) {
-        // C_0: x_j = D_j^-1 g_j, g_j from E_0 in f
+        // C_0: x_j = D_j^-1 g_j
         const int64_t j = 2 * bi + 1;
         t.blk = j;
-        t.map[0] = kMapDinv; t.mblk[0] = j; t.vblk[0] = j; t.nmat = 1;
+        t.map[0] = kMapDinv; t.mblk[0] = j; t.in[0] = h.g + j * S;
+        t.out = h.x + j * S;
     } else {
         // E_0: g_j = c_j - L_j x_{j-1} - U_j x_{j+1} from the padded coupling rows
-        const int64_t q = 2 * bi + 1;
-        t.blk = q;
-        t.hasl = true;
-        t.hasr = q + 1 < lv_s[0].Kl;
-        t.vblk[0] = q - 1; t.vblk[1] = q + 1;
+        t.blk = 2 * bi + 1;
+        t.nmat = 0;
+        t.in[0] = h.x;
+        t.out = h.g + t.blk * S;
     }
 }
 
@@ -270,10 +307,7 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
     uint64_t *empty = full + nst;
     C *vbuf = reinterpret_cast<C *>(empty + nst);   // 2 x nvec input vectors (each warp fills its columns)
     __shared__ C red[2][kTmaConsumerWarps][33];   // per-warp partial sums, by tile parity
-    __shared__ BcrLevel lv_s[kMaxLevels];
-    __shared__ int64_t st_begin[3 * kMaxLevels + 2];
-    __shared__ int tiles[3 * kMaxLevels + 2];   // per block of a stage, by its counter
-    __shared__ long long ready;      // highest tile of this CTA whose inputs are complete
+    __shared__ SweepShape h;
     {
         bool all = true;
         for (int s = 0; s < ns; ++s)
@@ -285,40 +319,43 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
     const int64_t np = (int64_t)K * S;
     const int ntile = (S + kTileRows - 1) / kTileRows;
     const int nstage = L > 0 ? 3 * L + 2 : 1;
-    if (tid < L) lv_s[tid] = a.levs[tid];
+    if (tid < L) h.lv[tid] = a.levs[tid];
     if (tid == 0) {
         for (int i = 0; i < nst; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], kTmaConsumerWarps); }
         mbar_fence_init();
-        ready = -1;
     }
     if (tid == kTmaConsumers) for (int i = 0; i < 8; ++i) tma_prefetch_desc(&P.maps[i]);
     __syncthreads();
     if (tid == 0) {
+        h.S = S; h.L = L; h.K = K;
+        h.x = np;
+        h.g = 2 * np;
+        int64_t f = 3 * np;
+        for (int l = 1; l <= L; ++l) {
+            h.fo[l] = f;
+            f += (int64_t)h.lv[l - 1].neven * S;
+        }
         int64_t acc = 0;
         for (int k = 0; k < nstage; ++k) {
-            st_begin[k] = acc;
+            h.begin[k] = acc;
             int nblk;
-            if (k < 2 * L) nblk = (k & 1) ? lv_s[k >> 1].neven : lv_s[k >> 1].nodd;
+            if (k < 2 * L) nblk = (k & 1) ? h.lv[k >> 1].neven : h.lv[k >> 1].nodd;
             else if (k == 2 * L) nblk = 1;
-            else if (k < 3 * L) nblk = lv_s[3 * L - k].nodd;
-            else nblk = lv_s[0].nodd;   // E_0, C_0
+            else if (k < 3 * L) nblk = h.lv[3 * L - k].nodd;
+            else nblk = h.lv[0].nodd;   // E_0, C_0
             // the sparse stages B_0 and E_0 keep 32 rows
             const bool sparse = L > 0 && (k == 1 || k == 3 * L);
             const bool low = !sparse && nblk * ntile * ns <= P.low_tiles;
-            const int nt = low ? (S + kLowRows - 1) / kLowRows : ntile;
-            tiles[counter_of(k, L)] = nt;
-            acc += (int64_t)nblk * nt * ns;
+            h.tiles[k] = low ? (S + kLowRows - 1) / kLowRows : ntile;
+            acc += (int64_t)nblk * h.tiles[k] * ns;
         }
-        st_begin[nstage] = acc;
+        h.begin[nstage] = acc;
     }
     __syncthreads();
-    const int64_t total = st_begin[nstage];
+    const int64_t total = h.begin[nstage];
     auto live = [&](int64_t s) -> bool {
         return mask_has(a.live_mask, s) && !(a.skip && a.skip[s * a.skip_stride] != 0);
     };
-    auto ctr = [&](int64_t s, int sid, int64_t blk) -> int * { return a.cnt + ((s * nstage + sid) * K + blk); };
-    // counter of the stage that finishes x of a block
-    auto xstage = [&](int64_t blk) -> int { return blk == 0 ? 2 * L : 2 * L + __ffsll(blk); };
 
     if (w == kTmaConsumerWarps) {
         // ------------------------------------------------------------------ producer
@@ -328,7 +365,7 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
             uint64_t issued = 0;
             TileJob t;
             for (int64_t g = blockIdx.x; g < total; g += gridDim.x) {
-                decode_tile(g, k, st_begin, lv_s, L, tiles, S, t);
+                decode_tile(g, k, h, t);
                 if (!live(t.s)) continue;
 #pragma unroll
                 for (int m = 0; m < 2; ++m) {
@@ -351,72 +388,24 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
         }
         return;
     }
-    auto vec = [&](void *base, int64_t s) -> C * { return static_cast<C *>(base) + s * np; };
-    if (w == kTmaConsumerWarps + 1) {
-        // ------------------------------------------------------------------ dependency checker
-        // Runs ahead of the consumers through the CTA's tiles: waits (bounded, one lane
-        // per counter) for the completion counters of the blocks a tile reads and
-        // publishes the tile in `ready`, so that the consumers find their inputs complete
-        // without a round trip to global memory of their own.  A timed-out wait sets the
-        // error flag and the tile is published all the same.
-        int k = 0;
-        TileJob t;
-        for (int64_t g = blockIdx.x; g < total; g += gridDim.x) {
-            decode_tile(g, k, st_begin, lv_s, L, tiles, S, t);
-            const int64_t s = t.s;
-            if (live(s)) {
-                // the counters this tile needs (at most three), one lane waiting on each
-                int sid = -1;
-                int64_t blk = t.blk;
-                if (t.kind == 0) {
-                    if (t.l > 0 && lane == 0) sid = L + t.l - 1;
-                } else if (t.kind == 1) {
-                    const int64_t st = lv_s[t.l].stride;
-                    if (lane == 0 && t.hasl) { sid = t.l; blk = t.blk - st; }
-                    if (lane == 1 && t.hasr) { sid = t.l; blk = t.blk + st; }
-                    if (lane == 2 && t.l > 0) sid = L + t.l - 1;
-                } else if (t.kind == 2) {
-                    if (L > 0 && lane == 0) { sid = 2 * L - 1; blk = 0; }
-                } else if (t.kind == 3 && t.l == 0) {
-                    if (lane == 0) sid = 3 * L + 1;
-                } else if (lane == 0 || (lane == 1 && t.hasr)) {   // E_0, C_l: x of the neighbours
-                    blk = lane == 0 ? t.vblk[0] : t.vblk[1];
-                    sid = xstage(blk);
-                }
-                if (sid >= 0) wait_count(ctr(s, sid, blk), tiles[sid], a.err);
-                __syncwarp();
-            }
-            if (lane == 0) st_release_cta(&ready, (long long)g);
-        }
-        return;
-    }
-
     // ---------------------------------------------------------------------- consumers
-    // Each warp follows the CTA's tiles on its own: it waits for `ready`, loads the
-    // entries of the input vectors that its columns of the chunks multiply, consumes
-    // its columns of every chunk of the ring, and leaves its partial sums in red; one
-    // named barrier per tile gathers them, after which warp 0 reduces and writes the
-    // rows and signals the tile's completion while the other warps go on.
-    auto emit = [&](int64_t s, int64_t p, C val, double2 prev) {
-        stcg(vec(a.x, s) + p, val);
-        const double bn = a.bnorm[s];
-        const double2 d = ((bn > 0.0) ? bn : 1.0) * to_c128(val);
-        a.out[s * np + p] = a.accumulate ? prev + d : d;
-    };
+    // Each warp follows the CTA's tiles on its own: it waits for and loads the entries of the
+    // input vectors that its columns of the chunks multiply, consumes its columns of every
+    // chunk of the ring, and leaves its partial sums in red; one named barrier per tile
+    // gathers them, after which warp 0 reduces and writes the rows while the other warps go on.
     uint32_t slot = 0, ph = 0;
     int k = 0;
     TileJob t;
     int64_t i = 0;
     int64_t scaled = -1;     // the shift of bscale (an FP64 division, kept off the tiles' path)
     double bscale = 1.0;
-    for (int64_t g = blockIdx.x; g < total; g += gridDim.x, ++i) {
-        decode_tile(g, k, st_begin, lv_s, L, tiles, S, t);
+    for (int64_t g = blockIdx.x; g < total; g += gridDim.x) {
+        decode_tile(g, k, h, t);
         const int64_t s = t.s;
-        const int sid = t.kind == 0 ? t.l
-                      : (t.kind == 1 ? L + t.l : (t.kind == 2 ? 2 * L : (t.kind == 3 ? 2 * L + 1 + t.l : 3 * L + 1)));
-        int *done = ctr(s, sid, t.blk);
-        C (*rd)[33] = red[i & 1];
+        C (*rd)[33] = red[i & 1];   // i counts the tiles worked on: two in a row never share
         if (live(s)) {
+            ++i;
+            C *vs = static_cast<C *>(a.vecs) + s * a.vec_stride;
             // level-0 couplings (B_0, E_0): this thread's padded entries are loaded before
             // the wait, as they do not depend on the sweep; lane = row, warp w = entries w + 8u
             const bool ell = (t.kind == 1 && t.l == 0) || t.kind == 4;
@@ -437,39 +426,23 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
             const bool wr = w == 0 && r < S && !(t.low && lane >= kLowRows);
             C zf = czero<C>();
             double2 prev = mk(0.0, 0.0);
-            const bool from_b = (t.kind == 0 && t.l == 0) || (t.kind == 2 && L == 0);
-            if ((from_b || ell) && scaled != s) {
+            if ((t.from_b || ell) && scaled != s) {
                 const double bn = a.bnorm[s];
                 bscale = (bn > 0.0) ? 1.0 / bn : 1.0;
                 scaled = s;
             }
             if (wr && ell) zf = from_c128<C>((a.rscale[s * np + p] * bscale) * a.b[s * np + p]);
-            if (lane == 0) {
-                // the checker has seen this tile's inputs complete (acquire; __syncwarp
-                // orders the rest of the warp after this lane)
-                unsigned spins = 0;
-                while (ld_acquire_cta(&ready) < (long long)g) {
-                    if (++spins > KORE_SPIN_LIMIT) { atomicCAS(a.err, 0, KORE_DEVERR_FLAG); break; }
-                    if (spins > 64) __nanosleep(16);
-                }
-            }
-            __syncwarp();
-            // what the write combines with (read early)
-            if (wr) {
-                if (t.kind == 1 && t.l > 0) zf = ldcg(vec(a.f, s) + p);
-                else if (t.kind == 3 && t.l > 0) zf = ldcg(vec(a.z, s) + p);
-                if ((t.kind == 2 || t.kind == 3) && a.accumulate) prev = a.out[s * np + p];
-            }
+            if (wr && (t.kind == 2 || t.kind == 3) && a.accumulate) prev = a.out[s * np + p];
             if (!ell && t.nmat > 0) {
-                // this warp's slice of the input vectors: columns ch kCols + w kCpw + u
-                const C *src = (t.kind == 0 || t.kind == 2 || (t.kind == 3 && t.l == 0))
-                                   ? vec(a.f, s) : (t.kind == 1 ? vec(a.z, s) : vec(a.x, s));
+                // this warp's slice of the input vectors.  A lane per vector waits for one of its
+                // entries first, so that tiles far ahead poll little.
+                if (!t.from_b && lane < t.nmat) wait_entry(vs + (lane ? t.in[1] : t.in[0]) + S - 1, a.err);
+                __syncwarp();
                 const int per = nvec / kTmaConsumerWarps;   // zeros past S: the chunks reach there
                 const int ne = t.nmat * per;
-                const int64_t vb0 = t.vblk[0] * S, vb1 = t.vblk[1] * S;
                 for (int e0 = 0; e0 < ne; e0 += 32 * kFill) {
                     C v[kFill];
-                    int cv[kFill];
+                    int cv[kFill];   // column of the entry, + S for the second vector; -1: none
 #pragma unroll
                     for (int u = 0; u < kFill; ++u) {
                         const int e = e0 + u * 32 + lane;
@@ -480,26 +453,40 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
                         cv[u] = (e < ne) ? m * nvec + c : -1;
                         v[u] = czero<C>();
                         if (e < ne && c < S) {
-                            const int64_t q = (m ? vb1 : vb0) + c;
-                            v[u] = from_b ? from_c128<C>((a.rscale[s * np + q] * bscale) * a.b[s * np + q])
-                                          : ldcg(src + q);
+                            if (t.from_b) {
+                                const int64_t q = s * np + t.blk * S + c;
+                                v[u] = from_c128<C>((a.rscale[q] * bscale) * a.b[q]);
+                            } else v[u] = ld_entry(vs + (m ? t.in[1] : t.in[0]) + c);
                         }
                     }
 #pragma unroll
                     for (int u = 0; u < kFill; ++u)
-                        if (cv[u] >= 0) vbuf[cv[u]] = v[u];
+                        if (cv[u] >= 0) {
+                            if (!t.from_b && unset(v[u])) {
+                                const int m = cv[u] >= nvec ? 1 : 0;
+                                v[u] = wait_entry(vs + (m ? t.in[1] : t.in[0]) + cv[u] - m * nvec, a.err);
+                            }
+                            vbuf[cv[u]] = v[u];
+                        }
                 }
                 __syncwarp();
             }
+            if (wr && t.add >= 0) zf = ld_entry(vs + t.add + r);
             C acc = czero<C>();
             if (ell) {
-                const C *z = vec(t.kind == 4 ? a.x : a.z, s);   // E_0 couples to x, B_0 to z
+                const C *z = vs + t.in[0];   // E_0 couples to x, B_0 to z
+                C zv[kEllReg];
+#pragma unroll
+                for (int u = 0; u < kEllReg; ++u) zv[u] = ecol[u] >= 0 ? ld_entry(z + ecol[u]) : czero<C>();
 #pragma unroll
                 for (int u = 0; u < kEllReg; ++u)
-                    if (ecol[u] >= 0) acc = cfma(acc, eval[u], ldcg(z + ecol[u]));
+                    if (ecol[u] >= 0) {
+                        if (unset(zv[u])) zv[u] = wait_entry(z + ecol[u], a.err);
+                        acc = cfma(acc, eval[u], zv[u]);
+                    }
                 for (int kk = w + kEllReg * kTmaConsumerWarps; kk < a.ell_w; kk += kTmaConsumerWarps) {
                     const int c = __ldg(a.ell_col + ebase + (int64_t)kk * 32);
-                    if (c >= 0) acc = cfma(acc, ldg(ellv + ebase + (int64_t)kk * 32), ldcg(z + c));
+                    if (c >= 0) acc = cfma(acc, ldg(ellv + ebase + (int64_t)kk * 32), wait_entry(z + c, a.err));
                 }
             } else if (t.nmat > 0) {
 #pragma unroll
@@ -550,17 +537,16 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
 #pragma unroll
                 for (int q = 0; q < kTmaConsumerWarps; ++q) val = val + rd[q][lane];
                 if (wr) {
-                    if (ell) stcg(vec(a.f, s) + p, zf - val);
-                    else if (t.kind == 0) stcg(vec(a.z, s) + p, val);
-                    else if (t.kind == 1) stcg(vec(a.f, s) + p, zf - val);
-                    else if (t.kind == 2 || t.l == 0) emit(s, p, val, prev);
-                    else emit(s, p, zf - val, prev);
+                    if (t.add >= 0 && unset(zf)) zf = wait_entry(vs + t.add + r, a.err);
+                    if (ell || t.add >= 0) val = zf - val;
+                    st_entry(vs + t.out + r, val);
+                    if (t.kind == 2 || t.kind == 3) {   // an entry of the solution
+                        const double bn = a.bnorm[s];
+                        const double2 d = ((bn > 0.0) ? bn : 1.0) * to_c128(val);
+                        a.out[s * np + p] = a.accumulate ? prev + d : d;
+                    }
                 }
             }
-        }
-        if (w == 0) {
-            __syncwarp();
-            if (lane == 0) signal_count(done);
         }
     }
 }
@@ -814,6 +800,7 @@ SweepArgs sweep_args(const kore_plan *p, int nshift) {
     a.f_stride = p->f_stride(); a.lu_stride = p->lu_stride();
     a.ell_col = p->d_ell_col; a.ell_val = p->d_ell_val; a.ell_w = p->ell_w; a.ell_stride = p->ell_stride();
     a.rscale = p->d_rscale;
+    a.vec_stride = p->sweep_vec_elems();
     a.live_mask = ~0u;
     return a;
 }
@@ -826,7 +813,7 @@ SweepArgs sweep_args(const kore_plan *p, int nshift) {
 int sweep_low_tiles(const kore_plan *p) { return p->prec == KORE_PREC_FP64 ? p->num_sms : 2 * p->num_sms; }
 
 // Tensor maps, ring depth and the cooperative launch of the k_sweep_tma variant v (CTAs
-// per SM, chunk bytes); the completion counters a.cnt are zeroed first.
+// per SM, chunk bytes); all bits of the sweep's vectors are set first.
 template <typename C>
 int launch_sweep(const kore_plan *p, const SweepArgs &a, cudaStream_t st, TmaVariant v = kTmaDefault) {
     SweepTmaParams P;
@@ -865,7 +852,7 @@ int launch_sweep(const kore_plan *p, const SweepArgs &a, cudaStream_t st, TmaVar
     KORE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kTmaThreads, smem));
     if (occ < 1) return KORE_EINVAL;
     occ = std::min(occ, cps);
-    KORE_CUDA_TRY(cudaMemsetAsync(a.cnt, 0, (size_t)ns * p->sweep_stages() * p->K * sizeof(int), st));
+    KORE_CUDA_TRY(cudaMemsetAsync(a.vecs, 0xff, (size_t)ns * a.vec_stride * sizeof(C), st));
     void *args[] = {&P};
     dim3 grid(p->num_sms * occ), block(kTmaThreads);
     KORE_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)kern, grid, block, args, smem, st));
@@ -922,8 +909,8 @@ int sweep(kore_plan *p, const double2 *b, const double *bnorm, double2 *x, int a
     SweepArgs a = sweep_args(p, p->nshift);
     a.live_mask = live_mask;
     a.b = b; a.bnorm = bnorm;
-    a.f = p->d_flo; a.z = p->d_zlo; a.x = p->d_xlo;
-    a.out = x; a.accumulate = accumulate; a.cnt = p->d_cnt; a.err = p->d_err;
+    a.vecs = p->d_sweep;
+    a.out = x; a.accumulate = accumulate; a.err = p->d_err;
     a.skip = skip; a.skip_stride = (int)(sizeof(IrState) / sizeof(int));
     a.count = &p->d_ir->sweeps; a.count_total = &p->d_ir->sweeps_total;
     const bool fp64 = p->prec == KORE_PREC_FP64;
@@ -1305,20 +1292,20 @@ int kore_ir_read(kore_plan *p, IrState *out) {
 namespace {
 
 constexpr int64_t kNoAllocMaxNp = 16384;
-constexpr int64_t kNoAllocMaxCnt = 32768;   // sweep completion counters: (3 levels + 2) x blocks
+constexpr int64_t kNoAllocMaxCnt = 32768;   // stages x blocks of a sweep: (3 levels + 2) x blocks
 constexpr int64_t kNoAllocMaxSpmvCta = (kNoAllocMaxNp * kRowLanes + 255) / 256 + kNoAllocMaxNp / 8 + 1;
 
 struct NoAllocScratch {
     double2 bp[kNoAllocMaxNp];      // padded right-hand side (complex128)
     double2 xp[kNoAllocMaxNp];      // padded solution
     double2 r[kNoAllocMaxNp];       // FP64 residual of the refinement loop
-    double2 f[kNoAllocMaxNp];       // sweep reduction vectors, room for complex128
-    double2 z[kNoAllocMaxNp];
-    double2 x[kNoAllocMaxNp];
+    // sweep vectors, room for complex128: z, x, g and the levels' f, which take fewer than
+    // blocks + levels blocks (20480 entries hold those of 16384 unknowns: at most 4 blocks of
+    // 1024 more than the blocks themselves)
+    double2 vecs[3 * kNoAllocMaxNp + 20480];
     double part[2 * kNoAllocMaxSpmvCta];   // per-CTA maxima of the residual kernel
     double red[2048 + 8];                  // ||b||_inf partials [0, 2048), then scalars
     IrState ir;
-    int cnt[kNoAllocMaxCnt];              // sweep completion counters
     int err;
 };
 
@@ -1351,8 +1338,8 @@ int noalloc_sweep(kore_plan *p, NoAllocScratch *s, const double2 *b, const doubl
                   const int *skip, cudaStream_t st) {
     SweepArgs a = sweep_args(p, 1);   // shift 0
     a.b = b; a.bnorm = bnorm;
-    a.f = s->f; a.z = s->z; a.x = s->x;
-    a.out = x; a.accumulate = accumulate; a.cnt = s->cnt; a.err = &s->err;
+    a.vecs = s->vecs;
+    a.out = x; a.accumulate = accumulate; a.err = &s->err;
     a.skip = skip; a.skip_stride = 0; a.count = &s->ir.sweeps; a.count_total = &s->ir.sweeps_total;
     return launch_sweep<C>(p, a, st, p->sweep_cps > 0 ? TmaVariant{p->sweep_cps, p->sweep_chunk} : kTmaDefault);
 }
@@ -1397,7 +1384,7 @@ int noalloc_solve(kore_plan *p, NoAllocScratch *s, const double2 *b_dev, double2
 
 extern "C" int kore_solve_dev_noalloc(kore_plan *p, const void *b_dev, void *x_dev, double refine_tol, void *stream) {
     if (!p || !b_dev || !x_dev) return KORE_EINVAL;
-    if (p->np > kNoAllocMaxNp || (int64_t)p->sweep_stages() * p->K > kNoAllocMaxCnt) {
+    if (p->np > kNoAllocMaxNp || (int64_t)(p->nlev > 0 ? 3 * p->nlev + 2 : 1) * p->K > kNoAllocMaxCnt) {
         std::fprintf(stderr,
                      "kore_solve_dev_noalloc: %lld padded unknowns in %d blocks exceed the fixed scratch "
                      "(%lld unknowns, %lld block counters); use kore_solve_dev\n",
