@@ -713,7 +713,7 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
     void **bufs[] = {&p->d_Dinv, &p->d_Gm, &p->d_Hm, &p->d_Dw, &p->d_LU, &p->d_T, &p->d_sweep,
                      (void **)&p->d_rscale, (void **)&p->d_piv, (void **)&p->d_used,
                      (void **)&p->d_sigma, (void **)&p->d_minf, (void **)&p->d_bb, (void **)&p->d_xb, (void **)&p->d_rb,
-                     (void **)&p->d_bn, (void **)&p->d_rn, (void **)&p->d_part, (void **)&p->d_ir,
+                     (void **)&p->d_bn, (void **)&p->d_rn, (void **)&p->d_part, (void **)&p->d_ir, (void **)&p->d_tick,
                      &p->d_ell_val, &p->d_tctab, &p->d_oz};
     for (void **b : bufs) {
         if (*b) cudaFree(*b);
@@ -757,6 +757,9 @@ int ensure_factor_storage(kore_plan *p, int cap, size_t elt) {
     KORE_CUDA_TRY(cudaMemset(p->d_piv, 0, c * p->p_stride() * sizeof(int)));
     KORE_CUDA_TRY(cudaMemset(p->d_used, 0, c * p->p_stride() * sizeof(int)));
     KORE_CUDA_TRY(cudaMemset(p->d_ir, 0, c * sizeof(IrState)));
+    KORE_TRY(kore_alloc(p, (void **)&p->d_tick, c * sizeof(unsigned)));
+    KORE_CUDA_TRY(cudaMemset(p->d_tick, 0, c * sizeof(unsigned)));
+    p->sweep_launch.reset();
     p->factor_bytes = p->bytes - before;
     p->factor_elt = elt;
     p->shift_cap = cap;

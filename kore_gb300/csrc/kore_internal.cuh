@@ -1,6 +1,7 @@
 // Internal plan structure and cross-file declarations of libkoregpu.
 #pragma once
 
+#include <memory>
 #include <vector>
 #include "kore_common.cuh"
 
@@ -148,6 +149,8 @@ struct kore_plan {
     double *d_part = nullptr;         // per-CTA maxima of the residual kernel (2 per CTA, per shift)
     double *h_red = nullptr;          // pinned host mirror
     int *d_err = nullptr;
+    unsigned *d_tick = nullptr;       // one per shift: arrivals of a launch's CTAs (0 between launches)
+    std::shared_ptr<void> sweep_launch;   // the last sweep launch's maps and shape (sweep.cu)
     int *d_flag = nullptr;            // a solve's non-finite flag
     IrState *d_ir = nullptr;          // one per shift
 
@@ -187,6 +190,8 @@ int kore_prof_collect(kore_plan *p);
 
 // plan.cu
 int kore_check_device_error(kore_plan *p);
+// the status of an error flag that was read; a set flag is cleared on the device
+int kore_device_error(kore_plan *p, int flag);
 int kore_alloc(kore_plan *p, void **ptr, size_t bytes);
 
 // factor.cu
@@ -226,7 +231,8 @@ int64_t kore_oz_workspace_bytes(int S, int64_t K, int64_t cap);
 int kore_apply_inverse(kore_plan *p, const double2 *b, double2 *x, double tol, unsigned live_mask = ~0u,
                        const double *shift_tols = nullptr);
 int kore_ir_reset(kore_plan *p);
-int kore_ir_read(kore_plan *p, IrState *out);
+// err (may be null) receives the device error flag as it stands after the plan's work
+int kore_ir_read(kore_plan *p, IrState *out, int *err = nullptr);
 // once per plan, before the sparse products run: their launch attributes
 int kore_spmv_prepare(kore_plan *p);
 // y = B x on padded vectors

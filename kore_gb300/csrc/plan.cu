@@ -31,13 +31,17 @@ int kore_alloc(kore_plan *p, void **ptr, size_t bytes) {
     return KORE_OK;
 }
 
+int kore_device_error(kore_plan *p, int flag) {
+    if (flag == 0) return KORE_OK;
+    KORE_CUDA_TRY(cudaMemset(p->d_err, 0, sizeof(int)));
+    if (flag == KORE_DEVERR_PIVOT) return KORE_ESINGULAR;
+    return KORE_ETIMEOUT;
+}
+
 int kore_check_device_error(kore_plan *p) {
     int h = 0;
     KORE_CUDA_TRY(cudaMemcpy(&h, p->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (h == 0) return KORE_OK;
-    KORE_CUDA_TRY(cudaMemset(p->d_err, 0, sizeof(int)));
-    if (h == KORE_DEVERR_PIVOT) return KORE_ESINGULAR;
-    return KORE_ETIMEOUT;
+    return kore_device_error(p, h);
 }
 
 int kore_prof_mark(kore_plan *p, int kind, bool begin) {
@@ -95,7 +99,7 @@ void free_plan(kore_plan *p) {
     void *ptrs[] = {p->d_arow, p->d_acol, p->d_asplit, p->d_aval, p->d_brow, p->d_bcol, p->d_bval,
                     p->d_slot2orig, p->d_bsz, p->d_Dinv, p->d_Gm, p->d_Hm, p->d_Dw, p->d_LU, p->d_lev,
                     p->d_rscale, p->d_T, p->d_piv, p->d_used, p->d_sweep,
-                    p->d_red, p->d_part, p->d_err, p->d_flag, p->d_ir, p->d_V, p->d_Vtmp, p->d_ksx, p->d_small, p->d_warm,
+                    p->d_red, p->d_part, p->d_err, p->d_flag, p->d_ir, p->d_tick, p->d_V, p->d_Vtmp, p->d_ksx, p->d_small, p->d_warm,
                     p->d_sigma, p->d_minf, p->d_bb, p->d_xb, p->d_rb, p->d_bn, p->d_rn,
                     p->d_ell_col, p->d_ell_src, p->d_ell_val, p->d_long_rows, p->d_srow, p->d_smid,
                     p->d_scol, p->d_sval, p->d_cc_ptr, p->d_cc_row, p->d_cc_src, p->d_tctab, p->d_oz};
@@ -386,14 +390,15 @@ int solve_dev_impl(kore_plan *p, const double2 *b, double2 *x, int nrhs, double 
         else KORE_TRY(kore_scatter_shifts(p, p->d_xb, x + (int64_t)g * p->n));
     }
     IrState s;
-    KORE_TRY(kore_ir_read(p, &s));
+    int err = 0;
+    KORE_TRY(kore_ir_read(p, &s, &err));
     if (st) {
         st->sweeps = s.sweeps;
         st->refine_iters_max = s.iters_max;
         st->solve_resid_max = s.eta_max;
     }
-    if (s.nan) return KORE_ENAN;
-    return KORE_OK;
+    const int rc = kore_device_error(p, err);
+    return s.nan ? KORE_ENAN : rc;
 }
 
 // The host-pointer solves: copies, solve, and the test of the solution for NaN or Inf
@@ -424,7 +429,6 @@ int solve_host(kore_plan *p, const double *b, double *x, int nrhs, double refine
     cudaFreeAsync(db, p->stream);
     cudaFreeAsync(dx, p->stream);
     if (cudaStreamSynchronize(p->stream) != cudaSuccess && s == KORE_OK) s = KORE_ECUDA;
-    if (s == KORE_OK) s = kore_check_device_error(p);
     if (s == KORE_OK && bad) s = KORE_ENAN;
     if (stats) stats->iterate_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     return s;
@@ -476,7 +480,6 @@ int kore_solve_dev(kore_plan *p, const void *b_dev, void *x_dev, int nrhs, doubl
     KORE_CUDA_TRY(cudaEventRecord(ev, p->stream));
     KORE_CUDA_TRY(cudaStreamWaitEvent(cs, ev, 0));
     cudaEventDestroy(ev);
-    if (s == KORE_OK) s = kore_check_device_error(p);
     return s;
 }
 

@@ -23,6 +23,8 @@
 #include "kore_internal.cuh"
 #include "kore_tma.cuh"
 #include <cstddef>
+#include <cstring>
+#include <memory>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -551,38 +553,83 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
     }
 }
 
-// max |v_p| per shift: grid (x, shift) -> red[s * gridDim.x + blockIdx.x]
-__global__ void k_absmax(int64_t np, const double2 *__restrict__ v, double *__restrict__ red) {
-    const int64_t s = blockIdx.y;
-    v += s * np;
-    double mx = 0.0;
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np; p += (int64_t)gridDim.x * blockDim.x)
-        mx = fmax(mx, fmax(fabs(v[p].x), fabs(v[p].y)));
-    mx = warp_max_d(mx);
-    __shared__ double sm[32];
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double t = (threadIdx.x < (blockDim.x >> 5)) ? sm[threadIdx.x] : 0.0;
-        t = warp_max_d(t);
-        if (threadIdx.x == 0) red[s * gridDim.x + blockIdx.x] = t;
-    }
+// |v| of a double as the bits of its absolute value: for non-negative IEEE doubles the
+// integer order is the numeric order, so maxima run on the integer units, not on the
+// FP64 pipe, and a NaN (above +inf as bits) is kept instead of dropped as fmax drops it
+__device__ __forceinline__ unsigned long long abs_bits(double v) {
+    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v) {
+    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_down_sync(0xffffffffu, v, o));
+    return v;
 }
 
-// out[s] = max of in[s * n .. s * n + n), one CTA per shift
-__global__ void k_reduce_max(const double *__restrict__ in, int n, double *__restrict__ out) {
-    const int s = blockIdx.x;
-    in += (int64_t)s * n;
-    double mx = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) mx = fmax(mx, in[i]);
-    mx = warp_max_d(mx);
-    __shared__ double sm[32];
+// True in every thread of the last CTA of a grid row to get here (the CTAs' earlier writes
+// are then visible to it); *tick is 0 before and after the launch.
+__device__ __forceinline__ bool last_cta(unsigned *tick, unsigned ctas) {
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(tick, 1u) == ctas - 1;
+        if (last) {
+            *tick = 0;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    return last;
+}
+
+// Set all bits of the sweep's vectors of shift s (st_entry), this CTA's share of them.
+__device__ __forceinline__ void reset_vecs(void *vecs, int64_t bytes, int64_t s) {
+    uint4 *v = reinterpret_cast<uint4 *>(static_cast<unsigned char *>(vecs) + s * bytes);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < bytes / 16; i += (int64_t)gridDim.x * blockDim.x)
+        v[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+}
+
+// What a sweep of the right-hand sides b needs first, per shift (grid y): ||b||_inf (a NaN
+// does not count), the sweep's vectors set, and with ir the refinement state of a new
+// application (a shift outside live_mask has nothing to refine).  Bound by its launch: one
+// kernel here for two maxima kernels, a state kernel and a memset, and the check in the
+// residual product's last CTA, took a solve of 704 unknowns in FP64 from 123 to 102 us and
+// four mixed targets of the 1.9k-unknown shell from 74.9 to 68.5 ms.
+__global__ void __launch_bounds__(256) k_begin(int64_t np, const double2 *__restrict__ v, double *__restrict__ part,
+                                               double *__restrict__ bnorm, unsigned *tick, void *vecs, int64_t vbytes,
+                                               IrState *ir, unsigned live_mask) {
+    const int s = blockIdx.y;
+    reset_vecs(vecs, vbytes, s);
+    v += s * np;
+    part += (int64_t)s * gridDim.x;
+    unsigned long long mx = 0;
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np; p += (int64_t)gridDim.x * blockDim.x) {
+        const unsigned long long x = abs_bits(v[p].x), y = abs_bits(v[p].y);
+        if (x <= 0x7ff0000000000000ull) mx = max(mx, x);
+        if (y <= 0x7ff0000000000000ull) mx = max(mx, y);
+    }
+    __shared__ unsigned long long sm[8];
+    mx = warp_max_bits(mx);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = mx;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        double t = (threadIdx.x < (blockDim.x >> 5)) ? sm[threadIdx.x] : 0.0;
-        t = warp_max_d(t);
-        if (threadIdx.x == 0) out[s] = t;
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) mx = max(mx, sm[w]);
+        part[blockIdx.x] = __longlong_as_double((long long)mx);
+    }
+    if (!last_cta(tick + s, gridDim.x)) return;
+    mx = 0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) mx = max(mx, abs_bits(__ldcg(part + i)));
+    mx = warp_max_bits(mx);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 8; ++w) mx = max(mx, sm[w]);
+    bnorm[s] = __longlong_as_double((long long)mx);
+    if (!ir) return;
+    const bool on = mask_has(live_mask, s);
+    ir[s].done = on ? 0 : 1;
+    if (on) {
+        ir[s].prev = 1e300;
+        ir[s].applies += 1;
     }
 }
 
@@ -677,18 +724,63 @@ __device__ __forceinline__ void row_dot(const SpmvArgs &a, int64_t p, int sub, c
 // x entries of the window of a CTA of 256 short rows: at most (255 / S + 4) blocks
 __host__ __device__ __forceinline__ int64_t spmv_window(int S) { return (int64_t)(255 / S + 4) * S; }
 
-// |v| of a double as the bits of its absolute value: for non-negative IEEE doubles the
-// integer order is the numeric order, so maxima run on the integer units, not on the
-// FP64 pipe, and a NaN (above +inf as bits) is kept instead of dropped as fmax drops it
-__device__ __forceinline__ unsigned long long abs_bits(double v) {
-    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
-}
-__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v) {
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_down_sync(0xffffffffu, v, o));
-    return v;
+// Per-shift refinement tolerances of one application (shifts past 31 use the scalar).
+struct ShiftTols {
+    double t[32];
+    int valid;
+};
+
+// The refinement's test, run by the last CTA of a shift's residual product: eta = ||r||_inf /
+// (||M||_inf ||x||_inf + ||b||_inf) from the CTAs' maxima; stop when eta <= tol or when it no
+// longer decreases (FP64 floor).
+struct IrCheck {
+    IrState *ir;             // null: no test
+    const double *bnorm, *minf;
+    double *rn;              // ||r||_inf for the next correction
+    double tol;
+    ShiftTols tols;
+    unsigned *tick;
+    void *vecs;              // the next sweep's vectors, set here
+    int64_t vbytes;
+};
+
+__device__ __forceinline__ void ir_check(const IrCheck &c, int s, const double *part, int n) {
+    // maxima of non-negative doubles as bits (a NaN among them stays, and is caught below)
+    unsigned long long rb = 0, xb = 0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        rb = max(rb, abs_bits(__ldcg(part + 2 * i)));
+        xb = max(xb, abs_bits(__ldcg(part + 2 * i + 1)));
+    }
+    rb = warp_max_bits(rb);
+    xb = warp_max_bits(xb);
+    __shared__ unsigned long long s0[8], s1[8];
+    if ((threadIdx.x & 31) == 0) { s0[threadIdx.x >> 5] = rb; s1[threadIdx.x >> 5] = xb; }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 8; ++w) { rb = max(rb, s0[w]); xb = max(xb, s1[w]); }
+    const double rm = __longlong_as_double((long long)rb), xm = __longlong_as_double((long long)xb);
+    const double den = c.minf[s] * xm + c.bnorm[s];
+    const double tol = (c.tols.valid && s < 32) ? c.tols.t[s] : c.tol;
+    // a NaN in r, x or b makes eta NaN (a NaN denominator must not read as converged)
+    const double eta = (den == 0.0) ? 0.0 : rm / den;
+    IrState *st = c.ir + s;
+    if (!(eta == eta)) {
+        st->nan = 1;
+        st->done = 1;
+        return;
+    }
+    if (eta <= tol || eta > 0.9 * st->prev) {
+        st->done = 1;
+        st->eta_max = fmax(st->eta_max, eta);
+        return;
+    }
+    st->prev = eta;
+    st->iters += 1;
+    st->iters_cur += 1;
+    c.rn[s] = rm;
 }
 
-__global__ void __launch_bounds__(256) k_spmv(SpmvArgs a) {
+__global__ void __launch_bounds__(256) k_spmv(const SpmvArgs a, const __grid_constant__ IrCheck chk) {
     extern __shared__ double2 xsh[];   // spmv_window(S) entries
     const int64_t s = blockIdx.y;
     if (!mask_has(a.live_mask, s) || (a.skip && a.skip[s * a.skip_stride])) return;
@@ -755,6 +847,10 @@ __global__ void __launch_bounds__(256) k_spmv(SpmvArgs a) {
             a.part[s * 2 * gridDim.x + 2 * blockIdx.x] = __longlong_as_double((long long)rmax);
             a.part[s * 2 * gridDim.x + 2 * blockIdx.x + 1] = __longlong_as_double((long long)xmax);
         }
+        if (chk.ir) {
+            reset_vecs(chk.vecs, chk.vbytes, s);
+            if (last_cta(chk.tick + s, gridDim.x)) ir_check(chk, (int)s, a.part + s * 2 * gridDim.x, (int)gridDim.x);
+        }
     }
 }
 
@@ -812,17 +908,21 @@ SweepArgs sweep_args(const kore_plan *p, int nshift) {
 // 730 us; 240k shell in complex64 (7 sweeps) 5.26, 5.06, 4.98, 4.98, 4.90, 4.88 ms.
 int sweep_low_tiles(const kore_plan *p) { return p->prec == KORE_PREC_FP64 ? p->num_sms : 2 * p->num_sms; }
 
-// Tensor maps, ring depth and the cooperative launch of the k_sweep_tma variant v (CTAs
-// per SM, chunk bytes); all bits of the sweep's vectors are set first.
-template <typename C>
-int launch_sweep(const kore_plan *p, const SweepArgs &a, cudaStream_t st, TmaVariant v = kTmaDefault) {
+// What a launch of a variant needs besides its arguments.  The plan keeps its last one: maps
+// and occupancy depend on the variant, the factors' storage and the number of shifts alone,
+// and encoding and asking for them takes the host longer than a small sweep runs.
+struct SweepLaunch {
+    int prec, nshift, cps, chunk, occ;
+    size_t smem;
     SweepTmaParams P;
-    P.a = a;
+};
+
+template <typename C>
+int prepare_sweep(const kore_plan *p, TmaVariant v, int ns, SweepLaunch &l) {
     const int rb = (int)sizeof(C) / 2;
-    const int cps = v.cps;
     if (v.chunk != 8192 && v.chunk != 16384) return KORE_EINVAL;
     const int kCols = v.chunk / (kTileRows * (int)sizeof(C));
-    const int ns = a.nshift;
+    SweepTmaParams &P = l.P;
     for (int low = 0; low < 2; ++low) {
         const int rows = low ? kLowRows : kTileRows, cols = low ? 4 * kCols : kCols, o = 4 * low;
         KORE_TRY(kore_encode_block_map(&P.maps[o + kMapDinv], p->d_Dinv, rb, p->S, p->K, ns, p->f_stride(), rows, cols));
@@ -840,24 +940,49 @@ int launch_sweep(const kore_plan *p, const SweepArgs &a, cudaStream_t st, TmaVar
     cudaFuncAttributes fa;
     KORE_CUDA_TRY(cudaFuncGetAttributes(&fa, kern));
     const size_t static_smem = fa.sharedSizeBytes + 1024;   // + the per-CTA reserve of the SM
-    const size_t budget = std::min<size_t>((size_t)smem_sm / cps - static_smem,
+    const size_t budget = std::min<size_t>((size_t)smem_sm / v.cps - static_smem,
                                            (size_t)smem_blk - fa.sharedSizeBytes);
     int nst = kMaxRing;
     while (nst > 2 && tma_smem<C>(p->S, nst, v.chunk) > budget) --nst;
     if (tma_smem<C>(p->S, nst, v.chunk) > budget) return KORE_EINVAL;
     P.nst = nst;
-    const size_t smem = tma_smem<C>(p->S, nst, v.chunk);
+    l.smem = tma_smem<C>(p->S, nst, v.chunk);
     KORE_TRY(kore_allow_max_dyn_smem(kern, p->device));
     int occ = 0;
-    KORE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kTmaThreads, smem));
+    KORE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kTmaThreads, l.smem));
     if (occ < 1) return KORE_EINVAL;
-    occ = std::min(occ, cps);
-    KORE_CUDA_TRY(cudaMemsetAsync(a.vecs, 0xff, (size_t)ns * a.vec_stride * sizeof(C), st));
-    void *args[] = {&P};
-    dim3 grid(p->num_sms * occ), block(kTmaThreads);
-    KORE_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)kern, grid, block, args, smem, st));
+    l.occ = std::min(occ, v.cps);
+    l.prec = p->prec; l.nshift = ns; l.cps = v.cps; l.chunk = v.chunk;
+    return KORE_OK;
+}
+
+// The cooperative launch of a prepared k_sweep_tma on the vectors that the kernel before it set
+template <typename C>
+int launch_prepared(SweepLaunch &l, const SweepArgs &a, int num_sms, cudaStream_t st) {
+    l.P.a = a;
+    void *args[] = {&l.P};
+    KORE_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)sweep_kernel<C>(TmaVariant{l.cps, l.chunk}),
+                                              dim3(num_sms * l.occ), dim3(kTmaThreads), args, l.smem, st));
     KORE_LAUNCHED(1);
     return KORE_OK;
+}
+
+// The same on the plan's own stream, prepared when the plan's last one was of another shape
+template <typename C>
+int launch_sweep(kore_plan *p, const SweepArgs &a, TmaVariant v) {
+    SweepLaunch *l = static_cast<SweepLaunch *>(p->sweep_launch.get());
+    if (!l || l->prec != p->prec || l->nshift != a.nshift || l->cps != v.cps || l->chunk != v.chunk) {
+        std::shared_ptr<SweepLaunch> made = std::make_shared<SweepLaunch>();
+        KORE_TRY(prepare_sweep<C>(p, v, a.nshift, *made));
+        p->sweep_launch = made;
+        l = made.get();
+    }
+    return launch_prepared<C>(*l, a, p->num_sms, p->stream);
+}
+
+// bytes of one shift's sweep vectors (16-byte entries or pairs: S is a multiple of 4)
+int64_t vec_bytes(const kore_plan *p) {
+    return p->sweep_vec_elems() * (int64_t)(p->prec == KORE_PREC_FP64 ? sizeof(double2) : sizeof(float2));
 }
 
 // Autotuner of the sweep's variant (CTAs per SM, chunk size), keyed on the plan's shape: the first
@@ -876,6 +1001,12 @@ std::map<TuneKey, TmaVariant> g_tune;
 TmaVariant g_force{0, 0};   // kore_sweep_variant: every sweep uses it instead of the autotuner's choice
 
 template <typename C>
+int reset_and_sweep(kore_plan *p, const SweepArgs &a, TmaVariant v) {
+    KORE_CUDA_TRY(cudaMemsetAsync(a.vecs, 0xff, (size_t)a.nshift * vec_bytes(p), p->stream));
+    return launch_sweep<C>(p, a, v);
+}
+
+template <typename C>
 int tune_sweep(kore_plan *p, const SweepArgs &a, TmaVariant *best) {
     cudaEvent_t e0, e1;
     KORE_CUDA_TRY(cudaEventCreate(&e0));
@@ -887,7 +1018,7 @@ int tune_sweep(kore_plan *p, const SweepArgs &a, TmaVariant *best) {
         float ms = 0.f;
         for (int rep = 0; rep < 2 && rc == KORE_OK; ++rep) {   // the second run is timed
             if (cudaEventRecord(e0, p->stream) != cudaSuccess) rc = KORE_ECUDA;
-            if (rc == KORE_OK) rc = launch_sweep<C>(p, a, p->stream, v);
+            if (rc == KORE_OK) rc = reset_and_sweep<C>(p, a, v);
             if (rc == KORE_OK && cudaEventRecord(e1, p->stream) != cudaSuccess) rc = KORE_ECUDA;
             if (rc == KORE_OK && cudaEventSynchronize(e1) != cudaSuccess) rc = KORE_ECUDA;
             if (rc == KORE_OK && cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) rc = KORE_ECUDA;
@@ -897,7 +1028,7 @@ int tune_sweep(kore_plan *p, const SweepArgs &a, TmaVariant *best) {
         if (ms < best_ms) { best_ms = ms; *best = v; }
     }
     // the chosen variant runs last, so the sweep's outputs are its own
-    if (rc == KORE_OK) rc = launch_sweep<C>(p, a, p->stream, *best);
+    if (rc == KORE_OK) rc = reset_and_sweep<C>(p, a, *best);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     return rc;
@@ -932,7 +1063,7 @@ int sweep(kore_plan *p, const double2 *b, const double *bnorm, double2 *x, int a
         }
     } else {
         if (v.cps == 0) v = kTmaDefault;
-        s = fp64 ? launch_sweep<double2>(p, a, p->stream, v) : launch_sweep<float2>(p, a, p->stream, v);
+        s = fp64 ? launch_sweep<double2>(p, a, v) : launch_sweep<float2>(p, a, v);
     }
     p->sweep_cps = v.cps;
     p->sweep_chunk = v.chunk;
@@ -953,17 +1084,7 @@ extern "C" int kore_sweep_variant(int ctas_per_sm, int chunk_bytes) {
 
 namespace {
 
-unsigned absmax_grid(int64_t np) { return std::min<unsigned>(kore_div_up(np, 256), 1024u); }
-
-// ||v_s||_inf of nshift padded vectors into out[s] (device); scratch: g * nshift doubles
-int absmax(kore_plan *p, const double2 *v, double *out, double *scratch) {
-    const unsigned g = absmax_grid(p->np);
-    k_absmax<<<dim3(g, p->nshift), 256, 0, p->stream>>>(p->np, v, scratch);
-    k_reduce_max<<<p->nshift, 1024, 0, p->stream>>>(scratch, (int)g, out);
-    KORE_LAUNCHED(2);
-    KORE_CUDA_TRY(cudaGetLastError());
-    return KORE_OK;
-}
+unsigned begin_grid(const kore_plan *p) { return std::min<unsigned>(kore_div_up(p->np, 256), 2u * p->num_sms); }
 
 // CTAs of one sparse product: the 4-lane part, then 8 long rows per CTA
 unsigned spmv_short_blocks(int64_t np) { return kore_div_up(np * kRowLanes, 256); }
@@ -993,7 +1114,7 @@ int kore_spmv_prepare(kore_plan *p) {
 int kore_spmv_b(kore_plan *p, const double2 *x, double2 *y) {
     if (!p->has_b) return KORE_EINVAL;
     if (p->prof) KORE_TRY(kore_prof_mark(p, 2, true));
-    k_spmv<<<spmv_grid(p), 256, spmv_smem(p), p->stream>>>(spmv_args(p, 0, x, y));
+    k_spmv<<<spmv_grid(p), 256, spmv_smem(p), p->stream>>>(spmv_args(p, 0, x, y), IrCheck{});
     KORE_LAUNCHED(1);
     if (p->prof) KORE_TRY(kore_prof_mark(p, 2, false));
     KORE_CUDA_TRY(cudaGetLastError());
@@ -1005,7 +1126,7 @@ int kore_spmv_b_shifts(kore_plan *p, const double2 *x, double2 *y, unsigned live
     if (p->prof) KORE_TRY(kore_prof_mark(p, 2, true));
     SpmvArgs a = spmv_args(p, 0, x, y);
     a.live_mask = live_mask;
-    k_spmv<<<dim3(spmv_grid(p), std::max(1, p->nshift)), 256, spmv_smem(p), p->stream>>>(a);
+    k_spmv<<<dim3(spmv_grid(p), std::max(1, p->nshift)), 256, spmv_smem(p), p->stream>>>(a, IrCheck{});
     KORE_LAUNCHED(1);
     if (p->prof) KORE_TRY(kore_prof_mark(p, 2, false));
     KORE_CUDA_TRY(cudaGetLastError());
@@ -1017,7 +1138,7 @@ int kore_spmv_a_shifts(kore_plan *p, const double2 *x, double2 *y, unsigned live
     SpmvArgs a = spmv_args(p, 1, x, y);   // A x - 0 B x
     a.has_b = 0;
     a.live_mask = live_mask;
-    k_spmv<<<dim3(spmv_grid(p), std::max(1, p->nshift)), 256, spmv_smem(p), p->stream>>>(a);
+    k_spmv<<<dim3(spmv_grid(p), std::max(1, p->nshift)), 256, spmv_smem(p), p->stream>>>(a, IrCheck{});
     KORE_LAUNCHED(1);
     if (p->prof) KORE_TRY(kore_prof_mark(p, 2, false));
     KORE_CUDA_TRY(cudaGetLastError());
@@ -1027,7 +1148,7 @@ int kore_spmv_a_shifts(kore_plan *p, const double2 *x, double2 *y, unsigned live
 int kore_spmv_pencil(kore_plan *p, double lre, double lim, const double2 *x, double2 *y) {
     SpmvArgs a = spmv_args(p, 1, x, y);
     a.lam = mk(lre, lim);
-    k_spmv<<<spmv_grid(p), 256, spmv_smem(p), p->stream>>>(a);
+    k_spmv<<<spmv_grid(p), 256, spmv_smem(p), p->stream>>>(a, IrCheck{});
     KORE_LAUNCHED(1);
     KORE_CUDA_TRY(cudaGetLastError());
     return KORE_OK;
@@ -1137,68 +1258,6 @@ int kore_check_finite(kore_plan *p, const double2 *v, int64_t n, int *flag) {
 
 namespace {
 
-// one thread per shift
-__global__ void k_ir_begin(IrState *st, int nshift, unsigned live_mask) {
-    const int s = threadIdx.x;
-    if (s >= nshift) return;
-    if (!mask_has(live_mask, s)) {   // not part of this application: nothing to refine
-        st[s].done = 1;
-        return;
-    }
-    st[s].done = 0;
-    st[s].prev = 1e300;
-    st[s].applies += 1;
-}
-
-// One CTA per shift s: eta = ||r||_inf / (||M||_inf ||x||_inf + ||b||_inf) from the
-// per-CTA maxima of the residual kernel; stop when eta <= tol or when it no longer
-// decreases (FP64 floor).
-// Per-shift refinement tolerances of one application (shifts past 31 use the scalar).
-struct ShiftTols {
-    double t[32];
-    int valid;
-};
-
-__global__ void k_ir_check(const double *__restrict__ part, int n, const double *__restrict__ bnorm,
-                           const double *__restrict__ minf, double tol0, ShiftTols tols, IrState *stall, double *rn) {
-    const int s = blockIdx.x;
-    const double tol = (tols.valid && s < 32) ? tols.t[s] : tol0;
-    IrState *st = stall + s;
-    if (st->done) return;
-    part += (int64_t)s * 2 * n;
-    // maxima of non-negative doubles as bits (a NaN among them stays, and is caught below)
-    unsigned long long rb = 0, xb = 0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        rb = max(rb, abs_bits(part[2 * i]));
-        xb = max(xb, abs_bits(part[2 * i + 1]));
-    }
-    rb = warp_max_bits(rb);
-    xb = warp_max_bits(xb);
-    __shared__ unsigned long long s0[32], s1[32];
-    if ((threadIdx.x & 31) == 0) { s0[threadIdx.x >> 5] = rb; s1[threadIdx.x >> 5] = xb; }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { rb = max(rb, s0[w]); xb = max(xb, s1[w]); }
-    const double rm = __longlong_as_double((long long)rb), xm = __longlong_as_double((long long)xb);
-    const double den = minf[s] * xm + bnorm[s];
-    // a NaN in r, x or b makes eta NaN (a NaN denominator must not read as converged)
-    const double eta = (den == 0.0) ? 0.0 : rm / den;
-    if (!(eta == eta)) {
-        st->nan = 1;
-        st->done = 1;
-        return;
-    }
-    if (eta <= tol || eta > 0.9 * st->prev) {
-        st->done = 1;
-        st->eta_max = fmax(st->eta_max, eta);
-        return;
-    }
-    st->prev = eta;
-    st->iters += 1;
-    st->iters_cur += 1;
-    rn[s] = rm;
-}
-
 __global__ void k_ir_end(IrState *st, int nshift) {
     const int s = threadIdx.x;
     if (s >= nshift) return;
@@ -1212,8 +1271,8 @@ __global__ void k_ir_end(IrState *st, int nshift) {
 }  // namespace
 
 // Mixed precision: the refinement loop runs without host synchronisation.  Its length
-// is bounded (kIrMax corrections); each step is a residual kernel, a convergence check
-// (one CTA per shift) and a correction sweep, and once the check marks a shift done
+// is bounded (kIrMax corrections); each step is a residual kernel, whose last CTA of a shift
+// runs the convergence check, and a correction sweep, and once the check marks a shift done
 // the remaining work of that shift is skipped (kernels return at once when every
 // shift is done).
 constexpr int kIrMax = 6;
@@ -1221,26 +1280,29 @@ int kore_apply_inverse(kore_plan *p, const double2 *b, double2 *x, double tol, u
                        const double *shift_tols) {
     if (!p->factored) return KORE_ENOTFACTORED;
     double *bn = p->d_bn, *rn = p->d_rn;
-    KORE_TRY(absmax(p, b, bn, p->d_part));
-    if (p->prec != KORE_PREC_MIXED) return sweep(p, b, bn, x, 0, nullptr, live_mask);
-    if (!(tol > 0.0)) tol = 1e-14;
-    ShiftTols tols{};
-    tols.valid = shift_tols ? 1 : 0;
-    for (int s = 0; s < 32 && shift_tols && s < p->nshift; ++s) tols.t[s] = (shift_tols[s] > 0.0) ? shift_tols[s] : tol;
     const int ns = p->nshift;
-    const int skip_stride = (int)(sizeof(IrState) / sizeof(int));
-    k_ir_begin<<<1, ns, 0, p->stream>>>(p->d_ir, ns, live_mask);
+    const bool mixed = p->prec == KORE_PREC_MIXED;
+    k_begin<<<dim3(begin_grid(p), ns), 256, 0, p->stream>>>(p->np, b, p->d_part, bn, p->d_tick, p->d_sweep, vec_bytes(p),
+                                                            mixed ? p->d_ir : nullptr, live_mask);
     KORE_LAUNCHED(1);
     KORE_TRY(sweep(p, b, bn, x, 0, nullptr, live_mask));
+    if (!mixed) return KORE_OK;
+    if (!(tol > 0.0)) tol = 1e-14;
+    IrCheck chk{};
+    chk.ir = p->d_ir; chk.bnorm = bn; chk.minf = p->d_minf; chk.rn = rn; chk.tol = tol;
+    chk.tick = p->d_tick; chk.vecs = p->d_sweep; chk.vbytes = vec_bytes(p);
+    chk.tols.valid = shift_tols ? 1 : 0;
+    for (int s = 0; s < 32 && shift_tols && s < p->nshift; ++s)
+        chk.tols.t[s] = (shift_tols[s] > 0.0) ? shift_tols[s] : tol;
+    const int skip_stride = (int)(sizeof(IrState) / sizeof(int));
     const unsigned grid = spmv_grid(p);
     SpmvArgs ra = spmv_args(p, 2, x, p->d_rb);
     ra.sig = p->d_sigma; ra.rhs = b; ra.part = p->d_part; ra.skip = &p->d_ir->done; ra.skip_stride = skip_stride;
     ra.live_mask = live_mask;
     for (int it = 0; it < kIrMax; ++it) {
         if (p->prof) KORE_TRY(kore_prof_mark(p, 2, true));
-        k_spmv<<<dim3(grid, ns), 256, spmv_smem(p), p->stream>>>(ra);
-        k_ir_check<<<ns, 1024, 0, p->stream>>>(p->d_part, (int)grid, bn, p->d_minf, tol, tols, p->d_ir, rn);
-        KORE_LAUNCHED(2);
+        k_spmv<<<dim3(grid, ns), 256, spmv_smem(p), p->stream>>>(ra, chk);
+        KORE_LAUNCHED(1);
         if (p->prof) KORE_TRY(kore_prof_mark(p, 2, false));
         KORE_TRY(sweep(p, p->d_rb, rn, x, 1, &p->d_ir->done, live_mask));
     }
@@ -1251,19 +1313,25 @@ int kore_apply_inverse(kore_plan *p, const double2 *b, double2 *x, double tol, u
 }
 
 int kore_ir_reset(kore_plan *p) {
-    // everything but the lifetime sweep counter of shift 0
-    for (int s = 0; s < std::max(1, p->nshift); ++s)
-        KORE_CUDA_TRY(cudaMemsetAsync(p->d_ir + s, 0, offsetof(IrState, sweeps_total), p->stream));
+    // everything but the lifetime sweep counters
+    KORE_CUDA_TRY(cudaMemset2DAsync(p->d_ir, sizeof(IrState), 0, offsetof(IrState, sweeps_total), std::max(1, p->nshift),
+                                    p->stream));
     return KORE_OK;
 }
 
 // Aggregate over the factorised shifts: sweep counts of shift 0 (every launch counts
 // there), worst refinement count and eta, NaN in any shift.
-int kore_ir_read(kore_plan *p, IrState *out) {
+int kore_ir_read(kore_plan *p, IrState *out, int *err) {
+    // through the plan's pinned buffer, with the error flag: one wait
     const int ns = std::max(1, p->nshift);
     std::vector<IrState> all(ns);
-    KORE_CUDA_TRY(cudaMemcpyAsync(all.data(), p->d_ir, ns * sizeof(IrState), cudaMemcpyDeviceToHost, p->stream));
+    const size_t bytes = ns * sizeof(IrState);
+    IrState *h = 8 + bytes <= 8192 * sizeof(double) ? reinterpret_cast<IrState *>(p->h_red + 1) : all.data();
+    KORE_CUDA_TRY(cudaMemcpyAsync(h, p->d_ir, bytes, cudaMemcpyDeviceToHost, p->stream));
+    if (err) KORE_CUDA_TRY(cudaMemcpyAsync(p->h_red, p->d_err, sizeof(int), cudaMemcpyDeviceToHost, p->stream));
     KORE_CUDA_TRY(cudaStreamSynchronize(p->stream));
+    if (h != all.data()) memcpy(all.data(), h, bytes);
+    if (err) *err = *reinterpret_cast<int *>(p->h_red);
     *out = all[0];
     for (int s = 1; s < ns; ++s) {
         out->nan |= all[s].nan;
@@ -1286,7 +1354,7 @@ int kore_ir_read(kore_plan *p, IrState *out) {
 // norm partials, the refinement state, the sweep's completion counters and the error
 // flag) lives in the file-scope array below instead of in buffers of the plan or of a
 // caller.  Its size
-// is fixed at kNoAllocMaxNp padded unknowns (about 1.6 MB, held by every GPU that
+// is fixed at kNoAllocMaxNp padded unknowns (about 2 MB, held by every GPU that
 // loads the library until the process exits); larger problems are rejected.
 // The kernels are the ones of kore_solve_dev; only their scratch pointers differ.
 namespace {
@@ -1307,6 +1375,7 @@ struct NoAllocScratch {
     double red[2048 + 8];                  // ||b||_inf partials [0, 2048), then scalars
     IrState ir;
     int err;
+    unsigned tick;
 };
 
 static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
@@ -1333,44 +1402,40 @@ int noalloc_scratch(int device, NoAllocScratch **out) {
     return KORE_OK;
 }
 
+// The launch is prepared per call, not kept in the plan: calls with scratches of their own
+// may come from several threads.
 template <typename C>
-int noalloc_sweep(kore_plan *p, NoAllocScratch *s, const double2 *b, const double *bnorm, double2 *x, int accumulate,
-                  const int *skip, cudaStream_t st) {
-    SweepArgs a = sweep_args(p, 1);   // shift 0
-    a.b = b; a.bnorm = bnorm;
-    a.vecs = s->vecs;
-    a.out = x; a.accumulate = accumulate; a.err = &s->err;
-    a.skip = skip; a.skip_stride = 0; a.count = &s->ir.sweeps; a.count_total = &s->ir.sweeps_total;
-    return launch_sweep<C>(p, a, st, p->sweep_cps > 0 ? TmaVariant{p->sweep_cps, p->sweep_chunk} : kTmaDefault);
-}
-
 int noalloc_solve(kore_plan *p, NoAllocScratch *s, const double2 *b_dev, double2 *x_dev, double tol, cudaStream_t st) {
     const bool mixed = p->prec == KORE_PREC_MIXED;
-    const unsigned g = std::min<unsigned>(kore_div_up(p->np, 256), 1024u);
     double *bn = s->red + 2048, *rn = s->red + 2049;
-    // every call starts from a cleared error flag and refinement state
-    KORE_CUDA_TRY(cudaMemsetAsync(&s->err, 0, sizeof(int), st));
+    SweepLaunch l;
+    KORE_TRY(prepare_sweep<C>(p, p->sweep_cps > 0 ? TmaVariant{p->sweep_cps, p->sweep_chunk} : kTmaDefault, 1, l));
+    SweepArgs a = sweep_args(p, 1);   // shift 0
+    a.b = s->bp; a.bnorm = bn;
+    a.vecs = s->vecs;
+    a.out = s->xp; a.accumulate = 0; a.err = &s->err;
+    a.skip = nullptr; a.skip_stride = 0; a.count = &s->ir.sweeps; a.count_total = &s->ir.sweeps_total;
+    // every call starts from a cleared error flag, tick and refinement state
+    KORE_CUDA_TRY(cudaMemsetAsync(&s->err, 0, 2 * sizeof(int), st));
     KORE_CUDA_TRY(cudaMemsetAsync(&s->ir, 0, sizeof(IrState), st));
     k_gather<<<std::min<unsigned>(kore_div_up(p->np, 256), 2048u), 256, 0, st>>>(p->np, p->n, p->d_slot2orig, b_dev,
                                                                                  s->bp);
-    k_absmax<<<g, 256, 0, st>>>(p->np, s->bp, s->red);
-    k_reduce_max<<<1, 1024, 0, st>>>(s->red, (int)g, bn);
-    KORE_LAUNCHED(3);
-    if (!mixed) {
-        KORE_TRY(noalloc_sweep<double2>(p, s, s->bp, bn, s->xp, 0, nullptr, st));
-    } else {
-        if (!(tol > 0.0)) tol = 1e-14;
-        k_ir_begin<<<1, 1, 0, st>>>(&s->ir, 1, ~0u);
-        KORE_LAUNCHED(1);
-        KORE_TRY(noalloc_sweep<float2>(p, s, s->bp, bn, s->xp, 0, nullptr, st));
+    k_begin<<<kore_div_up(p->np, 256), 256, 0, st>>>(p->np, s->bp, s->red, bn, &s->tick, s->vecs, vec_bytes(p),
+                                                     mixed ? &s->ir : nullptr, ~0u);
+    KORE_LAUNCHED(2);
+    KORE_TRY(launch_prepared<C>(l, a, p->num_sms, st));
+    if (mixed) {
         const unsigned grid = spmv_grid(p);
         SpmvArgs ra = spmv_args(p, 2, s->xp, s->r);
         ra.lam = mk(p->sigma_re, p->sigma_im); ra.rhs = s->bp; ra.part = s->part; ra.skip = &s->ir.done;
+        IrCheck chk{};
+        chk.ir = &s->ir; chk.bnorm = bn; chk.minf = p->d_minf; chk.rn = rn; chk.tol = tol > 0.0 ? tol : 1e-14;
+        chk.tick = &s->tick; chk.vecs = s->vecs; chk.vbytes = vec_bytes(p);
+        a.b = s->r; a.bnorm = rn; a.accumulate = 1; a.skip = &s->ir.done;
         for (int it = 0; it < kIrMax; ++it) {
-            k_spmv<<<grid, 256, spmv_smem(p), st>>>(ra);
-            k_ir_check<<<1, 1024, 0, st>>>(s->part, (int)grid, bn, p->d_minf, tol, ShiftTols{}, &s->ir, rn);
-            KORE_LAUNCHED(2);
-            KORE_TRY(noalloc_sweep<float2>(p, s, s->r, rn, s->xp, 1, &s->ir.done, st));
+            k_spmv<<<grid, 256, spmv_smem(p), st>>>(ra, chk);
+            KORE_LAUNCHED(1);
+            KORE_TRY(launch_prepared<C>(l, a, p->num_sms, st));
         }
     }
     k_scatter<<<std::min<unsigned>(kore_div_up(p->np, 256), 2048u), 256, 0, st>>>(p->np, p->n, p->d_slot2orig, s->xp,
@@ -1387,7 +1452,7 @@ extern "C" int kore_solve_dev_noalloc(kore_plan *p, const void *b_dev, void *x_d
     if (p->np > kNoAllocMaxNp || (int64_t)(p->nlev > 0 ? 3 * p->nlev + 2 : 1) * p->K > kNoAllocMaxCnt) {
         std::fprintf(stderr,
                      "kore_solve_dev_noalloc: %lld padded unknowns in %d blocks exceed the fixed scratch "
-                     "(%lld unknowns, %lld block counters); use kore_solve_dev\n",
+                     "(%lld unknowns, %lld block entries); use kore_solve_dev\n",
                      (long long)p->np, p->K, (long long)kNoAllocMaxNp, (long long)kNoAllocMaxCnt);
         return KORE_EINVAL;
     }
@@ -1403,8 +1468,11 @@ extern "C" int kore_solve_dev_noalloc(kore_plan *p, const void *b_dev, void *x_d
     NoAllocScratch *s = nullptr;
     int rc = noalloc_scratch(p->device, &s);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (rc == KORE_OK) rc = noalloc_solve(p, s, static_cast<const double2 *>(b_dev), static_cast<double2 *>(x_dev),
-                                          refine_tol, st);
+    const double2 *b = static_cast<const double2 *>(b_dev);
+    double2 *x = static_cast<double2 *>(x_dev);
+    if (rc == KORE_OK)
+        rc = p->prec == KORE_PREC_MIXED ? noalloc_solve<float2>(p, s, b, x, refine_tol, st)
+                                        : noalloc_solve<double2>(p, s, b, x, refine_tol, st);
     if (rc == KORE_OK) {
         // wait for this call's kernels, then read its error flag and NaN state
         int flags[2] = {0, 0};
