@@ -354,10 +354,52 @@ __global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0, int nb, int str
 // and walks the rows in chunks of 128: a thread holds 4 rows x TW / 8 columns, so that
 // one step of the sum costs 4 + TW / 8 shared-memory loads for TW / 2 complex products
 // and FP32 arithmetic, not shared memory, is the bound (complex128: the FP64 pipe).
+// The last chunk computes only the 32-row groups that it has (S = 400 has 13 of 16: one
+// solve of the 240k-unknown shell 40.7 -> 39.1 ms).  Packed FP32 pairs instead of single
+// multiply-adds were slower (72k-unknown shell, 16 shifts: 16.7 ms in this kernel against 13.6),
+// as the pivot rows then take twice the shared-memory reads.
 constexpr int kUpdRows = 128;
+
+// NI groups of 32 rows from r0 on: the sums of the panel's columns, added and stored
+template <typename C, int NB, int TW, int NI, typename Column>
+__device__ __forceinline__ void update_rows(const C *src, C *T, const C (*es)[kUpdRows], const C (*tp)[TW],
+                                            const int *used, int S, int r0, int k0, int nb, int nt, Column column) {
+    constexpr int CT = TW / 8;   // columns per thread
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    C acc[NI][CT];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        const int r = r0 + tx + 32 * i;
+        // a pivot row of the panel starts from zero
+        const bool keep = r < S && !(used[r] > k0 && used[r] <= k0 + nb);
+#pragma unroll
+        for (int t = 0; t < CT; ++t)
+            acc[i][t] = (keep && ty * CT + t < nt) ? src[r + (int64_t)column(ty * CT + t) * S] : czero<C>();
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int c = 0; c < NB; ++c) {
+        C e[NI], t4[CT];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) e[i] = es[c][tx + 32 * i];
+#pragma unroll
+        for (int t = 0; t < CT; ++t) t4[t] = tp[c][ty * CT + t];
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+#pragma unroll
+            for (int t = 0; t < CT; ++t) acc[i][t] = cfma(acc[i][t], e[i], t4[t]);
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        const int r = r0 + tx + 32 * i;
+#pragma unroll
+        for (int t = 0; t < CT; ++t)
+            if (r < S && ty * CT + t < nt) T[r + (int64_t)column(ty * CT + t) * S] = acc[i][t];
+    }
+}
+
 template <typename C, int NB, int TW>
 __global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb, int c0, int c1, int stride) {
-    constexpr int CT = TW / 8;   // columns per thread
     __shared__ __align__(16) C tp[NB][TW];
     __shared__ __align__(16) C es[NB][kUpdRows];
     const int S = v.S;
@@ -366,50 +408,23 @@ __global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb, int c0,
     const C *src = k0 == 0 ? diag_block(v, o, sh, stride) : T;
     const int *piv = v.piv + sh * v.p_stride + o * S, *used = v.used + sh * v.p_stride + o * S;
     // columns of this CTA, counted from c0 without the panel's own
-    const int j0 = blockIdx.x * TW, ncols = c1 - c0 - nb;
+    const int j0 = blockIdx.x * TW, nt = c1 - c0 - nb - j0;
     auto column = [&](int t) { const int j = c0 + j0 + t; return j < k0 ? j : j + nb; };
     for (int idx = threadIdx.x; idx < TW * NB; idx += 256) {
         const int c = idx % NB, t = idx / NB;
-        tp[c][t] = (j0 + t < ncols && c < nb) ? src[piv[k0 + c] + (int64_t)column(t) * S] : czero<C>();
+        tp[c][t] = (t < nt && c < nb) ? src[piv[k0 + c] + (int64_t)column(t) * S] : czero<C>();
     }
     const C *E = T + (int64_t)k0 * S;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     for (int r0 = 0; r0 < S; r0 += kUpdRows) {
         __syncthreads();
         for (int idx = threadIdx.x; idx < NB * kUpdRows; idx += 256) {
             const int rr = idx % kUpdRows, c = idx / kUpdRows;
             es[c][rr] = (r0 + rr < S && c < nb) ? E[r0 + rr + (int64_t)c * S] : czero<C>();
         }
-        C acc[4][CT];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = r0 + tx + 32 * i;
-            // a pivot row of the panel starts from zero
-            const bool keep = r < S && !(used[r] > k0 && used[r] <= k0 + nb);
-#pragma unroll
-            for (int t = 0; t < CT; ++t)
-                acc[i][t] = (keep && j0 + ty * CT + t < ncols) ? src[r + (int64_t)column(ty * CT + t) * S] : czero<C>();
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int c = 0; c < NB; ++c) {
-            C e[4], t4[CT];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) e[i] = es[c][tx + 32 * i];
-#pragma unroll
-            for (int t = 0; t < CT; ++t) t4[t] = tp[c][ty * CT + t];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int t = 0; t < CT; ++t) acc[i][t] = cfma(acc[i][t], e[i], t4[t]);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = r0 + tx + 32 * i;
-#pragma unroll
-            for (int t = 0; t < CT; ++t)
-                if (r < S && j0 + ty * CT + t < ncols) T[r + (int64_t)column(ty * CT + t) * S] = acc[i][t];
-        }
+        if (S - r0 > 96) update_rows<C, NB, TW, 4>(src, T, es, tp, used, S, r0, k0, nb, nt, column);
+        else if (S - r0 > 64) update_rows<C, NB, TW, 3>(src, T, es, tp, used, S, r0, k0, nb, nt, column);
+        else if (S - r0 > 32) update_rows<C, NB, TW, 2>(src, T, es, tp, used, S, r0, k0, nb, nt, column);
+        else update_rows<C, NB, TW, 1>(src, T, es, tp, used, S, r0, k0, nb, nt, column);
     }
 }
 
