@@ -463,9 +463,10 @@ __device__ __forceinline__ double2 couple(double2 acc, double2 a, double2 b) {
 // row's coupling entries once, as padded rows (the level-0 rows of the sweep, with the row
 // scale folded in), and accumulates the CW columns in registers.  The CW columns of the
 // four matrices are staged in shared memory: an entry (about 30 per row) costs 2 CW reads
-// of them, and gathered from L2 those reads were what the kernel took its time for
-// (14.0 ms for 16 shifts of the 72k-unknown shell in complex64; complex128 is bound by
-// the FP64 pipe).
+// of them, which gathered from L2 took 14.0 ms for 16 shifts of the 72k-unknown shell in
+// complex64.  What was left was the wait for the entries, 15 of 20 stalled warps: loaded one
+// batch ahead they took it from 7.3 to 4.1 ms (complex128 is bound by the FP64 pipe, and
+// deeper batches only cost it registers: four shifts 8.5 ms with 1, 9.4 with 4).
 template <typename C, int CW>
 __global__ void __launch_bounds__(512) k_even_l0(FV<C> v, BcrLevel lv) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -499,11 +500,20 @@ __global__ void __launch_bounds__(512) k_even_l0(FV<C> v, BcrLevel lv) {
 #pragma unroll
         for (int t = 0; t < CW; ++t) dsum[t] = lsum[t] = usum[t] = czero<C>();
         const int64_t ebase = ((q * ntile + r / 32) * (int64_t)v.ell_w) * 32 + (r & 31);
-#pragma unroll 4
-        for (int k = 0; k < v.ell_w; ++k) {
-            const int col = v.ell_col[ebase + (int64_t)k * 32];
-            const C a = ev[ebase + (int64_t)k * 32];
-            if (col < 0) continue;
+        // kAhead entries are loaded while the kAhead before them are summed (ell_w is a
+        // multiple of 8)
+        constexpr int kAhead = sizeof(C) == 8 ? 4 : 1;
+        int ncol[kAhead];
+        C na[kAhead];
+        auto load = [&](int k) {
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                ncol[u] = k < v.ell_w ? v.ell_col[ebase + (int64_t)(k + u) * 32] : -1;
+                if (k < v.ell_w) na[u] = ev[ebase + (int64_t)(k + u) * 32];
+            }
+        };
+        auto sum = [&](int col, C a) {
+            if (col < 0) return;
             if (col < first) {   // left neighbour j = q - 1
                 const C *x = sm + (col - first + S);
 #pragma unroll
@@ -519,6 +529,19 @@ __global__ void __launch_bounds__(512) k_even_l0(FV<C> v, BcrLevel lv) {
                     if (outr) usum[t] = couple(usum[t], a, x[(CW + t) * S]);
                 }
             }
+        };
+        load(0);
+        for (int k = 0; k < v.ell_w; k += kAhead) {
+            int col[kAhead];
+            C a[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                col[u] = ncol[u];
+                a[u] = na[u];
+            }
+            load(k + kAhead);
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) sum(col[u], a[u]);
         }
 #pragma unroll
         for (int t = 0; t < CW; ++t)
@@ -647,11 +670,14 @@ int factor_levels(kore_plan *p) {
             k_gh_l0<C><<<dim3(kore_div_up(S, kGhCW), lv.nodd, ns), th, 0, st>>>(v);
             KORE_LAUNCHED(1);
             if (sizeof(C) == sizeof(float2)) KORE_TRY(kore_gh_update_tc(p, lv, 1));
-            // columns per CTA: 8 while four blocks of 8 columns leave room for two CTAs per SM
-            // in shared memory (S = 400 in complex64: 102 KB), else fewer
+            // columns per CTA: 4 while they leave room for two CTAs per SM in shared memory
+            // (S = 800 in complex64: 102 KB), else 2.  8 took 97 registers in complex64, which
+            // left too few warps to cover the entries' loads: 6.0 against 4.1 ms for 16 shifts
+            // of the 72k-unknown shell, 2.7 against 1.7 ms for one of the 240k-unknown shell;
+            // 2 took 5.3 and 2.2 ms.
             const size_t per = (size_t)4 * S * sizeof(C);
-            const int cw = 8 * per <= 110 * 1024 ? 8 : 4 * per <= 110 * 1024 ? 4 : 2;
-            auto even = cw == 8 ? k_even_l0<C, 8> : cw == 4 ? k_even_l0<C, 4> : k_even_l0<C, 2>;
+            const int cw = 4 * per <= 110 * 1024 ? 4 : 2;
+            auto even = cw == 4 ? k_even_l0<C, 4> : k_even_l0<C, 2>;
             KORE_TRY(kore_allow_max_dyn_smem(even, p->device));
             even<<<dim3(kore_div_up(S, cw), lv.neven, ns), th, cw * per, st>>>(v, lv);
             KORE_LAUNCHED(1);
