@@ -416,9 +416,8 @@ static int tc_upload_run(kore_plan *p, const std::vector<TcJob> &jobs) {
     return tc_run(p->stream, p->device, p->S, static_cast<const TcJob *>(p->d_tctab), (int)jobs.size(), p->d_err);
 }
 
-// Even-block update of level l >= 1 for every shift (complex64 factors), the
-// tensor-core form of k_even_gemm: D_i -= L_q H_jl + U_q G_jr;  L' = -L_q G_jl;
-// U' = -U_q H_jr.
+// Even-block update of level l >= 1 for every shift (complex64 factors):
+// D_i -= L_q H_jl + U_q G_jr;  L' = -L_q G_jl;  U' = -U_q H_jr.
 int kore_even_update_tc(kore_plan *p, const BcrLevel &lv) {
     const int S = p->S, ns = p->fw_n;
     const int64_t lo = p->fw_lo;   // shift sh of the factor window is shift lo + sh of the plan
