@@ -273,39 +273,84 @@ __device__ __forceinline__ const C *diag_block(const FV<C> &v, int64_t o, int64_
 // product; here it is two barriers, an integer search and one broadcast load per two
 // columns.  The first panel and its update
 // read the diagonal block itself, which stays as it is.
+// With Helper (up to 512 rows) one more warp shortens the chain: a step updates the next
+// pivot column first and hands its candidates over, and while the row warps update the
+// other columns the helper picks the pivot and inverts it.
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+constexpr int panel_threads(int rows) { return rows <= 512 ? rows + 32 : rows; }
+
 template <typename C, int NB, int MAXT>
-__global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0, int nb, int stride) {
+__global__ void __launch_bounds__(panel_threads(MAXT)) k_panel(FV<C> v, int k0, int nb, int stride) {
+    constexpr bool Helper = MAXT <= 512;
     __shared__ __align__(16) C prow[NB];
+    __shared__ __align__(16) C wval[32];
+    __shared__ C s_inv;
     __shared__ unsigned long long wkey[32];
     __shared__ int wrow[32];
-    __shared__ int s_piv[NB];
+    __shared__ int s_piv[NB], s_p;
     const int S = v.S;
     const int64_t o = blockIdx.x, sh = blockIdx.y;
     C *T = v.T + sh * v.t_stride + o * v.t_block + (int64_t)k0 * S;
     const C *src = k0 == 0 ? diag_block(v, o, sh, stride) : T;
     int *piv = v.piv + sh * v.p_stride + o * S;
     int *used = v.used + sh * v.p_stride + o * S;
-    const int r = threadIdx.x, lane = r & 31, w = r >> 5, nw = blockDim.x >> 5;
-    const bool in = r < S;
+    const int threads = blockDim.x;
+    const int r = threadIdx.x, lane = r & 31, w = r >> 5, nw = (threads >> 5) - (Helper ? 1 : 0);
 
+    // the largest candidate: its row, or -1 when there is none; with inv also its inverse
+    auto choose = [&](C *inv) {
+        int wl;
+        const unsigned long long best = warp_argmax<C>(lane < nw ? wkey[lane] : 0ull, wl);
+        if (best == 0ull) return -1;
+        if (inv) *inv = inverse(wval[wl]);
+        return wrow[wl];
+    };
+    if (Helper && w == nw) {
+        for (int c = 0; c < nb; ++c) {
+            bar_sync(1, threads);   // the candidates of column c
+            C inv = czero<C>();
+            const int p = choose(&inv);
+            if (lane == 0) {
+                s_p = p;
+                s_inv = inv;
+            }
+            bar_sync(0, threads);
+            if (p < 0) break;
+            bar_sync(0, threads);
+        }
+        return;
+    }
+
+    const bool in = r < S;
     C P[NB];
 #pragma unroll
     for (int c = 0; c < NB; ++c) P[c] = (in && c < nb) ? src[r + (int64_t)c * S] : czero<C>();
     int mine = (in && k0 != 0) ? used[r] : 0;   // 1 + the column this row is the pivot of, or 0
     bool u = !in || mine != 0;
+    auto propose = [&](C x) {   // this warp's candidate for the next pivot
+        int l;
+        const unsigned long long k = warp_argmax<C>(u ? 0ull : pivot_key(x), l);
+        if (lane == l) {
+            wkey[w] = k;
+            wrow[w] = r;
+            wval[w] = x;
+        }
+        if (Helper) bar_arrive(1, threads);
+    };
+    propose(P[0]);
     int c = 0;
     for (; c < nb; ++c) {
-        int l;
-        const unsigned long long k = warp_argmax<C>(u ? 0ull : pivot_key(P[0]), l);
-        if (lane == 0) { wkey[w] = k; wrow[w] = w * 32 + l; }
-        __syncthreads();
-        int wl;
-        const unsigned long long best = warp_argmax<C>(lane < nw ? wkey[lane] : 0ull, wl);
-        if (best == 0ull) {   // uniform over the CTA
+        bar_sync(0, threads);
+        const int p = Helper ? s_p : choose(nullptr);
+        if (p < 0) {   // uniform over the CTA
             if (r == 0) atomicCAS(v.err, 0, KORE_DEVERR_PIVOT);
             break;
         }
-        const int p = wrow[wl];
         if (w == p >> 5) {   // the pivot row's warp publishes the row, scaled by 1 / pivot
             if (r == p) {
                 u = true;
@@ -315,20 +360,22 @@ __global__ void __launch_bounds__(MAXT) k_panel(FV<C> v, int k0, int nb, int str
                 for (int q = 0; q < NB; ++q) prow[q] = P[q];
             }
             __syncwarp();
-            const C dinv = inverse(prow[0]);
+            const C dinv = Helper ? s_inv : inverse(prow[0]);
             const C own = lane < NB ? prow[lane] : czero<C>();
             __syncwarp();
             if (lane < NB) prow[lane] = lane == 0 ? dinv : own * dinv;
         }
-        __syncthreads();
+        bar_sync(0, threads);
         const C dinv = prow[0], mult = P[0];
+        P[0] = r == p ? prow[1] : cfms(P[1], mult, prow[1]);
+        if (c + 1 < nb) propose(P[0]);
         if (r == p) {
 #pragma unroll
-            for (int q = 1; q < NB; ++q) P[q - 1] = prow[q];
+            for (int q = 2; q < NB; ++q) P[q - 1] = prow[q];
             P[NB - 1] = dinv;
         } else {
 #pragma unroll
-            for (int q = 1; q < NB; ++q) P[q - 1] = cfms(P[q], mult, prow[q]);
+            for (int q = 2; q < NB; ++q) P[q - 1] = cfms(P[q], mult, prow[q]);
             P[NB - 1] = -(mult * dinv);
         }
     }
@@ -627,7 +674,7 @@ int gauss_jordan(kore_plan *p, const FV<C> &v, const BcrLevel &lv, int nodd, int
         const int g1 = std::min(S, g0 + group);
         for (int k0 = g0; k0 < g1; k0 += NB) {
             const int nb = std::min(NB, g1 - k0), ncols = g1 - g0 - nb;
-            k_panel<C, NB, MAXT><<<dim3(nodd, nshift), pthreads, 0, p->stream>>>(v, k0, nb, lv.stride);
+            k_panel<C, NB, MAXT><<<dim3(nodd, nshift), panel_threads(pthreads), 0, p->stream>>>(v, k0, nb, lv.stride);
             KORE_LAUNCHED(1);
             if (ncols == 0) continue;
             // 32 columns per CTA re-read the panel least; levels with few blocks take 8, so
