@@ -263,6 +263,14 @@ __device__ __forceinline__ const C *diag_block(const FV<C> &v, int64_t o, int64_
     return v.Dw + sh * v.f_stride + (2 * o + 1) * stride * (int64_t)v.S * v.S;
 }
 
+// A kernel that launch_chained() launches calls after_previous() before it touches memory,
+// as its CTAs may start while the launch before it in the stream runs, and before_next() once
+// its main loop is done: the next launch's CTAs then take the places that become free, and
+// wait there.  (Called at the start instead, they held places from the kernel's own CTAs:
+// four FP64 shifts of the 72k-unknown shell 94.6 -> 95.8 ms.)
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void before_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Panel reduction of columns [k0, k0+nb) of T_o; one CTA per (odd block o = blockIdx.x,
 // shift = blockIdx.y), one thread per row, which holds its NB entries of the panel in
 // registers.  Every elimination step works on register 0 and shifts the others down by
@@ -301,6 +309,7 @@ __global__ void __launch_bounds__(panel_threads(MAXT)) k_panel(FV<C> v, int k0, 
     int *used = v.used + sh * v.p_stride + o * S;
     const int threads = blockDim.x;
     const int r = threadIdx.x, lane = r & 31, w = r >> 5, nw = (threads >> 5) - (Helper ? 1 : 0);
+    after_previous();
 
     // the largest candidate: its row, or -1 when there is none; with inv also its inverse
     auto choose = [&](C *inv) {
@@ -379,6 +388,7 @@ __global__ void __launch_bounds__(panel_threads(MAXT)) k_panel(FV<C> v, int k0, 
             P[NB - 1] = -(mult * dinv);
         }
     }
+    before_next();
     const int done = c;
     if (in) {
         if (done == nb) {
@@ -455,6 +465,7 @@ __global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb, int c0,
     const C *src = k0 == 0 ? diag_block(v, o, sh, stride) : T;
     const int *piv = v.piv + sh * v.p_stride + o * S, *used = v.used + sh * v.p_stride + o * S;
     // columns of this CTA, counted from c0 without the panel's own
+    after_previous();
     const int part = blockIdx.x % split;
     const int j0 = blockIdx.x / split * TW, nt = c1 - c0 - nb - j0;
     auto column = [&](int t) { const int j = c0 + j0 + t; return j < k0 ? j : j + nb; };
@@ -476,6 +487,7 @@ __global__ void __launch_bounds__(256) k_update(FV<C> v, int k0, int nb, int c0,
         else if (S - r0 > 32) update_rows<C, NB, TW, 2>(src, T, es, tp, used, S, r0, k0, nb, nt, column);
         else update_rows<C, NB, TW, 1>(src, T, es, tp, used, S, r0, k0, nb, nt, column);
     }
+    before_next();
 }
 
 // The inverse from the reduced work matrix: row piv[k] of T is row k of the inverse and
@@ -655,23 +667,24 @@ unsigned grid_for(int64_t work, int threads, int num_sms) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>((work + threads - 1) / threads, 16LL * num_sms));
 }
 
-template <typename C, int NB>
-int launch_update(kore_plan *p, const FV<C> &v, int k0, int nb, int g0, int g1, int stride, int nodd, int nshift) {
-    const int ncols = g1 - g0 - nb;
-    const bool wide = (int64_t)nodd * nshift * kore_div_up(ncols, 32) >= 2 * p->num_sms;
-    const int split = wide ? 1 : (int)kore_div_up(p->S, kUpdRows);   // at most 8, a portable cluster
+// Launch of a kernel that begins with after_previous(): it is set up while the kernel before
+// it in the stream still runs, and split CTAs along x form a cluster.
+template <typename... P, typename... A>
+int launch_chained(kore_plan *p, void (*kern)(P...), dim3 grid, unsigned threads, int split, const A &...args) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(kore_div_up(ncols, wide ? 32 : 8) * split, nodd, nshift);
-    cfg.blockDim = dim3(256);
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
     cfg.stream = p->stream;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = split;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = split > 1 ? 1 : 0;
-    KORE_CUDA_TRY(wide ? cudaLaunchKernelEx(&cfg, k_update<C, NB, 32>, v, k0, nb, g0, g1, stride, split)
-                       : cudaLaunchKernelEx(&cfg, k_update<C, NB, 8>, v, k0, nb, g0, g1, stride, split));
+    cudaLaunchAttribute at[2]{};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = split;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = split > 1 ? 2 : 1;
+    KORE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P(args)...));
+    KORE_LAUNCHED(1);
     return KORE_OK;
 }
 
@@ -697,15 +710,21 @@ int gauss_jordan(kore_plan *p, const FV<C> &v, const BcrLevel &lv, int nodd, int
         const int g1 = std::min(S, g0 + group);
         for (int k0 = g0; k0 < g1; k0 += NB) {
             const int nb = std::min(NB, g1 - k0), ncols = g1 - g0 - nb;
-            k_panel<C, NB, MAXT><<<dim3(nodd, nshift), panel_threads(pthreads), 0, p->stream>>>(v, k0, nb, lv.stride);
-            KORE_LAUNCHED(1);
+            KORE_TRY(launch_chained(p, k_panel<C, NB, MAXT>, dim3(nodd, nshift), panel_threads(pthreads), 1, v, k0, nb,
+                                    lv.stride));
             if (ncols == 0) continue;
             // 32 columns per CTA re-read the panel least; levels with few blocks take 8, so
             // that their CTAs still cover the GPU, and share the row chunks among a cluster's
             // CTAs, as a chunk then is a chain of loads and a few products (two shifts of the MAC
             // shell, S = 360: 9.37 -> 9.31 ms; the 240k-unknown shell: 38.4 -> 38.2 ms)
-            KORE_TRY((launch_update<C, NB>(p, v, k0, nb, g0, g1, lv.stride, nodd, nshift)));
-            KORE_LAUNCHED(1);
+            if ((int64_t)nodd * nshift * kore_div_up(ncols, 32) >= 2 * p->num_sms) {
+                KORE_TRY(launch_chained(p, k_update<C, NB, 32>, dim3(kore_div_up(ncols, 32), nodd, nshift), 256, 1, v, k0, nb,
+                                        g0, g1, lv.stride, 1));
+            } else {
+                const int split = (int)kore_div_up(S, kUpdRows);   // at most 8, a portable cluster
+                KORE_TRY(launch_chained(p, k_update<C, NB, 8>, dim3(kore_div_up(ncols, 8) * split, nodd, nshift), 256,
+                                        split, v, k0, nb, g0, g1, lv.stride, split));
+            }
         }
         if (g1 - g0 < S) KORE_TRY(kore_group_update_oz(p, lv, nodd, g0, g1));
     }
