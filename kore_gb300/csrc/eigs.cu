@@ -487,13 +487,14 @@ __device__ __forceinline__ double warp_transpose_sum16(double (&v)[16], int lane
 // run (may be null): target t returns at once unless run[t] != 0.  grid.z shares the chunks of
 // columns: with few rows the products of one SM's FP64 pipe are the time (1,920 rows, 40
 // columns: 28 us on 8 CTAs, 10 us with the chunks on CTAs of their own; the same sums).
-__global__ void __launch_bounds__(kDotThreads) k_mdot(int64_t np, TVec V, TVec w, double2 *__restrict__ partial0,
-                                                      int with_norm, const int *__restrict__ run, TCols tc) {
+__global__ void __launch_bounds__(kDotThreads) k_mdot(int64_t np, TVec V, TVec w, double2 *partial0,
+                                                      int with_norm, const int *run, TCols tc) {
+    after_previous();
     const int tg = blockIdx.y;
     if (!in_mask(tc.mask, tg) || (run && run[tg] == 0)) return;
-    const double2 *__restrict__ Vt = V.p[tg];
-    const double2 *__restrict__ wt = w.p[tg];
-    double2 *__restrict__ partial = partial0 + tg * kPartStride;
+    const double2 *Vt = V.p[tg];
+    const double2 *wt = w.p[tg];
+    double2 *partial = partial0 + tg * kPartStride;
     __shared__ double sm[kDotThreads / 32][2 * kDotChunk];
     const int ncol = tc.n[tg];
     const int nc = ncol + with_norm;
@@ -542,20 +543,22 @@ __global__ void __launch_bounds__(kDotThreads) k_mdot(int64_t np, TVec V, TVec w
         }
         __syncthreads();
     }
+    before_next();
 }
 
 // Target t (grid.y), column c (grid.x): h_t[c] (+)= sum_b partial_t[b*nc + c] with
 // nc = ncol_t + with_norm; returns at once unless run[t] != 0 (when run is given).
-__global__ void k_mdot_reduce(int nblk, const double2 *__restrict__ partial0, int64_t pstride,
-                              double2 *__restrict__ h0, int accumulate, const int *__restrict__ run, TCols tc,
+__global__ void k_mdot_reduce(int nblk, const double2 *partial0, int64_t pstride,
+                              double2 *h0, int accumulate, const int *run, TCols tc,
                               int with_norm) {
+    after_previous();
     const int tg = blockIdx.y;
     if (!in_mask(tc.mask, tg) || (run && run[tg] == 0)) return;
     const int nc = tc.n[tg] + with_norm;
     const int c = blockIdx.x;
     if (c >= nc) return;
-    const double2 *__restrict__ partial = partial0 + tg * pstride;
-    double2 *__restrict__ h = h0 + tg * kHStride;
+    const double2 *partial = partial0 + tg * pstride;
+    double2 *h = h0 + tg * kHStride;
     double2 s = mk(0.0, 0.0);
     for (int b = threadIdx.x; b < nblk; b += blockDim.x) s = s + partial[(int64_t)b * nc + c];
     s = warp_sum(s);
@@ -567,15 +570,17 @@ __global__ void k_mdot_reduce(int nblk, const double2 *__restrict__ partial0, in
         for (int wv = 0; wv < (int)(blockDim.x >> 5); ++wv) t = t + sm[wv];
         h[c] = accumulate ? h[c] + t : t;
     }
+    before_next();
 }
 
 // w_t -= V_t h_t (ncol_t columns); returns at once unless run[t] != 0 (when run is given)
-__global__ void k_mgs_update(int64_t np, TVec V, const double2 *__restrict__ h0, TVec w,
-                             const int *__restrict__ run, TCols tc) {
+__global__ void k_mgs_update(int64_t np, TVec V, const double2 *h0, TVec w,
+                             const int *run, TCols tc) {
+    after_previous();
     const int tg = blockIdx.y;
     if (!in_mask(tc.mask, tg) || (run && run[tg] == 0)) return;
-    const double2 *__restrict__ Vt = V.p[tg];
-    double2 *__restrict__ wt = w.p[tg];
+    const double2 *Vt = V.p[tg];
+    double2 *wt = w.p[tg];
     const int ncol = tc.n[tg];
     __shared__ double2 hs[kMaxNcv + 1];
     for (int c = threadIdx.x; c < ncol; c += blockDim.x) hs[c] = h0[tg * kHStride + c];
@@ -585,16 +590,18 @@ __global__ void k_mgs_update(int64_t np, TVec V, const double2 *__restrict__ h0,
         for (int c = 0; c < ncol; ++c) acc = cfms(acc, Vt[r + (int64_t)c * np], hs[c]);
         wt[r] = acc;
     }
+    before_next();
 }
 
 // The same for few rows: a thread per real or imaginary part, so that twice as many warps,
 // on SMs of their own, share the FP64 work (the same operations in the same order).
-__global__ void __launch_bounds__(128) k_mgs_update_parts(int64_t np, TVec V, const double2 *__restrict__ h0, TVec w,
-                                                          const int *__restrict__ run, TCols tc) {
+__global__ void __launch_bounds__(128) k_mgs_update_parts(int64_t np, TVec V, const double2 *h0, TVec w,
+                                                          const int *run, TCols tc) {
+    after_previous();
     const int tg = blockIdx.y;
     if (!in_mask(tc.mask, tg) || (run && run[tg] == 0)) return;
-    const double2 *__restrict__ Vt = V.p[tg];
-    double *__restrict__ wt = reinterpret_cast<double *>(w.p[tg]);
+    const double2 *Vt = V.p[tg];
+    double *wt = reinterpret_cast<double *>(w.p[tg]);
     const int ncol = tc.n[tg];
     __shared__ double2 hs[kMaxNcv + 1];
     for (int c = threadIdx.x; c < ncol; c += blockDim.x) hs[c] = h0[tg * kHStride + c];
@@ -610,13 +617,15 @@ __global__ void __launch_bounds__(128) k_mgs_update_parts(int64_t np, TVec V, co
         acc = fma(-v.x, im ? h.y : h.x, fma(im ? -v.y : v.y, im ? h.x : h.y, acc));
     }
     wt[i] = acc;
+    before_next();
 }
 
 // partial_t[b] = sum of |w_t|^2 over CTA b's rows (grid.y = target)
-__global__ void k_nrm2_partial(int64_t np, TVec w, double *__restrict__ partial0, unsigned mask) {
+__global__ void k_nrm2_partial(int64_t np, TVec w, double *partial0, unsigned mask) {
+    after_previous();
     const int tg = blockIdx.y;
     if (!in_mask(mask, tg)) return;
-    const double2 *__restrict__ wt = w.p[tg];
+    const double2 *wt = w.p[tg];
     double s = 0.0;
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < np; r += (int64_t)gridDim.x * blockDim.x)
         s += abs2(wt[r]);
@@ -629,6 +638,7 @@ __global__ void k_nrm2_partial(int64_t np, TVec w, double *__restrict__ partial0
         for (int wv = 0; wv < (int)(blockDim.x >> 5); ++wv) t += sm[wv];
         partial0[tg * (int64_t)kGridMax + blockIdx.x] = t;
     }
+    before_next();
 }
 
 // Refinement decision of classical Gram-Schmidt (SLEPc's default, refinement "if needed"
@@ -636,11 +646,12 @@ __global__ void k_nrm2_partial(int64_t np, TVec w, double *__restrict__ partial0
 // the norm after it is sqrt(||w||^2 - sum |h1_c|^2) (exact for orthonormal V); a second
 // pass runs when that is below eta ||w||.  Clears h2, which a skipped second pass leaves
 // untouched.
-__global__ void k_refine_decide(double2 *__restrict__ h0, int *__restrict__ run2, TCols tc) {
+__global__ void k_refine_decide(double2 *h0, int *run2, TCols tc) {
+    after_previous();
     const int tg = blockIdx.x;
     if (!in_mask(tc.mask, tg)) return;
-    const double2 *__restrict__ h1 = h0 + tg * kHStride;
-    double2 *__restrict__ h2 = h0 + tg * kHStride + (kMaxNcv + 1);
+    const double2 *h1 = h0 + tg * kHStride;
+    double2 *h2 = h0 + tg * kHStride + (kMaxNcv + 1);
     const int ncol = tc.n[tg];
     __shared__ double sm[32];
     double s = 0.0;
@@ -657,22 +668,24 @@ __global__ void k_refine_decide(double2 *__restrict__ h0, int *__restrict__ run2
         const double onrm2 = h1[ncol].x;
         run2[tg] = (onrm2 - t < 0.5 * onrm2) ? 1 : 0;
     }
+    before_next();
 }
 
 // One CTA per target: beta_t = sqrt(sum of its partials); with set_col, Hbar_t[j+1, j] =
 // beta_t and h_t (ncol_t entries) becomes column j of Hbar_t (j = tc.j[t], ld tc.ld[t]).
-__global__ void k_finish_col(int nblk, const double *__restrict__ partial0, const double2 *__restrict__ h0,
-                             double2 *__restrict__ Hbar0, double *__restrict__ beta0, TCols tc, int set_col) {
+__global__ void k_finish_col(int nblk, const double *partial0, const double2 *h0,
+                             double2 *Hbar0, double *beta0, TCols tc, int set_col) {
+    after_previous();
     const int tg = blockIdx.x;
     if (!in_mask(tc.mask, tg)) return;
-    const double *__restrict__ partial = partial0 + tg * (int64_t)kGridMax;
+    const double *partial = partial0 + tg * (int64_t)kGridMax;
     __shared__ double sm[32];
     double s = 0.0;
     for (int b = threadIdx.x; b < nblk; b += blockDim.x) s += partial[b];
     s = warp_sum_d(s);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
     __syncthreads();
-    double2 *__restrict__ Hbar = Hbar0 + tg * kHbarStride;
+    double2 *Hbar = Hbar0 + tg * kHbarStride;
     const int j = tc.j[tg], ld = tc.ld[tg];
     if (threadIdx.x == 0) {
         double t = 0.0;
@@ -683,18 +696,21 @@ __global__ void k_finish_col(int nblk, const double *__restrict__ partial0, cons
     }
     if (set_col)
         for (int c = threadIdx.x; c < tc.n[tg]; c += blockDim.x) Hbar[c + (int64_t)j * ld] = h0[tg * kHStride + c];
+    before_next();
 }
 
 // dst_t = src_t / beta_t (beta_t > 0), else 0; src and dst may be the same vector
-__global__ void k_scale_copy(int64_t np, TVec src, const double *__restrict__ beta0, TVec dst, unsigned mask) {
+__global__ void k_scale_copy(int64_t np, TVec src, const double *beta0, TVec dst, unsigned mask) {
+    after_previous();
     const int tg = blockIdx.y;
     if (!in_mask(mask, tg)) return;
     const double s = beta0[tg];
     const double inv = (s > 0.0) ? 1.0 / s : 0.0;
-    const double2 *__restrict__ a = src.p[tg];
-    double2 *__restrict__ b = dst.p[tg];
+    const double2 *a = src.p[tg];
+    double2 *b = dst.p[tg];
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < np; r += (int64_t)gridDim.x * blockDim.x)
         b[r] = inv * a[r];
+    before_next();
 }
 
 // dst_t = src_t (np entries)
@@ -941,13 +957,12 @@ unsigned chunk_grid(const Ctx &c, int chunks) {
 }
 
 // w_t -= V_t h_t
-void mgs_update(Ctx &c, const TVec &V, const double2 *h, const TVec &w, const int *run, const TCols &tc) {
+int mgs_update(Ctx &c, const TVec &V, const double2 *h, const TVec &w, const int *run, const TCols &tc) {
     // one warp per SM sub-partition at most: below that the component form is the faster
     if (2 * c.np * c.T <= 128LL * 4 * c.p->num_sms)
-        k_mgs_update_parts<<<dim3(kore_div_up(2 * c.np, 128), c.T), 128, 0, c.p->stream>>>(c.np, V, h, w, run, tc);
-    else
-        k_mgs_update<<<dim3(c.grid, c.T), 256, 0, c.p->stream>>>(c.np, V, h, w, run, tc);
-    KORE_LAUNCHED(1);
+        return kore_launch_chained(c.p->stream, k_mgs_update_parts, dim3(kore_div_up(2 * c.np, 128), c.T), 128, 1, c.np, V,
+                                   h, w, run, tc);
+    return kore_launch_chained(c.p->stream, k_mgs_update, dim3(c.grid, c.T), 256, 1, c.np, V, h, w, run, tc);
 }
 
 // For each target t in tc.mask: orthogonalise w_t against V_t[:, 0:ncol_t] (classical
@@ -963,26 +978,27 @@ int orthonormalise(Ctx &c, const TVec &V, const TCols &tc) {
     double2 *h1 = c.h, *h2 = c.h + (kMaxNcv + 1);
     const dim3 g2(c.grid, c.T);
     const dim3 g3(c.grid, c.T, chunk_grid(c, kore_div_up(nmax + 1, kDotChunk)));
+    cudaStream_t st = p->stream;
+    const int nblk = (int)c.grid, *all = nullptr;
     // first pass, with ||w||^2 as entry ncol of h1
-    k_mdot<<<g3, kDotThreads, 0, p->stream>>>(c.np, V, w, c.partial, 1, nullptr, tc);
-    k_mdot_reduce<<<dim3(nmax + 1, c.T), 256, 0, p->stream>>>((int)c.grid, c.partial, kPartStride, h1, 0, nullptr,
-                                                               tc, 1);
-    mgs_update(c, V, h1, w, nullptr, tc);
-    k_refine_decide<<<c.T, 256, 0, p->stream>>>(c.h, c.run2, tc);
+    KORE_TRY(kore_launch_chained(st, k_mdot, g3, kDotThreads, 1, c.np, V, w, c.partial, 1, all, tc));
+    KORE_TRY(kore_launch_chained(st, k_mdot_reduce, dim3(nmax + 1, c.T), 256, 1, nblk, c.partial, kPartStride, h1, 0, all,
+                                 tc, 1));
+    KORE_TRY(mgs_update(c, V, h1, w, all, tc));
+    KORE_TRY(kore_launch_chained(st, k_refine_decide, dim3(c.T), 256, 1, c.h, c.run2, tc));
     // second pass if needed
-    k_mdot<<<g3, kDotThreads, 0, p->stream>>>(c.np, V, w, c.partial, 0, c.run2, tc);
-    k_mdot_reduce<<<dim3(nmax, c.T), 256, 0, p->stream>>>((int)c.grid, c.partial, kPartStride, h2, 0, c.run2, tc, 0);
-    mgs_update(c, V, h2, w, c.run2, tc);
-    KORE_LAUNCHED(5);
+    KORE_TRY(kore_launch_chained(st, k_mdot, g3, kDotThreads, 1, c.np, V, w, c.partial, 0, c.run2, tc));
+    KORE_TRY(kore_launch_chained(st, k_mdot_reduce, dim3(nmax, c.T), 256, 1, nblk, c.partial, kPartStride, h2, 0, c.run2,
+                                 tc, 0));
+    KORE_TRY(mgs_update(c, V, h2, w, c.run2, tc));
     // h = h1 + h2
-    k_mdot_reduce<<<dim3(nmax, c.T), 32, 0, p->stream>>>(1, h2, kHStride, h1, 1, nullptr, tc, 0);
-    k_nrm2_partial<<<g2, 256, 0, p->stream>>>(c.np, w, c.dpart, tc.mask);
-    k_finish_col<<<c.T, 256, 0, p->stream>>>((int)c.grid, c.dpart, c.h, c.Hbar, c.beta, tc, 1);
+    KORE_TRY(kore_launch_chained(st, k_mdot_reduce, dim3(nmax, c.T), 32, 1, 1, h2, kHStride, h1, 1, all, tc, 0));
+    KORE_TRY(kore_launch_chained(st, k_nrm2_partial, g2, 256, 1, c.np, w, c.dpart, tc.mask));
+    KORE_TRY(kore_launch_chained(st, k_finish_col, dim3(c.T), 256, 1, nblk, c.dpart, c.h, c.Hbar, c.beta, tc, 1));
     TVec vnext;
     for (int t = 0; t < kMaxTargets; ++t)
         vnext.p[t] = (t < c.T && ((tc.mask >> t) & 1u)) ? V.p[t] + (int64_t)(tc.j[t] + 1) * c.np : nullptr;
-    k_scale_copy<<<g2, 256, 0, p->stream>>>(c.np, w, c.beta, vnext, tc.mask);
-    KORE_LAUNCHED(4);
+    KORE_TRY(kore_launch_chained(st, k_scale_copy, g2, 256, 1, c.np, w, c.beta, vnext, tc.mask));
     if (p->prof) KORE_TRY(kore_prof_mark(p, 3, false));
     KORE_CUDA_TRY(cudaGetLastError());
     return KORE_OK;

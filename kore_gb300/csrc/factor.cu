@@ -263,14 +263,6 @@ __device__ __forceinline__ const C *diag_block(const FV<C> &v, int64_t o, int64_
     return v.Dw + sh * v.f_stride + (2 * o + 1) * stride * (int64_t)v.S * v.S;
 }
 
-// A kernel that launch_chained() launches calls after_previous() before it touches memory,
-// as its CTAs may start while the launch before it in the stream runs, and before_next() once
-// its main loop is done: the next launch's CTAs then take the places that become free, and
-// wait there.  (Called at the start instead, they held places from the kernel's own CTAs:
-// four FP64 shifts of the 72k-unknown shell 94.6 -> 95.8 ms.)
-__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void before_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // Panel reduction of columns [k0, k0+nb) of T_o; one CTA per (odd block o = blockIdx.x,
 // shift = blockIdx.y), one thread per row, which holds its NB entries of the panel in
 // registers.  Every elimination step works on register 0 and shifts the others down by
@@ -667,27 +659,6 @@ unsigned grid_for(int64_t work, int threads, int num_sms) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>((work + threads - 1) / threads, 16LL * num_sms));
 }
 
-// Launch of a kernel that begins with after_previous(): it is set up while the kernel before
-// it in the stream still runs, and split CTAs along x form a cluster.
-template <typename... P, typename... A>
-int launch_chained(kore_plan *p, void (*kern)(P...), dim3 grid, unsigned threads, int split, const A &...args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.stream = p->stream;
-    cudaLaunchAttribute at[2]{};
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = split;
-    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = split > 1 ? 2 : 1;
-    KORE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, P(args)...));
-    KORE_LAUNCHED(1);
-    return KORE_OK;
-}
-
 // Gauss-Jordan of the nodd work matrices T_o of every shift, then extraction.  Complex64:
 // panels of NB columns, each followed by the update of all other columns.  Complex128, where
 // that update would keep the FP64 pipe busy: the panels' updates stay within a group of
@@ -710,7 +681,7 @@ int gauss_jordan(kore_plan *p, const FV<C> &v, const BcrLevel &lv, int nodd, int
         const int g1 = std::min(S, g0 + group);
         for (int k0 = g0; k0 < g1; k0 += NB) {
             const int nb = std::min(NB, g1 - k0), ncols = g1 - g0 - nb;
-            KORE_TRY(launch_chained(p, k_panel<C, NB, MAXT>, dim3(nodd, nshift), panel_threads(pthreads), 1, v, k0, nb,
+            KORE_TRY(kore_launch_chained(p->stream, k_panel<C, NB, MAXT>, dim3(nodd, nshift), panel_threads(pthreads), 1, v, k0, nb,
                                     lv.stride));
             if (ncols == 0) continue;
             // 32 columns per CTA re-read the panel least; levels with few blocks take 8, so
@@ -718,11 +689,11 @@ int gauss_jordan(kore_plan *p, const FV<C> &v, const BcrLevel &lv, int nodd, int
             // CTAs, as a chunk then is a chain of loads and a few products (two shifts of the MAC
             // shell, S = 360: 9.37 -> 9.31 ms; the 240k-unknown shell: 38.4 -> 38.2 ms)
             if ((int64_t)nodd * nshift * kore_div_up(ncols, 32) >= 2 * p->num_sms) {
-                KORE_TRY(launch_chained(p, k_update<C, NB, 32>, dim3(kore_div_up(ncols, 32), nodd, nshift), 256, 1, v, k0, nb,
+                KORE_TRY(kore_launch_chained(p->stream, k_update<C, NB, 32>, dim3(kore_div_up(ncols, 32), nodd, nshift), 256, 1, v, k0, nb,
                                         g0, g1, lv.stride, 1));
             } else {
                 const int split = (int)kore_div_up(S, kUpdRows);   // at most 8, a portable cluster
-                KORE_TRY(launch_chained(p, k_update<C, NB, 8>, dim3(kore_div_up(ncols, 8) * split, nodd, nshift), 256,
+                KORE_TRY(kore_launch_chained(p->stream, k_update<C, NB, 8>, dim3(kore_div_up(ncols, 8) * split, nodd, nshift), 256,
                                         split, v, k0, nb, g0, g1, lv.stride, split));
             }
         }
