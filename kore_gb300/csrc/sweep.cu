@@ -592,8 +592,8 @@ __device__ __forceinline__ void reset_vecs(void *vecs, int64_t bytes, int64_t s)
 // does not count), the sweep's vectors set, and with ir the refinement state of a new
 // application (a shift outside live_mask has nothing to refine).  Bound by its launch: one
 // kernel here for two maxima kernels, a state kernel and a memset, and the check in the
-// residual product's last CTA, took a solve of 704 unknowns in FP64 from 123 to 102 us and
-// four mixed targets of the 1.9k-unknown shell from 74.9 to 68.5 ms.
+// residual product's last CTA, took a solve of 480 unknowns in FP64 from 123 to 102 us and
+// four mixed targets of a 5.8k-unknown shell from 74.9 to 68.5 ms.
 __global__ void __launch_bounds__(256) k_begin(int64_t np, const double2 *__restrict__ v, double *__restrict__ part,
                                                double *__restrict__ bnorm, unsigned *tick, void *vecs, int64_t vbytes,
                                                IrState *ir, unsigned live_mask) {
