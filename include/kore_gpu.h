@@ -343,6 +343,15 @@ int kore_batch_destroy(kore_batch *batch);
 int kore_tc_selftest(int device, int S, int nmat, double *max_rel_err);
 
 /*
+ * Self-test of the FP64 products on the tensor cores (digits): column-major S x S complex
+ * host matrices, C = beta C + alpha (A1 B1 [+ A2 B2]) with alpha = -1 when negate, else 1,
+ * beta = 1 or 0, and A2 = B2 = NULL for one product.  S <= 1024.
+ * No counterpart in the reference; a diagnostic for the kernel.
+ */
+int kore_oz_selftest(int device, int S, const double *A1, const double *B1, const double *A2, const double *B2,
+                     double *C, int negate, int beta);
+
+/*
  * Multiplication operator of the Gegenbauer (ultraspherical) basis, computed on
  * `device`: M multiplies a C^(lam) series by the function whose N C^(lam) coefficients
  * are a0 (lam >= 0; lam = 0 is the Chebyshev basis).  M is banded with half-width

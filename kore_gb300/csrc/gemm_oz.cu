@@ -11,13 +11,21 @@
 // the radial order, the rows of G fall as fast).
 //
 // Digits.  An entry is rounded to 63 bits and written as nine digits in [-64, 64] of base
-// 128, exact in FP16:  x = sum_i x_i 128^-(i+1).  The product keeps the 45 digit pairs with
-// i + i' = d <= 8:  sum_d 128^-(d+2) (sum over pairs and k of x_i y_i').  Each inner sum is
-// a sum of at most 9 K products of at most 2^12, hence an integer below 2^24 for K <= 448,
-// and exact in the MMA's FP32 accumulators; longer inner dimensions are cut into pieces of
-// 448.  The nine sums are put together as integers and rounded to FP64 once.  What is lost
-// is below K 2^-60 of (largest entry of A's row) x (largest of B's column): in solves with
-// these factors the error against 64 bits is that of FP64 products or smaller.
+// 128, exact in FP16:  x = 2 sum_i x_i 128^-(i+1).  The product keeps the 45 digit pairs with
+// i + i' = d <= 8:  4 sum_d 128^-(d+2) (sum over pairs and k of x_i y_i').  A real or imaginary
+// part takes two real products per k, so the inner sum of one d is a sum of 2 (d + 1) K
+// products of at most 2^12: an integer of at most 2^24 for (d + 1) K <= 2048, and exact in the
+// MMA's FP32 accumulators.  Longer inner dimensions are cut: at 224 for d = 8-6, 336 for 5-3 and
+// 672 for 2-0.  The nine sums are put together as integers and rounded to FP64 once.
+//
+// What is lost, in units of the powers of two that scale row and column: 2^-62 per real product
+// by rounding the entries, 1.01 x 2^-60 by the pairs left out (d >= 9), two such products per
+// k.  The powers are below twice the largest components, so a real or imaginary part of C is
+// off by at most 10.1 K 2^-60 of (largest of A's row) x (largest of B's column), after the
+// scaling by rho, and one rounding.  That is a bound by rows and columns.  An entry of C whose
+// own sum |a||b| is far below that product of maxima, which rho cannot repair when the grading
+// is not one of rows, columns and inner index (blocks of weakly coupled unknowns), has less
+// relative accuracy than FP64 multiply-adds would give it.
 //
 // Data flow.  k_oz_rho finds rho; k_oz_split_a and k_oz_split_b write the digit planes in
 // the order the MMA reads them (8 x 16-byte core matrices, K-major, no swizzle), nine slices
@@ -39,7 +47,6 @@ namespace {
 
 constexpr int kOzSlices = 9, kOzBits = 7;
 constexpr int kOzM = 128, kOzN = 64, kOzK = 16;
-constexpr int kOzMaxSteps = 28;                    // steps of K whose sums stay below 2^24
 constexpr int kOzSliceA = 2 * kOzM * kOzK * 2;     // bytes of one slice of a step: Re, Im
 constexpr int kOzSliceB = 2 * kOzN * kOzK * 2;
 constexpr int kOzStepA = kOzSlices * kOzSliceA, kOzStepB = kOzSlices * kOzSliceB;
@@ -51,7 +58,16 @@ constexpr size_t kOzSmem = (size_t)kOzStages * kOzStage + 128 + 128;
 constexpr int kOzNone = -100000;                   // exponent of an all-zero row
 constexpr int kOzBad = 100000;                     // exponent of a row with an infinity or NaN
 
-static_assert((int64_t)kOzSlices * kOzMaxSteps * kOzK * 4096 <= (1 << 24), "exact FP32 sums");
+// A pass g sums the pairs of d = 8 - 3 g, 7 - 3 g, 6 - 3 g.  Steps of K that one pass may take:
+// two real products of 9 - 3 g pairs at most per k, each at most 64^2, stay within 2^24.
+constexpr int kOzPasses = 3;
+__host__ __device__ constexpr int oz_max_steps(int g) { return (1 << 24) / (2 * (kOzSlices - 3 * g) * kOzK * 4096); }
+static_assert(oz_max_steps(0) == 14 && oz_max_steps(1) == 21 && oz_max_steps(2) == 42, "exact FP32 sums");
+// `steps` of K are cut into this many pieces for pass g, piece p being [p steps / n, (p + 1) steps / n).
+// The pieces of the last pass are segments: each is a product of its own, rounded and added to
+// C, whose passes 0 and 1 are cut further but summed as integers.
+__host__ __device__ constexpr int oz_pieces(int steps, int g) { return (steps + oz_max_steps(g) - 1) / oz_max_steps(g); }
+constexpr int kOzPlainSteps = oz_max_steps(0);   // up to this many nothing is cut
 
 int oz_mt(int S) { return (S + kOzM - 1) / kOzM; }
 int oz_nt(int S) { return (S + kOzN - 1) / kOzN; }
@@ -364,8 +380,11 @@ __device__ __forceinline__ double from_digits(long long h, long long g, int e) {
     return neg ? -r : r;
 }
 
-// One 128 x 64 tile (blockIdx.x) of job (of the group update: block) blockIdx.y.
-template <bool GROUP>
+// One 128 x 64 tile (blockIdx.x) of job (of the group update: block) blockIdx.y.  CUT: more
+// than kOzPlainSteps steps.  (The 64 registers of a thread's integer sums leave too few for the
+// rest: of the 96 that eighteen warps have, 516 bytes a thread spill with CUT, 312 without and
+// 200 in the group update.)
+template <bool GROUP, bool CUT>
 __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzParams P) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
@@ -386,8 +405,8 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzParams P) {
     } else job = P.jobs[blockIdx.y];
     const int ncols = GROUP ? S - (P.group.g1 - P.group.g0) : S;
     const int mt = blockIdx.x / P.nt, nt = blockIdx.x - mt * P.nt;
-    const int pieces = (steps + kOzMaxSteps - 1) / kOzMaxSteps;   // of the inner dimension
-    const int nseg = (job.a2 >= 0 ? 2 : 1) * pieces;              // pieces of all products
+    const int parts = CUT ? oz_pieces(steps, 2) : 1;   // segments of a product
+    const int nseg = (job.a2 >= 0 ? 2 : 1) * parts;
     if (tid == 0) {
         for (int s = 0; s < kOzStages; ++s) {
             mbar_init(&full[s], 1);
@@ -411,13 +430,13 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzParams P) {
         if (lane == 0) {
             uint32_t it = 0;
             for (int sg = 0; sg < nseg; ++sg) {
-                const int prod = sg / pieces, k0 = (sg - prod * pieces) * kOzMaxSteps;
-                const int k1 = min(steps, k0 + kOzMaxSteps);
+                const int prod = sg / parts, part = sg - prod * parts;
+                const int k0 = part * steps / parts, k1 = (part + 1) * steps / parts;
                 const unsigned char *pa = P.pa + (prod ? job.a2 : job.a1) * P.bytes_a + (int64_t)mt * steps * kOzStepA;
                 const unsigned char *pb = P.pb + (prod ? job.b2 : job.b1) * P.bytes_b + (int64_t)nt * steps * kOzStepB;
-                for (int g = 0; g < 3; ++g) {
+                for (int g = 0; g < kOzPasses; ++g) {
                     const uint32_t ns = kOzSlices - 3 * g;
-                    for (int k = k0; k < k1; ++k, ++it) {
+                    for (int k = k0; k < k1; ++k, ++it) {   // the pieces of a pass follow one another
                         const int s = it % kOzStages;
                         if (!mbar_wait(&empty[s], ((it / kOzStages) & 1u) ^ 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
                         mbar_arrive_expect_tx(&full[s], ns * (kOzSliceA + kOzSliceB));
@@ -432,10 +451,13 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzParams P) {
     } else if (warp == kOzEpiWarps + 1) {
         if (lane == 0) {
             uint32_t it = 0, pass = 0;
-            for (int sg = 0; sg < nseg; ++sg) {
-                const int prod = sg / pieces, k0 = (sg - prod * pieces) * kOzMaxSteps;
-                const int k1 = min(steps, k0 + kOzMaxSteps);
-                for (int g = 0; g < 3; ++g, ++pass) {
+            // the passes of all segments, each in its pieces
+            for (int g3 = 0; g3 < nseg * kOzPasses; ++g3) {
+                const int sg = g3 / kOzPasses, g = g3 - sg * kOzPasses, part = sg % parts;
+                const int s0 = part * steps / parts, n = (part + 1) * steps / parts - s0;
+                const int np = CUT ? oz_pieces(n, g) : 1;
+                for (int p = 0; p < np; ++p, ++pass) {
+                    const int k0 = s0 + p * n / np, k1 = s0 + (p + 1) * n / np;
                     if (pass > 0 && !mbar_wait(drained, (pass - 1) & 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
                     oz_fence_after();
                     for (int k = k0; k < k1; ++k, ++it) {
@@ -473,33 +495,37 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzParams P) {
         const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cb;
         uint32_t pass = 0;
         for (int sg = 0; sg < nseg; ++sg) {
-            const int prod = sg / pieces;
-            long long gr[16], gi[16];   // sums of d = 3 .. 8 in units of 128^-10
+            const int prod = sg / parts, part = sg - prod * parts;
+            const int n = (part + 1) * steps / parts - part * steps / parts;
+            long long gr[16], gi[16];   // sums of d = 3 .. 8 in units of 128^-10, below 2^61
 #pragma unroll
             for (int c = 0; c < 16; ++c) gr[c] = gi[c] = 0;
 #pragma unroll
-            for (int g = 0; g < 2; ++g, ++pass) {
-                if (!mbar_wait(accum, pass & 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
-                oz_fence_after();
+            for (int g = 0; g < 2; ++g) {
+                const int np = CUT ? oz_pieces(n, g) : 1;
+                for (int p = 0; p < np; ++p, ++pass) {
+                    if (!mbar_wait(accum, pass & 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
+                    oz_fence_after();
 #pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    const int sh = kOzBits * (3 * g + q);
+                    for (int q = 0; q < 3; ++q) {
+                        const int sh = kOzBits * (3 * g + q);
 #pragma unroll
-                    for (int h = 0; h < 16; h += 8) {
-                        float vr[8], vi[8];
-                        oz_ld8(tl + (uint32_t)(q * 2 * kOzN + h), vr);
-                        oz_ld8(tl + (uint32_t)(q * 2 * kOzN + kOzN + h), vi);
-                        oz_ld_wait();
+                        for (int h = 0; h < 16; h += 8) {
+                            float vr[8], vi[8];
+                            oz_ld8(tl + (uint32_t)(q * 2 * kOzN + h), vr);
+                            oz_ld8(tl + (uint32_t)(q * 2 * kOzN + kOzN + h), vi);
+                            oz_ld_wait();
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) {
-                            gr[h + c] += (long long)__float2int_rn(vr[c]) << sh;
-                            gi[h + c] += (long long)__float2int_rn(vi[c]) << sh;
+                            for (int c = 0; c < 8; ++c) {
+                                gr[h + c] += (long long)__float2int_rn(vr[c]) << sh;
+                                gi[h + c] += (long long)__float2int_rn(vi[c]) << sh;
+                            }
                         }
                     }
+                    oz_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(drained);
                 }
-                oz_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(drained);
             }
             if (!mbar_wait(accum, pass & 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
             oz_fence_after();
@@ -611,8 +637,9 @@ int oz_run(cudaStream_t st, int device, int S, const OzBatch &w, unsigned char *
     P.pa = pa; P.pb = pb; P.ea = ea; P.eb = eb;
     P.bytes_a = oz_bytes_a(S, S); P.bytes_b = oz_bytes_b(S, S);
     P.S = S; P.nt = oz_nt(S); P.steps = oz_steps(S); P.err = err;
-    KORE_TRY(kore_allow_max_dyn_smem(k_oz_gemm<false>, device));
-    k_oz_gemm<false><<<dim3(oz_mt(S) * oz_nt(S), (unsigned)w.jobs.size()), kOzThreads, kOzSmem, st>>>(P);
+    auto gemm = P.steps > kOzPlainSteps ? k_oz_gemm<false, true> : k_oz_gemm<false, false>;
+    KORE_TRY(kore_allow_max_dyn_smem(gemm, device));
+    gemm<<<dim3(oz_mt(S) * oz_nt(S), (unsigned)w.jobs.size()), kOzThreads, kOzSmem, st>>>(P);
     KORE_LAUNCHED(4);
     KORE_CUDA_TRY(cudaGetLastError());
     return KORE_OK;
@@ -753,8 +780,8 @@ int kore_group_update_oz(kore_plan *p, const BcrLevel &lv, int nodd, int g0, int
               p->f_stride(), p->p_stride(), nodd, lv.stride, S, g0, g1, 0};
     const int total = nodd * p->fw_n;
     const int per = (int)std::min<int64_t>(std::min(total, 65535), p->oz_bytes / oz_group_bytes(S, W));
-    if (per < 1) return KORE_EINVAL;
-    KORE_TRY(kore_allow_max_dyn_smem(k_oz_gemm<true>, p->device));
+    if (per < 1 || oz_steps(W) > kOzPlainSteps) return KORE_EINVAL;
+    KORE_TRY(kore_allow_max_dyn_smem(k_oz_gemm<true, false>, p->device));
     for (q.first = 0; q.first < total; q.first += per) {
         const int nb = std::min(per, total - q.first);
         unsigned char *pa = static_cast<unsigned char *>(p->d_oz), *pb = pa + nb * oz_bytes_a(S, W);
@@ -767,9 +794,49 @@ int kore_group_update_oz(kore_plan *p, const BcrLevel &lv, int nodd, int g0, int
         P.pa = pa; P.pb = pb; P.ea = ea; P.eb = eb;
         P.bytes_a = oz_bytes_a(S, W); P.bytes_b = oz_bytes_b(S, W);
         P.S = S; P.nt = oz_nt(n); P.steps = oz_steps(W); P.err = p->d_err; P.group = q;
-        k_oz_gemm<true><<<dim3(oz_mt(S) * P.nt, nb), kOzThreads, kOzSmem, p->stream>>>(P);
+        k_oz_gemm<true, false><<<dim3(oz_mt(S) * P.nt, nb), kOzThreads, kOzSmem, p->stream>>>(P);
         KORE_LAUNCHED(4);
     }
     KORE_CUDA_TRY(cudaGetLastError());
     return KORE_OK;
+}
+
+extern "C" int kore_oz_selftest(int device, int S, const double *A1, const double *B1, const double *A2, const double *B2,
+                                double *C, int negate, int beta) {
+    if (S <= 0 || S > 1024 || !A1 || !B1 || !C || !A2 != !B2) return KORE_EINVAL;
+    int prev = -1;
+    cudaGetDevice(&prev);
+    KORE_CUDA_TRY(cudaSetDevice(device));
+    const size_t SS = (size_t)S * S, bytes = SS * sizeof(double2);
+    const double *host[] = {A1, B1, A2, B2, C};
+    double2 *m = nullptr;   // A1, B1, A2, B2, C
+    unsigned char *ws = nullptr;
+    int *flag = nullptr;
+    int rc = KORE_OK;
+    auto ck = [&](cudaError_t e) { if (e != cudaSuccess && rc == KORE_OK) rc = (e == cudaErrorMemoryAllocation) ? KORE_ENOMEM : KORE_ECUDA; };
+    ck(cudaMalloc(&m, 5 * bytes));
+    ck(cudaMalloc(&ws, oz_batch_bytes(S, 2, 2, 2, 1)));
+    ck(cudaMalloc(&flag, sizeof(int)));
+    if (rc == KORE_OK) {
+        for (int i = 0; i < 5; ++i)
+            if (host[i]) ck(cudaMemcpy(m + i * SS, host[i], bytes, cudaMemcpyHostToDevice));
+        ck(cudaMemset(flag, 0, sizeof(int)));
+        OzBatch w;
+        for (int q = 0; q < (A2 ? 2 : 1); ++q) {
+            w.pairs.push_back({m + (2 * q + 1) * SS, nullptr});
+            w.a.push_back({m + 2 * q * SS, q});
+            w.b.push_back({m + (2 * q + 1) * SS, q});
+        }
+        w.jobs.push_back({0, 0, A2 ? 1 : -1, A2 ? 1 : -1, m + 4 * SS, negate != 0, beta != 0});
+        if (rc == KORE_OK) rc = oz_run(0, device, S, w, ws, flag);
+        int h = 0;
+        if (rc == KORE_OK) {
+            ck(cudaMemcpy(&h, flag, sizeof(int), cudaMemcpyDeviceToHost));
+            ck(cudaMemcpy(C, m + 4 * SS, bytes, cudaMemcpyDeviceToHost));
+            if (rc == KORE_OK && h != 0) rc = KORE_ETIMEOUT;
+        }
+    }
+    cudaFree(m); cudaFree(ws); cudaFree(flag);
+    if (prev >= 0) cudaSetDevice(prev);
+    return rc;
 }
