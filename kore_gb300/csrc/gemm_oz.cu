@@ -118,11 +118,12 @@ struct OzGroup {
     __device__ int column(int t) const { return t < g0 ? t : t + g1 - g0; }   // t-th column outside the group
 };
 
-// exponent e with |v| < 2^e of a finite nonzero double, from its bits (subnormals count as zero)
+// exponent e with |v| < 2^e of a finite nonzero double, from its bits (all subnormals: -1022)
 __device__ __forceinline__ int exp_of(double2 v) {
     const int a = (__double2hiint(v.x) >> 20) & 0x7ff, b = (__double2hiint(v.y) >> 20) & 0x7ff;
     const int m = max(a, b);
-    return m == 0x7ff ? kOzBad : m == 0 ? kOzNone : m - 1022;
+    if (m == 0) return ((__double_as_longlong(v.x) | __double_as_longlong(v.y)) << 1) == 0 ? kOzNone : -1022;
+    return m == 0x7ff ? kOzBad : m - 1022;
 }
 
 // rho[pair][k] = largest exponent in row k of the pair's matrices.  CTA = 32 rows, warps
@@ -151,11 +152,11 @@ __global__ void __launch_bounds__(256) k_oz_rho(const OzPair *__restrict__ pairs
 __device__ __forceinline__ long long fixed63(double v, int e) {
     const long long b = __double_as_longlong(v);
     const int ex = (int)(b >> 52) & 0x7ff;
-    if (ex == 0 || ex == 0x7ff) return 0;
-    const long long m = (b & 0xfffffffffffffll) | (1ll << 52);
-    const int sh = ex - 1075 + 62 - e;
+    if (ex == 0x7ff) return 0;
+    const long long m = (b & 0xfffffffffffffll) | (ex ? 1ll << 52 : 0);
+    const int sh = max(ex, 1) - 1075 + 62 - e;
     long long x;
-    if (sh >= 0) x = sh < 10 ? m << sh : 0;   // sh <= 9 by |v| < 2^e
+    if (sh >= 0) x = sh <= 10 ? m << sh : 0;   // sh <= 9 by |v| < 2^e, 10 for a subnormal
     else x = sh > -55 ? (m + (1ll << (-sh - 1))) >> -sh : 0;
     return b < 0 ? -x : x;
 }

@@ -110,9 +110,9 @@ def test_two_products(gpu_lib, S, graded):
         assert abs(C[i, j] - ref) <= 1.5 * (10 * 2.0 ** -53 * mag + lost[i, j]), (i, j, C[i, j], ref)
 
 
-def test_zeros_infinities(gpu_lib):
+def test_zeros_infinities_subnormals(gpu_lib):
     """A zero row, column and inner index give zeros; rows and columns with an infinity or a NaN
-    give NaN and touch nothing else."""
+    give NaN and touch nothing else; subnormal operands keep their bits."""
     S = 70
     rng = np.random.default_rng(0)
     A = rng.standard_normal((S, S)) + 1j * rng.standard_normal((S, S))
@@ -130,3 +130,9 @@ def test_zeros_infinities(gpu_lib):
     bad = np.zeros((S, S), bool)
     bad[10] = bad[:, 13] = True
     assert np.all(np.isnan(C[bad].real)) and np.all(np.isnan(C[bad].imag)) and np.all(np.isfinite(C[~bad]))
+    # subnormals: integers below 2^40 in units of 2^-1074 against integers, sums below 2^53
+    T = rng.integers(-(1 << 20), 1 << 20, size=(S, S)) * 2.0 ** -1074 * (1 + 0j)
+    N = rng.integers(-(1 << 10), 1 << 10, size=(S, S)) * (1.0 + 0j)
+    exact = (np.rint(T.real * 2.0 ** 1000 * 2.0 ** 74) @ N.real) * 2.0 ** -1074
+    np.testing.assert_array_equal(product(gpu_lib, T, N).real, exact)
+    np.testing.assert_array_equal(product(gpu_lib, N, T).real, (N.real @ np.rint(T.real * 2.0 ** 1000 * 2.0 ** 74)) * 2.0 ** -1074)
