@@ -57,6 +57,12 @@ constexpr int kOzThreads = 32 * (kOzEpiWarps + 2); // + the copying and the MMA 
 constexpr size_t kOzSmem = (size_t)kOzStages * kOzStage + 128 + 128;
 constexpr int kOzNone = -100000;                   // exponent of an all-zero row
 constexpr int kOzBad = 100000;                     // exponent of a row with an infinity or NaN
+// rho of a zero row of B: the column of A that meets it takes no part in the scale of A's rows.
+// (Left as it stands it decides that scale wherever its entries are the largest, and the others
+// lose their digits: boundary rows have no couplings, so L has zero rows, and solutions that
+// fall off with the degree had blocks of 1e-12 of the largest off by 1e-6 of themselves, 1e-12
+// with it.)
+constexpr int kOzUnused = -4096;
 
 // A pass g sums the pairs of d = 8 - 3 g, 7 - 3 g, 6 - 3 g.  Steps of K that one pass may take:
 // two real products of 9 - 3 g pairs at most per k, each at most 64^2, stay within 2^24.
@@ -126,6 +132,9 @@ __device__ __forceinline__ int exp_of(double2 v) {
     return m == 0x7ff ? kOzBad : m - 1022;
 }
 
+// rho of a row of B with largest exponent e
+__device__ __forceinline__ int rho_of(int e) { return e == kOzNone ? kOzUnused : e == kOzBad ? 0 : e; }
+
 // rho[pair][k] = largest exponent in row k of the pair's matrices.  CTA = 32 rows, warps
 // over the columns.
 __global__ void __launch_bounds__(256) k_oz_rho(const OzPair *__restrict__ pairs, int S, int *__restrict__ rho) {
@@ -143,8 +152,7 @@ __global__ void __launch_bounds__(256) k_oz_rho(const OzPair *__restrict__ pairs
     if (w == 0 && r < S) {
 #pragma unroll
         for (int q = 1; q < 8; ++q) e = max(e, sm[q][lane]);
-        // a row without finite nonzero entries is left unscaled
-        rho[(int64_t)blockIdx.y * S + r] = (e == kOzNone || e == kOzBad) ? 0 : e;
+        rho[(int64_t)blockIdx.y * S + r] = rho_of(e);
     }
 }
 
@@ -303,7 +311,7 @@ __global__ void __launch_bounds__(512) k_oz_group_rho(const OzGroup q, int *__re
         int e = kOzNone;
         for (int t = lane; t < n; t += 32) e = max(e, exp_of(X[piv[k] + (int64_t)q.column(t) * q.S]));
         e = __reduce_max_sync(0xffffffffu, e);
-        if (lane == 0) rho[(int64_t)blockIdx.x * W + k] = (e == kOzNone || e == kOzBad) ? 0 : e;
+        if (lane == 0) rho[(int64_t)blockIdx.x * W + k] = rho_of(e);
     }
 }
 
