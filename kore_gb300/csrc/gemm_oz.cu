@@ -455,6 +455,9 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzParams P) {
                     }
                 }
             }
+            // every copy has landed before the CTA may exit (normally already read)
+            for (uint32_t i = it > kOzStages ? it - kOzStages : 0; i < it; ++i)
+                if (!mbar_wait(&full[i % kOzStages], (i / kOzStages) & 1u)) atomicCAS(P.err, 0, KORE_DEVERR_FLAG);
         }
         __syncwarp();
     } else if (warp == kOzEpiWarps + 1) {
