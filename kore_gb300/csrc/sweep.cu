@@ -72,15 +72,22 @@ __host__ __device__ __forceinline__ bool mask_has(unsigned mask, int64_t s) {
 }
 
 // An entry of the sweep's vectors is written once per sweep.  Before the sweep all its bits
-// are set, a NaN that no arithmetic produces, so a reader sees by the entry itself whether
-// it is there: no counter, fence or flag stands between a tile's result and its use.  The 8
+// are set, a NaN that is never stored, so a reader sees by the entry itself whether
+// it is there: no counter, fence or flag stands between a tile's result and its use.
+// (FP32 arithmetic gives one NaN of other bits.  FP64 addition and multiplication keep the bits
+// of a NaN operand, so one of all bits set could come from a caller's vector: it is stored as
+// another NaN.)  The 8
 // bytes of a complex64 entry and each half of a complex128 one are written and read as one
 // access (relaxed, at L2), and a complex128 entry is there when both halves are.
 __device__ __forceinline__ void st_entry(float2 *p, float2 v) {
     const unsigned long long b = (unsigned long long)__float_as_uint(v.x) | ((unsigned long long)__float_as_uint(v.y) << 32);
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(b) : "memory");
 }
+__device__ __forceinline__ double not_the_mark(double v) {
+    return __double_as_longlong(v) == -1ll ? __longlong_as_double(0x7ff8000000000000ll) : v;
+}
 __device__ __forceinline__ void st_entry(double2 *p, double2 v) {
+    v = mk(not_the_mark(v.x), not_the_mark(v.y));
     asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v.x), "d"(v.y) : "memory");
 }
 __device__ __forceinline__ float2 ld_entry(const float2 *p) {
