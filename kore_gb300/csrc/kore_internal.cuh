@@ -190,8 +190,8 @@ int kore_prof_collect(kore_plan *p);
 
 // plan.cu
 int kore_check_device_error(kore_plan *p);
-// the status of an error flag that was read; a set flag is cleared on the device
-int kore_device_error(kore_plan *p, int flag);
+// the status of an error flag and NaN state that were read; a set flag is cleared on the device
+int kore_device_error(kore_plan *p, int flag, int nan);
 int kore_alloc(kore_plan *p, void **ptr, size_t bytes);
 
 // factor.cu

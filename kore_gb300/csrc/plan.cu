@@ -31,17 +31,23 @@ int kore_alloc(kore_plan *p, void **ptr, size_t bytes) {
     return KORE_OK;
 }
 
-int kore_device_error(kore_plan *p, int flag) {
-    if (flag == 0) return KORE_OK;
-    KORE_CUDA_TRY(cudaMemset(p->d_err, 0, sizeof(int)));
+// The status of a device error flag and a solve's NaN state.  An error comes first: what a wait
+// that ran out leaves in the solution may read as a NaN.
+extern "C" int kore_outcome(int flag, int nan) {
     if (flag == KORE_DEVERR_PIVOT) return KORE_ESINGULAR;
-    return KORE_ETIMEOUT;
+    if (flag != 0) return KORE_ETIMEOUT;
+    return nan ? KORE_ENAN : KORE_OK;
+}
+
+int kore_device_error(kore_plan *p, int flag, int nan) {
+    if (flag != 0) KORE_CUDA_TRY(cudaMemset(p->d_err, 0, sizeof(int)));
+    return kore_outcome(flag, nan);
 }
 
 int kore_check_device_error(kore_plan *p) {
     int h = 0;
     KORE_CUDA_TRY(cudaMemcpy(&h, p->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    return kore_device_error(p, h);
+    return kore_device_error(p, h, 0);
 }
 
 int kore_prof_mark(kore_plan *p, int kind, bool begin) {
@@ -397,8 +403,7 @@ int solve_dev_impl(kore_plan *p, const double2 *b, double2 *x, int nrhs, double 
         st->refine_iters_max = s.iters_max;
         st->solve_resid_max = s.eta_max;
     }
-    const int rc = kore_device_error(p, err);
-    return s.nan ? KORE_ENAN : rc;
+    return kore_device_error(p, err, s.nan);
 }
 
 // The host-pointer solves: copies, solve, and the test of the solution for NaN or Inf
