@@ -675,10 +675,15 @@ int gauss_jordan(kore_plan *p, const FV<C> &v, const BcrLevel &lv, int nodd, int
     const int S = p->S;
     const int pthreads = ((S + 31) / 32) * 32;
     // A group's product has fixed costs of about 50 us (four launches, one tile's chain); the
-    // FP64 products that it replaces, four multiply-adds each, run at two per SM and clock.
-    // (30 blocks of S = 96: 6.4 ms per solve with groups at every level, 5.9 without.)
-    const int64_t fma = 4LL * nodd * nshift * S * std::max(0, S - kGroup) * kGroup;
-    const int group = (sizeof(C) == 16 && fma / (2 * p->num_sms) > 200000) ? kGroup : S;
+    // FP64 products that it replaces, four multiply-adds each, run at two per SM and clock.  Per
+    // shift, as the two forms round differently and a shift's factors must not depend on how
+    // many others share the launches.  Limits of 200,000, 100,000, 50,000 and 20,000 cycles,
+    // factorisation of 1, 4 and 8 shifts: 60 blocks of S = 96, 4.45, 6.1, 8.6 ms; 4.45, 6.0, 8.7;
+    // 4.43, 5.6, 8.0; 4.64, 5.7, 7.5; 300 of S = 240, 35.2, 92.6, 172; 35.3, 91.6, 169; 35.7, 91.4,
+    // 169; 36.8, 91.9, 168.  (With a right-hand side one shift of S = 96 takes 4.67 ms ungrouped,
+    // 4.75 with level 0 grouped, which is at 87,000.)
+    const int64_t fma = 4LL * nodd * S * std::max(0, S - kGroup) * kGroup;
+    const int group = (sizeof(C) == 16 && fma / (2 * p->num_sms) > 90000) ? kGroup : S;
     for (int g0 = 0; g0 < S; g0 += group) {
         const int g1 = std::min(S, g0 + group);
         for (int k0 = g0; k0 < g1; k0 += NB) {

@@ -169,9 +169,10 @@ constexpr int kTileRows = 32;
 // columns and four times as many SMs work on the stage.  These stages are the chain of the
 // upper levels, where a tile's own time counts.  complex128: its products (10.5 us per matrix
 // of S = 240 on the FP64 pipe of one SM), so a warp's lanes share each row four ways (lane =
-// row + 8 x column mod 4).  complex64: its chunks' waits (2.8 us per matrix at S = 400; a
-// quarter of the chunks, 0.7 us); a warp keeps its columns and their order, so the sums are
-// those of 32-row tiles bit for bit.  See sweep_low_tiles for the rule.
+// row + 8 x column mod 4), with the four sums that a lane of a 32-row tile keeps.  complex64:
+// its chunks' waits (2.8 us per matrix at S = 400; a quarter of the chunks, 0.7 us); a warp
+// keeps its columns and their order.  The sums of both heights are the same bit for bit, as the
+// height depends on the number of shifts (sweep_low_tiles).
 constexpr int kLowRows = 8;
 constexpr int kMaxRing = 24;
 constexpr int kEllReg = 4;   // level-0 coupling entries per thread held in registers (width 32)
@@ -193,7 +194,6 @@ struct SweepTmaParams {
 
 template <typename C, int CHUNK> struct TmaShape {
     static constexpr int kCols = CHUNK / (kTileRows * (int)sizeof(C));   // columns per chunk
-    static constexpr int kColsPerWarp = kCols / kTmaConsumerWarps;
 };
 
 // One tile of the sweep: stage kind (0 A, 1 B, 2 top, 3 C, 4 E_0), level, shift, block
@@ -298,14 +298,17 @@ __device__ __forceinline__ void decode_tile(int64_t n, int &k, const SweepShape 
 template <typename C, int CPS, int CHUNK>
 __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_constant__ SweepTmaParams P) {
     using Shape = TmaShape<C, CHUNK>;
-    constexpr int kCols = Shape::kCols, kCpw = Shape::kColsPerWarp;
+    constexpr int kCols = Shape::kCols;
     constexpr int kFill = fill_of<C, CPS>();
     constexpr bool kSplit = sizeof(C) == 16;   // low tiles: lanes share a row
-    // Columns of a warp: runs of kRun, 4 kRun apart.  complex64: the same in every variant, so
-    // that a sweep's sums do not depend on the autotuner's choice (with 8 KB chunks of 32 rows
-    // a warp then works on every other chunk).
-    constexpr int kRun = sizeof(C) == 8 ? 16 : kCpw;
+    // Columns of a warp: runs of kRun, 4 kRun apart, the same in every variant, so that a sweep's
+    // sums do not depend on the autotuner's choice (complex64: with 8 KB chunks of 32 rows a warp
+    // then works on every other chunk).  complex128 keeps a sum for each of the run's four
+    // columns, as low tiles have them on four lanes: the sums then depend neither on the height
+    // of the tiles nor with it on the number of shifts.
+    constexpr int kRun = sizeof(C) == 8 ? 16 : 4;
     constexpr bool kHalf = kCols < 4 * kRun;
+    constexpr int kAcc = kSplit ? 4 : 1;
     const SweepArgs &a = P.a;
     const int nst = P.nst;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -456,9 +459,7 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
                     for (int u = 0; u < kFill; ++u) {
                         const int e = e0 + u * 32 + lane;
                         const int m = e >= per ? 1 : 0, rem = e - m * per;
-                        // low tiles of complex128: runs of kCols columns, 4 kCols apart
-                        const int c = t.low && kSplit ? (rem / kCols) * 4 * kCols + w * kCols + rem % kCols
-                                            : (rem / kRun) * 4 * kRun + w * kRun + rem % kRun;
+                        const int c = (rem / kRun) * 4 * kRun + w * kRun + rem % kRun;
                         cv[u] = (e < ne) ? m * nvec + c : -1;
                         v[u] = czero<C>();
                         if (e < ne && c < S) {
@@ -481,7 +482,10 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
                 __syncwarp();
             }
             if (wr && t.add >= 0) zf = ld_entry(vs + t.add + r);
-            C acc = czero<C>();
+            C sums[kAcc];
+#pragma unroll
+            for (int q = 0; q < kAcc; ++q) sums[q] = czero<C>();
+            C &acc = sums[0];
             if (ell) {
                 const C *z = vs + t.in[0];   // E_0 couples to x, B_0 to z
                 C zv[kEllReg];
@@ -502,7 +506,7 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
                 for (int m = 0; m < 2; ++m) {
                     if (m >= t.nmat) break;
                     // the warp's columns of a chunk; in low tiles of complex128 column
-                    // w kCols + 4 u + lane / 8
+                    // 16 u + 4 w + lane / 8
                     const bool split = t.low && kSplit;
                     const C *vv = vbuf + m * nvec;
                     const int cols = t.low ? 4 * kCols : kCols;
@@ -511,10 +515,10 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
                         const C *cb = reinterpret_cast<const C *>(ring + (size_t)slot * CHUNK);
                         const C *vc = vv + ch * cols;
                         if (split) {
-                            const C *bc = cb + w * kCpw * kTileRows + lane;
-                            vc += w * kCols + (lane >> 3);
+                            const C *bc = cb + 4 * w * kLowRows + lane;
+                            vc += 4 * w + (lane >> 3);
 #pragma unroll
-                            for (int u = 0; u < kCpw; ++u) acc = cfma(acc, bc[u * kTileRows], vc[4 * u]);
+                            for (int u = 0; u < kCols / 4; ++u) acc = cfma(acc, bc[u * 16 * kLowRows], vc[16 * u]);
                         } else if (t.low) {
 #pragma unroll
                             for (int h = 0; h < kCols / kRun; ++h) {
@@ -522,6 +526,14 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
                                 const C *bc = cb + c0 * kLowRows + (lane & 7);
 #pragma unroll
                                 for (int u = 0; u < kRun; ++u) acc = cfma(acc, bc[u * kLowRows], vc[c0 + u]);
+                            }
+                        } else if (kSplit) {
+#pragma unroll
+                            for (int h = 0; h < kCols / 16; ++h) {
+                                const int c0 = 16 * h + 4 * w;
+                                const C *bc = cb + c0 * kTileRows + lane;
+#pragma unroll
+                                for (int q = 0; q < kAcc; ++q) sums[q] = cfma(sums[q], bc[q * kTileRows], vc[c0 + q]);
                             }
                         } else if (!kHalf || (ch & 1) == (w >> 1)) {
                             const int c0 = kHalf ? (w & 1) * kRun : w * kRun;
@@ -535,9 +547,11 @@ __global__ void __launch_bounds__(kTmaThreads, CPS) k_sweep_tma(const __grid_con
                     }
                 }
             }
-            if (t.low && kSplit) {   // the four column classes of a row
-                acc = acc + shfl_xor(acc, 8);
-                acc = acc + shfl_xor(acc, 16);
+            if (kSplit && !ell) {   // the four column classes of a row
+                if (t.low) {
+                    acc = acc + shfl_xor(acc, 8);
+                    acc = acc + shfl_xor(acc, 16);
+                } else acc = (acc + sums[kAcc > 1 ? 1 : 0]) + (sums[kAcc > 2 ? 2 : 0] + sums[kAcc > 3 ? 3 : 0]);
             }
             rd[w][lane] = acc;
             named_sync(1, kTmaConsumers);
