@@ -234,6 +234,8 @@ def forced_sweep(pencil, omegas, b, precision="mixed", group=16, refine_tol=0.0,
                 pencil.factor_shifts(1j * om[sl], "fp64")
                 x = pencil.solve(rhs)
                 escalated += k
+        if x.shape != (pencil.n, k):   # a right-hand side of another length than the pencil's
+            raise ValueError(f"right-hand side of shape {b.shape} for {F} frequencies and {pencil.n} unknowns")
         if X is None:
             X = x   # a single group
         else:
