@@ -1,6 +1,5 @@
 // Common device/host helpers of libkoregpu: complex arithmetic on float2/double2,
-// the bounded grid barrier used by the persistent kernels, status plumbing and
-// launch accounting.
+// launches set up while the one before runs, status plumbing and launch accounting.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -89,52 +88,14 @@ __device__ __forceinline__ double warp_max_d(double v) {
 
 // ----------------------------------------------------------------------------- errors
 // Device error flag values (plan->d_err); the first writer wins.
-#define KORE_DEVERR_BARRIER 1   // a grid barrier wait ran out
 #define KORE_DEVERR_PIVOT   2   // zero pivot in Gauss-Jordan
-#define KORE_DEVERR_FLAG    3   // a dataflow flag wait ran out
+#define KORE_DEVERR_FLAG    3   // a bounded wait (sweep entry, mbarrier) ran out
 
-// Iteration limit of every device spin-wait: ~2^26 polls with 64 ns sleeps is a few
-// seconds, far above any legitimate wait, far below a watchdog.
-#define KORE_SPIN_LIMIT (1u << 26)
-
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 __device__ __forceinline__ int ld_relaxed_i32(const int *p) {
     int v;
     asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-
-// Grid-wide barrier for a cooperative (co-resident) launch.  `counter` is a
-// monotonically increasing arrival count zeroed before the launch; episode e
-// completes when counter reaches (e+1)*gridDim.x.  Every wait is bounded: on
-// timeout the error flag is set and the barrier returns, and once the flag is set
-// all later barriers return immediately so the kernel drains instead of hanging.
-struct GridBarrier {
-    unsigned *counter;
-    int *err;
-    unsigned target;
-    __device__ __forceinline__ void init(unsigned *c, int *e) { counter = c; err = e; target = 0; }
-    __device__ __forceinline__ void sync() {
-        __syncthreads();
-        target += gridDim.x;
-        if (threadIdx.x == 0) {
-            __threadfence();
-            atomicAdd(counter, 1u);
-            unsigned spins = 0;
-            while (ld_acquire_u32(counter) < target) {
-                if (ld_relaxed_i32(err) != 0) break;
-                if (++spins > KORE_SPIN_LIMIT) { atomicCAS(err, 0, KORE_DEVERR_BARRIER); break; }
-                __nanosleep(64);
-            }
-            __threadfence();
-        }
-        __syncthreads();
-    }
-};
 
 // ----------------------------------------------------------------------------- host side
 extern std::atomic<long long> g_kore_launches;

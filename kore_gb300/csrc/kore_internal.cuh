@@ -145,9 +145,8 @@ struct kore_plan {
     void *d_sweep = nullptr;
     double2 *d_bb = nullptr, *d_xb = nullptr, *d_rb = nullptr;
     double *d_bn = nullptr, *d_rn = nullptr;   // per-shift ||b||_inf and ||r||_inf
-    double *d_red = nullptr;          // reduction scratch (8192 doubles)
     double *d_part = nullptr;         // per-CTA maxima of the residual kernel (2 per CTA, per shift)
-    double *h_red = nullptr;          // pinned host mirror
+    double *h_red = nullptr;          // pinned (8192 doubles): refinement states and error flag of a solve
     int *d_err = nullptr;
     unsigned *d_tick = nullptr;       // one per shift: arrivals of a launch's CTAs (0 between launches)
     std::shared_ptr<void> sweep_launch;   // the last sweep launch's maps and shape (sweep.cu)

@@ -105,7 +105,7 @@ void free_plan(kore_plan *p) {
     void *ptrs[] = {p->d_arow, p->d_acol, p->d_asplit, p->d_aval, p->d_brow, p->d_bcol, p->d_bval,
                     p->d_slot2orig, p->d_bsz, p->d_Dinv, p->d_Gm, p->d_Hm, p->d_Dw, p->d_LU, p->d_lev,
                     p->d_rscale, p->d_T, p->d_piv, p->d_used, p->d_sweep,
-                    p->d_red, p->d_part, p->d_err, p->d_flag, p->d_ir, p->d_tick, p->d_V, p->d_Vtmp, p->d_ksx, p->d_small, p->d_warm,
+                    p->d_part, p->d_err, p->d_flag, p->d_ir, p->d_tick, p->d_V, p->d_Vtmp, p->d_ksx, p->d_small, p->d_warm,
                     p->d_sigma, p->d_minf, p->d_bb, p->d_xb, p->d_rb, p->d_bn, p->d_rn,
                     p->d_ell_col, p->d_ell_src, p->d_ell_val, p->d_long_rows, p->d_srow, p->d_smid,
                     p->d_scol, p->d_sval, p->d_cc_ptr, p->d_cc_row, p->d_cc_src, p->d_tctab, p->d_oz};
@@ -368,11 +368,9 @@ int create(const kore_pencil_desc *d, int device, kore_plan **out) {
         KORE_CUDA_TRY(cudaMemcpy(p->d_lev, p->lev.data(), p->lev.size() * sizeof(BcrLevel), cudaMemcpyHostToDevice));
     }
     for (auto &v : p->d_v) KORE_TRY(kore_alloc(p, (void **)&v, p->np * sizeof(double2)));
-    KORE_TRY(kore_alloc(p, (void **)&p->d_red, 8192 * sizeof(double)));
     KORE_TRY(kore_alloc(p, (void **)&p->d_err, sizeof(int)));
     KORE_TRY(kore_alloc(p, (void **)&p->d_flag, 64));
     KORE_CUDA_TRY(cudaMemset(p->d_err, 0, sizeof(int)));
-    KORE_CUDA_TRY(cudaMemset(p->d_red, 0, 8192 * sizeof(double)));
     KORE_CUDA_TRY(cudaMallocHost(&p->h_red, 8192 * sizeof(double)));
     // the set-up copies and memsets ran on the legacy default stream; plans' own streams
     // are non-blocking, so this waits for this plan's set-up only
@@ -614,7 +612,7 @@ int kore_plan_estimate_bytes(const kore_pencil_desc *d, int precision, int nshif
     b += (2 * np + 1) * 4 + 2 * na * 12;
     b += 2 * ell * 4 + np * 4;
     b += (np + 1) * 4 + nb * 12;
-    b += np * 8 + K * 4 + nlev * (int64_t)sizeof(BcrLevel) + 6 * np * 16 + 8192 * 8 + 1024;
+    b += np * 8 + K * 4 + nlev * (int64_t)sizeof(BcrLevel) + 6 * np * 16 + 1024;
     // factors and solve workspace of c shifts
     b += c * (4 * K * SS * e + lu * SS * e + nodd_max * (e == 8 ? 2 : 1) * SS * e + (4 * np + nlev * S) * e + np * 8 + 2 * nodd_max * S * 4);
     // level-0 couplings by column; job table of the tensor-core products

@@ -9,10 +9,10 @@
 //     level l >= 1, odd blocks j:   x_j = z_j - G_j x_jl - H_j x_jr,
 //     level 0, odd blocks j:        g_j = c_j - L_j x_{j-1} - U_j x_{j+1},  x_j = D_j^-1 g_j
 // then x <- s x.  At level 0 the couplings are sparse, so forming g_j from them and
-// multiplying by D_j^-1 reads one dense block instead of the two of G_j, H_j.  One cooperative persistent kernel runs all phases (about 3 log2 K of
-// them) as a dataflow over tiles of 32 rows: a tile starts as soon as the blocks it
-// reads are complete (per-block completion counters), and the factor blocks stream
-// from HBM through shared memory by TMA.
+// multiplying by D_j^-1 reads one dense block instead of the two of G_j, H_j.  One cooperative
+// persistent kernel runs all phases (about 3 log2 K of them) as a dataflow over tiles of 32
+// (or 8) rows: a tile starts as soon as the entries it reads are there (each entry shows its
+// own readiness), and the factor blocks stream from HBM through shared memory by TMA.
 //
 // Every kernel here works on all factorised shifts at once (shift s: its own factors,
 // row scales and vectors at offset s * stride), so a batch of forcing frequencies is
@@ -893,7 +893,6 @@ __global__ void k_scatter(int64_t np, int64_t n, const int64_t *__restrict__ s2o
     }
 }
 
-
 template <typename C>
 size_t tma_smem(int S, int nst, int chunk) {
     const int kCols = chunk / (kTileRows * (int)sizeof(C));
@@ -1372,16 +1371,16 @@ int kore_ir_read(kore_plan *p, IrState *out, int *err) {
 // latency-critical loop, or a host library that is handed only a stream.  For them the
 // scratch of one solve (padded right-hand side and solution, the reduction vectors of
 // the sweep, the FP64 residual and the per-CTA maxima of the refinement loop, the
-// norm partials, the refinement state, the sweep's completion counters and the error
-// flag) lives in the file-scope array below instead of in buffers of the plan or of a
-// caller.  Its size
-// is fixed at kNoAllocMaxNp padded unknowns (about 2 MB, held by every GPU that
+// norm partials, the refinement state and the error flag) lives in the file-scope array
+// below instead of in buffers of the plan or of a caller.  Its size is fixed at kNoAllocMaxNp padded unknowns (about 2 MB, held by every GPU that
 // loads the library until the process exits); larger problems are rejected.
 // The kernels are the ones of kore_solve_dev; only their scratch pointers differ.
 namespace {
 
 constexpr int64_t kNoAllocMaxNp = 16384;
-constexpr int64_t kNoAllocMaxCnt = 32768;   // stages x blocks of a sweep: (3 levels + 2) x blocks
+// stages x blocks of a sweep, (3 levels + 2) x blocks: a limit of the entry point, not of the
+// scratch, which grows with the unknowns alone
+constexpr int64_t kNoAllocMaxCnt = 32768;
 constexpr int64_t kNoAllocMaxSpmvCta = (kNoAllocMaxNp * kRowLanes + 255) / 256 + kNoAllocMaxNp / 8 + 1;
 
 struct NoAllocScratch {
@@ -1473,7 +1472,7 @@ extern "C" int kore_solve_dev_noalloc(kore_plan *p, const void *b_dev, void *x_d
     if (p->np > kNoAllocMaxNp || (int64_t)(p->nlev > 0 ? 3 * p->nlev + 2 : 1) * p->K > kNoAllocMaxCnt) {
         std::fprintf(stderr,
                      "kore_solve_dev_noalloc: %lld padded unknowns in %d blocks exceed the fixed scratch "
-                     "(%lld unknowns, %lld block entries); use kore_solve_dev\n",
+                     "(%lld unknowns, %lld stages x blocks); use kore_solve_dev\n",
                      (long long)p->np, p->K, (long long)kNoAllocMaxNp, (long long)kNoAllocMaxCnt);
         return KORE_EINVAL;
     }

@@ -1,6 +1,6 @@
-// Host-side encoding of the tensor maps that the TMA copies of the sweep and of the
-// tensor-core GEMMs read.  The encoder is the driver's cuTensorMapEncodeTiled, fetched
-// at run time through the runtime API (no link against libcuda).
+// Host-side encoding of the tensor maps that the TMA copies of the sweep read.  The encoder
+// is the driver's cuTensorMapEncodeTiled, fetched at run time through the runtime API (no
+// link against libcuda).
 #include "kore_tma.cuh"
 #include <cstdio>
 namespace {
@@ -40,28 +40,6 @@ int kore_encode_block_map(CUtensorMap *map, const void *base, int real_bytes, in
     if (r != CUDA_SUCCESS) {
         std::fprintf(stderr, "kore: cuTensorMapEncodeTiled failed (%d): S=%d blocks=%lld shifts=%d\n", (int)r, S,
                      (long long)nblk, nshift);
-        return KORE_ECUDA;
-    }
-    return KORE_OK;
-}
-
-int kore_encode_f32_3d(CUtensorMap *map, const void *base, const uint64_t dims[3], const uint64_t strides[2],
-                       const uint32_t box[3], int swizzle128) {
-    EncodeTiledFn fn = encode_tiled_fn();
-    if (!fn) {
-        std::fprintf(stderr, "kore: cuTensorMapEncodeTiled is not available from the driver\n");
-        return KORE_ECUDA;
-    }
-    const cuuint64_t d[3] = {dims[0], dims[1], dims[2]};
-    const cuuint64_t st[2] = {strides[0], strides[1]};
-    const cuuint32_t b[3] = {box[0], box[1], box[2]};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void *>(base), d, st, b, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        std::fprintf(stderr, "kore: cuTensorMapEncodeTiled (3-D float) failed (%d)\n", (int)r);
         return KORE_ECUDA;
     }
     return KORE_OK;
