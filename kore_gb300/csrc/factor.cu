@@ -275,7 +275,7 @@ __device__ __forceinline__ const C *diag_block(const FV<C> &v, int64_t o, int64_
 // read the diagonal block itself, which stays as it is.
 // With Helper (up to 512 rows) one more warp shortens the chain: a step updates the next
 // pivot column first and hands its candidates over, and while the row warps update the
-// other columns the helper picks the pivot and inverts it (30 blocks of 96 in complex128,
+// other columns the helper picks the pivot and inverts it (60 blocks of 96 in complex128,
 // factorised and solved: 5.20 -> 4.86 ms; two shifts of the MAC shell, S = 360, in complex64:
 // 9.58 -> 9.37 ms).
 __device__ __forceinline__ void bar_sync(int id, int threads) {
